@@ -535,6 +535,54 @@ int moe_b200_block_bwd(const void* grad_out, const float* grad_aux, const void* 
                        size_t scratch_bytes, void* side_stream_a, void* side_stream_b,
                        int32_t* n_launches, int32_t* status, void* stream);
 
+/* The same with every option of the block (src/model/moe.py:96-418), described by one struct; the
+ * kept tensors are one buffer whose layout is the library's own. Zero-initialise the struct; a NULL
+ * pointer means the option is absent. x, the weights, biases, residual, grad_out and the results
+ * are bf16 and contiguous, 32-byte aligned. */
+typedef struct moe_b200_block_desc {
+  int64_t n_tokens;
+  int32_t d_model, d_hidden, n_experts, n_shared, top_k;
+  int32_t normalize, full_softmax, activation;
+  int32_t store_combine;         /* 0: rows added in the GEMM epilogues; 1: fp32 sum in pair order */
+  int32_t capacity;              /* > 0: pairs a routed expert keeps; the rest are dropped */
+  float aux_coef;
+  const void* x;                 /* [T, D] */
+  const void* router_w;          /* [D, E] */
+  const void* logits_in;         /* [T, E]: the router's logits when the caller has formed them */
+  const float* logit_bias;       /* [E] */
+  const float* noise;            /* [T, E] */
+  const void *w_in, *w_out;      /* [E, D, 2H], [E, H, D] */
+  const void *w_sh_in, *w_sh_out;/* [S, D, 2H], [S, H, D] */
+  const void *b_in, *b_out;      /* [E, 2H], [E, D] */
+  const void *b_sh_in, *b_sh_out;/* [S, 2H], [S, D] */
+  const void* residual;          /* [T, D], added to out */
+  int32_t* status;
+} moe_b200_block_desc;
+
+/* Bytes of the kept buffer (train != 0: what the backward reads; 0: the plan alone) and of the two
+ * directions' scratch; 0 for a bad shape. */
+size_t moe_b200_block_kept_bytes(const moe_b200_block_desc* desc, int32_t train);
+size_t moe_b200_block_forward_scratch_bytes(const moe_b200_block_desc* desc);
+size_t moe_b200_block_backward_scratch_bytes(const moe_b200_block_desc* desc);
+
+/* out [T, D]; aux: the balance loss (fp32), or zero when full_softmax is 0 (written as a 16-bit zero
+ * when aux_is_16bit); counts [E] the routing decisions; dropped (int64, may be NULL) the pairs over
+ * capacity. train == 0 keeps no rows for a backward and gathers the token rows in the up GEMM. */
+int moe_b200_block_forward(const moe_b200_block_desc* desc, int32_t train, void* out, void* aux,
+                           int32_t aux_is_16bit, int32_t* counts, int64_t* dropped, void* kept,
+                           size_t kept_bytes, void* scratch, size_t scratch_bytes,
+                           int32_t* n_launches, void* stream);
+
+/* The backward on the desc and kept buffer of a forward with train != 0: dx [T, D], d_router [D, E],
+ * weight gradients in the weights' shapes, db_in [E + S, 2H] / db_out [E + S, D] (routed experts
+ * first) when the block has biases. Side streams as for moe_b200_block_bwd. */
+int moe_b200_block_backward(const moe_b200_block_desc* desc, const void* grad_out,
+                            const float* grad_aux, const void* kept, size_t kept_bytes, void* dx,
+                            void* d_router, void* dw_in, void* dw_out, void* dw_sh_in,
+                            void* dw_sh_out, void* db_in, void* db_out, void* scratch,
+                            size_t scratch_bytes, void* side_stream_a, void* side_stream_b,
+                            int32_t* n_launches, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,22 +1,27 @@
 // The whole block's forward and backward as ONE host call each: the stage sequence of
 // nanospeaker_b200/moe_kernel.py (router GEMM, routing + dispatch, permute, up/gate GEMM + GLU,
-// down GEMM with the atomic combine, balance loss; and the backward with its three independent
+// down GEMM, combine, balance loss; and the backward with its three independent
 // branches on three streams) issued from C++, for hosts that pay per call into this library -- a
 // Python caller's ~22 ctypes calls per step cost it more than the GPU needs for the work.
-// Everything here is host code over the other entry points of include/moe_b200.h, plus four
+// Everything here is host code over the other entry points of include/moe_b200.h, plus a few
 // trivial kernels: zero / copy a few words (memset and device-to-device copy nodes go to a copy
 // engine, where they queue behind a caller's large host-to-device copy in flight: the end-to-end
 // step lost 13 us to that), and the forward's first and last launch, which fold what would
-// otherwise be small launches of their own on the critical path (pad the router weight + clear
-// the column sums; counts for the caller + balance loss). All of them wait for their
+// otherwise be small launches of their own on the critical path (pad the router weight, stack the
+// biases, clear the column sums; counts for the caller, balance loss, dropped pairs). All of them wait for their
 // predecessors programmatically like the library's other kernels, so none of them breaks the
-// chain of early launches. Training form only: pre-activations and permuted rows are kept,
-// combine mode "atomic", no residual, no per-expert biases.
+// chain of early launches.
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <mutex>
+#include <vector>
+
 #include "../../include/moe_b200.h"
 #include "pdl.cuh"
+#include "routing.cuh"
 
 namespace {
 
@@ -47,48 +52,81 @@ inline int copy_words(const void* src, void* dst, int64_t n_words, cudaStream_t 
   return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
 }
 
-// The forward's first launch: the router weight [D, E] zero-padded to [D, ld] (what
-// moe_b200_copy_cols does) and, in the same launch, the column sums of the balance loss cleared.
-__global__ void __launch_bounds__(256)
-    pad_router_kernel(const uint16_t* __restrict__ src, int64_t rows, int32_t cols,
-                      uint16_t* __restrict__ dst, int32_t dst_ld, float* __restrict__ colsum) {
+// The forward's first launch: up to PREP_JOBS small 16-bit matrices copied into zero-padded places
+// (the router weight [D, E] -> [D, ld] as the tensor maps want it; the biases of both weight stacks
+// one under the other) and, in the same launch, the column sums of the balance loss cleared.
+constexpr int PREP_JOBS = 6;
+struct PrepJob {
+  const uint16_t* src;      // null: zeros
+  uint16_t* dst;
+  int32_t rows, cols;       // of src
+  int32_t dst_rows, dst_ld; // of dst; what src does not cover is zero
+};
+struct PrepArgs {
+  PrepJob job[PREP_JOBS];
+  int32_t n_jobs;
+  int32_t n_clear;
+  float* clear;
+};
+__global__ void __launch_bounds__(256) prep_kernel(const PrepArgs a) {
   moe::pdl_trigger();
   moe::pdl_wait();
-  const int64_t first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (colsum != nullptr && first < cols) colsum[first] = 0.f;
-  const int64_t total = rows * dst_ld;
-  for (int64_t i = first; i < total; i += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t r = i / dst_ld;
-    const int32_t c = int32_t(i - r * dst_ld);
-    dst[i] = c < cols ? src[r * cols + c] : uint16_t(0);
+  const int first = int(blockIdx.x * blockDim.x + threadIdx.x);
+  const int step = int(gridDim.x * blockDim.x);
+  for (int i = first; i < a.n_clear; i += step) a.clear[i] = 0.f;
+  for (int k = 0; k < a.n_jobs; ++k) {
+    const PrepJob j = a.job[k];
+    const int total = j.dst_rows * j.dst_ld;
+    for (int i = first; i < total; i += step) {
+      const int r = i / j.dst_ld, c = i - r * j.dst_ld;
+      j.dst[i] = j.src != nullptr && r < j.rows && c < j.cols ? j.src[r * j.cols + c] : uint16_t(0);
+    }
   }
 }
-inline int pad_router(const void* src, int64_t rows, int32_t cols, void* dst, int32_t dst_ld,
-                      float* colsum, cudaStream_t st) {
-  int64_t blocks = (rows * dst_ld + 255) / 256;
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  if (blocks * 256 < cols) return MOE_B200_ERR_SHAPE;   // (the clearing threads are the first `cols`)
-  moe::launch_pdl(pad_router_kernel, dim3(unsigned(blocks)), dim3(256), 0, st,
-                  static_cast<const uint16_t*>(src), rows, cols, static_cast<uint16_t*>(dst),
-                  dst_ld, colsum);
+inline int prep(const PrepArgs& a, cudaStream_t st) {
+  int64_t most = a.n_clear;
+  for (int k = 0; k < a.n_jobs; ++k)
+    most = std::max(most, int64_t(a.job[k].dst_rows) * a.job[k].dst_ld);
+  if (most > INT32_MAX) return MOE_B200_ERR_SHAPE;
+  const int64_t blocks = std::min<int64_t>((most + 255) / 256, 148 * 8);
+  moe::launch_pdl(prep_kernel, dim3(unsigned(std::max<int64_t>(blocks, 1))), dim3(256), 0, st, a);
+  return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
+}
+
+// fp32 -> bf16 (the bias gradients' last step).
+__global__ void __launch_bounds__(256)
+    to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int32_t n) {
+  moe::pdl_trigger();
+  moe::pdl_wait();
+  for (int i = int(blockIdx.x * blockDim.x + threadIdx.x); i < n; i += int(gridDim.x * blockDim.x))
+    dst[i] = __float2bfloat16(src[i]);
+}
+inline int to_bf16(const float* src, void* dst, int32_t n, cudaStream_t st) {
+  const int blocks = std::min((n + 255) / 256, 592);
+  moe::launch_pdl(to_bf16_kernel, dim3(unsigned(blocks)), dim3(256), 0, st, src,
+                  static_cast<__nv_bfloat16*>(dst), n);
   return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
 }
 
 // The forward's last launch: the routed experts' counts for the caller and the balance loss
 // aux = coef * E * sum_e (counts[e] / sum counts) * (colsum[e] / T) -- the arithmetic of
-// moe_b200_balance_loss, same order -- or zero when the loss is off (colsum == nullptr). One warp.
+// moe_b200_balance_loss, same order -- or zero when the loss is off (colsum == nullptr); with a
+// capacity also the number of pairs over it. One warp.
 // It does not release its dependents early: when a backward follows in the same graph, letting
 // that backward's first kernel become resident under the down GEMM cost the step 2 us.
 __global__ void finish_fwd_kernel(const int32_t* __restrict__ counts_all,
                                   int32_t* __restrict__ counts, const float* __restrict__ colsum,
                                   int n_experts, int64_t n_tokens, float coef,
-                                  float* __restrict__ aux) {
+                                  float* __restrict__ aux, int aux_is_16bit, int32_t capacity,
+                                  int64_t* __restrict__ dropped) {
   moe::pdl_wait();
   const int lane = threadIdx.x;
   float dot = 0.f, tot = 0.f;
+  int over = 0;
   for (int e = lane; e < n_experts; e += 32) {
     const int32_t ci = counts_all[e];
     counts[e] = ci;
+    if (capacity > 0) over += max(ci - capacity, 0);
     if (colsum != nullptr) {
       const float c = float(ci);
       dot += c * colsum[e];
@@ -99,16 +137,24 @@ __global__ void finish_fwd_kernel(const int32_t* __restrict__ counts_all,
   for (int o = 16; o; o >>= 1) {
     dot += __shfl_xor_sync(0xffffffffu, dot, o);
     tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    over += __shfl_xor_sync(0xffffffffu, over, o);
   }
-  if (lane == 0)
-    aux[0] = colsum == nullptr ? 0.f
-                               : coef * float(n_experts) * dot / fmaxf(tot, 1.f) /
-                                     float(n_tokens > 0 ? n_tokens : 1);
+  if (lane == 0) {
+    if (dropped != nullptr) *dropped = over;
+    if (aux_is_16bit)
+      *reinterpret_cast<uint16_t*>(aux) = 0;
+    else
+      aux[0] = colsum == nullptr ? 0.f
+                                 : coef * float(n_experts) * dot / fmaxf(tot, 1.f) /
+                                       float(n_tokens > 0 ? n_tokens : 1);
+  }
 }
+
 inline int finish_fwd(const int32_t* counts_all, int32_t* counts, const float* colsum,
-                      int n_experts, int64_t n_tokens, float coef, float* aux, cudaStream_t st) {
+                      int n_experts, int64_t n_tokens, float coef, float* aux, int aux_is_16bit,
+                      int32_t capacity, int64_t* dropped, cudaStream_t st) {
   moe::launch_pdl(finish_fwd_kernel, dim3(1), dim3(32), 0, st, counts_all, counts, colsum,
-                  n_experts, n_tokens, coef, aux);
+                  n_experts, n_tokens, coef, aux, aux_is_16bit, capacity, dropped);
   return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
 }
 
@@ -141,62 +187,83 @@ inline Sizes sizes(int64_t n_tokens, int32_t n_experts, int32_t n_shared, int32_
   return s;
 }
 
+// What the forward makes besides its results. A training forward keeps all of it for the backward.
+struct Kept {
+  void *xs, *a1;                  // [L, D] permuted rows, [L, 2H] pre-activations (training only)
+  void *logits, *w_all;           // [T, ld] unless the caller brought logits; [T, kS]
+  int64_t* idx_all;
+  int32_t *sorted_ids, *expert_ids, *pad_offsets, *counts_all, *n_post_pad, *inv_ids;
+  void* router_wp;                // [D, ld]
+  void *bias_in, *bias_out;       // [E + S, 2H], [E + S, D]: both weight stacks' biases
+  void* bias_out_k;               // [ld, D]: the routed experts' b_out, rows past E zero
+  size_t total;
+};
+struct Has {                      // the optional parts that the layout depends on
+  bool train, logits_in, bias_in, bias_out;
+};
+Kept carve_kept(void* p, int64_t n_tokens, int32_t d_model, int32_t d_hidden, int32_t n_experts,
+                int32_t n_shared, int32_t top_k, const Has& h) {
+  const Sizes z = sizes(n_tokens, n_experts, n_shared, top_k);
+  Carver c(p);
+  Kept k{};
+  if (h.train) {
+    k.xs = c.take(size_t(z.l_cap) * d_model * 2);
+    k.a1 = c.take(size_t(z.l_cap) * 2 * d_hidden * 2);
+  }
+  if (!h.logits_in) k.logits = c.take(size_t(n_tokens) * z.ld * 2);
+  k.w_all = c.take(size_t(z.m) * 2);
+  k.idx_all = static_cast<int64_t*>(c.take(size_t(z.m) * 8));
+  k.sorted_ids = static_cast<int32_t*>(c.take(size_t(z.l_cap) * 4));
+  k.expert_ids = static_cast<int32_t*>(c.take(size_t(z.l_cap / 128 + 1) * 4));
+  k.pad_offsets = static_cast<int32_t*>(c.take(size_t(z.n_all + 1) * 4));
+  k.counts_all = static_cast<int32_t*>(c.take(size_t(z.n_all) * 4));
+  k.n_post_pad = static_cast<int32_t*>(c.take(4));
+  k.inv_ids = static_cast<int32_t*>(c.take(size_t(z.m) * 4));
+  k.router_wp = c.take(size_t(d_model) * z.ld * 2);
+  if (h.bias_in) k.bias_in = c.take(size_t(z.n_all) * 2 * d_hidden * 2);
+  if (h.bias_out) {
+    k.bias_out = c.take(size_t(z.n_all) * d_model * 2);
+    k.bias_out_k = c.take(size_t(z.ld) * d_model * 2);
+  }
+  k.total = c.used;
+  return k;
+}
+
+// Scratch of the forward: dead when it returns.
 struct FwdScratch {
-  void* hid;
+  void *hid, *y;                  // [L, H]; [L, D] (store combine only)
   void* block_hist;
   size_t block_hist_bytes;
   float* colsum;
   size_t total;
 };
-FwdScratch carve_fwd(void* p, int64_t n_tokens, int32_t d_hidden, int32_t n_experts,
-                     int32_t n_shared, int32_t top_k) {
+FwdScratch carve_fwd(void* p, int64_t n_tokens, int32_t d_model, int32_t d_hidden,
+                     int32_t n_experts, int32_t n_shared, int32_t top_k, bool store) {
   const Sizes z = sizes(n_tokens, n_experts, n_shared, top_k);
   Carver c(p);
-  FwdScratch f;
+  FwdScratch f{};
   f.hid = c.take(size_t(z.l_cap) * d_hidden * 2);
   f.block_hist_bytes = moe_b200_router_dispatch_scratch_bytes(n_tokens, z.n_all);
   f.block_hist = c.take(f.block_hist_bytes);
   f.colsum = static_cast<float*>(c.take(size_t(n_experts) * 4));
-  f.total = c.used;
-  return f;
-}
-
-struct InferScratch {
-  void *logits, *w_all, *hid, *y, *block_hist;
-  int64_t* idx_all;
-  int32_t *sorted_ids, *expert_ids, *pad_offsets, *counts, *n_post_pad, *inv_ids;
-  size_t block_hist_bytes, total;
-};
-InferScratch carve_infer(void* p, int64_t n_tokens, int32_t d_model, int32_t d_hidden,
-                         int32_t n_experts, int32_t n_shared, int32_t top_k) {
-  const Sizes z = sizes(n_tokens, n_experts, n_shared, top_k);
-  Carver c(p);
-  InferScratch f;
-  f.logits = c.take(size_t(n_tokens) * z.ld * 2);
-  f.w_all = c.take(size_t(z.m) * 2);
-  f.idx_all = static_cast<int64_t*>(c.take(size_t(z.m) * 8));
-  f.sorted_ids = static_cast<int32_t*>(c.take(size_t(z.l_cap) * 4));
-  f.expert_ids = static_cast<int32_t*>(c.take(size_t(z.l_cap / 128 + 1) * 4));
-  f.pad_offsets = static_cast<int32_t*>(c.take(size_t(z.n_all + 1) * 4));
-  f.counts = static_cast<int32_t*>(c.take(size_t(z.n_all) * 4));
-  f.n_post_pad = static_cast<int32_t*>(c.take(4));
-  f.inv_ids = static_cast<int32_t*>(c.take(size_t(z.m) * 4));
-  f.block_hist_bytes = moe_b200_router_dispatch_scratch_bytes(n_tokens, z.n_all);
-  f.block_hist = c.take(f.block_hist_bytes);
-  f.hid = c.take(size_t(z.l_cap) * d_hidden * 2);
-  f.y = c.take(size_t(z.l_cap) * d_model * 2);
+  if (store) f.y = c.take(size_t(z.l_cap) * d_model * 2);
   f.total = c.used;
   return f;
 }
 
 struct BwdScratch {
   void *douts, *da1, *hidw, *dtw, *dl, *d_router_padded, *part_in, *part_out, *part_r;
+  void *ydx, *dx_router;          // store combine only
+  void* b_extra;                  // [T, ld]: <dOut[t], b_out[e]> (with b_out only)
+  float *db_in, *db_out;          // fp32 column sums (with biases only); one buffer
   size_t part_in_bytes, part_out_bytes, part_r_bytes, total;
 };
 int carve_bwd(void* p, int64_t n_tokens, int32_t d_model, int32_t d_hidden, int32_t n_experts,
-              int32_t n_shared, int32_t top_k, BwdScratch* b) {
+              int32_t n_shared, int32_t top_k, bool store, bool bias_in, bool bias_out,
+              BwdScratch* b) {
   const Sizes z = sizes(n_tokens, n_experts, n_shared, top_k);
   Carver c(p);
+  *b = BwdScratch{};
   b->douts = c.take(size_t(z.l_cap) * d_model * 2);
   b->da1 = c.take(size_t(z.l_cap) * 2 * d_hidden * 2);
   b->hidw = c.take(size_t(z.l_cap) * d_hidden * 2);
@@ -213,6 +280,13 @@ int carve_bwd(void* p, int64_t n_tokens, int32_t d_model, int32_t d_hidden, int3
   b->part_in = c.take(b->part_in_bytes);
   b->part_out = c.take(b->part_out_bytes);
   b->part_r = c.take(b->part_r_bytes);
+  if (store) {
+    b->ydx = c.take(size_t(z.l_cap) * d_model * 2);
+    b->dx_router = c.take(size_t(n_tokens) * d_model * 2);
+  }
+  if (bias_out) b->b_extra = c.take(size_t(n_tokens) * z.ld * 2);
+  if (bias_in) b->db_in = static_cast<float*>(c.take(size_t(z.n_all) * 2 * d_hidden * 4));
+  if (bias_out) b->db_out = static_cast<float*>(c.take(size_t(z.n_all) * d_model * 4));
   b->total = c.used;
   return MOE_B200_OK;
 }
@@ -230,20 +304,428 @@ inline bool bad_shape(int64_t n_tokens, int32_t d_model, int32_t d_hidden, int32
     ++launched;                      \
   } while (0)
 
+// Everything a forward reads and writes, resolved to pointers. desc.router_w may be null when
+// kept.router_wp already holds the padded weight.
+struct Fwd {
+  moe_b200_block_desc d;
+  Kept k;
+  FwdScratch s;
+  void* out;
+  float* aux;                     // null with counts: the caller wants neither
+  int32_t aux_is_16bit;
+  int32_t* counts;
+  int64_t* dropped;
+  bool train;
+};
+
+int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
+  const moe_b200_block_desc& d = f.d;
+  const Sizes z = sizes(d.n_tokens, d.n_experts, d.n_shared, d.top_k);
+  const int64_t T = d.n_tokens;
+  const int32_t D = d.d_model, H = d.d_hidden, E = d.n_experts, S = d.n_shared;
+  void* stream = st;
+  int launched = 0;
+  const int32_t* first_shared = f.k.pad_offsets + E;   // start of the first shared run
+  float* colsum = d.full_softmax ? f.s.colsum : nullptr;
+
+  PrepArgs pa{};
+  auto job = [&](const void* src, int32_t rows, int32_t cols, void* dst, int32_t dst_rows,
+                 int32_t dst_ld) {
+    pa.job[pa.n_jobs++] = PrepJob{static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst),
+                                  src ? rows : 0, cols, dst_rows, dst_ld};
+  };
+  auto below = [](void* p, int64_t values) { return static_cast<uint16_t*>(p) + values; };
+  if (d.router_w) job(d.router_w, D, E, f.k.router_wp, D, z.ld);
+  if (f.k.bias_in) {
+    job(d.b_in, E, 2 * H, f.k.bias_in, E, 2 * H);
+    if (S) job(d.b_sh_in, S, 2 * H, below(f.k.bias_in, int64_t(E) * 2 * H), S, 2 * H);
+  }
+  if (f.k.bias_out) {
+    job(d.b_out, E, D, f.k.bias_out, E, D);
+    if (S) job(d.b_sh_out, S, D, below(f.k.bias_out, int64_t(E) * D), S, D);
+    job(d.b_out, E, D, f.k.bias_out_k, z.ld, D);
+  }
+  if (colsum) {
+    pa.clear = colsum;
+    pa.n_clear = E;
+  }
+  if (pa.n_jobs || pa.n_clear) STEP(prep(pa, st));
+
+  // router: logits GEMM against the padded weight (one fixed group, no pair weights), then
+  // routing + dispatch
+  const void* logits = d.logits_in ? d.logits_in : f.k.logits;
+  const int32_t ld = d.logits_in ? E : z.ld;
+  if (!d.logits_in)
+    STEP(moe_b200_down_gemm(d.x, T, D, f.k.router_wp, 1, nullptr, 0, z.ld, nullptr, nullptr, 1,
+                            nullptr, nullptr, 0, f.k.logits, nullptr, d.status, stream));
+  int n_disp = 0;
+  STEP(moe::router_dispatch(logits, ld, d.logit_bias, d.noise, T, E, d.top_k, S, d.normalize,
+                            d.full_softmax, f.k.w_all, f.k.idx_all, colsum, f.k.sorted_ids,
+                            f.k.expert_ids, f.k.pad_offsets, f.k.counts_all, f.k.n_post_pad,
+                            f.k.inv_ids, f.s.block_hist, f.s.block_hist_bytes, d.capacity, d.status,
+                            stream, &n_disp));
+  launched += n_disp - 1;
+  // experts: up/gate + GLU over the permuted rows, which the backward needs again, or (nothing kept)
+  // gathering the token rows itself
+  if (f.train) {
+    STEP(moe_b200_permute(d.x, T, D, z.ks, f.k.sorted_ids, S ? first_shared : f.k.n_post_pad,
+                          z.l_cap, f.k.xs, stream));
+    STEP(moe_b200_up_gemm(f.k.xs, z.l_cap, D, d.w_in, E, d.w_sh_in, S, H, f.k.expert_ids,
+                          f.k.n_post_pad, 0, nullptr, 0, 0, d.activation, f.s.hid, f.k.a1,
+                          S ? d.x : nullptr, S ? T : 0, f.k.pad_offsets, f.k.bias_in, d.status,
+                          stream));
+  } else {
+    STEP(moe_b200_up_gemm(d.x, z.l_cap, D, d.w_in, E, d.w_sh_in, S, H, f.k.expert_ids,
+                          f.k.n_post_pad, 0, f.k.sorted_ids, z.ks, z.m, d.activation, f.s.hid,
+                          nullptr, nullptr, 0, nullptr, f.k.bias_in, d.status, stream));
+  }
+  // down + combine
+  if (d.store_combine) {
+    STEP(moe_b200_down_gemm(f.s.hid, z.l_cap, H, d.w_out, E, d.w_sh_out, S, D, f.k.expert_ids,
+                            f.k.n_post_pad, 0, f.k.sorted_ids, f.k.w_all, z.m, f.s.y,
+                            f.k.bias_out, d.status, stream));
+    STEP(moe_b200_combine(f.s.y, f.k.inv_ids, T, z.ks, D, d.residual, nullptr, f.out, stream));
+  } else if (S && !d.residual && !f.k.bias_out) {
+    // the shared experts' share, stored, is the accumulator's first value
+    STEP(moe_b200_down_gemm_sum(f.s.hid, z.l_cap, H, d.w_sh_out, S, D, first_shared, T, f.out,
+                                d.status, stream));
+    STEP(moe_b200_down_gemm_acc(f.s.hid, z.l_cap, H, d.w_out, E, nullptr, 0, D, f.k.expert_ids,
+                                first_shared, 0, f.k.sorted_ids, f.k.w_all, z.m, z.ks, f.out, T,
+                                nullptr, d.status, stream));
+  } else {
+    if (d.residual) STEP(copy_words(d.residual, f.out, T * D / 2, st));
+    else STEP(zero_words(f.out, T * D / 2, st));
+    STEP(moe_b200_down_gemm_acc(f.s.hid, z.l_cap, H, d.w_out, E, d.w_sh_out, S, D,
+                                f.k.expert_ids, f.k.n_post_pad, 0, f.k.sorted_ids, f.k.w_all, z.m,
+                                z.ks, f.out, T, f.k.bias_out, d.status, stream));
+  }
+  if (f.counts)
+    STEP(finish_fwd(f.k.counts_all, f.counts, colsum, E, T, d.aux_coef, f.aux, f.aux_is_16bit,
+                    d.capacity, f.dropped, st));
+  if (n_launches) *n_launches = launched;
+  return MOE_B200_OK;
+}
+
+struct Bwd {
+  moe_b200_block_desc d;
+  Kept k;
+  BwdScratch s;
+  const void* grad_out;
+  const float* grad_aux;
+  void *dx, *d_router, *dw_in, *dw_out, *dw_sh_in, *dw_sh_out, *db_in, *db_out;
+  void *side_a, *side_b;
+};
+
+// The four events of the fork and the join. Sets are kept between calls, one per call in progress at
+// once, and live as long as the process (there is no point at which a static could destroy them:
+// the runtime may already be gone).
+struct ForkEvents {
+  cudaEvent_t fork = nullptr, dx = nullptr, a = nullptr, b = nullptr;
+};
+class ForkEventsLease {
+ public:
+  ForkEventsLease() {
+    if (cudaGetDevice(&dev_) != cudaSuccess || dev_ < 0 || dev_ >= MAX_DEVICES) return;
+    {
+      std::lock_guard<std::mutex> lock(mutex());
+      std::vector<ForkEvents>& pool = pools()[dev_];
+      if (!pool.empty()) {
+        ev = pool.back();
+        pool.pop_back();
+        ok = true;
+        return;
+      }
+    }
+    ok = true;
+    for (cudaEvent_t* p : {&ev.fork, &ev.dx, &ev.a, &ev.b})
+      ok = ok && cudaEventCreateWithFlags(p, cudaEventDisableTiming) == cudaSuccess;
+  }
+  ~ForkEventsLease() {
+    if (!ok) return;
+    std::lock_guard<std::mutex> lock(mutex());
+    pools()[dev_].push_back(ev);
+  }
+  ForkEventsLease(const ForkEventsLease&) = delete;
+  ForkEvents ev;
+  bool ok = false;
+
+ private:
+  static constexpr int MAX_DEVICES = 64;
+  static std::mutex& mutex() {
+    static std::mutex* m = new std::mutex;
+    return *m;
+  }
+  static std::vector<ForkEvents>* pools() {
+    static std::vector<ForkEvents>* p = new std::vector<ForkEvents>[MAX_DEVICES];
+    return p;
+  }
+  int dev_ = -1;
+};
+
+int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
+  const moe_b200_block_desc& d = b.d;
+  const Sizes z = sizes(d.n_tokens, d.n_experts, d.n_shared, d.top_k);
+  const int64_t T = d.n_tokens;
+  const int32_t D = d.d_model, H = d.d_hidden, E = d.n_experts, S = d.n_shared;
+  void* stream = main_st;
+  // the two side branches run on the caller's side streams, or in line when none are given
+  cudaStream_t sa = b.side_a ? static_cast<cudaStream_t>(b.side_a) : main_st;
+  cudaStream_t sb = b.side_b ? static_cast<cudaStream_t>(b.side_b) : main_st;
+  int launched = 0;
+  const int32_t* first_shared = b.k.pad_offsets + E;
+  const int32_t* live = S ? first_shared : b.k.n_post_pad;
+  const bool store = d.store_combine != 0;
+  const int32_t* offs = S ? b.k.pad_offsets : nullptr;
+
+  STEP(moe_b200_permute(b.grad_out, T, D, z.ks, b.k.sorted_ids, live, z.l_cap, b.s.douts, stream));
+  STEP(moe_b200_dhidden_glu_bwd(b.s.douts, z.l_cap, D, d.w_out, E, d.w_sh_out, S, H,
+                                b.k.expert_ids, b.k.n_post_pad, 0, b.k.sorted_ids, 0, b.k.w_all,
+                                z.m, b.k.a1, d.activation, b.s.da1, b.s.hidw, b.s.dtw,
+                                S ? b.grad_out : nullptr, S ? T : 0, offs, d.status, stream));
+  // fork: everything below depends only on the two launches above
+  const ForkEventsLease lease;
+  if (!lease.ok) return MOE_B200_ERR_CUDA;
+  const ForkEvents* ev = &lease.ev;
+#define CU(call) \
+  if ((call) != cudaSuccess) return MOE_B200_ERR_CUDA
+  CU(cudaEventRecord(ev->fork, main_st));
+  if (sa != main_st) CU(cudaStreamWaitEvent(sa, ev->fork, 0));
+  if (sb != main_st) CU(cudaStreamWaitEvent(sb, ev->fork, 0));
+
+  // main: dx's first value (the shared experts' share, stored), dW_in, the routed rows of dx
+  if (!store) {
+    if (S) {
+      STEP(moe_b200_dx_gemm_sum(b.s.da1, z.l_cap, H, d.w_sh_in, S, D, first_shared, T, b.dx,
+                                d.status, stream));
+    } else {
+      STEP(zero_words(b.dx, T * D / 2, main_st));
+    }
+    CU(cudaEventRecord(ev->dx, main_st));
+  }
+  STEP(moe_b200_wgrad(b.k.xs, 0, D, b.s.da1, 0, 2 * H, z.l_cap, b.k.pad_offsets, z.n_all, 0,
+                      nullptr, 0, 0, 0, b.dw_in, E, S ? b.dw_sh_in : nullptr, b.s.part_in,
+                      b.s.part_in_bytes, S ? d.x : nullptr, S ? T : 0, S ? 1 : 0, d.status,
+                      stream));
+  if (store) {
+    STEP(moe_b200_dx_gemm(b.s.da1, z.l_cap, H, d.w_in, E, d.w_sh_in, S, D, b.k.expert_ids,
+                          b.k.n_post_pad, 0, b.s.ydx, d.status, stream));
+  } else {
+    STEP(moe_b200_dx_gemm_acc(b.s.da1, z.l_cap, H, d.w_in, E, nullptr, 0, D, b.k.expert_ids, live,
+                              0, b.k.sorted_ids, z.m, z.ks, b.dx, T, b.k.pad_offsets, d.status,
+                              stream));
+  }
+  // side a: dW_out, then the bias gradients (column sums over the runs)
+  STEP(moe_b200_wgrad(b.s.hidw, 0, H, b.s.douts, 0, D, z.l_cap, b.k.pad_offsets, z.n_all, 0,
+                      nullptr, 0, 0, 0, b.dw_out, E, S ? b.dw_sh_out : nullptr, b.s.part_out,
+                      b.s.part_out_bytes, S ? b.grad_out : nullptr, S ? T : 0, S ? 2 : 0, d.status,
+                      sa));
+  const int32_t n_bi = b.s.db_in ? z.n_all * 2 * H : 0, n_bo = b.s.db_out ? z.n_all * D : 0;
+  if (n_bi) {
+    STEP(zero_words(b.s.db_in, n_bi, sa));
+    STEP(moe_b200_segment_colsum(b.s.da1, z.l_cap, 2 * H, b.k.expert_ids, b.k.n_post_pad, nullptr,
+                                 z.n_all, nullptr, nullptr, 0, nullptr, 0, 0, b.s.db_in, sa));
+    STEP(to_bf16(b.s.db_in, b.db_in, n_bi, sa));
+  }
+  if (n_bo) {
+    STEP(zero_words(b.s.db_out, n_bo, sa));
+    STEP(moe_b200_segment_colsum(b.s.douts, z.l_cap, D, b.k.expert_ids, b.k.n_post_pad, offs,
+                                 z.n_all, b.k.sorted_ids, b.k.w_all, z.m,
+                                 S ? b.grad_out : nullptr, S ? T : 0, E, b.s.db_out, sa));
+    STEP(to_bf16(b.s.db_out, b.db_out, n_bo, sa));
+  }
+  // side b: the router's backward, its weight gradient, its share of dx. With b_out a pair's
+  // d(topk_w) gains <dOut[t], b_out[e]>: one row GEMM dOut @ b_out^T over all experts, read at the
+  // pair's column by the router kernel.
+  if (b.s.b_extra)
+    STEP(moe_b200_dx_gemm(b.grad_out, T, D / 2, b.k.bias_out_k, 1, nullptr, 0, z.ld, nullptr,
+                          nullptr, 1, b.s.b_extra, d.status, sb));
+  STEP(moe::router_fused_bwd(d.logits_in ? d.logits_in : b.k.logits, d.logits_in ? E : z.ld,
+                             d.logit_bias, d.noise, b.k.idx_all, b.s.dtw, b.s.b_extra, z.ld,
+                             d.capacity > 0 ? b.k.inv_ids : nullptr, T, E, d.top_k, S,
+                             d.normalize, d.full_softmax, b.grad_aux, b.k.counts_all, d.aux_coef,
+                             b.s.dl, z.ld, sb));
+  STEP(moe_b200_wgrad(d.x, 0, D, b.s.dl, 0, z.ld, T, nullptr, 1, 0, nullptr, 0, 0, 0,
+                      b.s.d_router_padded, 1, nullptr, b.s.part_r, b.s.part_r_bytes, nullptr, 0, 0,
+                      d.status, sb));
+  STEP(moe_b200_copy_cols(b.s.d_router_padded, D, E, z.ld, b.d_router, E, sb));
+  if (store) {
+    STEP(moe_b200_dx_gemm(b.s.dl, T, z.ld / 2, b.k.router_wp, 1, nullptr, 0, D, nullptr, nullptr,
+                          1, b.s.dx_router, d.status, sb));
+  } else {
+    if (sb != main_st) CU(cudaStreamWaitEvent(sb, ev->dx, 0));
+    STEP(moe_b200_dx_gemm_acc(b.s.dl, T, z.ld / 2, b.k.router_wp, 1, nullptr, 0, D, nullptr,
+                              nullptr, 1, nullptr, 0, 1, b.dx, T, nullptr, d.status, sb));
+  }
+  // join
+  if (sa != main_st) {
+    CU(cudaEventRecord(ev->a, sa));
+    CU(cudaStreamWaitEvent(main_st, ev->a, 0));
+  }
+  if (sb != main_st) {
+    CU(cudaEventRecord(ev->b, sb));
+    CU(cudaStreamWaitEvent(main_st, ev->b, 0));
+  }
+#undef CU
+  if (store)
+    STEP(moe_b200_combine(b.s.ydx, b.k.inv_ids, T, z.ks, D, b.s.dx_router, nullptr, b.dx, stream));
+  if (n_launches) *n_launches = launched + 3;   // the three weight gradients may add a reduction pass
+  return MOE_B200_OK;
+}
+
+// The checks every descriptor call makes before it touches a pointer.
+int check_desc(const moe_b200_block_desc* d) {
+  if (d == nullptr) return MOE_B200_ERR_NULL;
+  if (bad_shape(d->n_tokens, d->d_model, d->d_hidden, d->n_experts, d->n_shared, d->top_k) ||
+      d->capacity < 0)
+    return MOE_B200_ERR_SHAPE;
+  return MOE_B200_OK;
+}
+inline Has has_of(const moe_b200_block_desc* d, bool train) {
+  return Has{train, d->logits_in != nullptr, d->b_in || d->b_sh_in, d->b_out || d->b_sh_out};
+}
+inline Kept kept_of(const moe_b200_block_desc* d, void* p, bool train) {
+  return carve_kept(p, d->n_tokens, d->d_model, d->d_hidden, d->n_experts, d->n_shared, d->top_k,
+                    has_of(d, train));
+}
+
 }  // namespace
 
 extern "C" {
 
+size_t moe_b200_block_kept_bytes(const moe_b200_block_desc* d, int32_t train) {
+  if (check_desc(d) != MOE_B200_OK) return 0;
+  return kept_of(d, nullptr, train != 0).total;
+}
+
+size_t moe_b200_block_forward_scratch_bytes(const moe_b200_block_desc* d) {
+  if (check_desc(d) != MOE_B200_OK) return 0;
+  return carve_fwd(nullptr, d->n_tokens, d->d_model, d->d_hidden, d->n_experts, d->n_shared,
+                   d->top_k, d->store_combine != 0).total;
+}
+
+size_t moe_b200_block_backward_scratch_bytes(const moe_b200_block_desc* d) {
+  if (check_desc(d) != MOE_B200_OK) return 0;
+  BwdScratch b;
+  const Has h = has_of(d, true);
+  if (carve_bwd(nullptr, d->n_tokens, d->d_model, d->d_hidden, d->n_experts, d->n_shared, d->top_k,
+                d->store_combine != 0, h.bias_in, h.bias_out, &b) != MOE_B200_OK)
+    return 0;
+  return b.total;
+}
+
+int moe_b200_block_forward(const moe_b200_block_desc* d, int32_t train, void* out, void* aux,
+                           int32_t aux_is_16bit, int32_t* counts, int64_t* dropped, void* kept,
+                           size_t kept_bytes, void* scratch, size_t scratch_bytes,
+                           int32_t* n_launches, void* stream) {
+  const int rc = check_desc(d);
+  if (rc != MOE_B200_OK) return rc;
+  if (!d->x || !d->router_w || !d->w_in || !d->w_out || !d->status || !out || !aux || !counts ||
+      !kept || !scratch)
+    return MOE_B200_ERR_NULL;
+  if (d->n_shared > 0 && (!d->w_sh_in || !d->w_sh_out)) return MOE_B200_ERR_NULL;
+  if (kept_bytes < moe_b200_block_kept_bytes(d, train) ||
+      scratch_bytes < moe_b200_block_forward_scratch_bytes(d))
+    return MOE_B200_ERR_SCRATCH;
+  Fwd f{};
+  f.d = *d;
+  f.train = train != 0;
+  f.k = kept_of(d, kept, f.train);
+  f.s = carve_fwd(scratch, d->n_tokens, d->d_model, d->d_hidden, d->n_experts, d->n_shared,
+                  d->top_k, d->store_combine != 0);
+  f.out = out;
+  f.aux = static_cast<float*>(aux);
+  f.aux_is_16bit = aux_is_16bit && !d->full_softmax;
+  f.counts = counts;
+  f.dropped = dropped;
+  return run_forward(f, n_launches, static_cast<cudaStream_t>(stream));
+}
+
+int moe_b200_block_backward(const moe_b200_block_desc* d, const void* grad_out,
+                            const float* grad_aux, const void* kept, size_t kept_bytes, void* dx,
+                            void* d_router, void* dw_in, void* dw_out, void* dw_sh_in,
+                            void* dw_sh_out, void* db_in, void* db_out, void* scratch,
+                            size_t scratch_bytes, void* side_stream_a, void* side_stream_b,
+                            int32_t* n_launches, void* stream) {
+  const int rc = check_desc(d);
+  if (rc != MOE_B200_OK) return rc;
+  if (!d->x || !d->w_in || !d->w_out || !d->status || !grad_out || !kept || !dx || !d_router ||
+      !dw_in || !dw_out || !scratch)
+    return MOE_B200_ERR_NULL;
+  if (d->n_shared > 0 && (!d->w_sh_in || !d->w_sh_out || !dw_sh_in || !dw_sh_out))
+    return MOE_B200_ERR_NULL;
+  const Has h = has_of(d, true);
+  if ((h.bias_in && !db_in) || (h.bias_out && !db_out)) return MOE_B200_ERR_NULL;
+  if (kept_bytes < moe_b200_block_kept_bytes(d, 1)) return MOE_B200_ERR_SCRATCH;
+  Bwd b{};
+  b.d = *d;
+  b.k = kept_of(d, const_cast<void*>(kept), true);
+  const int rcb = carve_bwd(scratch, d->n_tokens, d->d_model, d->d_hidden, d->n_experts,
+                            d->n_shared, d->top_k, d->store_combine != 0, h.bias_in, h.bias_out,
+                            &b.s);
+  if (rcb != MOE_B200_OK) return rcb;
+  if (scratch_bytes < b.s.total) return MOE_B200_ERR_SCRATCH;
+  b.grad_out = grad_out;
+  b.grad_aux = grad_aux;
+  b.dx = dx;
+  b.d_router = d_router;
+  b.dw_in = dw_in;
+  b.dw_out = dw_out;
+  b.dw_sh_in = dw_sh_in;
+  b.dw_sh_out = dw_sh_out;
+  b.db_in = db_in;
+  b.db_out = db_out;
+  b.side_a = side_stream_a;
+  b.side_b = side_stream_b;
+  return run_backward(b, n_launches, static_cast<cudaStream_t>(stream));
+}
+
+// The same sequences for hosts that hold every kept tensor as a buffer of its own.
+static moe_b200_block_desc plain_desc(const void* x, int64_t n_tokens, int32_t d_model,
+                                      const void* w_in, const void* w_out, int32_t n_experts,
+                                      int32_t d_hidden, const void* w_sh_in, const void* w_sh_out,
+                                      int32_t n_shared, int32_t top_k, int32_t normalize,
+                                      int32_t activation, const float* logit_bias,
+                                      int32_t* status) {
+  moe_b200_block_desc d{};
+  d.n_tokens = n_tokens;
+  d.d_model = d_model;
+  d.d_hidden = d_hidden;
+  d.n_experts = n_experts;
+  d.n_shared = n_shared;
+  d.top_k = top_k;
+  d.normalize = normalize;
+  d.activation = activation;
+  d.x = x;
+  d.w_in = w_in;
+  d.w_out = w_out;
+  d.w_sh_in = w_sh_in;
+  d.w_sh_out = w_sh_out;
+  d.logit_bias = logit_bias;
+  d.status = status;
+  return d;
+}
+
 size_t moe_b200_block_fwd_scratch_bytes(int64_t n_tokens, int32_t d_model, int32_t d_hidden,
                                         int32_t n_experts, int32_t n_shared, int32_t top_k) {
   if (bad_shape(n_tokens, d_model, d_hidden, n_experts, n_shared, top_k)) return 0;
-  return carve_fwd(nullptr, n_tokens, d_hidden, n_experts, n_shared, top_k).total;
+  return carve_fwd(nullptr, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, false).total;
 }
 
 size_t moe_b200_block_infer_scratch_bytes(int64_t n_tokens, int32_t d_model, int32_t d_hidden,
                                           int32_t n_experts, int32_t n_shared, int32_t top_k) {
   if (bad_shape(n_tokens, d_model, d_hidden, n_experts, n_shared, top_k)) return 0;
-  return carve_infer(nullptr, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k).total;
+  return carve_kept(nullptr, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, Has{}).total +
+         carve_fwd(nullptr, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, true).total;
+}
+
+size_t moe_b200_block_bwd_scratch_bytes(int64_t n_tokens, int32_t d_model, int32_t d_hidden,
+                                        int32_t n_experts, int32_t n_shared, int32_t top_k) {
+  if (bad_shape(n_tokens, d_model, d_hidden, n_experts, n_shared, top_k)) return 0;
+  BwdScratch b;
+  if (carve_bwd(nullptr, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, false, false,
+                false, &b) != MOE_B200_OK)
+    return 0;
+  return b.total;
 }
 
 int moe_b200_block_infer(const void* x, int64_t n_tokens, int32_t d_model,
@@ -258,46 +740,20 @@ int moe_b200_block_infer(const void* x, int64_t n_tokens, int32_t d_model,
   if (!x || !router_w_padded || !w_in || !w_out || !out || !scratch || !status)
     return MOE_B200_ERR_NULL;
   if (n_shared > 0 && (!w_sh_in || !w_sh_out)) return MOE_B200_ERR_NULL;
-  const InferScratch f = carve_infer(scratch, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k);
-  if (scratch_bytes < f.total) return MOE_B200_ERR_SCRATCH;
-  const Sizes z = sizes(n_tokens, n_experts, n_shared, top_k);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int launched = 0;
-  STEP(moe_b200_down_gemm(x, n_tokens, d_model, router_w_padded, 1, nullptr, 0, z.ld, nullptr,
-                          nullptr, 1, nullptr, nullptr, 0, f.logits, nullptr, status, stream));
-  STEP(moe_b200_router_dispatch(f.logits, z.ld, logit_bias, nullptr, n_tokens, n_experts, top_k,
-                                n_shared, normalize, 0, f.w_all, f.idx_all, nullptr, f.sorted_ids,
-                                f.expert_ids, f.pad_offsets, f.counts, f.n_post_pad, f.inv_ids,
-                                f.block_hist, f.block_hist_bytes, status, stream));
-  if (n_tokens > 128) ++launched;   // the dispatch's scatter pass is a launch of its own
-  // up/gate GEMM gathering the token rows itself (no permuted copy), then down GEMM + combine
-  STEP(moe_b200_up_gemm(x, z.l_cap, d_model, w_in, n_experts, w_sh_in, n_shared, d_hidden,
-                        f.expert_ids, f.n_post_pad, 0, f.sorted_ids, z.ks, z.m, activation, f.hid,
-                        nullptr, nullptr, 0, nullptr, nullptr, status, stream));
-  if (atomic_combine) {
-    if (residual) STEP(copy_words(residual, out, n_tokens * d_model / 2, st));
-    else STEP(zero_words(out, n_tokens * d_model / 2, st));
-    STEP(moe_b200_down_gemm_acc(f.hid, z.l_cap, d_hidden, w_out, n_experts, w_sh_out, n_shared,
-                                d_model, f.expert_ids, f.n_post_pad, 0, f.sorted_ids, f.w_all,
-                                z.m, z.ks, out, n_tokens, nullptr, status, stream));
-  } else {
-    STEP(moe_b200_down_gemm(f.hid, z.l_cap, d_hidden, w_out, n_experts, w_sh_out, n_shared,
-                            d_model, f.expert_ids, f.n_post_pad, 0, f.sorted_ids, f.w_all, z.m,
-                            f.y, nullptr, status, stream));
-    STEP(moe_b200_combine(f.y, f.inv_ids, n_tokens, z.ks, d_model, residual, nullptr, out, stream));
-  }
-  if (n_launches) *n_launches = launched;
-  return MOE_B200_OK;
-}
-
-size_t moe_b200_block_bwd_scratch_bytes(int64_t n_tokens, int32_t d_model, int32_t d_hidden,
-                                        int32_t n_experts, int32_t n_shared, int32_t top_k) {
-  if (bad_shape(n_tokens, d_model, d_hidden, n_experts, n_shared, top_k)) return 0;
-  BwdScratch b;
-  if (carve_bwd(nullptr, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, &b) !=
-      MOE_B200_OK)
-    return 0;
-  return b.total;
+  if (scratch_bytes < moe_b200_block_infer_scratch_bytes(n_tokens, d_model, d_hidden, n_experts,
+                                                         n_shared, top_k))
+    return MOE_B200_ERR_SCRATCH;
+  Fwd f{};
+  f.d = plain_desc(x, n_tokens, d_model, w_in, w_out, n_experts, d_hidden, w_sh_in, w_sh_out,
+                   n_shared, top_k, normalize, activation, logit_bias, status);
+  f.d.residual = residual;
+  f.d.store_combine = !atomic_combine;
+  f.k = carve_kept(scratch, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, Has{});
+  f.s = carve_fwd(static_cast<char*>(scratch) + f.k.total, n_tokens, d_model, d_hidden, n_experts,
+                  n_shared, top_k, true);
+  f.k.router_wp = const_cast<void*>(router_w_padded);
+  f.out = out;
+  return run_forward(f, n_launches, static_cast<cudaStream_t>(stream));
 }
 
 int moe_b200_block_fwd(const void* x, int64_t n_tokens, int32_t d_model, const void* router_w,
@@ -317,45 +773,32 @@ int moe_b200_block_fwd(const void* x, int64_t n_tokens, int32_t d_model, const v
       !n_post_pad || !inv_ids || !router_w_padded || !scratch || !status)
     return MOE_B200_ERR_NULL;
   if (n_shared > 0 && (!w_sh_in || !w_sh_out)) return MOE_B200_ERR_NULL;
-  const FwdScratch f = carve_fwd(scratch, n_tokens, d_hidden, n_experts, n_shared, top_k);
-  if (scratch_bytes < f.total) return MOE_B200_ERR_SCRATCH;
-  const Sizes z = sizes(n_tokens, n_experts, n_shared, top_k);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int launched = 0;
-  const int32_t* first_shared = pad_offsets + n_experts;   // start of the first shared run
-
-  // router: zero-padded weight, logits GEMM (one fixed group, no pair weights), routing + dispatch
-  float* colsum = full_softmax ? f.colsum : nullptr;
-  STEP(pad_router(router_w, d_model, n_experts, router_w_padded, z.ld, colsum, st));
-  STEP(moe_b200_down_gemm(x, n_tokens, d_model, router_w_padded, 1, nullptr, 0, z.ld, nullptr,
-                          nullptr, 1, nullptr, nullptr, 0, logits, nullptr, status, stream));
-  STEP(moe_b200_router_dispatch(logits, z.ld, logit_bias, noise, n_tokens, n_experts, top_k,
-                                n_shared, normalize, full_softmax, w_all, idx_all, colsum,
-                                sorted_ids, expert_ids, pad_offsets, counts_all, n_post_pad,
-                                inv_ids, f.block_hist, f.block_hist_bytes, status, stream));
-  ++launched;   // (two launches, one for batches of up to 128 tokens: counted as two)
-  // experts: permute the routed rows, up/gate + GLU, down with the combine in its epilogue
-  STEP(moe_b200_permute(x, n_tokens, d_model, z.ks, sorted_ids,
-                        n_shared ? first_shared : n_post_pad, z.l_cap, xs, stream));
-  STEP(moe_b200_up_gemm(xs, z.l_cap, d_model, w_in, n_experts, w_sh_in, n_shared, d_hidden,
-                        expert_ids, n_post_pad, 0, nullptr, 0, 0, activation, f.hid, a1,
-                        n_shared ? x : nullptr, n_shared ? n_tokens : 0, pad_offsets, nullptr,
-                        status, stream));
-  if (n_shared) {
-    STEP(moe_b200_down_gemm_sum(f.hid, z.l_cap, d_hidden, w_sh_out, n_shared, d_model,
-                                first_shared, n_tokens, out, status, stream));
-    STEP(moe_b200_down_gemm_acc(f.hid, z.l_cap, d_hidden, w_out, n_experts, nullptr, 0, d_model,
-                                expert_ids, first_shared, 0, sorted_ids, w_all, z.m, z.ks, out,
-                                n_tokens, nullptr, status, stream));
-  } else {
-    STEP(zero_words(out, n_tokens * d_model / 2, st));
-    STEP(moe_b200_down_gemm_acc(f.hid, z.l_cap, d_hidden, w_out, n_experts, nullptr, 0, d_model,
-                                expert_ids, n_post_pad, 0, sorted_ids, w_all, z.m, z.ks, out,
-                                n_tokens, nullptr, status, stream));
-  }
-  STEP(finish_fwd(counts_all, counts, colsum, n_experts, n_tokens, aux_coef, aux, st));
-  if (n_launches) *n_launches = launched;
-  return MOE_B200_OK;
+  Fwd f{};
+  f.s = carve_fwd(scratch, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, false);
+  if (scratch_bytes < f.s.total) return MOE_B200_ERR_SCRATCH;
+  f.d = plain_desc(x, n_tokens, d_model, w_in, w_out, n_experts, d_hidden, w_sh_in, w_sh_out,
+                   n_shared, top_k, normalize, activation, logit_bias, status);
+  f.d.router_w = router_w;
+  f.d.noise = noise;
+  f.d.full_softmax = full_softmax;
+  f.d.aux_coef = aux_coef;
+  f.train = true;
+  f.k.xs = xs;
+  f.k.a1 = a1;
+  f.k.logits = logits;
+  f.k.w_all = w_all;
+  f.k.idx_all = idx_all;
+  f.k.sorted_ids = sorted_ids;
+  f.k.expert_ids = expert_ids;
+  f.k.pad_offsets = pad_offsets;
+  f.k.counts_all = counts_all;
+  f.k.n_post_pad = n_post_pad;
+  f.k.inv_ids = inv_ids;
+  f.k.router_wp = router_w_padded;
+  f.out = out;
+  f.aux = aux;
+  f.counts = counts;
+  return run_forward(f, n_launches, static_cast<cudaStream_t>(stream));
 }
 
 int moe_b200_block_bwd(const void* grad_out, const float* grad_aux, const void* x,
@@ -378,94 +821,38 @@ int moe_b200_block_bwd(const void* grad_out, const float* grad_aux, const void* 
       !router_w_padded || !dx || !d_router || !dw_in || !dw_out || !scratch || !status)
     return MOE_B200_ERR_NULL;
   if (n_shared > 0 && (!w_sh_in || !w_sh_out || !dw_sh_in || !dw_sh_out)) return MOE_B200_ERR_NULL;
-  BwdScratch b;
-  const int rcb = carve_bwd(scratch, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, &b);
+  Bwd b{};
+  const int rcb = carve_bwd(scratch, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k,
+                            false, false, false, &b.s);
   if (rcb != MOE_B200_OK) return rcb;
-  if (scratch_bytes < b.total) return MOE_B200_ERR_SCRATCH;
-  const Sizes z = sizes(n_tokens, n_experts, n_shared, top_k);
-  cudaStream_t main_st = static_cast<cudaStream_t>(stream);
-  // the two side branches run on the caller's side streams, or in line when none are given
-  cudaStream_t sa = side_stream_a ? static_cast<cudaStream_t>(side_stream_a) : main_st;
-  cudaStream_t sb = side_stream_b ? static_cast<cudaStream_t>(side_stream_b) : main_st;
-  int launched = 0;
-  const int32_t* first_shared = pad_offsets + n_experts;
-  const int32_t* live = n_shared ? first_shared : n_post_pad;
-
-  STEP(moe_b200_permute(grad_out, n_tokens, d_model, z.ks, sorted_ids, live, z.l_cap, b.douts,
-                        stream));
-  STEP(moe_b200_dhidden_glu_bwd(b.douts, z.l_cap, d_model, w_out, n_experts, w_sh_out, n_shared,
-                                d_hidden, expert_ids, n_post_pad, 0, sorted_ids, 0, w_all, z.m,
-                                a1, activation, b.da1, b.hidw, b.dtw,
-                                n_shared ? grad_out : nullptr, n_shared ? n_tokens : 0,
-                                n_shared ? pad_offsets : nullptr, status, stream));
-  // fork: everything below depends only on the two launches above
-  cudaEvent_t ev_fork = nullptr, ev_dx = nullptr, ev_a = nullptr, ev_b = nullptr;
-  auto fail = [&](int code) {
-    for (cudaEvent_t e : {ev_fork, ev_dx, ev_a, ev_b})
-      if (e) cudaEventDestroy(e);
-    return code;
-  };
-  for (cudaEvent_t* e : {&ev_fork, &ev_dx, &ev_a, &ev_b})
-    if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess)
-      return fail(MOE_B200_ERR_CUDA);
-#define STEP_F(call)                          \
-  do {                                        \
-    const int rc_ = (call);                   \
-    if (rc_ != MOE_B200_OK) return fail(rc_); \
-    ++launched;                               \
-  } while (0)
-#define CU_F(call) \
-  if ((call) != cudaSuccess) return fail(MOE_B200_ERR_CUDA)
-  CU_F(cudaEventRecord(ev_fork, main_st));
-  if (sa != main_st) CU_F(cudaStreamWaitEvent(sa, ev_fork, 0));
-  if (sb != main_st) CU_F(cudaStreamWaitEvent(sb, ev_fork, 0));
-
-  // main: dx's first value (the shared experts' share, stored), dW_in, the routed rows of dx
-  if (n_shared) {
-    STEP_F(moe_b200_dx_gemm_sum(b.da1, z.l_cap, d_hidden, w_sh_in, n_shared, d_model,
-                                first_shared, n_tokens, dx, status, stream));
-  } else {
-    STEP_F(zero_words(dx, n_tokens * d_model / 2, main_st));
-  }
-  CU_F(cudaEventRecord(ev_dx, main_st));
-  STEP_F(moe_b200_wgrad(xs, 0, d_model, b.da1, 0, 2 * d_hidden, z.l_cap, pad_offsets, z.n_all, 0,
-                        nullptr, 0, 0, 0, dw_in, n_experts, n_shared ? dw_sh_in : nullptr,
-                        b.part_in, b.part_in_bytes, n_shared ? x : nullptr,
-                        n_shared ? n_tokens : 0, n_shared ? 1 : 0, status, stream));
-  STEP_F(moe_b200_dx_gemm_acc(b.da1, z.l_cap, d_hidden, w_in, n_experts, nullptr, 0, d_model,
-                              expert_ids, live, 0, sorted_ids, z.m, z.ks, dx, n_tokens,
-                              pad_offsets, status, stream));
-  // side a: dW_out
-  STEP_F(moe_b200_wgrad(b.hidw, 0, d_hidden, b.douts, 0, d_model, z.l_cap, pad_offsets, z.n_all,
-                        0, nullptr, 0, 0, 0, dw_out, n_experts, n_shared ? dw_sh_out : nullptr,
-                        b.part_out, b.part_out_bytes, n_shared ? grad_out : nullptr,
-                        n_shared ? n_tokens : 0, n_shared ? 2 : 0, status, sa));
-  // side b: the router's backward, its weight gradient, its share of dx
-  STEP_F(moe_b200_router_fused_bwd(logits, z.ld, logit_bias, noise, idx_all, b.dtw, n_tokens,
-                                   n_experts, top_k, n_shared, normalize, full_softmax, grad_aux,
-                                   counts_all, aux_coef, b.dl, z.ld, sb));
-  STEP_F(moe_b200_wgrad(x, 0, d_model, b.dl, 0, z.ld, n_tokens, nullptr, 1, 0, nullptr, 0, 0, 0,
-                        b.d_router_padded, 1, nullptr, b.part_r, b.part_r_bytes, nullptr, 0, 0,
-                        status, sb));
-  STEP_F(moe_b200_copy_cols(b.d_router_padded, d_model, n_experts, z.ld, d_router, n_experts, sb));
-  if (sb != main_st) CU_F(cudaStreamWaitEvent(sb, ev_dx, 0));
-  STEP_F(moe_b200_dx_gemm_acc(b.dl, n_tokens, z.ld / 2, router_w_padded, 1, nullptr, 0, d_model,
-                              nullptr, nullptr, 1, nullptr, 0, 1, dx, n_tokens, nullptr, status,
-                              sb));
-  // join
-  if (sa != main_st) {
-    CU_F(cudaEventRecord(ev_a, sa));
-    CU_F(cudaStreamWaitEvent(main_st, ev_a, 0));
-  }
-  if (sb != main_st) {
-    CU_F(cudaEventRecord(ev_b, sb));
-    CU_F(cudaStreamWaitEvent(main_st, ev_b, 0));
-  }
-#undef STEP_F
-#undef CU_F
-  fail(0);   // the events are released once their work has completed
-  if (n_launches) *n_launches = launched + 3;   // the three weight gradients may add a reduction pass
-  return MOE_B200_OK;
+  if (scratch_bytes < b.s.total) return MOE_B200_ERR_SCRATCH;
+  b.d = plain_desc(x, n_tokens, d_model, w_in, w_out, n_experts, d_hidden, w_sh_in, w_sh_out,
+                   n_shared, top_k, normalize, activation, logit_bias, status);
+  b.d.noise = noise;
+  b.d.full_softmax = full_softmax;
+  b.d.aux_coef = aux_coef;
+  b.k.xs = const_cast<void*>(xs);
+  b.k.a1 = const_cast<void*>(a1);
+  b.k.logits = const_cast<void*>(logits);
+  b.k.w_all = const_cast<void*>(w_all);
+  b.k.idx_all = const_cast<int64_t*>(idx_all);
+  b.k.sorted_ids = const_cast<int32_t*>(sorted_ids);
+  b.k.expert_ids = const_cast<int32_t*>(expert_ids);
+  b.k.pad_offsets = const_cast<int32_t*>(pad_offsets);
+  b.k.counts_all = const_cast<int32_t*>(counts_all);
+  b.k.n_post_pad = const_cast<int32_t*>(n_post_pad);
+  b.k.router_wp = const_cast<void*>(router_w_padded);
+  b.grad_out = grad_out;
+  b.grad_aux = grad_aux;
+  b.dx = dx;
+  b.d_router = d_router;
+  b.dw_in = dw_in;
+  b.dw_out = dw_out;
+  b.dw_sh_in = dw_sh_in;
+  b.dw_sh_out = dw_sh_out;
+  b.side_a = side_stream_a;
+  b.side_b = side_stream_b;
+  return run_backward(b, n_launches, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

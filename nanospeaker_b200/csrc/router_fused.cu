@@ -395,7 +395,8 @@ __global__ void __launch_bounds__(RF4_THREADS)
       __syncthreads();
       dispatch_scatter_body<true>(idx_all, n_pairs, n_experts + n_shared, tokens_per_block * kS, 1,
                                   block_hist, sc.counts, sc.pad_offsets, sc.n_post_pad,
-                                  sc.expert_ids, sc.n_tiles_cap, sorted_ids, sc.inv_ids, 0, 0, 0, 1);
+                                  sc.expert_ids, sc.n_tiles_cap, sorted_ids, sc.inv_ids,
+                                  sc.capacity, sc.n_capped, 0, 1);
     }
   }
 }
@@ -427,7 +428,9 @@ template <int NSLOT>
 __global__ void __launch_bounds__(RF_WARPS * 32)
     router_fused_bwd_kernel(const __nv_bfloat16* __restrict__ logits, int ld,
                             const float* __restrict__ bias, const float* __restrict__ noise, const int64_t* __restrict__ idx_all,
-                            const __nv_bfloat16* __restrict__ dw_all, int64_t n_tokens,
+                            const __nv_bfloat16* __restrict__ dw_all,
+                            const __nv_bfloat16* __restrict__ extra_dw, int extra_ld,
+                            const int32_t* __restrict__ inv_ids, int64_t n_tokens,
                             int n_experts, int top_k, int n_shared, int normalize,
                             int full_softmax, const float* __restrict__ d_aux,
                             const int32_t* __restrict__ counts, float aux_scale_T,
@@ -482,7 +485,9 @@ __global__ void __launch_bounds__(RF_WARPS * 32)
 
     const bool active = lane < top_k;
     const int my_idx = active ? int(idx_all[t * kS + lane]) : -1;
-    const float my_dw = active ? __bfloat162float(dw_all[t * kS + lane]) : 0.f;
+    float my_dw = active ? __bfloat162float(dw_all[t * kS + lane]) : 0.f;
+    if (active && extra_dw != nullptr) my_dw += __bfloat162float(extra_dw[t * extra_ld + my_idx]);
+    if (active && inv_ids != nullptr && inv_ids[t * kS + lane] < 0) my_dw = 0.f;   // dropped pair
     // my winner's logit, taken from the lane that holds it
     float my_l = -CUDART_INF_F;
     for (int j = 0; j < top_k; ++j) {
@@ -640,6 +645,41 @@ int launch_router_fused_chunked(const __nv_bfloat16* logits, int ld, const float
   return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
 }
 
+int router_fused_bwd(const void* logits, int32_t ld, const float* bias,
+                     const float* noise, const int64_t* idx_all, const void* dw_all, const void* extra_dw,
+                     int32_t extra_ld, const int32_t* inv_ids, int64_t n_tokens,
+                     int32_t n_experts, int32_t top_k, int32_t n_shared,
+                     int32_t normalize, int32_t full_softmax, const float* d_aux,
+                     const int32_t* counts, float aux_coef, void* d_logits,
+                     int32_t ld_out, void* stream) {
+  if (n_experts < 1 || n_experts > MAX_EXPERTS || top_k < 1 || top_k > n_experts ||
+      n_shared < 0 || top_k + n_shared > 32 || top_k > MAX_TOPK || n_tokens < 0 ||
+      ld < n_experts || ld_out < n_experts)
+    return MOE_B200_ERR_SHAPE;
+  if (n_tokens == 0) return MOE_B200_OK;
+  if (!logits || !idx_all || !dw_all || !d_logits || (d_aux && !counts)) return MOE_B200_ERR_NULL;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const unsigned grid = rf_grid(n_tokens);
+  const float scale = aux_coef * float(n_experts) / float(n_tokens);
+  const __nv_bfloat16* lg = static_cast<const __nv_bfloat16*>(logits);
+  const __nv_bfloat16* dw = static_cast<const __nv_bfloat16*>(dw_all);
+  __nv_bfloat16* out = static_cast<__nv_bfloat16*>(d_logits);
+#define LAUNCH(NS)                                                                               \
+  launch_pdl(router_fused_bwd_kernel<NS>, dim3(grid), dim3(RF_WARPS * 32), 0, st,                                     \
+      lg, ld, bias, noise, idx_all, dw, static_cast<const __nv_bfloat16*>(extra_dw), extra_ld,     \
+      inv_ids, n_tokens, n_experts, top_k, n_shared, normalize,          \
+      full_softmax,                                                                                \
+      d_aux, counts, scale, out, ld_out)
+  const int nslot = (n_experts + 31) / 32;
+  if (nslot <= 1) LAUNCH(1);
+  else if (nslot <= 2) LAUNCH(2);
+  else if (nslot <= 3) LAUNCH(3);
+  else if (nslot <= 4) LAUNCH(4);
+  else LAUNCH(8);
+#undef LAUNCH
+  return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
+}
+
 }  // namespace moe
 
 using namespace moe;
@@ -693,31 +733,9 @@ int moe_b200_router_fused_bwd(const void* logits, int32_t ld, const float* bias,
                               int32_t normalize, int32_t full_softmax, const float* d_aux,
                               const int32_t* counts, float aux_coef, void* d_logits,
                               int32_t ld_out, void* stream) {
-  if (n_experts < 1 || n_experts > MAX_EXPERTS || top_k < 1 || top_k > n_experts ||
-      n_shared < 0 || top_k + n_shared > 32 || top_k > MAX_TOPK || n_tokens < 0 ||
-      ld < n_experts || ld_out < n_experts)
-    return MOE_B200_ERR_SHAPE;
-  if (n_tokens == 0) return MOE_B200_OK;
-  if (!logits || !idx_all || !dw_all || !d_logits || (d_aux && !counts)) return MOE_B200_ERR_NULL;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const unsigned grid = rf_grid(n_tokens);
-  const float scale = aux_coef * float(n_experts) / float(n_tokens);
-  const __nv_bfloat16* lg = static_cast<const __nv_bfloat16*>(logits);
-  const __nv_bfloat16* dw = static_cast<const __nv_bfloat16*>(dw_all);
-  __nv_bfloat16* out = static_cast<__nv_bfloat16*>(d_logits);
-#define LAUNCH(NS)                                                                               \
-  launch_pdl(router_fused_bwd_kernel<NS>, dim3(grid), dim3(RF_WARPS * 32), 0, st,                                     \
-      lg, ld, bias, noise, idx_all, dw, n_tokens, n_experts, top_k, n_shared, normalize,          \
-      full_softmax,                                                                                \
-      d_aux, counts, scale, out, ld_out)
-  const int nslot = (n_experts + 31) / 32;
-  if (nslot <= 1) LAUNCH(1);
-  else if (nslot <= 2) LAUNCH(2);
-  else if (nslot <= 3) LAUNCH(3);
-  else if (nslot <= 4) LAUNCH(4);
-  else LAUNCH(8);
-#undef LAUNCH
-  return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
+  return router_fused_bwd(logits, ld, bias, noise, idx_all, dw_all, nullptr, 0, nullptr, n_tokens,
+                          n_experts, top_k, n_shared, normalize, full_softmax, d_aux, counts,
+                          aux_coef, d_logits, ld_out, stream);
 }
 
 int moe_b200_balance_loss(const float* colsum, const int32_t* counts, int32_t n_experts,

@@ -432,10 +432,28 @@ int moe_b200_router_dispatch(const void* logits, int32_t ld, const float* bias,
                              int32_t* expert_ids, int32_t* pad_offsets, int32_t* counts,
                              int32_t* n_post_pad, int32_t* inv_ids, void* scratch,
                              size_t scratch_bytes, int32_t* status, void* stream) {
+  return router_dispatch(logits, ld, bias, noise, n_tokens, n_experts, top_k, n_shared, normalize,
+                         full_softmax, w_all, idx_all, colsum, sorted_ids, expert_ids, pad_offsets,
+                         counts, n_post_pad, inv_ids, scratch, scratch_bytes, 0, status, stream,
+                         nullptr);
+}
+
+}  // extern "C"
+
+namespace moe {
+int router_dispatch(const void* logits, int32_t ld, const float* bias,
+                    const float* noise, int64_t n_tokens,
+                    int32_t n_experts, int32_t top_k, int32_t n_shared,
+                    int32_t normalize, int32_t full_softmax, void* w_all,
+                    int64_t* idx_all, float* colsum, int32_t* sorted_ids,
+                    int32_t* expert_ids, int32_t* pad_offsets, int32_t* counts,
+                    int32_t* n_post_pad, int32_t* inv_ids, void* scratch,
+                    size_t scratch_bytes, int32_t capacity, int32_t* status, void* stream,
+                    int* launches) {
   const int32_t n_all = n_experts + n_shared;
   if (n_experts < 1 || n_all > MAX_EXPERTS || top_k < 1 || top_k > n_experts || n_shared < 0 ||
       top_k + n_shared > 32 || top_k > MAX_TOPK || n_tokens < 1 || ld < n_experts ||
-      n_tokens * (top_k + n_shared) > (int64_t(1) << 30))
+      capacity < 0 || n_tokens * (top_k + n_shared) > (int64_t(1) << 30))
     return MOE_B200_ERR_SHAPE;
   if (!logits || !w_all || !idx_all || !sorted_ids || !pad_offsets || !counts || !n_post_pad ||
       !inv_ids || !status)
@@ -450,7 +468,8 @@ int moe_b200_router_dispatch(const void* logits, int32_t ld, const float* bias,
   int32_t* block_hist = static_cast<int32_t*>(scratch);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // a batch that fits one block (128 tokens) is routed, planned and scattered by ONE launch
-  const ScatterArgs sc{counts, pad_offsets, n_post_pad, expert_ids, l_cap / ALIGN_M, inv_ids};
+  const ScatterArgs sc{counts,  pad_offsets, n_post_pad, expert_ids, l_cap / ALIGN_M,
+                       inv_ids, capacity,    n_experts};
   bool did_scatter = false;
   const int rc = launch_router_fused_chunked(
       static_cast<const __nv_bfloat16*>(logits), ld, bias, noise, n_tokens, n_experts, top_k,
@@ -458,15 +477,15 @@ int moe_b200_router_dispatch(const void* logits, int32_t ld, const float* bias,
       normalize, full_softmax, static_cast<__nv_bfloat16*>(w_all), idx_all, colsum, tpb, blocks,
       block_hist, sorted_ids, l_cap, st, &sc, &did_scatter);
   if (rc != MOE_B200_OK) return rc;
+  if (launches) *launches = did_scatter ? 1 : 2;
   if (did_scatter) return MOE_B200_OK;
   launch_pdl(dispatch_scatter_kernel, dim3(blocks), dim3(DISPATCH_THREADS), 0, st,
              static_cast<const int64_t*>(idx_all), n_pairs, int(n_all), tpb * kS, blocks,
              static_cast<const int32_t*>(block_hist), counts, pad_offsets, n_post_pad, expert_ids,
-             l_cap / ALIGN_M, sorted_ids, inv_ids, 0, 0);
+             l_cap / ALIGN_M, sorted_ids, inv_ids, capacity, n_experts);
   return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
 }
-
-}  // extern "C"
+}  // namespace moe
 
 // ------------------------------------------------------- dispatch without caller scratch
 // Some hosts cannot hand this library a scratch buffer: a serving process that fixed its whole

@@ -35,6 +35,8 @@ struct ScatterArgs {
   int32_t* expert_ids;
   int64_t n_tiles_cap;
   int32_t* inv_ids;
+  int32_t capacity;   // > 0: experts below n_capped keep the first `capacity` pairs of their runs
+  int32_t n_capped;
 };
 int launch_router_fused_chunked(const __nv_bfloat16* logits, int ld, const float* bias,
                                 const float* noise,
@@ -44,4 +46,22 @@ int launch_router_fused_chunked(const __nv_bfloat16* logits, int ld, const float
                                 int32_t* block_hist, int32_t* sorted_ids, int64_t l_cap,
                                 cudaStream_t st, const ScatterArgs* sc = nullptr,
                                 bool* did_scatter = nullptr);
+// routing.cu: moe_b200_router_dispatch with an expert capacity (0 = dropless) on the first n_experts
+// experts; *launches (may be null) receives the number of kernels.
+int router_dispatch(const void* logits, int32_t ld, const float* bias, const float* noise,
+                    int64_t n_tokens, int32_t n_experts, int32_t top_k, int32_t n_shared,
+                    int32_t normalize, int32_t full_softmax, void* w_all, int64_t* idx_all,
+                    float* colsum, int32_t* sorted_ids, int32_t* expert_ids, int32_t* pad_offsets,
+                    int32_t* counts, int32_t* n_post_pad, int32_t* inv_ids, void* scratch,
+                    size_t scratch_bytes, int32_t capacity, int32_t* status, void* stream,
+                    int* launches);
+// router_fused.cu: moe_b200_router_fused_bwd with two more inputs. extra_dw [T, extra_ld] bf16: what
+// d(topk_w) of a pair gains, read at its expert's column; inv_ids [T * (k + S)]: pairs without a slot
+// (dropped by a capacity) have no d(topk_w). Either may be null.
+int router_fused_bwd(const void* logits, int32_t ld, const float* bias, const float* noise,
+                     const int64_t* idx_all, const void* dw_all, const void* extra_dw,
+                     int32_t extra_ld, const int32_t* inv_ids, int64_t n_tokens, int32_t n_experts,
+                     int32_t top_k, int32_t n_shared, int32_t normalize, int32_t full_softmax,
+                     const float* d_aux, const int32_t* counts, float aux_coef, void* d_logits,
+                     int32_t ld_out, void* stream);
 }  // namespace moe

@@ -24,13 +24,42 @@ def _need_cuda(*tensors) -> None:
             raise RuntimeError("moe_b200 kernels take CUDA tensors only; there is no CPU path")
 
 
-# Number of CUDA kernels this module has launched (every entry point launches a fixed number).
-LAUNCHES = 0
+# kernels.LAUNCHES: number of CUDA kernels launched, by this module (every entry point launches a fixed
+# number) and by the pybind shim.
+_launches = 0
 
 
 def _count(n: int) -> None:
-    global LAUNCHES
-    LAUNCHES += n
+    global _launches
+    _launches += n
+
+
+def __getattr__(name: str):
+    if name == "LAUNCHES":
+        return _launches + (_shim.launches() if _shim is not None else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+
+_shim = None
+
+
+def shim():
+    """The pybind shim (csrc/shim.cpp, built by `python -m nanospeaker_b200.build`), bound to the same
+    library as the ctypes entry points."""
+    global _shim
+    if _shim is None:
+        import ctypes
+        lib = _lib.load()
+        try:
+            from . import _moe_shim
+        except ImportError as e:
+            raise RuntimeError("nanospeaker_b200/_moe_shim.so is missing or does not load: build it "
+                               "with `python -m nanospeaker_b200.build`") from e
+        _moe_shim.bind({n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value
+                        for n in _lib.SIGNATURES},
+                       lambda dev: status_word(torch.device("cuda", dev)).data_ptr())
+        _shim = _moe_shim
+    return _shim
 
 
 _status_words = {}

@@ -197,24 +197,46 @@ class MoEBlock(nn.Module):
         if x.shape[-1] != self.d_model:
             raise ValueError(f"expected last dim {self.d_model}, got {tuple(x.shape)}.")
         shape = x.shape
-        x = x.reshape(-1, self.d_model)
+        if x.dim() != 2:
+            x = x.reshape(-1, self.d_model)
         if x.shape[0] == 0:
             return x.clone().view(shape)
-        if self._whole_block_ok(x):
-            # whole block as one op: router GEMM, top-k, dispatch, experts, combine, balance loss
-            full = self.router.wants_probs()
+        router = self.router
+        if self._kernels_take(x):
+            capacity = self.capacity_factor
+            plain = capacity is None and self.b_in is None and self.b_sh_in is None
+            full = router.wants_probs()
+            native = MK.native_ok(x)
             noise = None
-            if self.training and self.router.noise_std:
+            if self.training and router.noise_std and (plain or native):
                 # exploration noise on the logits (src/model/router.py:76-77), drawn here so that
-                # the op stays a pure function of its inputs
+                # the block stays a pure function of its inputs
                 noise = torch.randn(x.shape[0], self.n_experts, device=x.device,
-                                    dtype=torch.float32) * self.router.noise_std
-            out, aux, counts = fused_moe_block(
-                x, self.router, self.W_in, self.W_out, self.W_sh_in, self.W_sh_out,
-                self._kernel_act, full, combine=self.combine_mode, noise=noise)
-            self.expert_counts = counts.detach()
-            self.aux_loss = aux if full else torch.zeros((), device=x.device, dtype=x.dtype)
-            return out.view(shape)
+                                    dtype=torch.float32) * router.noise_std
+            if plain:
+                # whole block as one op: router GEMM, top-k, dispatch, experts, combine, balance loss
+                out, aux, counts = fused_moe_block(
+                    x, router, self.W_in, self.W_out, self.W_sh_in, self.W_sh_out,
+                    self._kernel_act, full, combine=self.combine_mode, noise=noise)
+            elif native:
+                # biases or a capacity: the same launches with these options. The logits are torch's
+                # matmul, as in the traced form below: another summation order would move bf16 ties.
+                cap = self._capacity(x.shape[0]) if capacity is not None else 0
+                out, aux, counts, dropped = MK.K.shim().block(
+                    x, router.W, router.logit_bias, noise, self.W_in, self.W_out, self.W_sh_in,
+                    self.W_sh_out, self.b_in, self.b_out, self.b_sh_in, self.b_sh_out, None,
+                    router.top_k, bool(router.normalize_weights), full, router.aux_loss_coef,
+                    KERNEL_ACTIVATIONS[self._kernel_act], cap, not MK._atomic(self.combine_mode),
+                    True, MK._DEBUG_ONE_STREAM)
+                if cap:
+                    self.dropped = dropped
+            if plain or native:
+                self.expert_counts = counts.detach()
+                if full or aux.dtype == x.dtype:
+                    self.aux_loss = aux
+                else:
+                    self.aux_loss = torch.zeros((), device=x.device, dtype=x.dtype)
+                return out if len(shape) == 2 else out.view(shape)
 
         topk_w, topk_idx, probs = self.router(x)
         cap = self._capacity(x.shape[0]) if self.capacity_factor is not None else 0

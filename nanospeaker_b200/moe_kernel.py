@@ -507,9 +507,10 @@ _T6 = Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor
 _SIDE_STREAMS = {}
 # Debugging aid, off in normal use: True keeps every launch of the backward on the caller's stream.
 _DEBUG_ONE_STREAM = False
-# The whole-block op's common training form (atomic combine, no residual) is issued by ONE call into
-# the library per direction (moe_b200_block_fwd / _bwd) instead of ~22 calls from Python; False
-# keeps the stage-by-stage sequence below, which is the same launches.
+# The block's launches are issued by ONE call into the library per direction instead of ~22 calls from
+# Python: eager calls go through the pybind shim (native autograd node, every option of the block),
+# the registered ops through ctypes in their common training form (atomic combine, no residual).
+# False keeps the stage-by-stage sequence below, which is the same launches.
 _ONE_CALL = True
 
 
@@ -802,7 +803,7 @@ moe_block.register_autograd(_block_backward, setup_context=_block_setup)
 
 class _BlockFn(torch.autograd.Function):
     """The same forward / backward as the registered op `moe_b200::moe_block`, as a plain autograd
-    node. Eager training calls go through this: a Python-registered torch.library op costs the
+    node. Eager training calls that the shim does not take go through this: a Python-registered torch.library op costs the
     host ~100 us per call in dispatcher and schema work (twice per step), which at T = 16384 is a
     quarter of what the GPU needs for the whole step. The registered ops remain what
     torch.compile, fake tensors and opcheck see."""
@@ -841,12 +842,26 @@ def _call_block(*args):
     return moe_block(*args)
 
 
+def native_ok(x: torch.Tensor) -> bool:
+    """Whether an eager call can go through the shim: plain tensors, nothing tracing or intercepting
+    the dispatch (torch.compile, fake tensors, functional transforms see the registered ops)."""
+    return (_ONE_CALL and type(x) in (torch.Tensor, torch.nn.Parameter)
+            and not torch.compiler.is_compiling()
+            and torch._C._len_torch_dispatch_stack() == 0
+            and torch._C._functorch.peek_interpreter_stack() is None)
+
+
 def fused_moe_block(x, router, w_in, w_out, w_sh_in, w_sh_out, activation, full_softmax,
                     combine: Optional[str] = None, noise: Optional[torch.Tensor] = None):
-    """(out, aux_loss fp32, counts int32 [E]) for a TopKRouter-like `router` (attributes W,
+    """(out, aux_loss (fp32; zero in eager calls' x.dtype without the loss), counts int32 [E]) for a TopKRouter-like `router` (attributes W,
     logit_bias, top_k, normalize_weights, aux_loss_coef) -- the path MoEBlock.forward takes
     whenever no exploration noise has to be added to the logits."""
-    _act_id(activation)
+    act = _act_id(activation)
+    if _aux_reduce is None and native_ok(x):
+        return K.shim().block(
+            x, router.W, router.logit_bias, noise, w_in, w_out, w_sh_in, w_sh_out, None, None, None,
+            None, None, router.top_k, bool(router.normalize_weights), full_softmax,
+            router.aux_loss_coef, act, 0, not _atomic(combine), False, _DEBUG_ONE_STREAM)[:3]
     cast = lambda t: None if t is None else t.to(x.dtype)
     tensors = (x, router.W, w_in, w_out, w_sh_in, w_sh_out)
     save = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)

@@ -87,11 +87,20 @@ class MoEFFNSublayer(nn.Module):
 
     def forward(self, x: torch.Tensor):
         shape = x.shape
-        x2 = x.reshape(-1, shape[-1])
+        x2 = x if x.dim() == 2 else x.reshape(-1, shape[-1])
         f = self.ffn
         if x2.shape[0] > 0 and self._fused_ok(x2):
             full = f.router.wants_probs()
             bias = f.router.logit_bias
+            if MK.native_ok(x2):
+                out, aux, counts = K.shim().sublayer(
+                    x2, self.norm_gamma, self.epsilon, f.router.W, bias, f.W_in, f.W_out,
+                    f.W_sh_in, f.W_sh_out, f.router.top_k, bool(f.router.normalize_weights), full,
+                    f.router.aux_loss_coef, MK._act_id(f._kernel_act),
+                    not MK._atomic(f.combine_mode), MK._DEBUG_ONE_STREAM)
+                f.expert_counts = counts
+                f.aux_loss = aux
+                return out if len(shape) == 2 else out.view(shape), aux
             if bias is not None:
                 bias = bias.to(torch.float32).contiguous()
             out, aux, counts = _FFNSublayerFn.apply(

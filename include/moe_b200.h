@@ -583,6 +583,31 @@ int moe_b200_block_backward(const moe_b200_block_desc* desc, const void* grad_ou
                             size_t scratch_bytes, void* side_stream_a, void* side_stream_b,
                             int32_t* n_launches, void* stream);
 
+/* ---- A stack of blocks on a small batch in one kernel -------------------------------------------
+ * x <- x + block_l(x) for n_layers blocks of one shape on up to 256 tokens (the decode loop of
+ * src/model/nanospeaker.py:254-269 without attention and norms): one persistent kernel, launched
+ * cooperatively, per-pair rows summed in fp32 in a fixed order (bit-reproducible).
+ * moe_b200_stack_supported: 1 where the shape is covered, 0 where the layers are called one by one
+ * (moe_b200_block_infer). moe_b200_stack_plan fills layer `layer` of a host buffer of
+ * moe_b200_stack_plan_bytes bytes with the addresses of that layer's tensors (router_w [D, E]
+ * unpadded, weights as for moe_b200_block_fwd, all 16-byte aligned); the caller copies the whole
+ * buffer to the device once (64-byte aligned) and keeps it as long as the weights stay where they are.
+ * out must not be x. */
+int moe_b200_stack_supported(int64_t n_tokens, int32_t d_model, int32_t d_hidden,
+                             int32_t n_experts, int32_t n_shared, int32_t top_k);
+size_t moe_b200_stack_plan_bytes(int32_t n_layers);
+size_t moe_b200_stack_scratch_bytes(int64_t n_tokens, int32_t d_model, int32_t n_shared,
+                                    int32_t top_k);
+int moe_b200_stack_plan(void* host_plan, int32_t n_layers, int32_t layer, const void* router_w,
+                        const float* logit_bias, const void* w_in, const void* w_out,
+                        const void* w_sh_in, const void* w_sh_out, int32_t n_experts,
+                        int32_t n_shared, int32_t d_model, int32_t d_hidden);
+int moe_b200_stack_infer(const void* plan, int32_t n_layers, const void* x, void* out,
+                         int64_t n_tokens, int32_t d_model, int32_t d_hidden, int32_t n_experts,
+                         int32_t n_shared, int32_t top_k, int32_t normalize, int32_t activation,
+                         void* scratch, size_t scratch_bytes, int32_t* n_launches, int32_t* status,
+                         void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -130,6 +130,16 @@ SIGNATURES = {
     "moe_b200_block_backward": (
         ctypes.c_int, [_c_vp, _c_vp, _c_vp, _c_vp, _c_sz, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp,
                        _c_vp, _c_vp, _c_vp, _c_sz, _c_vp, _c_vp, ctypes.POINTER(_c_i32), _c_vp]),
+    "moe_b200_stack_supported": (
+        ctypes.c_int, [_c_i64, _c_i32, _c_i32, _c_i32, _c_i32, _c_i32]),
+    "moe_b200_stack_plan_bytes": (_c_sz, [_c_i32]),
+    "moe_b200_stack_scratch_bytes": (_c_sz, [_c_i64, _c_i32, _c_i32, _c_i32]),
+    "moe_b200_stack_plan": (
+        ctypes.c_int, [_c_vp, _c_i32, _c_i32, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_i32,
+                       _c_i32, _c_i32, _c_i32]),
+    "moe_b200_stack_infer": (
+        ctypes.c_int, [_c_vp, _c_i32, _c_vp, _c_vp, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32, _c_i32,
+                       _c_i32, _c_i32, _c_vp, _c_sz, ctypes.POINTER(_c_i32), _c_vp, _c_vp]),
     "moe_b200_ep_plan": (
         ctypes.c_int, [_c_vp, _c_vp, _c_i32, _c_i32, _c_i32, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp,
                        _c_vp, _c_i64, _c_vp]),

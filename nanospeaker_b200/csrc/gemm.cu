@@ -1,6 +1,7 @@
 // Host side of the grouped tcgen05 GEMMs: builds the TMA tensor maps for each stage's operands and
 // launches the matching instantiation of grouped_gemm_kernel (gemm.cuh).
 #include "gemm.cuh"
+#include "tma_map.cuh"
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -31,45 +32,6 @@
 #endif
 
 namespace moe {
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  });
-  return fn;
-}
-
-// bf16 tensor map, 128-byte swizzle, zero fill out of bounds. dims/box innermost first;
-// strides (bytes) for dims 1..rank-1.
-static bool make_map(CUtensorMap* m, const void* base, int rank, const uint64_t* dims,
-                     const uint64_t* strides, const uint32_t* box) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  cuuint64_t gd[5];
-  cuuint64_t gs[4];
-  cuuint32_t bx[5], es[5];
-  for (int i = 0; i < rank; ++i) {
-    gd[i] = dims[i];
-    bx[i] = box[i];
-    es[i] = 1;
-  }
-  for (int i = 0; i + 1 < rank; ++i) gs[i] = strides[i];
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, cuuint32_t(rank), const_cast<void*>(base), gd, gs,
-            bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
 
 // [groups, rows, cols] row-major activation buffer as the K-major A operand: 64 cols x 128 rows.
 static bool map_rows_kmajor(CUtensorMap* m, const void* base, int64_t groups, int64_t rows,

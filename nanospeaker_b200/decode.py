@@ -1,9 +1,9 @@
 """Decode-shaped use of the MoE block: a stack of blocks on a small, fixed batch of tokens (one
 token per sequence), forward only, replayed from one CUDA graph.
 
-At T = 64 every expert sees a handful of rows and each block's launches take a few
-microseconds: the cost is launch latency, not arithmetic, so the whole stack is captured once and
-replayed. The caller loop this stands for is `generate` -> `Block.forward` -> `MoEBlock.forward`
+At T = 64 every expert sees a handful of rows: layer by layer the cost is launch latency, not
+arithmetic, so blocks of one shape run as ONE persistent kernel (csrc/stack.cu), and what it does not
+cover is captured once and replayed. The caller loop this stands for is `generate` -> `Block.forward` -> `MoEBlock.forward`
 with T = batch size in eval mode (src/model/nanospeaker.py:254-269, 165-169); attention, norms and
 the KV cache of that loop are outside this package, so the stack here chains the blocks through
 the residual only: x <- x + block_l(x).
@@ -36,6 +36,7 @@ class StackedMoEDecoder:
             b.eval()
         self._graphs = {}
         self._consts = {}
+        self._plans = {}
 
     def _fast_args(self, b: MoEBlock, x: torch.Tensor):
         """Per-block constants of the kernel path (weights are fixed while decoding): the padded
@@ -55,13 +56,45 @@ class StackedMoEDecoder:
                 b.n_experts, b.router.top_k, bool(b.router.normalize_weights), b._kernel_act)
         return self._consts[key]
 
+    def _stack_plan(self, x: torch.Tensor):
+        """(plan, shape arguments) of the one-kernel stack, or None where it does not apply: blocks
+        of different shapes, blocks the kernels decline, more tokens than it takes. The plan holds
+        the addresses of the tensors in self._consts."""
+        from . import kernels as K
+        key = (x.dtype, x.device)
+        if key not in self._plans:
+            plan = None
+            args = [self._fast_args(b, x) for b in self.blocks]
+            if all(a is not None for a in args):
+                shapes = {(b.d_model, b.d_hidden, b.n_experts, b.n_shared) + a[7:]
+                          for b, a in zip(self.blocks, args)}
+                if len(shapes) == 1:
+                    d, h, e, s, k, normalize, act = shapes.pop()
+                    if K.stack_supported(1, d, h, e, s, k):
+                        routers = [b.router.W.detach().to(x.dtype).contiguous()
+                                   for b in self.blocks]
+                        plan = (K.stack_plan([(w,) + a[1:6] for w, a in zip(routers, args)], s),
+                                (d, h, e, s, k), (h, e, s, k, normalize, K.KERNEL_ACTIVATIONS[act]),
+                                routers)
+            self._plans[key] = plan
+        plan = self._plans[key]
+        if plan is None or x.shape[0] < 1 or not K.stack_supported(x.shape[0], *plan[1]):
+            return None
+        return plan
+
     @torch.no_grad()
     def eager(self, x: torch.Tensor) -> torch.Tensor:
-        """x <- x + block(x) through the stack. On the kernel path a block is six launches: the
-        residual is added inside the combine, the padded router weight is kept between steps,
-        and the per-call bookkeeping of MoEBlock.forward (expert_counts, aux_loss) is skipped."""
+        """x <- x + block(x) through the stack: one persistent kernel for blocks of one shape and up
+        to 256 tokens (per-pair rows summed in fp32 in a fixed order, whatever the combine mode).
+        Otherwise block by block, five launches each: the residual is added inside the combine,
+        the padded router weight is kept between steps, and the per-call bookkeeping of
+        MoEBlock.forward (expert_counts, aux_loss) is skipped."""
+        from . import kernels as K
         from . import moe_kernel as MK
         x = x.contiguous()
+        plan = self._stack_plan(x) if x.dim() == 2 and MK._ONE_CALL else None
+        if plan is not None:
+            return K.stack_infer(plan[0], len(self.blocks), x, *plan[2])
         for b in self.blocks:
             args = self._fast_args(b, x)
             x = x + b(x) if args is None else MK.moe_block_inference(x, *args, residual=x,

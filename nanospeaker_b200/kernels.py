@@ -636,6 +636,48 @@ def block_infer(x, router_w_padded, logit_bias, w_in, w_out, w_sh_in, w_sh_out, 
     return out
 
 
+def stack_plan(layers, n_shared: int) -> torch.Tensor:
+    """Device buffer with the addresses of a stack's tensors (moe_b200_stack_plan), one
+    (router_w [D, E], logit_bias | None, w_in, w_out, w_sh_in | None, w_sh_out | None) per layer; valid
+    while those tensors stay where they are."""
+    lib = _lib.load()
+    n = len(layers)
+    host = torch.zeros(lib.moe_b200_stack_plan_bytes(n), dtype=torch.uint8)
+    for i, (rw, bias, w_in, w_out, sh_in, sh_out) in enumerate(layers):
+        _need_cuda(rw, bias, w_in, w_out, sh_in, sh_out)
+        e, d, h2 = w_in.shape
+        _lib.check(lib.moe_b200_stack_plan(
+            host.data_ptr(), n, i, rw.data_ptr(), _lib.ptr(bias), w_in.data_ptr(),
+            w_out.data_ptr(), _lib.ptr(sh_in), _lib.ptr(sh_out), e, n_shared, d, h2 // 2),
+            "moe_b200_stack_plan")
+    return host.to(layers[0][0].device)
+
+
+def stack_supported(n_tokens: int, d_model: int, d_hidden: int, n_experts: int, n_shared: int,
+                    top_k: int) -> bool:
+    return bool(_lib.load().moe_b200_stack_supported(n_tokens, d_model, d_hidden, n_experts,
+                                                     n_shared, top_k))
+
+
+def stack_infer(plan: torch.Tensor, n_layers: int, x: torch.Tensor, d_hidden: int, n_experts: int,
+                n_shared: int, top_k: int, normalize: bool, act: int) -> torch.Tensor:
+    """x <- x + block_l(x) through a stack of blocks in one persistent kernel."""
+    import ctypes
+    _need_cuda(x, plan)
+    t, d = x.shape
+    lib = _lib.load()
+    out = torch.empty_like(x)
+    nbytes = lib.moe_b200_stack_scratch_bytes(t, d, n_shared, top_k)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    n_l = ctypes.c_int32(0)
+    _lib.check(lib.moe_b200_stack_infer(
+        plan.data_ptr(), n_layers, x.data_ptr(), out.data_ptr(), t, d, d_hidden, n_experts,
+        n_shared, top_k, int(normalize), act, scratch.data_ptr(), nbytes, ctypes.byref(n_l),
+        status_word(x.device).data_ptr(), _stream(x)), "moe_b200_stack_infer")
+    _count(n_l.value)
+    return out
+
+
 def block_bwd(grad_out, grad_aux, x, logit_bias, noise, w_in, w_out, w_sh_in, w_sh_out, xs, a1,
               logits, w_all, idx_all, sids, eids, offs, counts_all, npp, wp, top_k: int,
               normalize: bool, full_softmax: bool, aux_coef: float, act: int, side_streams):

@@ -20,6 +20,11 @@
 // Everything is summed in a fixed order: results are bit-reproducible.
 //
 // The grid is launched cooperatively (its CTAs wait on one another); every wait is bounded.
+//
+// Nearly every instruction runs once or twice per layer, so the code is as much on the critical path as
+// the data: straight-line code that misses the small instruction caches costs some 20 cycles an
+// instruction. Loops are kept rolled, rare variants out of line, and the weight loads are a few
+// instructions of one warp (176 KB of unrolled code: 27 us a layer at 64 tokens).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math_constants.h>
@@ -43,9 +48,10 @@ constexpr int ST_SLICE = 32;               // of them in one work item
 constexpr int ST_SLICES = ST_H / ST_SLICE;
 constexpr int ST_STAGE = 8192;             // ring stage: [64 d x (32 gate + 32 up)] or [32 units x 128 d]
 constexpr int ST_HALF = ST_STAGE / 2;      // one TMA box
-// 8 warps: with one more (a warp of its own for the TMA loads) a thread is left with 168 registers, and
-// the spills, which find no room in the L1 that 227 KB of shared memory leave, cost more than the work.
-constexpr int ST_WARPS = 8;
+// 16 warps: the phases are chains of dependent instructions, so what counts is how few of them a warp
+// has. (A 17th warp for the TMA loads would leave a thread 96 registers, and the spills find no room in
+// the L1 that 227 KB of shared memory leave.)
+constexpr int ST_WARPS = 16;
 constexpr int ST_THREADS = ST_WARPS * 32;
 constexpr int ST_PASS = 16;                // tokens per pass over an item (two mma column tiles)
 constexpr int ST_ACC_LD = 68;              // floats between tokens of the up accumulators
@@ -56,10 +62,15 @@ constexpr int ST_MAX_ITEMS = 8;            // items of one CTA and layer
 constexpr int ST_MAX_STAGES = 24;
 constexpr int ST_PARTS = 32;               // barriers for the two parts of an item; more than stages
 constexpr int ST_MAX_SLOTS = 4;            // tokens of one CTA
-// Router weight chunks (four columns of a row) that a thread holds across the hand-over, in registers;
-// as many more as fit go to the row buffers, which are free then (all 45 at 76 experts and d_model
-// 576). Loaded after the hand-over, they cost an L2 latency a batch.
-constexpr int ST_ROUTER_PRE = 27;
+constexpr int ST_RED_BYTES = 16 * ST_THREADS;   // token phase: partial sums, then the router's
+static_assert(ST_RED_BYTES <= ST_ACC_BYTES, "they share the accumulators' place");
+// Router weight chunks (four columns of a row; a thread has 23 at 76 experts and d_model 576): the
+// first ST_ROUTER_PRE are held in registers across the hand-over, the next are copied to the row
+// buffer and the accumulators, which are free then, and ST_ROUTER_LATE more are fetched when the
+// partial rows are in. Chunks loaded at their use cost an L2 latency a batch.
+constexpr int ST_ROUTER_PRE = 12, ST_ROUTER_LATE = 8;
+static_assert(ST_PASS == ST_WARPS, "a warp has one token of a pass");
+static_assert(ST_MAX_STAGES <= 32, "a lane has one stage of the ring");
 static_assert(ST_MAX_ITEMS <= ST_WARPS, "a warp lists one item's tokens");
 
 struct alignas(64) StackLayer {
@@ -72,8 +83,6 @@ struct StackArgs {
   const StackLayer* layers;
   int32_t n_layers, T, D, E, S, k, normalize, act;
   int32_t n_stages;                        // of the ring
-  int32_t xs_bufs;                         // token row buffers: 2 (the next pass's rows arrive under
-                                           // this one's work) or 1
   int32_t kshift;                          // idx rows hold 1 << kshift entries: 8 or 16
   int32_t sh_tokens, sh_blocks;            // a shared expert's tokens are cut into blocks
   int32_t n_items;                         // per layer: S * slices * sh_blocks, then E * slices
@@ -125,7 +134,7 @@ __device__ __forceinline__ void ldsm4_t(uint32_t addr, uint32_t* r) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -145,21 +154,28 @@ __device__ __forceinline__ uint32_t load_gpu(const uint32_t* ctr) {
 __device__ __forceinline__ float4 ldcg4(const float* p) {
   return __ldcg(reinterpret_cast<const float4*>(p));
 }
-__device__ __forceinline__ float stack_act(int act, float g) {
+__device__ __noinline__ float stack_other_act(int act, float g) {
   switch (act) {
-    case ACT_SILU: return act_f<ACT_SILU>(g);
     case ACT_GELU: return act_f<ACT_GELU>(g);
     case ACT_RELU: return act_f<ACT_RELU>(g);
     case ACT_SIGMOID: return act_f<ACT_SIGMOID>(g);
     default: return act_f<ACT_TANH>(g);
   }
 }
+__device__ __forceinline__ float stack_act(int act, float g) {
+  return act == ACT_SILU ? act_f<ACT_SILU>(g) : stack_other_act(act, g);
+}
+// A value that the compiler cannot reason about: keeps it from cloning loops for their special cases.
+__device__ __forceinline__ int opaque(int v) {
+  asm volatile("" : "+r"(v));
+  return v;
+}
 
 // Shared memory behind the ring, in order.
 struct StackSmem {
   int xs, acc, hid, list, xrow, res, tokw, lg, bars, misc, total;
 };
-__host__ __device__ inline StackSmem stack_smem(int T, int D, int n_stages, int xs_bufs) {
+__host__ __device__ inline StackSmem stack_smem(int T, int D, int n_stages) {
   const int dpad = (D + 63) / 64 * 64;
   StackSmem s;
   int at = n_stages * ST_STAGE;
@@ -168,7 +184,7 @@ __host__ __device__ inline StackSmem stack_smem(int T, int D, int n_stages, int 
     at += (bytes + 15) / 16 * 16;
     return r;
   };
-  s.xs = take(xs_bufs * ST_PASS * (dpad * 2 + 16));    // token rows of a pass
+  s.xs = take(ST_PASS * (dpad * 2 + 16));              // token rows of a pass
   s.acc = take(ST_ACC_BYTES);                          // up accumulators; token phase: partial sums
   s.hid = take((T + ST_PASS - 1) / ST_PASS * ST_PASS * ST_HID_LD * 2);
   s.list = take(2 * ST_MAX_ITEMS * T * 2);             // an item's tokens, and their pairs
@@ -208,6 +224,7 @@ __device__ __forceinline__ void stack_select(const float* lg, int E, int k, int 
     for (int o = 16; o; o >>= 1) denom += __shfl_xor_sync(0xffffffffu, denom, o);
   }
   int sel = 0;
+#pragma unroll 1
   for (int j = 0; j < k; ++j) {
     uint32_t best = key[0];
 #pragma unroll
@@ -240,11 +257,12 @@ __device__ __forceinline__ void stack_select(const float* lg, int E, int k, int 
   *weight = active ? __bfloat162float(__float2bfloat16(w)) : 1.f;   // past k: the shared experts
 }
 
+template <int SELECT>   // values per lane in the expert selection: at most 32 * SELECT experts
 __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~uintptr_t(1023));
-  const StackSmem L = stack_smem(p.T, p.D, p.n_stages, p.xs_bufs);
+  // (aligned by an offset, not through an integer: the accesses stay shared-memory ones)
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const StackSmem L = stack_smem(p.T, p.D, p.n_stages);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.bars);   // [ST_PARTS] up / down weights of an item
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.misc);
   int* cnt = reinterpret_cast<int*>(smem + L.misc + 16);
@@ -252,7 +270,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = int(gridDim.x), cta = int(blockIdx.x);
   const int D = p.D, dpad = (D + 63) / 64 * 64;
-  const int n_in = dpad / 64, n_box = n_in, n_out = (n_box + 1) / 2;   // ring stages of one item
+  const int n_in = dpad / 64, n_out = (n_in + 1) / 2, n_st = n_in + n_out;   // ring stages of one item
   const int NS = p.n_stages;
   const int kS = p.k + p.S;
   // this CTA's items (all but the last round are full)
@@ -268,55 +286,53 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   __syncthreads();
   pdl_wait();   // the counters, x and the weights may come from the kernels before this one
 
-  // The ring is filled from where it is emptied: whenever an item's stages are free, one warp issues as
-  // many of the coming loads as there is room for. (The loads' state lives in that warp.)
+  // The ring is filled from where it is emptied, by one warp: lane s owns stage s of the ring and knows
+  // what it holds next (item stages are numbered through: items of a layer, layers). When the stages
+  // [ring_s, ring_s + n) are free again, their lanes issue their loads side by side.
   constexpr int FILL_WARP = ST_WARPS - 1;
-  const uint32_t ring_u = smem_u32(smem);
-  int f_s = 0, f_free = NS, f_layer = 0, f_item = 0, f_stage = 0, f_part = 0;
-  auto refill = [&](int freed) {
-    f_free += freed;
-    while (f_free > 0 && f_layer < p.n_layers && n_mine > 0) {
-      const StackItem item = items[f_item];
-      const StackLayer* ly = p.layers + f_layer;
-      const bool shared = item.expert >= p.E, down = f_stage >= n_in;
-      const int g = shared ? item.expert - p.E : item.expert;
-      const int n = min(f_free, (down ? n_in + n_out : n_in) - f_stage);   // stages of this part
-      uint64_t* bar = full + f_part % ST_PARTS;
-      if (lane == 0 && f_stage == (down ? n_in : 0))
-        mbar_expect_tx(bar, down ? n_box * ST_HALF : n_in * ST_STAGE);
-      __syncwarp();
-      const CUtensorMap* map = down ? (shared ? &ly->sh_out : &ly->out) : (shared ? &ly->sh_in : &ly->in);
-      for (int i = lane; i < n; i += 32) {
-        const int st = f_s + i < NS ? f_s + i : f_s + i - NS;
-        uint8_t* dst = smem + st * ST_STAGE;
-        if (down) {
-          const int b = 2 * (f_stage - n_in + i);
-          tma_load_3d(dst, map, bar, b * 64, item.slice * ST_SLICE, g);
-          if (b + 1 < n_box) tma_load_3d(dst + ST_HALF, map, bar, b * 64 + 64, item.slice * ST_SLICE, g);
-        } else {
-          tma_load_3d(dst, map, bar, item.slice * ST_SLICE, (f_stage + i) * 64, g);
-          tma_load_3d(dst + ST_HALF, map, bar, ST_H + item.slice * ST_SLICE, (f_stage + i) * 64, g);
-        }
-      }
-      __syncwarp();
-      f_s = f_s + n < NS ? f_s + n : f_s + n - NS;
-      f_free -= n;
-      f_stage += n;
-      if (f_stage == n_in) ++f_part;
-      if (f_stage == n_in + n_out) {
-        ++f_part;
-        f_stage = 0;
-        if (++f_item == n_mine) {
-          f_item = 0;
-          ++f_layer;
-        }
+  int f_layer = 0, f_item = 0, f_stage = lane, f_part = 0;   // of this lane's stage
+  auto f_normalise = [&] {
+#pragma unroll 1
+    while (f_stage >= n_st) {
+      f_stage -= n_st;
+      f_part += 2;
+      if (++f_item == n_mine) {
+        f_item = 0;
+        ++f_layer;
       }
     }
   };
-  if (warp == FILL_WARP) refill(0);
+  auto refill = [&](int from, int n) {   // n <= NS stages, from `from` on around the ring
+    const int off = lane >= from ? lane - from : lane + NS - from;
+    if (lane < NS && off < n && f_layer < p.n_layers) {
+      const StackItem item = items[f_item];
+      const StackLayer* ly = p.layers + f_layer;
+      const bool shared = item.expert >= p.E, down = f_stage >= n_in;
+      const CUtensorMap* map = shared ? &ly->sh_in : &ly->in;
+      if (down) ++map;   // (the maps lie in the order in, out, sh_in, sh_out)
+      const int g = shared ? item.expert - p.E : item.expert;
+      uint64_t* bar = full + (f_part + (down ? 1 : 0)) % ST_PARTS;
+      if (f_stage == 0) mbar_expect_tx(bar, n_in * ST_STAGE);
+      if (f_stage == n_in) mbar_expect_tx(bar, n_in * ST_HALF);
+      const int c = f_stage - n_in;   // down: boxes 2c, 2c + 1
+      const int x = down ? c * 128 : item.slice * ST_SLICE, y = down ? item.slice * ST_SLICE : f_stage * 64;
+      tma_load_3d(smem + lane * ST_STAGE, map, bar, x, y, g);
+      if (!down || 2 * c + 1 < n_in)
+        tma_load_3d(smem + lane * ST_STAGE + ST_HALF, map, bar, down ? x + 64 : x + ST_H, y, g);
+      f_stage += NS;
+      f_normalise();
+    }
+    __syncwarp();
+  };
+  if (warp == FILL_WARP && n_mine > 0) {
+    f_normalise();
+    refill(0, NS);
+  }
 
-  const uint32_t xs_ld = dpad * 2 + 16, xs_bytes = ST_PASS * xs_ld;
+  const uint32_t ring_u = smem_u32(smem), xs_u = smem_u32(smem + L.xs);
+  const uint32_t xs_ld = dpad * 2 + 16;
   float* acc_s = reinterpret_cast<float*>(smem + L.acc);
+  float* red_s = reinterpret_cast<float*>(smem + L.acc + ST_ACC_BYTES - ST_RED_BYTES);
   __nv_bfloat16* hid_s = reinterpret_cast<__nv_bfloat16*>(smem + L.hid);
   uint16_t* list = reinterpret_cast<uint16_t*>(smem + L.list);   // [item][tokens | pairs][T]
   float* xrow = reinterpret_cast<float*>(smem + L.xrow);
@@ -331,6 +347,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   auto grid_wait = [&](const uint32_t* ctr, uint32_t target) {
     if (tid == 0) {
       uint32_t n = 0;
+#pragma unroll 1
       while (load_gpu(ctr) < target) {
         if (++n > (1u << 22) || ((n & 1023u) == 0 && *reinterpret_cast<volatile int32_t*>(p.status))) {
           atomicExch(p.status, ST_WAIT_TIMEOUT);
@@ -341,7 +358,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
     }
     __syncthreads();
     if (*abort_flag == 0) return true;
-    for (int n = 0; n < 1000; ++n) __nanosleep(1000);   // let the loads in flight land
+    __nanosleep(1000000);   // let the loads in flight land
     return false;
   };
   int ring_s = 0, part = 0;   // the ring as the consumers see it: the current item's first stage, its part
@@ -351,88 +368,82 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
       *abort_flag = 1;
     }
   };
-  auto stage_of = [&](int c) {   // (an item may have more stages than the ring)
-    int s = ring_s + c;
-    while (s >= NS) s -= NS;
-    return s;
-  };
-  auto item_done = [&] {
-    ring_s = stage_of(n_in + n_out);
-    part += 2;
-  };
 
   // router weight: a thread owns four columns (4 * (tid % P)) of every Q-th row
   const int P = p.E / 4, Q = ST_THREADS / P;
   const int rp = tid % P, rq = tid / P;
-  const int router_more =   // chunks of this thread in the row buffers
-      max(0, min((D - rq + Q - 1) / Q - ST_ROUTER_PRE, int(p.xs_bufs * xs_bytes / (ST_THREADS * 8))));
-  const int cg = D / 4;   // token phase: 16-byte column groups
+  const int router_rows = rq < Q ? (D - rq + Q - 1) / Q : 0;
+  const int router_room = (L.acc - L.xs + ST_ACC_BYTES - ST_RED_BYTES) / (ST_THREADS * 8);
+  const int cg = D / 4, groups = ST_THREADS / cg;   // token phase: 16-byte column groups, sets of pairs
   const __nv_bfloat16* rw = p.layers[0].router_w;   // (the next layer's are fetched a layer ahead)
   const float* bias = p.layers[0].bias;
 
-  for (int l = 0; l <= p.n_layers; ++l) {
-    const bool last = l == p.n_layers;
+#pragma unroll 1
+  for (int l = 0;; l = opaque(l + 1)) {   // (leaves in the token phase behind the last layer)
+    const bool last = opaque(l) == p.n_layers;
     // ------------------------------------------------------------------ token phase
     if (has_token) {
       uint2 wr[ST_ROUTER_PRE];   // (on its way while this CTA waits for the others' partial rows)
+      const uint2* rsrc = reinterpret_cast<const uint2*>(rw + rq * p.E + 4 * rp);
+      const int rstep = Q * P, rn = last ? 0 : router_rows;   // (in chunks of four columns)
 #pragma unroll
-      for (int i = 0; i < ST_ROUTER_PRE; ++i) {
-        const int d = rq + i * Q;
-        wr[i] = !last && rq < Q && d < D
-                    ? __ldg(reinterpret_cast<const uint2*>(rw + d * p.E + 4 * rp))
-                    : make_uint2(0u, 0u);
-      }
-      if (!last && rq < Q) {
-        const __nv_bfloat16* src = rw + (rq + ST_ROUTER_PRE * Q) * p.E + 4 * rp;
-        for (int i = 0; i < router_more; ++i)
-          cp_async_8(smem_u32(smem + L.xs) + (i * ST_THREADS + tid) * 8, src + i * Q * p.E);
-      }
+      for (int i = 0; i < ST_ROUTER_PRE; ++i)
+        wr[i] = i < rn ? __ldg(rsrc + i * rstep) : make_uint2(0u, 0u);
+#pragma unroll 1
+      for (int i = ST_ROUTER_PRE; i < min(rn, ST_ROUTER_PRE + router_room); ++i)
+        cp_async_8(xs_u + ((i - ST_ROUTER_PRE) * ST_THREADS + tid) * 8, rsrc + i * rstep);
       cp_async_commit();
-      if (l > 0 && !grid_wait(p.ctr + 1, uint32_t(l) * G)) return;
+      if (opaque(l) > 0 && !grid_wait(p.ctr + 1, uint32_t(l) * G)) return;
+#pragma unroll 1
       for (int t = cta, slot = 0; t < p.T; t += G, ++slot) {
+        const bool first = opaque(l) == 0, last = opaque(l) == p.n_layers;
         __nv_bfloat16* my_res = res + slot * D;
         float* my_w = tokw + slot * 16;
-        // the row: residual + the pairs' partial rows, in order; four columns per thread and step,
-        // the rows cut into `groups` interleaved sets when there are threads for it
-        const int groups = max(1, ST_THREADS / cg);
-        if (l > 0) {
-          const int R = kS * ST_SLICES;
-          const float* base = p.partial + int64_t(t) * R * D;
-          for (int i = tid; i < groups * cg; i += ST_THREADS) {
-            const int g = i / cg, c = i - g * cg;
-            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int r0 = g; r0 < R; r0 += 16 * groups) {
-              float4 v[16];
+        // the row: residual + the pairs' rows in order, each the sum of its slices' partial rows; four
+        // columns per thread, the pairs cut into `groups` interleaved sets
+        if (!first && tid < groups * cg) {
+          const int g = tid / cg, c = tid - g * cg;
+          const float* base = p.partial + int64_t(t) * kS * ST_SLICES * D + 4 * c;
+          float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+          for (int j0 = g; j0 < kS; j0 += 3 * groups) {
+            float4 v[3][ST_SLICES];
 #pragma unroll
-              for (int u = 0; u < 16; ++u) {
-                const int r = r0 + u * groups;
-                v[u] = r < R ? ldcg4(base + r * D + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
-              }
+            for (int u = 0; u < 3; ++u)
 #pragma unroll
-              for (int u = 0; u < 16; ++u) {
-                const int r = r0 + u * groups;
-                const float w = r < R ? my_w[r / ST_SLICES] : 0.f;
-                a.x += w * v[u].x;
-                a.y += w * v[u].y;
-                a.z += w * v[u].z;
-                a.w += w * v[u].w;
-              }
+              for (int q = 0; q < ST_SLICES; ++q)
+                v[u][q] = ldcg4(base + (min(j0 + u * groups, kS - 1) * ST_SLICES + q) * D);
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+              const float w = j0 + u * groups < kS ? my_w[j0 + u * groups] : 0.f;
+              a.x += w * ((v[u][0].x + v[u][1].x) + (v[u][2].x + v[u][3].x));
+              a.y += w * ((v[u][0].y + v[u][1].y) + (v[u][2].y + v[u][3].y));
+              a.z += w * ((v[u][0].z + v[u][1].z) + (v[u][2].z + v[u][3].z));
+              a.w += w * ((v[u][0].w + v[u][1].w) + (v[u][2].w + v[u][3].w));
             }
-            *reinterpret_cast<float4*>(acc_s + g * D + 4 * c) = a;
           }
-          __syncthreads();
+          *reinterpret_cast<float4*>(red_s + g * D + 4 * c) = a;
         }
+        uint2 wl[ST_ROUTER_LATE];
+        const int i_late = ST_ROUTER_PRE + router_room;
+#pragma unroll
+        for (int u = 0; u < ST_ROUTER_LATE; ++u)
+          wl[u] = i_late + u < rn ? __ldg(rsrc + (i_late + u) * rstep) : make_uint2(0u, 0u);
+        __syncthreads();
+#pragma unroll 1
         for (int d = 2 * tid; d < dpad; d += 2 * ST_THREADS) {
           float v0 = 0.f, v1 = 0.f;
           if (d < D) {
             __nv_bfloat162 h;
-            if (l > 0) {
+            if (!first) {
               const float2 f = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(my_res + d));
               v0 = f.x;
               v1 = f.y;
+#pragma unroll 1
               for (int g = 0; g < groups; ++g) {
-                v0 += acc_s[g * D + d];
-                v1 += acc_s[g * D + d + 1];
+                const float2 r = *reinterpret_cast<const float2*>(red_s + g * D + d);
+                v0 += r.x;
+                v1 += r.y;
               }
               h = __floats2bfloat162_rn(v0, v1);
             } else {
@@ -444,8 +455,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
             v0 = f.x;
             v1 = f.y;
           }
-          xrow[d] = v0;
-          xrow[d + 1] = v1;
+          *reinterpret_cast<float2*>(xrow + d) = make_float2(v0, v1);
         }
         __syncthreads();
         if (last) continue;
@@ -458,44 +468,37 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
             a3 += x * __uint_as_float(w.y & 0xffff0000u);
           };
 #pragma unroll
-          for (int i = 0; i < ST_ROUTER_PRE; ++i) {
-            const int d = rq + i * Q;
-            if (d < D) add(wr[i], xrow[d]);
-          }
+          for (int i = 0; i < ST_ROUTER_PRE; ++i) add(wr[i], xrow[min(rq + i * Q, D - 1)]);
           cp_async_wait<0>();   // (a thread reads back what it copied itself)
           const uint2* ws = reinterpret_cast<const uint2*>(smem + L.xs) + tid;
-#pragma unroll 4
-          for (int i = 0; i < router_more; ++i) add(ws[i * ST_THREADS], xrow[rq + (ST_ROUTER_PRE + i) * Q]);
-          for (int d0 = rq + (ST_ROUTER_PRE + router_more) * Q; d0 < D; d0 += 16 * Q) {
-            uint2 w[16];
+          int i = ST_ROUTER_PRE;
+#pragma unroll 2
+          for (; i < min(rn, ST_ROUTER_PRE + router_room); ++i)
+            add(ws[(i - ST_ROUTER_PRE) * ST_THREADS], xrow[rq + i * Q]);
+#pragma unroll 1
+          for (; i < rn; i += ST_ROUTER_LATE) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-              w[i] = d0 + i * Q < D ? __ldg(reinterpret_cast<const uint2*>(
-                                          rw + (d0 + i * Q) * p.E + 4 * rp))
-                                    : make_uint2(0u, 0u);
+            for (int u = 0; u < ST_ROUTER_LATE; ++u) add(wl[u], xrow[min(rq + (i + u) * Q, D - 1)]);
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (d0 + i * Q < D) add(w[i], xrow[d0 + i * Q]);
+            for (int u = 0; u < ST_ROUTER_LATE; ++u)
+              wl[u] = i + ST_ROUTER_LATE + u < rn ? __ldg(rsrc + (i + ST_ROUTER_LATE + u) * rstep)
+                                                  : make_uint2(0u, 0u);
           }
-          *reinterpret_cast<float4*>(acc_s + rq * p.E + 4 * rp) = make_float4(a0, a1, a2, a3);
+          *reinterpret_cast<float4*>(red_s + rq * p.E + 4 * rp) = make_float4(a0, a1, a2, a3);
         }
         const float b = bias != nullptr && tid < p.E ? __ldg(bias + tid) : 0.f;
         __syncthreads();
         if (tid < p.E) {   // (at most 256 experts: one thread each)
           float s = 0.f;
-#pragma unroll 16
-          for (int q = 0; q < Q; ++q) s += acc_s[q * p.E + tid];
+#pragma unroll 4
+          for (int q = 0; q < Q; ++q) s += red_s[q * p.E + tid];
           lg[tid] = __bfloat162float(__float2bfloat16(s)) + b;
         }
         __syncthreads();
         if (warp == 0) {
           int sel;
           float w;
-          if (p.E <= 32) stack_select<1>(lg, p.E, p.k, p.normalize, lane, &sel, &w);
-          else if (p.E <= 64) stack_select<2>(lg, p.E, p.k, p.normalize, lane, &sel, &w);
-          else if (p.E <= 96) stack_select<3>(lg, p.E, p.k, p.normalize, lane, &sel, &w);
-          else if (p.E <= 128) stack_select<4>(lg, p.E, p.k, p.normalize, lane, &sel, &w);
-          else stack_select<8>(lg, p.E, p.k, p.normalize, lane, &sel, &w);
+          stack_select<SELECT>(lg, p.E, p.k, p.normalize, lane, &sel, &w);
           if (lane < kpad) p.idx[t * kpad + lane] = uint16_t(sel);
           if (lane < kS) my_w[lane] = w;
         }
@@ -520,23 +523,23 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
       uint16_t *tok = list + 2 * warp * p.T, *pair = tok + p.T;
       int n = 0;
       if (item.n >= 0) {
+#pragma unroll 1
         for (int i = lane; i < item.n; i += 32) {
           tok[i] = uint16_t(item.t0 + i);
           pair[i] = uint16_t((item.t0 + i) * kS + p.k + (item.expert - p.E));
         }
         n = item.n;
       } else {
+#pragma unroll 1
         for (int b = lane * 8; b - lane * 8 < p.T * kpad; b += 256) {
           uint4 v = make_uint4(~0u, ~0u, ~0u, ~0u);
           if (b < p.T * kpad) v = __ldcg(reinterpret_cast<const uint4*>(p.idx + b));
-          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-          uint32_t hits = 0;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            hits |= uint32_t((w[i] & 0xffffu) == uint32_t(item.expert)) << (2 * i);
-            hits |= uint32_t((w[i] >> 16) == uint32_t(item.expert)) << (2 * i + 1);
-          }
-          // a token chooses an expert once; eight entries are one token's (or half of one's)
+          // the place of the expert among the eight entries: a token chooses an expert once, and
+          // eight entries are one token's (or half of one's)
+          const uint32_t e2 = uint32_t(item.expert) * 0x10001u;
+          const uint32_t h0 = __vcmpeq2(v.x, e2) & 0x00020001u, h1 = __vcmpeq2(v.y, e2) & 0x00080004u;
+          const uint32_t h2 = __vcmpeq2(v.z, e2) & 0x00200010u, h3 = __vcmpeq2(v.w, e2) & 0x00800040u;
+          const uint32_t h = h0 | h1 | h2 | h3, hits = (h | (h >> 16)) & 0xffu;
           const unsigned m = __ballot_sync(0xffffffffu, hits != 0);
           if (hits) {
             const int i = n + __popc(m & ((1u << lane) - 1u)), at = b + __ffs(hits) - 1;
@@ -550,160 +553,141 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
       if (lane == 0) cnt[warp] = n;
     }
     __syncthreads();
-    // the rows of the tokens [n0, n0 + 16) of item r, into row buffer `buf`
-    auto gather = [&](int r, int n0, int buf) {
-      const uint16_t* tok = list + 2 * r * p.T + n0;
-      const int nn = min(ST_PASS, cnt[r] - n0), cpr = dpad / 8;
-      const uint32_t dst = smem_u32(smem + L.xs) + buf * xs_bytes;
-      for (int row = warp; row < nn; row += ST_WARPS) {
-        const __nv_bfloat16* src = p.xbuf + int64_t(tok[row]) * D;
-        for (int c = lane; c < cpr; c += 32)
-          cp_async_16(dst + row * xs_ld + c * 16, c * 8 < D ? src + c * 8 : src, c * 8 < D ? 16u : 0u);
-      }
-      cp_async_commit();
-    };
-    // the rows of the pass after (r, n0): the same item's next tokens, or the next item that has any
-    auto gather_next = [&](int r, int n0, int buf) {
+    // The rows of the pass after (r, n0) -- the same item's next tokens, or the next item that has any --
+    // are fetched as soon as this pass has read its own; a warp has one row.
+    auto gather_next = [&](int r, int n0) {
       n0 += ST_PASS;
       if (r < 0 || n0 >= cnt[r]) {
         n0 = 0;
+#pragma unroll 1
         do ++r;
         while (r < n_mine && cnt[r] == 0);
       }
-      if (r < n_mine) gather(r, n0, buf);
-    };
-    int buf = 0;
-    gather_next(-1, 0, 0);
-    for (int r = 0; r < n_mine; ++r) {
-      const int slice = items[r].slice;
-      const int n = cnt[r];
-      if (n == 0) {   // nobody chose it: the ring moves on
-        if (warp == FILL_WARP) {
-          part_wait(part);
-          refill(n_in);
-          part_wait(part + 1);
-          refill(n_out);
-        }
-        item_done();
-        continue;
+      if (r < n_mine && warp < cnt[r] - n0) {
+        const __nv_bfloat16* src = p.xbuf + int(list[2 * r * p.T + n0 + warp]) * D + lane * 8;
+        uint32_t dst = xs_u + warp * xs_ld + lane * 16;
+#pragma unroll 1
+        for (int c = lane * 8; c < dpad; c += 256, src += 256, dst += 512)
+          cp_async_16(dst, c < D ? src : p.xbuf, c < D ? 16u : 0u);
       }
-      // up/gate + GLU: 64 outputs (gate and up, two mma rows each) x 16 tokens; warps 2i, 2i + 1 take
-      // the i-th quarter of every 64-deep stage
-      const int mg = warp & 1, kp = warp >> 1;
-      for (int n0 = 0; n0 < n; n0 += ST_PASS) {
-        const int nn = min(ST_PASS, n - n0);
-        cp_async_wait<0>();
-        __syncthreads();
-        if (p.xs_bufs == 2) gather_next(r, n0, buf ^ 1);   // (under this pass's work)
-        if (n0 == 0) part_wait(part);
-        float acc[2][2][4] = {};
-        const int a_k = kp * 16 + (lane & 7) + ((lane >> 4) & 1) * 8;
-        const int a_c = (lane >> 3) & 1;
-        const uint32_t sw = (a_k >> 1) & 3;
-        const uint32_t a0 = mg * ST_HALF + a_k * 64 + ((a_c ^ sw) << 4);
-        const uint32_t a1 = mg * ST_HALF + a_k * 64 + (((a_c + 2) ^ sw) << 4);
-        uint32_t b_addr = smem_u32(smem + L.xs) + buf * xs_bytes + (kp * 16 + ((lane >> 3) & 1) * 8) * 2;
-        int s = ring_s;
-        if (nn > 8) {
-          b_addr += ((lane & 7) + ((lane >> 4) & 1) * 8) * xs_ld;
-#pragma unroll 3
-          for (int c = 0; c < n_in; ++c) {
-            uint32_t a[2][4], b[4];
-            ldsm4_t(ring_u + s * ST_STAGE + a0, a[0]);
-            ldsm4_t(ring_u + s * ST_STAGE + a1, a[1]);
-            ldsm4(b_addr + c * 128, b);
-            mma_bf16(acc[0][0], a[0], b[0], b[1]);
-            mma_bf16(acc[1][0], a[1], b[0], b[1]);
-            mma_bf16(acc[0][1], a[0], b[2], b[3]);
-            mma_bf16(acc[1][1], a[1], b[2], b[3]);
-            if (++s == NS) s = 0;
+      cp_async_commit();
+    };
+    gather_next(-1, 0);
+#pragma unroll 1
+    for (int r = 0; r < n_mine; ++r) {
+      const int n = cnt[r];
+      // (an item that nobody chose only moves the ring on)
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half, ++part) {   // up/gate, then down; each gives its stages back
+        if (n == 0) {
+          if (warp == FILL_WARP) part_wait(part);
+        } else if (half == 0) {
+          // up/gate + GLU: 64 outputs (gate, up: two mma rows each) x 16 tokens; the four warps of an
+          // mma row take a quarter of every 64-deep stage each
+          const int mt = warp & 3, kp = warp >> 2;
+#pragma unroll 1
+          for (int n0 = 0; n0 < n; n0 += ST_PASS) {
+            const int nn = min(ST_PASS, n - n0);
+            cp_async_wait<0>();
+            __syncthreads();
+            if (n0 == 0) part_wait(part);
+            float acc[2][2][4] = {};   // [even / odd stages][column tile]
+            const int a_k = kp * 16 + (lane & 7) + ((lane >> 4) & 1) * 8;
+            const int a_c = (mt & 1) * 2 + ((lane >> 3) & 1);
+            const uint32_t a0 = ring_u + (mt >> 1) * ST_HALF + a_k * 64 + ((a_c ^ ((a_k >> 1) & 3)) << 4);
+            // (the second column tile's rows may be stale: their columns are not used)
+            uint32_t b_addr = xs_u + (kp * 16 + ((lane >> 3) & 1) * 8) * 2 +
+                              ((lane & 7) + ((lane >> 4) & 1) * 8) * xs_ld;
+            uint32_t a_addr = a0 + ring_s * ST_STAGE;
+            const uint32_t a_end = a0 + NS * ST_STAGE;
+#pragma unroll 1
+            for (int c = 0; c < n_in; c += 3, b_addr += 384) {
+              uint32_t a[3][4], b[3][4];
+#pragma unroll
+              for (int u = 0; u < 3; ++u) {   // (behind the last stage: repeated, and not used)
+                ldsm4_t(a_addr, a[u]);
+                ldsm4(c + u < n_in ? b_addr + u * 128 : b_addr, b[u]);
+                a_addr += ST_STAGE;
+                if (a_addr == a_end) a_addr = a0;
+              }
+#pragma unroll
+              for (int u = 0; u < 3; ++u)
+                if (c + u < n_in) {
+                  mma_bf16(acc[u & 1][0], a[u], b[u][0], b[u][1]);
+                  mma_bf16(acc[u & 1][1], a[u], b[u][2], b[u][3]);
+                }
+            }
+            float* dst = acc_s + (kp * ST_PASS + 2 * (lane & 3)) * ST_ACC_LD + mt * 16 + (lane >> 2);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              float* d = dst + 8 * q * ST_ACC_LD;
+              d[0] = acc[0][q][0] + acc[1][q][0];
+              d[ST_ACC_LD] = acc[0][q][1] + acc[1][q][1];
+              d[8] = acc[0][q][2] + acc[1][q][2];
+              d[ST_ACC_LD + 8] = acc[0][q][3] + acc[1][q][3];
+            }
+            __syncthreads();
+            gather_next(r, n0);
+            if (warp < nn) {   // a warp: the 32 units of a token
+              float g = 0.f, up = 0.f;
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                g += acc_s[(q * ST_PASS + warp) * ST_ACC_LD + lane];
+                up += acc_s[(q * ST_PASS + warp) * ST_ACC_LD + 32 + lane];
+              }
+              hid_s[(n0 + warp) * ST_HID_LD + lane] = __float2bfloat16(stack_act(p.act, g) * up);
+            }
           }
         } else {
-          b_addr += (lane & 7) * xs_ld;
-#pragma unroll 3
-          for (int c = 0; c < n_in; ++c) {
-            uint32_t a[2][4], b[2];
-            ldsm4_t(ring_u + s * ST_STAGE + a0, a[0]);
-            ldsm4_t(ring_u + s * ST_STAGE + a1, a[1]);
-            ldsm2(b_addr + c * 128, b);
-            mma_bf16(acc[0][0], a[0], b[0], b[1]);
-            mma_bf16(acc[1][0], a[1], b[0], b[1]);
-            if (++s == NS) s = 0;
-          }
-        }
-        float* dst = acc_s + (kp * ST_PASS + 2 * (lane & 3)) * ST_ACC_LD + mg * 32 + (lane >> 2);
+          // down: D outputs in rows of 16, 32 deep; a warp takes every 16th row
+          part_wait(part);
+          const uint16_t* pair = list + (2 * r + 1) * p.T;
+          float* out0 = p.partial + items[r].slice * D + (lane >> 2);
+          const int u0 = (lane & 7) + ((lane >> 4) & 1) * 8, c0 = (lane >> 3) & 1;
+#pragma unroll 1
+          for (int n0 = 0; n0 < n; n0 += ST_PASS) {
+            uint32_t b[2][4];
+            const uint32_t h_addr = smem_u32(hid_s) +
+                                    (n0 + (lane & 7) + ((lane >> 4) & 1) * 8) * (ST_HID_LD * 2) +
+                                    ((lane >> 3) & 1) * 16;
+            ldsm4(h_addr, b[0]);
+            ldsm4(h_addr + 32, b[1]);
+            int dst[4];   // this thread's four tokens: where their rows begin, or -1
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            if (q == 1 && nn <= 8) break;
-            float* d = dst + 8 * q * ST_ACC_LD + m * 16;
-            d[0] = acc[m][q][0];
-            d[ST_ACC_LD] = acc[m][q][1];
-            d[8] = acc[m][q][2];
-            d[ST_ACC_LD + 8] = acc[m][q][3];
-          }
-        __syncthreads();
-        if (n0 + ST_PASS >= n && warp == FILL_WARP) refill(n_in);
-        if (p.xs_bufs == 1)
-          gather_next(r, n0, 0);
-        else
-          buf ^= 1;
-        for (int row = warp; row < nn; row += ST_WARPS) {   // 32 units of a token per warp
-          float g = 0.f, up = 0.f;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            g += acc_s[(q * ST_PASS + row) * ST_ACC_LD + lane];
-            up += acc_s[(q * ST_PASS + row) * ST_ACC_LD + 32 + lane];
-          }
-          hid_s[(n0 + row) * ST_HID_LD + lane] = __float2bfloat16(stack_act(p.act, g) * up);
-        }
-      }
-      __syncthreads();
-      // down: D outputs in rows of 16, 32 deep; a warp takes every 8th row
-      part_wait(part + 1);
-      const uint16_t* pair = list + (2 * r + 1) * p.T;
-      const int u0 = (lane & 7) + ((lane >> 4) & 1) * 8, c0 = (lane >> 3) & 1;
-      for (int n0 = 0; n0 < n; n0 += ST_PASS) {
-        uint32_t b[2][4];
-        const uint32_t h_addr = smem_u32(hid_s) +
-                                (n0 + (lane & 7) + ((lane >> 4) & 1) * 8) * (ST_HID_LD * 2) +
-                                ((lane >> 3) & 1) * 16;
-        ldsm4(h_addr, b[0]);
-        ldsm4(h_addr + 32, b[1]);
-        float* dst[4];   // this thread's four tokens
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int i = n0 + 8 * (q >> 1) + 2 * (lane & 3) + (q & 1);
-          dst[q] = i < n ? p.partial + (int64_t(pair[i]) * ST_SLICES + slice) * D + (lane >> 2)
-                         : nullptr;
-        }
-        const bool two = n - n0 > 8;
-#pragma unroll 2
-        for (int m = warp; m < D / 16; m += ST_WARPS) {
-          uint32_t a[2][4];
-          const uint32_t box = ring_u + stage_of(n_in + (m >> 3)) * ST_STAGE + ((m >> 2) & 1) * ST_HALF;
-          const uint32_t ch = (((m & 3) * 2 + c0) ^ (u0 & 7)) << 4;
-          ldsm4_t(box + u0 * 128 + ch, a[0]);
-          ldsm4_t(box + (u0 + 16) * 128 + ch, a[1]);
-          float acc[2][4] = {};
-          mma_bf16(acc[0], a[0], b[0][0], b[0][1]);
-          mma_bf16(acc[0], a[1], b[1][0], b[1][1]);
-          if (two) {
-            mma_bf16(acc[1], a[0], b[0][2], b[0][3]);
-            mma_bf16(acc[1], a[1], b[1][2], b[1][3]);
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (dst[q] != nullptr) {
-              dst[q][m * 16] = acc[q >> 1][q & 1];
-              dst[q][m * 16 + 8] = acc[q >> 1][2 + (q & 1)];
+            for (int q = 0; q < 4; ++q) {
+              const int i = n0 + 8 * (q >> 1) + 2 * (lane & 3) + (q & 1);
+              dst[q] = i < n ? int(pair[i]) * (ST_SLICES * D) : -1;
             }
+#pragma unroll 1
+            for (int m = warp; m < D / 16; m += ST_WARPS) {
+              uint32_t a[2][4];
+              int s = ring_s + (m >> 3);
+#pragma unroll 1
+              while (s >= NS) s -= NS;
+              const uint32_t box = ring_u + s * ST_STAGE + ((m >> 2) & 1) * ST_HALF +
+                                   u0 * 128 + ((((m & 3) * 2 + c0) ^ (u0 & 7)) << 4);
+              ldsm4_t(box, a[0]);
+              ldsm4_t(box + 16 * 128, a[1]);
+              float acc[2][4] = {};
+              mma_bf16(acc[0], a[0], b[0][0], b[0][1]);
+              mma_bf16(acc[1], a[0], b[0][2], b[0][3]);
+              mma_bf16(acc[0], a[1], b[1][0], b[1][1]);
+              mma_bf16(acc[1], a[1], b[1][2], b[1][3]);
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (dst[q] >= 0) {
+                  float* d = out0 + dst[q] + m * 16;
+                  d[0] = acc[q >> 1][q & 1];
+                  d[8] = acc[q >> 1][2 + (q & 1)];
+                }
+            }
+          }
         }
+        if (n > 0) __syncthreads();
+        const int freed = half == 0 ? n_in : n_out;
+        if (warp == FILL_WARP) refill(ring_s, freed);
+        ring_s = ring_s + freed < NS ? ring_s + freed : ring_s + freed - NS;
       }
-      __syncthreads();
-      if (warp == FILL_WARP) refill(n_out);
-      item_done();
     }
     if (tid == 0) arrive_gpu(p.ctr + 1);
   }
@@ -728,7 +712,7 @@ __global__ void stack_reset_kernel(uint32_t* ctr) {
 
 // The shape side of a launch; false: the layer-by-layer path is the one that takes it.
 struct StackShape {
-  int sh_tokens, sh_blocks, n_items, n_stages, xs_bufs, smem;
+  int sh_tokens, sh_blocks, n_items, n_stages, smem;
 };
 static bool stack_shape(int64_t T, int D, int H, int E, int S, int k, StackShape* o) {
   if (T < 1 || T > ST_MAX_T || H != ST_H || D < 64 || D % 32 != 0 || D > 1024 || E < 4 ||
@@ -736,20 +720,16 @@ static bool stack_shape(int64_t T, int D, int H, int E, int S, int k, StackShape
     return false;
   const int grid = stack_grid();
   if (T > int64_t(ST_MAX_SLOTS) * grid) return false;
-  // a shared expert sees every token: 32 of them per work item keep it in the range of the others
-  o->sh_tokens = int(std::min<int64_t>(T, 32));
+  // a shared expert sees every token: one pass's worth of them per work item keeps it in the range of
+  // the others, as long as that does not give every CTA more items
+  o->sh_tokens = int(std::min<int64_t>(T, T > 128 ? 2 * ST_PASS : ST_PASS));
   o->sh_blocks = int((T + o->sh_tokens - 1) / o->sh_tokens);
   o->n_items = ST_SLICES * (E + S * o->sh_blocks);
   if (o->n_items > ST_MAX_ITEMS * grid) return false;
-  // two row buffers unless they cost the ring the stages that an item's up weights need at once
-  const int limit = 232448 - 1024, n_in = (D + 63) / 64;
-  for (o->xs_bufs = 2; o->xs_bufs > 0; --o->xs_bufs) {
-    const int rest = stack_smem(int(T), D, 0, o->xs_bufs).total;
-    o->n_stages = std::min((limit - rest) / ST_STAGE, ST_MAX_STAGES);
-    if (limit > rest && o->n_stages >= n_in) break;
-  }
-  if (o->xs_bufs == 0) return false;
-  o->smem = stack_smem(int(T), D, o->n_stages, o->xs_bufs).total + 1024;
+  const int limit = 232448 - 1024, rest = stack_smem(int(T), D, 0).total, n_in = (D + 63) / 64;
+  o->n_stages = std::min((limit - rest) / ST_STAGE, ST_MAX_STAGES);
+  if (limit < rest || o->n_stages < n_in) return false;   // an item's up weights are there at once
+  o->smem = stack_smem(int(T), D, o->n_stages).total + 1024;
   return true;
 }
 
@@ -850,7 +830,9 @@ int moe_b200_stack_infer(const void* plan, int32_t n_layers, const void* x, void
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(stack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    attr_err = cudaFuncSetAttribute(stack_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    if (attr_err == cudaSuccess)
+      attr_err = cudaFuncSetAttribute(stack_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
   });
   if (attr_err != cudaSuccess) return MOE_B200_ERR_CUDA;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -866,7 +848,6 @@ int moe_b200_stack_infer(const void* plan, int32_t n_layers, const void* x, void
   a.normalize = normalize;
   a.act = activation;
   a.n_stages = o.n_stages;
-  a.xs_bufs = o.xs_bufs;
   a.kshift = top_k <= 8 ? 3 : 4;
   a.sh_tokens = o.sh_tokens;
   a.sh_blocks = o.sh_blocks;
@@ -888,7 +869,8 @@ int moe_b200_stack_infer(const void* plan, int32_t n_layers, const void* x, void
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, stack_kernel, a) != cudaSuccess) return MOE_B200_ERR_CUDA;
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, n_experts <= 96 ? stack_kernel<3> : stack_kernel<8>, a);
+  if (err != cudaSuccess) return MOE_B200_ERR_CUDA;
   if (n_launches) *n_launches = 2;
   return MOE_B200_OK;
 }

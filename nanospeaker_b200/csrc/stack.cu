@@ -46,8 +46,8 @@ namespace moe {
 constexpr int ST_H = 128;                  // hidden units per expert
 constexpr int ST_SLICE = 32;               // of them in one work item
 constexpr int ST_SLICES = ST_H / ST_SLICE;
-constexpr int ST_STAGE = 8192;             // ring stage: [64 d x (32 gate + 32 up)] or [32 units x 128 d]
-constexpr int ST_HALF = ST_STAGE / 2;      // one TMA box
+constexpr int ST_STAGE = 8192;             // ring stage: [gate | up][64 d][32 units] or [2][32 units][64 d]
+constexpr int ST_HALF = ST_STAGE / 2;
 // 16 warps: the phases are chains of dependent instructions, so what counts is how few of them a warp
 // has. (A 17th warp for the TMA loads would leave a thread 96 registers, and the spills find no room in
 // the L1 that 227 KB of shared memory leave.)
@@ -70,7 +70,7 @@ static_assert(ST_RED_BYTES <= ST_ACC_BYTES, "they share the accumulators' place"
 // partial rows are in. Chunks loaded at their use cost an L2 latency a batch.
 constexpr int ST_ROUTER_PRE = 12, ST_ROUTER_LATE = 8;
 static_assert(ST_PASS == ST_WARPS, "a warp has one token of a pass");
-static_assert(ST_MAX_STAGES <= 32, "a lane has one stage of the ring");
+static_assert(ST_MAX_STAGES <= 2 * ST_WARPS, "two lanes of a warp have one stage of the ring each");
 static_assert(ST_MAX_ITEMS <= ST_WARPS, "a warp lists one item's tokens");
 
 struct alignas(64) StackLayer {
@@ -83,6 +83,7 @@ struct StackArgs {
   const StackLayer* layers;
   int32_t n_layers, T, D, E, S, k, normalize, act;
   int32_t n_stages;                        // of the ring
+  int32_t out_boxes;                       // TMA boxes per down stage: 1, or 2 when d_model % 64 != 0
   int32_t kshift;                          // idx rows hold 1 << kshift entries: 8 or 16
   int32_t sh_tokens, sh_blocks;            // a shared expert's tokens are cut into blocks
   int32_t n_items;                         // per layer: S * slices * sh_blocks, then E * slices
@@ -191,38 +192,22 @@ __host__ __device__ inline StackSmem stack_smem(int T, int D, int n_stages) {
   s.xrow = take(dpad * 4);                             // token phase: the row, fp32
   s.res = take(ST_MAX_SLOTS * D * 2);                  // residual rows of this CTA's tokens
   s.tokw = take(ST_MAX_SLOTS * 16 * 4);                // their pairs' weights
-  s.lg = take(MAX_EXPERTS * 4);
+  s.lg = take(2 * MAX_EXPERTS * 4);                    // logits, their sort keys
   s.bars = take(ST_PARTS * 8);
   s.misc = take(16 + ST_MAX_ITEMS * 4 + ST_MAX_ITEMS * 16);   // abort flag, token counts, items
   s.total = at;
   return s;
 }
 
-// One warp: the k largest of lg[0, E) (value descending, ties to the lowest index) and their softmax
-// weights, rounded to bf16. NS = ceil(E / 32) values per lane. Lane j returns the j-th choice.
+// One warp: the k largest of lg[0, E) (value descending, ties to the lowest index; keys[e] is
+// float_key of lg[e], at least 1) and their softmax weights, rounded to bf16. NS = ceil(E / 32) values
+// per lane. Lane j returns the j-th choice.
 template <int NS>
-__device__ __forceinline__ void stack_select(const float* lg, int E, int k, int normalize, int lane,
-                                             int* idx, float* weight) {
-  float v[NS];
+__device__ __forceinline__ void stack_select(const float* lg, const uint32_t* keys, int E, int k,
+                                             int normalize, int lane, int* idx, float* weight) {
   uint32_t key[NS];
-  float mx = -CUDART_INF_F;
 #pragma unroll
-  for (int i = 0; i < NS; ++i) {
-    const int e = i * 32 + lane;
-    v[i] = e < E ? lg[e] : -CUDART_INF_F;
-    const uint32_t fk = float_key(v[i]);
-    key[i] = e < E ? (fk == 0u ? 1u : fk) : 0u;
-    mx = fmaxf(mx, v[i]);
-  }
-  float denom = 0.f;
-  if (!normalize) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-#pragma unroll
-    for (int i = 0; i < NS; ++i) denom += i * 32 + lane < E ? expf(v[i] - mx) : 0.f;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) denom += __shfl_xor_sync(0xffffffffu, denom, o);
-  }
+  for (int i = 0; i < NS; ++i) key[i] = i * 32 + lane < E ? keys[i * 32 + lane] : 0u;
   int sel = 0;
 #pragma unroll 1
   for (int j = 0; j < k; ++j) {
@@ -240,21 +225,23 @@ __device__ __forceinline__ void stack_select(const float* lg, int E, int k, int 
       if (i * 32 + lane == win) key[i] = 0u;
     if (lane == j) sel = win;
   }
-  const bool active = lane < k;
-  const float val = active ? lg[sel] : -CUDART_INF_F;
-  float w;
+  const bool active = lane < k;   // (k <= 16)
+  const float val = lg[sel];
+  const float top = __shfl_sync(0xffffffffu, val, 0);
+  const float ex = active ? expf(val - top) : 0.f;
+  float s = ex;
   if (normalize) {
-    const float top = __shfl_sync(0xffffffffu, val, 0);
-    const float ex = active ? expf(val - top) : 0.f;
-    float s = ex;
+#pragma unroll
+    for (int o = 8; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  } else {
+    s = 0.f;
+#pragma unroll 1
+    for (int e = lane; e < E; e += 32) s += expf(lg[e] - top);
 #pragma unroll
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    w = ex / s;
-  } else {
-    w = active ? expf(val - mx) / denom : 0.f;
   }
   *idx = active ? sel : 0xffff;
-  *weight = active ? __bfloat162float(__float2bfloat16(w)) : 1.f;   // past k: the shared experts
+  *weight = active ? __bfloat162float(__float2bfloat16(ex / s)) : 1.f;   // past k: the shared experts
 }
 
 template <int SELECT>   // values per lane in the expert selection: at most 32 * SELECT experts
@@ -286,11 +273,13 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   __syncthreads();
   pdl_wait();   // the counters, x and the weights may come from the kernels before this one
 
-  // The ring is filled from where it is emptied, by one warp: lane s owns stage s of the ring and knows
-  // what it holds next (item stages are numbered through: items of a layer, layers). When the stages
-  // [ring_s, ring_s + n) are free again, their lanes issue their loads side by side.
-  constexpr int FILL_WARP = ST_WARPS - 1;
-  int f_layer = 0, f_item = 0, f_stage = lane, f_part = 0;   // of this lane's stage
+  // The ring is filled from where it is emptied: stage s of the ring belongs to lane s / 16 of warp
+  // s % 16, which knows what it holds next (item stages are numbered through: items of a layer,
+  // layers). When the stages [from, from + n) are free again, their owners issue one load each (18
+  // loads from one warp took 0.6 us, twice per item).
+  const int f_slot = warp + ST_WARPS * lane;
+  const bool f_owner = lane < 2 && f_slot < NS && n_mine > 0;
+  int f_layer = 0, f_item = 0, f_stage = f_slot, f_part = 0;   // of this lane's stage
   auto f_normalise = [&] {
 #pragma unroll 1
     while (f_stage >= n_st) {
@@ -303,31 +292,36 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
     }
   };
   auto refill = [&](int from, int n) {   // n <= NS stages, from `from` on around the ring
-    const int off = lane >= from ? lane - from : lane + NS - from;
-    if (lane < NS && off < n && f_layer < p.n_layers) {
+    const int off = f_slot >= from ? f_slot - from : f_slot + NS - from;
+    if (f_owner && off < n && f_layer < p.n_layers) {
       const StackItem item = items[f_item];
-      const StackLayer* ly = p.layers + f_layer;
       const bool shared = item.expert >= p.E, down = f_stage >= n_in;
-      const CUtensorMap* map = shared ? &ly->sh_in : &ly->in;
-      if (down) ++map;   // (the maps lie in the order in, out, sh_in, sh_out)
-      const int g = shared ? item.expert - p.E : item.expert;
+      // (a layer's maps lie in the order in, out, sh_in, sh_out)
+      const CUtensorMap* map = &p.layers[f_layer].in + (shared ? 2 : 0) + (down ? 1 : 0);
+      const int g = shared ? item.expert - p.E : item.expert, u = item.slice * ST_SLICE;
       uint64_t* bar = full + (f_part + (down ? 1 : 0)) % ST_PARTS;
-      if (f_stage == 0) mbar_expect_tx(bar, n_in * ST_STAGE);
-      if (f_stage == n_in) mbar_expect_tx(bar, n_in * ST_HALF);
-      const int c = f_stage - n_in;   // down: boxes 2c, 2c + 1
-      const int x = down ? c * 128 : item.slice * ST_SLICE, y = down ? item.slice * ST_SLICE : f_stage * 64;
-      tma_load_3d(smem + lane * ST_STAGE, map, bar, x, y, g);
-      if (!down || 2 * c + 1 < n_in)
-        tma_load_3d(smem + lane * ST_STAGE + ST_HALF, map, bar, down ? x + 64 : x + ST_H, y, g);
+      uint8_t* dst = smem + f_slot * ST_STAGE;
+      if (!down) {
+        if (f_stage == 0) mbar_expect_tx(bar, n_in * ST_STAGE);
+        tma_load_4d(dst, map, bar, u, f_stage * 64, 0, g);
+      } else {
+        const int c = f_stage - n_in;
+        if (c == 0) mbar_expect_tx(bar, n_out * ST_STAGE);
+        if (p.out_boxes == 1) {
+          tma_load_4d(dst, map, bar, 0, u, 2 * c, g);
+        } else {
+          tma_load_3d(dst, map, bar, c * 128, u, g);
+          tma_load_3d(dst + ST_HALF, map, bar, c * 128 + 64, u, g);
+        }
+      }
       f_stage += NS;
       f_normalise();
     }
     __syncwarp();
   };
-  if (warp == FILL_WARP && n_mine > 0) {
-    f_normalise();
-    refill(0, NS);
-  }
+  if (f_owner) f_normalise();
+  __syncwarp();
+  refill(0, NS);
 
   const uint32_t ring_u = smem_u32(smem), xs_u = smem_u32(smem + L.xs);
   const uint32_t xs_ld = dpad * 2 + 16;
@@ -339,6 +333,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   __nv_bfloat16* res = reinterpret_cast<__nv_bfloat16*>(smem + L.res);
   float* tokw = reinterpret_cast<float*>(smem + L.tokw);
   float* lg = reinterpret_cast<float*>(smem + L.lg);
+  uint32_t* keys = reinterpret_cast<uint32_t*>(smem + L.lg) + MAX_EXPERTS;
   const int token_ctas = min(p.T, G);
   const bool has_token = cta < p.T;
   const int kpad = 1 << p.kshift;
@@ -492,13 +487,15 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
           float s = 0.f;
 #pragma unroll 4
           for (int q = 0; q < Q; ++q) s += red_s[q * p.E + tid];
-          lg[tid] = __bfloat162float(__float2bfloat16(s)) + b;
+          s = __bfloat162float(__float2bfloat16(s)) + b;
+          lg[tid] = s;
+          keys[tid] = max(float_key(s), 1u);
         }
         __syncthreads();
         if (warp == 0) {
           int sel;
           float w;
-          stack_select<SELECT>(lg, p.E, p.k, p.normalize, lane, &sel, &w);
+          stack_select<SELECT>(lg, keys, p.E, p.k, p.normalize, lane, &sel, &w);
           if (lane < kpad) p.idx[t * kpad + lane] = uint16_t(sel);
           if (lane < kS) my_w[lane] = w;
         }
@@ -530,10 +527,15 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
         }
         n = item.n;
       } else {
+        auto entries = [&](int b) {
+          return b < p.T * kpad ? __ldcg(reinterpret_cast<const uint4*>(p.idx + b))
+                                : make_uint4(~0u, ~0u, ~0u, ~0u);
+        };
+        uint4 next = entries(lane * 8);
 #pragma unroll 1
         for (int b = lane * 8; b - lane * 8 < p.T * kpad; b += 256) {
-          uint4 v = make_uint4(~0u, ~0u, ~0u, ~0u);
-          if (b < p.T * kpad) v = __ldcg(reinterpret_cast<const uint4*>(p.idx + b));
+          const uint4 v = next;
+          next = entries(b + 256);
           // the place of the expert among the eight entries: a token chooses an expert once, and
           // eight entries are one token's (or half of one's)
           const uint32_t e2 = uint32_t(item.expert) * 0x10001u;
@@ -573,6 +575,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
       cp_async_commit();
     };
     gather_next(-1, 0);
+    // The arrival does not wait for what only moves the ring on: a release stands in the memory pipe
+    // behind the loads issued before it.
+    int last_live = n_mine - 1;
+#pragma unroll 1
+    while (last_live >= 0 && cnt[last_live] == 0) --last_live;
+    if (last_live < 0 && tid == 0) arrive_gpu(p.ctr + 1);
 #pragma unroll 1
     for (int r = 0; r < n_mine; ++r) {
       const int n = cnt[r];
@@ -580,7 +588,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
 #pragma unroll 1
       for (int half = 0; half < 2; ++half, ++part) {   // up/gate, then down; each gives its stages back
         if (n == 0) {
-          if (warp == FILL_WARP) part_wait(part);
+          part_wait(part);
         } else if (half == 0) {
           // up/gate + GLU: 64 outputs (gate, up: two mma rows each) x 16 tokens; the four warps of an
           // mma row take a quarter of every 64-deep stage each
@@ -684,12 +692,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
           }
         }
         if (n > 0) __syncthreads();
+        if (r == last_live && half == 1 && tid == 0) arrive_gpu(p.ctr + 1);
         const int freed = half == 0 ? n_in : n_out;
-        if (warp == FILL_WARP) refill(ring_s, freed);
+        refill(ring_s, freed);
         ring_s = ring_s + freed < NS ? ring_s + freed : ring_s + freed - NS;
       }
     }
-    if (tid == 0) arrive_gpu(p.ctr + 1);
   }
 }
 
@@ -793,14 +801,22 @@ int moe_b200_stack_plan(void* host_plan, int32_t n_layers, int32_t layer, const 
   StackLayer ly;
   std::memset(&ly, 0, sizeof(ly));
   const auto maps = [&](CUtensorMap* in, CUtensorMap* out, const void* wi, const void* wo, int g) {
-    const uint64_t di[3] = {uint64_t(2 * d_hidden), uint64_t(d_model), uint64_t(g)};
-    const uint64_t si[2] = {uint64_t(4 * d_hidden), uint64_t(4 * d_hidden) * d_model};
-    const uint32_t bi[3] = {ST_SLICE, 64, 1};
+    // W_in [g][gate | up][d][128] (strides in that order of the box): 32 columns of 64 rows of both
+    const uint64_t di[4] = {uint64_t(d_hidden), uint64_t(d_model), 2, uint64_t(g)};
+    const uint64_t si[3] = {uint64_t(4 * d_hidden), uint64_t(2 * d_hidden),
+                            uint64_t(4 * d_hidden) * d_model};
+    const uint32_t bi[4] = {ST_SLICE, 64, 2, 1};
+    if (!make_map(in, wi, 4, di, si, bi, CU_TENSOR_MAP_SWIZZLE_64B)) return false;
+    if (d_model % 64 == 0) {   // W_out [g][128][d / 64][64]: two column blocks of 32 rows
+      const uint64_t dn[4] = {64, uint64_t(d_hidden), uint64_t(d_model / 64), uint64_t(g)};
+      const uint64_t sn[3] = {uint64_t(2 * d_model), 128, uint64_t(2 * d_model) * d_hidden};
+      const uint32_t bn[4] = {64, ST_SLICE, 2, 1};
+      return make_map(out, wo, 4, dn, sn, bn);
+    }
     const uint64_t dn[3] = {uint64_t(d_model), uint64_t(d_hidden), uint64_t(g)};
     const uint64_t sn[2] = {uint64_t(2 * d_model), uint64_t(2 * d_model) * d_hidden};
     const uint32_t bn[3] = {64, ST_SLICE, 1};
-    return make_map(in, wi, 3, di, si, bi, CU_TENSOR_MAP_SWIZZLE_64B) &&
-           make_map(out, wo, 3, dn, sn, bn);
+    return make_map(out, wo, 3, dn, sn, bn);
   };
   if (!maps(&ly.in, &ly.out, w_in, w_out, n_experts)) return MOE_B200_ERR_TMA;
   if (n_shared > 0 && !maps(&ly.sh_in, &ly.sh_out, w_sh_in, w_sh_out, n_shared))
@@ -848,6 +864,7 @@ int moe_b200_stack_infer(const void* plan, int32_t n_layers, const void* x, void
   a.normalize = normalize;
   a.act = activation;
   a.n_stages = o.n_stages;
+  a.out_boxes = d_model % 64 == 0 ? 1 : 2;
   a.kshift = top_k <= 8 ? 3 : 4;
   a.sh_tokens = o.sh_tokens;
   a.sh_blocks = o.sh_blocks;

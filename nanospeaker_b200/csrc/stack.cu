@@ -48,11 +48,13 @@ constexpr int ST_SLICE = 32;               // of them in one work item
 constexpr int ST_SLICES = ST_H / ST_SLICE;
 constexpr int ST_STAGE = 8192;             // ring stage: [gate | up][64 d][32 units] or [2][32 units][64 d]
 constexpr int ST_HALF = ST_STAGE / 2;
-// 16 warps: the phases are chains of dependent instructions, so what counts is how few of them a warp
-// has. (A 17th warp for the TMA loads would leave a thread 96 registers, and the spills find no room in
-// the L1 that 227 KB of shared memory leave.)
+// 16 compute warps: the phases are chains of dependent instructions, so what counts is how few of them a
+// warp has. One more warp issues the TMA loads: a box of 64-byte rows occupies the TMA unit for some
+// 200 cycles, and whoever issues a part's loads stands in that queue for a microsecond. (It leaves a
+// thread 96 registers; a spill would cost more, it finds no room in the L1 beside the shared memory.)
 constexpr int ST_WARPS = 16;
-constexpr int ST_THREADS = ST_WARPS * 32;
+constexpr int ST_CT = ST_WARPS * 32;       // compute threads
+constexpr int ST_THREADS = ST_CT + 32;
 constexpr int ST_PASS = 16;                // tokens per pass over an item (two mma column tiles)
 constexpr int ST_ACC_LD = 68;              // floats between tokens of the up accumulators
 constexpr int ST_ACC_BYTES = 4 * ST_PASS * ST_ACC_LD * 4;
@@ -62,15 +64,15 @@ constexpr int ST_MAX_ITEMS = 8;            // items of one CTA and layer
 constexpr int ST_MAX_STAGES = 24;
 constexpr int ST_PARTS = 32;               // barriers for the two parts of an item; more than stages
 constexpr int ST_MAX_SLOTS = 4;            // tokens of one CTA
-constexpr int ST_RED_BYTES = 16 * ST_THREADS;   // token phase: partial sums, then the router's
+constexpr int ST_RED_BYTES = 16 * ST_CT;   // token phase: partial sums, then the router's
 static_assert(ST_RED_BYTES <= ST_ACC_BYTES, "they share the accumulators' place");
 // Router weight chunks (four columns of a row; a thread has 23 at 76 experts and d_model 576): the
 // first ST_ROUTER_PRE are held in registers across the hand-over, the next are copied to the row
-// buffer and the accumulators, which are free then, and ST_ROUTER_LATE more are fetched when the
-// partial rows are in. Chunks loaded at their use cost an L2 latency a batch.
-constexpr int ST_ROUTER_PRE = 12, ST_ROUTER_LATE = 8;
+// buffer and the accumulators, which are free then, and ST_ROUTER_EXTRA bytes beside them, and
+// ST_ROUTER_LATE more are fetched when the partial rows are in. Chunks loaded at their use cost an L2
+// latency a batch.
+constexpr int ST_ROUTER_PRE = 5, ST_ROUTER_LATE = 10, ST_ROUTER_EXTRA = 8192;
 static_assert(ST_PASS == ST_WARPS, "a warp has one token of a pass");
-static_assert(ST_MAX_STAGES <= 2 * ST_WARPS, "two lanes of a warp have one stage of the ring each");
 static_assert(ST_MAX_ITEMS <= ST_WARPS, "a warp lists one item's tokens");
 
 struct alignas(64) StackLayer {
@@ -83,6 +85,7 @@ struct StackArgs {
   const StackLayer* layers;
   int32_t n_layers, T, D, E, S, k, normalize, act;
   int32_t n_stages;                        // of the ring
+  int32_t router_extra;                    // bytes of shared memory for router weight chunks alone
   int32_t out_boxes;                       // TMA boxes per down stage: 1, or 2 when d_model % 64 != 0
   int32_t kshift;                          // idx rows hold 1 << kshift entries: 8 or 16
   int32_t sh_tokens, sh_blocks;            // a shared expert's tokens are cut into blocks
@@ -144,6 +147,9 @@ __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b
 __device__ __forceinline__ void cp_async_8(uint32_t dst_smem, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst_smem), "l"(src) : "memory");
 }
+__device__ __forceinline__ void ct_sync() {   // the compute warps
+  asm volatile("bar.sync 1, %0;" ::"n"(ST_CT) : "memory");
+}
 __device__ __forceinline__ void arrive_gpu(uint32_t* ctr) {
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
 }
@@ -176,7 +182,7 @@ __device__ __forceinline__ int opaque(int v) {
 struct StackSmem {
   int xs, acc, hid, list, xrow, res, tokw, lg, bars, misc, total;
 };
-__host__ __device__ inline StackSmem stack_smem(int T, int D, int n_stages) {
+__host__ __device__ inline StackSmem stack_smem(int T, int D, int n_stages, int extra) {
   const int dpad = (D + 63) / 64 * 64;
   StackSmem s;
   int at = n_stages * ST_STAGE;
@@ -185,6 +191,7 @@ __host__ __device__ inline StackSmem stack_smem(int T, int D, int n_stages) {
     at += (bytes + 15) / 16 * 16;
     return r;
   };
+  take(extra);                                         // router weight chunks, with xs and acc
   s.xs = take(ST_PASS * (dpad * 2 + 16));              // token rows of a pass
   s.acc = take(ST_ACC_BYTES);                          // up accumulators; token phase: partial sums
   s.hid = take((T + ST_PASS - 1) / ST_PASS * ST_PASS * ST_HID_LD * 2);
@@ -193,7 +200,7 @@ __host__ __device__ inline StackSmem stack_smem(int T, int D, int n_stages) {
   s.res = take(ST_MAX_SLOTS * D * 2);                  // residual rows of this CTA's tokens
   s.tokw = take(ST_MAX_SLOTS * 16 * 4);                // their pairs' weights
   s.lg = take(2 * MAX_EXPERTS * 4);                    // logits, their sort keys
-  s.bars = take(ST_PARTS * 8);
+  s.bars = take(2 * ST_PARTS * 8);
   s.misc = take(16 + ST_MAX_ITEMS * 4 + ST_MAX_ITEMS * 16);   // abort flag, token counts, items
   s.total = at;
   return s;
@@ -249,15 +256,16 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   extern __shared__ uint8_t smem_raw[];
   // (aligned by an offset, not through an integer: the accesses stay shared-memory ones)
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  const StackSmem L = stack_smem(p.T, p.D, p.n_stages);
+  const StackSmem L = stack_smem(p.T, p.D, p.n_stages, p.router_extra);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.bars);   // [ST_PARTS] up / down weights of an item
+  uint64_t* empty = full + ST_PARTS;                             // [ST_PARTS] their stages are free again
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.misc);
   int* cnt = reinterpret_cast<int*>(smem + L.misc + 16);
   StackItem* items = reinterpret_cast<StackItem*>(smem + L.misc + 16 + ST_MAX_ITEMS * 4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = int(gridDim.x), cta = int(blockIdx.x);
   const int D = p.D, dpad = (D + 63) / 64 * 64;
-  const int n_in = dpad / 64, n_out = (n_in + 1) / 2, n_st = n_in + n_out;   // ring stages of one item
+  const int n_in = dpad / 64, n_out = (n_in + 1) / 2;   // ring stages of one item
   const int NS = p.n_stages;
   const int kS = p.k + p.S;
   // this CTA's items (all but the last round are full)
@@ -265,7 +273,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   const int n_mine = rounds - (stack_position(rounds - 1, cta, G) < p.n_items ? 0 : 1);
 
   if (tid == 0) {
-    for (int s = 0; s < ST_PARTS; ++s) mbar_init(full + s, 1);
+    for (int s = 0; s < 2 * ST_PARTS; ++s) mbar_init(full + s, 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -273,56 +281,57 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   __syncthreads();
   pdl_wait();   // the counters, x and the weights may come from the kernels before this one
 
-  // The ring is filled from where it is emptied: stage s of the ring belongs to lane s / 16 of warp
-  // s % 16, which knows what it holds next (item stages are numbered through: items of a layer,
-  // layers). When the stages [from, from + n) are free again, their owners issue one load each (18
-  // loads from one warp took 0.6 us, twice per item).
-  const int f_slot = warp + ST_WARPS * lane;
-  const bool f_owner = lane < 2 && f_slot < NS && n_mine > 0;
-  int f_layer = 0, f_item = 0, f_stage = f_slot, f_part = 0;   // of this lane's stage
-  auto f_normalise = [&] {
+  if (warp == ST_WARPS) {
+    // ------------------------------------------------------------------ weights by TMA
+    if (elect_one() && n_mine > 0) {
+      int slot = 0, part = 0;            // of the ring; of the loads
+      int ahead = NS, old_part = 0;      // stages until the next part's have to be free; that part
+      bool ok = true;
 #pragma unroll 1
-    while (f_stage >= n_st) {
-      f_stage -= n_st;
-      f_part += 2;
-      if (++f_item == n_mine) {
-        f_item = 0;
-        ++f_layer;
-      }
-    }
-  };
-  auto refill = [&](int from, int n) {   // n <= NS stages, from `from` on around the ring
-    const int off = f_slot >= from ? f_slot - from : f_slot + NS - from;
-    if (f_owner && off < n && f_layer < p.n_layers) {
-      const StackItem item = items[f_item];
-      const bool shared = item.expert >= p.E, down = f_stage >= n_in;
-      // (a layer's maps lie in the order in, out, sh_in, sh_out)
-      const CUtensorMap* map = &p.layers[f_layer].in + (shared ? 2 : 0) + (down ? 1 : 0);
-      const int g = shared ? item.expert - p.E : item.expert, u = item.slice * ST_SLICE;
-      uint64_t* bar = full + (f_part + (down ? 1 : 0)) % ST_PARTS;
-      uint8_t* dst = smem + f_slot * ST_STAGE;
-      if (!down) {
-        if (f_stage == 0) mbar_expect_tx(bar, n_in * ST_STAGE);
-        tma_load_4d(dst, map, bar, u, f_stage * 64, 0, g);
-      } else {
-        const int c = f_stage - n_in;
-        if (c == 0) mbar_expect_tx(bar, n_out * ST_STAGE);
-        if (p.out_boxes == 1) {
-          tma_load_4d(dst, map, bar, 0, u, 2 * c, g);
-        } else {
-          tma_load_3d(dst, map, bar, c * 128, u, g);
-          tma_load_3d(dst + ST_HALF, map, bar, c * 128 + 64, u, g);
+      for (int l = 0; l < p.n_layers && ok; ++l) {
+#pragma unroll 1
+        for (int r = 0; r < 2 * n_mine && ok; ++r, ++part) {   // up, down of every item
+          const StackItem item = items[r >> 1];
+          const bool shared = item.expert >= p.E, down = r & 1;
+          // (a layer's maps lie in the order in, out, sh_in, sh_out)
+          const CUtensorMap* map = &p.layers[l].in + (shared ? 2 : 0) + (down ? 1 : 0);
+          const int g = shared ? item.expert - p.E : item.expert, u = item.slice * ST_SLICE;
+          const int n = down ? n_out : n_in;
+          uint64_t* bar = full + part % ST_PARTS;
+#pragma unroll 1
+          for (int c = 0; c < n && ok; ++c) {
+            if (ahead == 0) {   // this stage was part old_part's
+              ok = mbar_wait(empty + old_part % ST_PARTS, (old_part / ST_PARTS) & 1, p.status) &&
+                   *abort_flag == 0;
+              if (!ok) break;
+              ahead = old_part & 1 ? n_out : n_in;
+              ++old_part;
+            }
+            --ahead;
+            if (c == 0) mbar_expect_tx(bar, n * ST_STAGE);
+            uint8_t* dst = smem + slot * ST_STAGE;
+            if (!down) {
+              tma_load_4d(dst, map, bar, u, c * 64, 0, g);
+            } else if (p.out_boxes == 1) {
+              tma_load_4d(dst, map, bar, 0, u, 2 * c, g);
+            } else {
+              tma_load_3d(dst, map, bar, c * 128, u, g);
+              tma_load_3d(dst + ST_HALF, map, bar, c * 128 + 64, u, g);
+            }
+            if (++slot == NS) slot = 0;
+          }
         }
       }
-      f_stage += NS;
-      f_normalise();
+      if (!ok) {   // given up: let what is in flight land before the CTA may leave
+        *abort_flag = 1;
+        atomicExch(p.status, ST_WAIT_TIMEOUT);
+        __nanosleep(1000000);
+      }
     }
-    __syncwarp();
-  };
-  if (f_owner) f_normalise();
-  __syncwarp();
-  refill(0, NS);
+    return;
+  }
 
+  // ---------------------------------------------------------------------- compute warps
   const uint32_t ring_u = smem_u32(smem), xs_u = smem_u32(smem + L.xs);
   const uint32_t xs_ld = dpad * 2 + 16;
   float* acc_s = reinterpret_cast<float*>(smem + L.acc);
@@ -351,10 +360,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
         }
       }
     }
-    __syncthreads();
-    if (*abort_flag == 0) return true;
-    __nanosleep(1000000);   // let the loads in flight land
-    return false;
+    ct_sync();
+    return *abort_flag == 0;
   };
   int ring_s = 0, part = 0;   // the ring as the consumers see it: the current item's first stage, its part
   auto part_wait = [&](int q) {
@@ -365,11 +372,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   };
 
   // router weight: a thread owns four columns (4 * (tid % P)) of every Q-th row
-  const int P = p.E / 4, Q = ST_THREADS / P;
+  const int P = p.E / 4, Q = ST_CT / P;
   const int rp = tid % P, rq = tid / P;
   const int router_rows = rq < Q ? (D - rq + Q - 1) / Q : 0;
-  const int router_room = (L.acc - L.xs + ST_ACC_BYTES - ST_RED_BYTES) / (ST_THREADS * 8);
-  const int cg = D / 4, groups = ST_THREADS / cg;   // token phase: 16-byte column groups, sets of pairs
+  const int router_room = (p.router_extra + L.acc - L.xs + ST_ACC_BYTES - ST_RED_BYTES) / (ST_CT * 8);
+  uint8_t* router_s = smem + L.xs - p.router_extra;
+  const int cg = D / 4, groups = ST_CT / cg;   // token phase: 16-byte column groups, sets of pairs
   const __nv_bfloat16* rw = p.layers[0].router_w;   // (the next layer's are fetched a layer ahead)
   const float* bias = p.layers[0].bias;
 
@@ -386,7 +394,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
         wr[i] = i < rn ? __ldg(rsrc + i * rstep) : make_uint2(0u, 0u);
 #pragma unroll 1
       for (int i = ST_ROUTER_PRE; i < min(rn, ST_ROUTER_PRE + router_room); ++i)
-        cp_async_8(xs_u + ((i - ST_ROUTER_PRE) * ST_THREADS + tid) * 8, rsrc + i * rstep);
+        cp_async_8(smem_u32(router_s) + ((i - ST_ROUTER_PRE) * ST_CT + tid) * 8, rsrc + i * rstep);
       cp_async_commit();
       if (opaque(l) > 0 && !grid_wait(p.ctr + 1, uint32_t(l) * G)) return;
 #pragma unroll 1
@@ -424,9 +432,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
 #pragma unroll
         for (int u = 0; u < ST_ROUTER_LATE; ++u)
           wl[u] = i_late + u < rn ? __ldg(rsrc + (i_late + u) * rstep) : make_uint2(0u, 0u);
-        __syncthreads();
+        ct_sync();
 #pragma unroll 1
-        for (int d = 2 * tid; d < dpad; d += 2 * ST_THREADS) {
+        for (int d = 2 * tid; d < dpad; d += 2 * ST_CT) {
           float v0 = 0.f, v1 = 0.f;
           if (d < D) {
             __nv_bfloat162 h;
@@ -452,7 +460,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
           }
           *reinterpret_cast<float2*>(xrow + d) = make_float2(v0, v1);
         }
-        __syncthreads();
+        ct_sync();
         if (last) continue;
         if (rq < Q) {
           float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
@@ -465,11 +473,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
 #pragma unroll
           for (int i = 0; i < ST_ROUTER_PRE; ++i) add(wr[i], xrow[min(rq + i * Q, D - 1)]);
           cp_async_wait<0>();   // (a thread reads back what it copied itself)
-          const uint2* ws = reinterpret_cast<const uint2*>(smem + L.xs) + tid;
+          const uint2* ws = reinterpret_cast<const uint2*>(router_s) + tid;
           int i = ST_ROUTER_PRE;
 #pragma unroll 2
           for (; i < min(rn, ST_ROUTER_PRE + router_room); ++i)
-            add(ws[(i - ST_ROUTER_PRE) * ST_THREADS], xrow[rq + i * Q]);
+            add(ws[(i - ST_ROUTER_PRE) * ST_CT], xrow[rq + i * Q]);
 #pragma unroll 1
           for (; i < rn; i += ST_ROUTER_LATE) {
 #pragma unroll
@@ -482,7 +490,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
           *reinterpret_cast<float4*>(red_s + rq * p.E + 4 * rp) = make_float4(a0, a1, a2, a3);
         }
         const float b = bias != nullptr && tid < p.E ? __ldg(bias + tid) : 0.f;
-        __syncthreads();
+        ct_sync();
         if (tid < p.E) {   // (at most 256 experts: one thread each)
           float s = 0.f;
 #pragma unroll 4
@@ -491,7 +499,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
           lg[tid] = s;
           keys[tid] = max(float_key(s), 1u);
         }
-        __syncthreads();
+        ct_sync();
         if (warp == 0) {
           int sel;
           float w;
@@ -499,7 +507,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
           if (lane < kpad) p.idx[t * kpad + lane] = uint16_t(sel);
           if (lane < kS) my_w[lane] = w;
         }
-        __syncthreads();
+        ct_sync();
       }
       if (last) return;
       if (tid == 0) arrive_gpu(p.ctr);   // (release: what the barrier above has collected)
@@ -554,7 +562,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
       }
       if (lane == 0) cnt[warp] = n;
     }
-    __syncthreads();
+    ct_sync();
     // The rows of the pass after (r, n0) -- the same item's next tokens, or the next item that has any --
     // are fetched as soon as this pass has read its own; a warp has one row.
     auto gather_next = [&](int r, int n0) {
@@ -588,7 +596,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
 #pragma unroll 1
       for (int half = 0; half < 2; ++half, ++part) {   // up/gate, then down; each gives its stages back
         if (n == 0) {
-          part_wait(part);
+          if (tid == 0) part_wait(part);
         } else if (half == 0) {
           // up/gate + GLU: 64 outputs (gate, up: two mma rows each) x 16 tokens; the four warps of an
           // mma row take a quarter of every 64-deep stage each
@@ -597,7 +605,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
           for (int n0 = 0; n0 < n; n0 += ST_PASS) {
             const int nn = min(ST_PASS, n - n0);
             cp_async_wait<0>();
-            __syncthreads();
+            ct_sync();
             if (n0 == 0) part_wait(part);
             float acc[2][2][4] = {};   // [even / odd stages][column tile]
             const int a_k = kp * 16 + (lane & 7) + ((lane >> 4) & 1) * 8;
@@ -634,7 +642,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
               d[8] = acc[0][q][2] + acc[1][q][2];
               d[ST_ACC_LD + 8] = acc[0][q][3] + acc[1][q][3];
             }
-            __syncthreads();
+            ct_sync();
             gather_next(r, n0);
             if (warp < nn) {   // a warp: the 32 units of a token
               float g = 0.f, up = 0.f;
@@ -691,10 +699,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
             }
           }
         }
-        if (n > 0) __syncthreads();
+        if (n > 0) ct_sync();
+        if (tid == 0) mbar_arrive(empty + part % ST_PARTS);
         if (r == last_live && half == 1 && tid == 0) arrive_gpu(p.ctr + 1);
         const int freed = half == 0 ? n_in : n_out;
-        refill(ring_s, freed);
         ring_s = ring_s + freed < NS ? ring_s + freed : ring_s + freed - NS;
       }
     }
@@ -720,7 +728,7 @@ __global__ void stack_reset_kernel(uint32_t* ctr) {
 
 // The shape side of a launch; false: the layer-by-layer path is the one that takes it.
 struct StackShape {
-  int sh_tokens, sh_blocks, n_items, n_stages, smem;
+  int sh_tokens, sh_blocks, n_items, n_stages, router_extra, smem;
 };
 static bool stack_shape(int64_t T, int D, int H, int E, int S, int k, StackShape* o) {
   if (T < 1 || T > ST_MAX_T || H != ST_H || D < 64 || D % 32 != 0 || D > 1024 || E < 4 ||
@@ -734,10 +742,15 @@ static bool stack_shape(int64_t T, int D, int H, int E, int S, int k, StackShape
   o->sh_blocks = int((T + o->sh_tokens - 1) / o->sh_tokens);
   o->n_items = ST_SLICES * (E + S * o->sh_blocks);
   if (o->n_items > ST_MAX_ITEMS * grid) return false;
-  const int limit = 232448 - 1024, rest = stack_smem(int(T), D, 0).total, n_in = (D + 63) / 64;
-  o->n_stages = std::min((limit - rest) / ST_STAGE, ST_MAX_STAGES);
-  if (limit < rest || o->n_stages < n_in) return false;   // an item's up weights are there at once
-  o->smem = stack_smem(int(T), D, o->n_stages).total + 1024;
+  const int limit = 232448 - 1024, n_in = (D + 63) / 64;
+  for (int extra : {ST_ROUTER_EXTRA, 0}) {
+    const int rest = stack_smem(int(T), D, 0, extra).total;
+    o->router_extra = extra;
+    o->n_stages = std::min((limit - rest) / ST_STAGE, ST_MAX_STAGES);
+    if (limit > rest && o->n_stages >= n_in) break;   // an item's up weights are there at once
+  }
+  if (o->n_stages < n_in) return false;
+  o->smem = stack_smem(int(T), D, o->n_stages, o->router_extra).total + 1024;
   return true;
 }
 
@@ -864,6 +877,7 @@ int moe_b200_stack_infer(const void* plan, int32_t n_layers, const void* x, void
   a.normalize = normalize;
   a.act = activation;
   a.n_stages = o.n_stages;
+  a.router_extra = o.router_extra;
   a.out_boxes = d_model % 64 == 0 ? 1 : 2;
   a.kshift = top_k <= 8 ? 3 : 4;
   a.sh_tokens = o.sh_tokens;

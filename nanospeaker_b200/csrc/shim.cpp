@@ -8,6 +8,7 @@
 // addresses the Python binding hands over (bind()), so that it and this file use one library.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAGraph.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -496,6 +497,130 @@ std::tuple<Tensor, Tensor, Tensor> sublayer(
   return {r.out, r.aux, r.counts};
 }
 
+// --------------------------------------------------------------------- replay from graphs
+// The block's training step for one input shape, forward and backward each captured in a CUDA graph
+// and replayed behind an autograd node. Inputs and incoming gradients are copied into the graphs'
+// own buffers; results are those buffers (overwritten by the next call).
+class GraphedBlock : public std::enable_shared_from_this<GraphedBlock> {
+ public:
+  GraphedBlock(const Tensor& x, const Tensor& router_w, const OptTensor& logit_bias,
+               const Tensor& w_in, const Tensor& w_out, const OptTensor& w_sh_in,
+               const OptTensor& w_sh_out, int64_t top_k, bool normalize, bool full_softmax,
+               double aux_coef, int64_t activation, bool store)
+      : opt_{top_k, activation, 0, normalize, full_softmax, store, false, false, aux_coef} {
+    at::NoGradGuard no_grad;
+    const c10::cuda::CUDAGuard on(x.device());
+    auto plain = [](const Tensor& t) { return t.defined() ? t.detach() : t; };
+    p_ = operands(x.clone(), router_w, logit_bias, OptTensor(), w_in, w_out, w_sh_in, w_sh_out);
+    for (Tensor* t : {&p_.x, &p_.router_w, &p_.w_in, &p_.w_out, &p_.w_sh_in, &p_.w_sh_out,
+                      &p_.logit_bias})
+      *t = plain(*t);
+    check_operands(p_, opt_);
+    grad_out_ = at::zeros_like(p_.x);
+    grad_aux_ = at::zeros({1}, p_.x.options().dtype(at::kFloat));
+    // once outside the capture: lazy initialisations, the status word, the side streams
+    const auto main = c10::cuda::getCurrentCUDAStream();
+    const auto side = c10::cuda::getStreamFromPool(false, p_.x.get_device());
+    C10_CUDA_CHECK(cudaStreamSynchronize(main.stream()));
+    {
+      const c10::cuda::CUDAStreamGuard work(side);
+      {
+        Results r = launch_forward(p_, opt_, true);
+        launch_backward(p_, opt_, r.kept, grad_out_, grad_aux_);
+      }
+      C10_CUDA_CHECK(cudaStreamSynchronize(side.stream()));
+      const int64_t l0 = n_launched;
+      fwd_.capture_begin();
+      r_ = launch_forward(p_, opt_, true);
+      fwd_.capture_end();
+      const int64_t l1 = n_launched;
+      bwd_.capture_begin(fwd_.pool());
+      g_ = launch_backward(p_, opt_, r_.kept, grad_out_, grad_aux_);
+      bwd_.capture_end();
+      n_fwd_ = l1 - l0;
+      n_bwd_ = n_launched - l1;
+    }
+  }
+
+  std::tuple<Tensor, Tensor, Tensor> run(const Tensor& x_in, const Tensor& router_w,
+                                         const Tensor& w_in, const Tensor& w_out,
+                                         const OptTensor& w_sh_in, const OptTensor& w_sh_out);
+  Grads backward(const Tensor& grad_out, const Tensor& grad_aux) {
+    const c10::cuda::CUDAGuard on(p_.x.device());
+    if (grad_out.defined())
+      grad_out_.copy_(grad_out, true);
+    else
+      grad_out_.zero_();
+    if (grad_aux.defined())
+      grad_aux_.copy_(grad_aux.reshape({1}), true);
+    else if (opt_.full_softmax)
+      grad_aux_.zero_();
+    bwd_.replay();
+    n_launched += n_bwd_;
+    return g_;
+  }
+
+ private:
+  Options opt_;
+  Operands p_;
+  Results r_;
+  Grads g_;
+  Tensor grad_out_, grad_aux_;
+  at::cuda::CUDAGraph fwd_, bwd_;
+  int64_t n_fwd_ = 0, n_bwd_ = 0;
+};
+
+// Edges: x, router_w, w_in, w_out, w_sh_in, w_sh_out.
+struct MoEGraphedBackward : public torch::autograd::Node {
+  std::shared_ptr<GraphedBlock> graphs;
+  std::string name() const override { return "MoEGraphedBackward"; }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    if (!grads[0].defined() && !grads[1].defined()) return variable_list(6);
+    at::NoGradGuard no_grad;
+    const Grads g = graphs->backward(grads[0], grads[1]);
+    auto out = [](const Tensor& t) { return t.defined() ? t.detach() : t; };
+    return {out(g.dx), out(g.d_router), out(g.dw_in), out(g.dw_out), out(g.dw_sh_in),
+            out(g.dw_sh_out)};
+  }
+};
+
+std::tuple<Tensor, Tensor, Tensor> GraphedBlock::run(const Tensor& x_in, const Tensor& router_w,
+                                                     const Tensor& w_in, const Tensor& w_out,
+                                                     const OptTensor& w_sh_in,
+                                                     const OptTensor& w_sh_out) {
+  TORCH_CHECK(x_in.sizes() == p_.x.sizes() && x_in.scalar_type() == p_.x.scalar_type() &&
+                  x_in.device() == p_.x.device(),
+              "the graphs were captured for another input shape");
+  const Tensor si = w_sh_in.value_or(Tensor()), so = w_sh_out.value_or(Tensor());
+  std::shared_ptr<MoEGraphedBackward> node;
+  if (any_grad(x_in, router_w, w_in, w_out, si, so)) {
+    node = new_node<MoEGraphedBackward>();
+    node->set_next_edges(
+        torch::autograd::collect_next_edges(x_in, router_w, w_in, w_out, si, so));
+    node->graphs = shared_from_this();
+  }
+  Tensor out, aux, counts;
+  {
+    at::NoGradGuard no_grad;
+    const c10::cuda::CUDAGuard on(p_.x.device());
+    p_.x.copy_(x_in, true);
+    fwd_.replay();
+    n_launched += n_fwd_;
+    out = r_.out.detach();
+    aux = r_.aux.detach();
+    counts = r_.counts.clone();   // (kept by callers for their logs)
+  }
+  if (node) {
+    torch::autograd::set_history(out, node);
+    if (opt_.full_softmax)
+      torch::autograd::set_history(aux, node);
+    else
+      node->add_input_metadata(torch::autograd::Node::undefined_input());
+  }
+  return {out, aux, counts};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_moe_shim, m) {
@@ -503,4 +628,9 @@ PYBIND11_MODULE(_moe_shim, m) {
   m.def("launches", [] { return n_launched.load(); });
   m.def("block", &block);
   m.def("sublayer", &sublayer);
+  py::class_<GraphedBlock, std::shared_ptr<GraphedBlock>>(m, "GraphedBlock")
+      .def(py::init<const Tensor&, const Tensor&, const OptTensor&, const Tensor&, const Tensor&,
+                    const OptTensor&, const OptTensor&, int64_t, bool, bool, double, int64_t,
+                    bool>())
+      .def("run", &GraphedBlock::run);
 }

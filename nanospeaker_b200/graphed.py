@@ -6,7 +6,8 @@ one from Python they cost more host time than the GPU needs to run them (about 1
 shape, so forward and backward can each be captured once per input shape and replayed.
 `GraphedMoEBlock` does that and stays a drop-in for the block: same call, same post-forward
 attributes (`aux_loss`, `expert_counts`, `dropped`), autograd works as usual (the two graphs are
-tied together by torch.cuda.make_graphed_callables), parameters stay those of the wrapped block.
+tied together by a native autograd node; by torch.cuda.make_graphed_callables where the weights are
+cast on every call), parameters stay those of the wrapped block.
 
 The caller loop this serves is the reference's micro-step, `loss, aux = model(x, y); (loss + aux)
 .backward()` (src/train/train.py:317-324), where the block is called once per layer and step with a
@@ -17,6 +18,7 @@ from typing import Dict, Tuple
 import torch
 from torch import nn
 
+from . import moe_kernel as MK
 from .moe import MoEBlock
 
 
@@ -66,6 +68,31 @@ class GraphedMoEBlock(nn.Module):
     def router(self):
         return self.block.router
 
+    def _weights(self):
+        b = self.block
+        return b.router.W, b.W_in, b.W_out, b.W_sh_in, b.W_sh_out
+
+    def _native_for(self, x2: torch.Tensor):
+        """The native forward / backward graph pair (csrc/shim.cpp) for this input shape, or None
+        where the block's weights or routing bias would have to be cast first."""
+        b = self.block
+        weights = self._weights()
+        key = ("native", tuple(x2.shape), x2.dtype, x2.device, b.training, MK._atomic(b.combine_mode),
+               b.router.logit_bias is None)
+        g = self._graphed.get(key)
+        if g is None:
+            bias = b.router.logit_bias
+            if (not all(w is None or (w.dtype == x2.dtype and w.is_contiguous()) for w in weights)
+                    or not (bias is None or (bias.dtype == torch.float32 and bias.is_contiguous()))):
+                return None
+            rw, w_in, w_out, sh_in, sh_out = weights
+            g = MK.K.shim().GraphedBlock(
+                torch.randn_like(x2), rw, bias, w_in, w_out, sh_in, sh_out,
+                b.router.top_k, bool(b.router.normalize_weights), b.router.wants_probs(),
+                b.router.aux_loss_coef, MK._act_id(b._kernel_act), not MK._atomic(b.combine_mode))
+            self._graphed[key] = g
+        return g
+
     def _callable_for(self, x: torch.Tensor):
         key = (tuple(x.shape), x.dtype, x.device, self.block.training, x.requires_grad)
         fn = self._graphed.get(key)
@@ -79,13 +106,20 @@ class GraphedMoEBlock(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         b = self.block
-        x2 = x.reshape(-1, x.shape[-1]) if x.dim() > 1 else x
+        x2 = x.reshape(-1, x.shape[-1]) if x.dim() not in (1, 2) else x
         # (without autograd there is no backward to pair the forward with: the block's own
         # inference path is the lighter one then, and nanospeaker_b200.decode graphs it)
         if (not x.is_cuda or x2.shape[0] == 0 or x.shape[-1] != b.d_model
                 or not torch.is_grad_enabled() or not b._whole_block_ok(x2)
                 or (b.training and b.router.noise_std)):   # noise: fresh random numbers every call
             return b(x)
+        if (x2.dim() == 2 and MK.native_ok(x2) and MK._aux_reduce is None
+                and not MK._DEBUG_ONE_STREAM):
+            g = self._native_for(x2)
+            if g is not None:
+                rw, w_in, w_out, sh_in, sh_out = self._weights()
+                out, b.aux_loss, b.expert_counts = g.run(x2, rw, w_in, w_out, sh_in, sh_out)
+                return out if x.dim() == 2 else out.view(x.shape)
         out, aux, counts = self._callable_for(x)(x)
         full = b.router.wants_probs()
         b.aux_loss = aux if full else torch.zeros((), device=x.device, dtype=x.dtype)

@@ -224,6 +224,26 @@ int moe_b200_group_sumsq(const void* x, int32_t groups, int64_t per_group, float
 int moe_b200_axpby(const void* x, const void* y, void* out, int32_t groups, int64_t per_group,
                    float alpha, float beta, const float* sumsq, float eps, void* stream);
 
+/* Muon's step (src/train/optim.py:75-105) on stacks of matrices, all in one call:
+ *   buf <- lerp(buf, grad, grad_weight), dir = lerp(grad, buf, momentum)
+ *   X = dir / (|dir| + eps), `steps` times X <- a X + (b A + c A A) X, A the Gram matrix of the short
+ *   side; delta = step * X, p <- p * decay + delta.
+ * norms[0] = sum |delta|^2, norms[1] = sum |p|^2, norms[2] is the library's. Shapes:
+ * moe_b200_muon_supported ([128, n] or [n, 256], the long side a multiple of 32). */
+typedef struct moe_b200_muon_param {
+  void* p;                 /* [groups, rows, cols], bf16 or fp32; every pointer 16-byte aligned */
+  const void* grad;        /* bf16 */
+  void* buf;               /* momentum, bf16 */
+  int32_t p_is_fp32, groups, rows, cols;
+  float step;              /* -lr * sqrt(max(1, rows / cols)) */
+} moe_b200_muon_param;
+int moe_b200_muon_supported(int32_t rows, int32_t cols);
+size_t moe_b200_muon_scratch_bytes(const moe_b200_muon_param* params, int32_t n);
+int moe_b200_muon_step(const moe_b200_muon_param* params, int32_t n, float grad_weight,
+                       float momentum, float decay, int32_t steps, float a, float b, float c,
+                       float eps, float* norms, void* scratch, size_t scratch_bytes,
+                       int32_t* n_launches, int32_t* status, void* stream);
+
 /* dst[r, c] = c < cols ? src[r, c] : 0 for 0 <= c < dst_ld; 16-bit elements, row strides src_ld /
  * dst_ld elements. Pads the router weight [d_model, n_experts] (src/model/router.py:51) to the
  * 64-column multiple the GEMM kernels' tensor maps need, and strips the pad columns from its

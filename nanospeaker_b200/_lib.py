@@ -140,6 +140,12 @@ SIGNATURES = {
     "moe_b200_stack_infer": (
         ctypes.c_int, [_c_vp, _c_i32, _c_vp, _c_vp, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32, _c_i32,
                        _c_i32, _c_i32, _c_vp, _c_sz, ctypes.POINTER(_c_i32), _c_vp, _c_vp]),
+    "moe_b200_muon_supported": (ctypes.c_int, [_c_i32, _c_i32]),
+    "moe_b200_muon_scratch_bytes": (_c_sz, [_c_vp, _c_i32]),
+    "moe_b200_muon_step": (
+        ctypes.c_int, [_c_vp, _c_i32, ctypes.c_float, ctypes.c_float, ctypes.c_float, _c_i32,
+                       ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float, _c_vp, _c_vp,
+                       _c_sz, ctypes.POINTER(_c_i32), _c_vp, _c_vp]),
     "moe_b200_ep_plan": (
         ctypes.c_int, [_c_vp, _c_vp, _c_i32, _c_i32, _c_i32, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp,
                        _c_vp, _c_i64, _c_vp]),

@@ -38,6 +38,8 @@ struct Abi {
   decltype(&moe_b200_block_backward_scratch_bytes) backward_scratch_bytes;
   decltype(&moe_b200_block_forward) forward;
   decltype(&moe_b200_block_backward) backward;
+  decltype(&moe_b200_muon_scratch_bytes) muon_scratch_bytes;
+  decltype(&moe_b200_muon_step) muon_step;
   decltype(&moe_b200_rmsnorm) rmsnorm;
   decltype(&moe_b200_rmsnorm_bwd) rmsnorm_bwd;
 } abi{};
@@ -56,6 +58,8 @@ void bind(const py::dict& d, const py::object& status) {
   take(d, "moe_b200_block_backward_scratch_bytes", abi.backward_scratch_bytes);
   take(d, "moe_b200_block_forward", abi.forward);
   take(d, "moe_b200_block_backward", abi.backward);
+  take(d, "moe_b200_muon_scratch_bytes", abi.muon_scratch_bytes);
+  take(d, "moe_b200_muon_step", abi.muon_step);
   take(d, "moe_b200_rmsnorm", abi.rmsnorm);
   take(d, "moe_b200_rmsnorm_bwd", abi.rmsnorm_bwd);
   status_word_of = new py::object(status);   // lives as long as the process
@@ -621,6 +625,53 @@ std::tuple<Tensor, Tensor, Tensor> GraphedBlock::run(const Tensor& x_in, const T
   return {out, aux, counts};
 }
 
+// ----------------------------------------------------------------------------------- Muon
+// One optimizer step over CUDA matrices or stacks of them, all of one device and of shapes
+// moe_b200_muon_supported takes. Returns fp32 [2]: |dW|^2 and |W|^2 over all of them.
+Tensor muon_step(const std::vector<Tensor>& params, const std::vector<Tensor>& grads,
+                 const std::vector<Tensor>& bufs, double lr, double momentum, double weight_decay,
+                 int64_t steps, double a, double b, double c, double eps) {
+  TORCH_CHECK(!params.empty() && params.size() == grads.size() && params.size() == bufs.size(),
+              "one gradient and one momentum buffer per parameter");
+  at::NoGradGuard no_grad;
+  const Tensor& first = params[0];
+  const c10::cuda::CUDAGuard on(first.device());
+  std::vector<moe_b200_muon_param> ps(params.size());
+  for (size_t i = 0; i < params.size(); ++i) {
+    const Tensor &p = params[i], &g = grads[i], &m = bufs[i];
+    TORCH_CHECK(p.device() == first.device() && g.device() == p.device() &&
+                    m.device() == p.device() && (p.dim() == 2 || p.dim() == 3) &&
+                    g.sizes() == p.sizes() && m.sizes() == p.sizes() && p.is_contiguous() &&
+                    g.is_contiguous() && m.is_contiguous() &&
+                    (p.scalar_type() == at::kBFloat16 || p.scalar_type() == at::kFloat) &&
+                    g.scalar_type() == at::kBFloat16 && m.scalar_type() == at::kBFloat16,
+                "parameter ", i, ": contiguous bf16 gradient and momentum beside it expected");
+    const int64_t rows = p.size(-2), cols = p.size(-1);
+    ps[i] = {p.mutable_data_ptr(),
+             g.const_data_ptr(),
+             m.mutable_data_ptr(),
+             p.scalar_type() == at::kFloat,
+             int32_t(p.dim() == 3 ? p.size(0) : 1),
+             int32_t(rows),
+             int32_t(cols),
+             float(-lr * std::sqrt(std::max(1.0, double(rows) / double(cols))))};
+  }
+  const int32_t n = int32_t(ps.size());
+  const Tensor norms = at::empty({3}, first.options().dtype(at::kFloat));
+  const Tensor scratch = bytes_like(first, abi.muon_scratch_bytes(ps.data(), n));
+  int32_t launched = 0;
+  check(abi.muon_step(ps.data(), n, float(1.0 - momentum), float(momentum),
+                      float(1.0 - lr * weight_decay), int32_t(steps), float(a), float(b), float(c),
+                      float(eps), norms.mutable_data_ptr<float>(), scratch.mutable_data_ptr(),
+                      size_t(scratch.numel()), &launched, status_word(first.get_device()),
+                      c10::cuda::getCurrentCUDAStream().stream()),
+        "moe_b200_muon_step");
+  for (const auto* v : {&params, &bufs})
+    for (const Tensor& t : *v) t.unsafeGetTensorImpl()->bump_version();
+  n_launched += launched;
+  return norms.narrow(0, 0, 2);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_moe_shim, m) {
@@ -628,6 +679,7 @@ PYBIND11_MODULE(_moe_shim, m) {
   m.def("launches", [] { return n_launched.load(); });
   m.def("block", &block);
   m.def("sublayer", &sublayer);
+  m.def("muon_step", &muon_step);
   py::class_<GraphedBlock, std::shared_ptr<GraphedBlock>>(m, "GraphedBlock")
       .def(py::init<const Tensor&, const Tensor&, const OptTensor&, const Tensor&, const Tensor&,
                     const OptTensor&, const OptTensor&, int64_t, bool, bool, double, int64_t,

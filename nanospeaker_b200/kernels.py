@@ -659,6 +659,11 @@ def stack_supported(n_tokens: int, d_model: int, d_hidden: int, n_experts: int, 
                                                      n_shared, top_k))
 
 
+def muon_supported(rows: int, cols: int) -> bool:
+    """Whether the fused Newton-Schulz iteration is built for [.., rows, cols] matrices."""
+    return bool(_lib.load().moe_b200_muon_supported(rows, cols))
+
+
 def stack_infer(plan: torch.Tensor, n_layers: int, x: torch.Tensor, d_hidden: int, n_experts: int,
                 n_shared: int, top_k: int, normalize: bool, act: int) -> torch.Tensor:
     """x <- x + block_l(x) through a stack of blocks in one persistent kernel."""

@@ -83,11 +83,23 @@ def newton_schulz5(g: torch.Tensor, steps: int = 5, eps: float = 1e-7) -> torch.
     return x[0] if single else x
 
 
+def _native_ok(p: torch.Tensor, buf: torch.Tensor) -> bool:
+    """Whether the native step (one call for all such parameters) takes this one: a CUDA matrix or
+    stack in bf16 or fp32 of a shape the fused iteration is built for."""
+    if not (p.is_cuda and p.dim() in (2, 3) and p.dtype in (torch.bfloat16, torch.float32)
+            and buf.dtype == torch.bfloat16 and p.is_contiguous() and buf.is_contiguous()
+            and (p.data_ptr() | buf.data_ptr()) % 16 == 0):
+        return False
+    return (p.numel() > 0 and (p.dim() == 2 or p.shape[0] <= 65535)
+            and max(p.shape[-2:]) <= 1 << 20 and K.muon_supported(p.shape[-2], p.shape[-1]))
+
+
 class Muon(torch.optim.Optimizer):
     """Nesterov momentum whose direction is replaced by its orthogonal factor
     (src/train/optim.py:43-105): momentum buffer in bf16, update scaled by sqrt(max(1, rows / cols)),
     decoupled weight decay, |dW| and |W| accumulated on the device for `update_norm_ratio`.
-    Stacked [E, rows, cols] parameters are orthogonalised per expert in one batched call."""
+    Stacked [E, rows, cols] parameters are orthogonalised per expert in one batched call. On CUDA the
+    whole step over parameters of supported shapes is one native call (csrc/muon.cu)."""
 
     def __init__(self, params: Iterable, lr: float = 0.02, momentum: float = 0.95,
                  weight_decay: float = 0.1, ns_steps: int = 5):
@@ -116,6 +128,7 @@ class Muon(torch.optim.Optimizer):
         self._update_sq = self._param_sq = 0.0
         for group in self.param_groups:
             lr, mom, wd = group["lr"], group["momentum"], group["weight_decay"]
+            native = {}
             for p in group["params"]:
                 if p.grad is None:
                     continue
@@ -124,6 +137,9 @@ class Muon(torch.optim.Optimizer):
                     state["momentum"] = torch.zeros_like(p, dtype=torch.bfloat16)
                 buf = state["momentum"]
                 grad = p.grad.to(buf.dtype)
+                if group["ns_steps"] > 0 and _native_ok(p, buf) and grad.is_contiguous() and grad.data_ptr() % 16 == 0:
+                    native.setdefault(p.device, []).append((p, grad, buf))
+                    continue
                 buf.lerp_(grad, 1 - mom)
                 update = newton_schulz5(grad.lerp(buf, mom), group["ns_steps"])
                 scale = max(1.0, p.size(-2) / p.size(-1)) ** 0.5
@@ -132,3 +148,9 @@ class Muon(torch.optim.Optimizer):
                 p.add_(delta)
                 self._update_sq = self._update_sq + delta.float().pow(2).sum()
                 self._param_sq = self._param_sq + p.detach().float().pow(2).sum()
+            for members in native.values():
+                params, grads, bufs = (list(t) for t in zip(*members))
+                norms = K.shim().muon_step(params, grads, bufs, lr, mom, wd, group["ns_steps"],
+                                           *NS_COEFFS, 1e-7)
+                self._update_sq = self._update_sq + norms[0]
+                self._param_sq = self._param_sq + norms[1]

@@ -82,3 +82,40 @@ def test_muon_step_on_the_blocks_gradients():
         assert rel_l2(p.detach().cpu(), w) < 1e-2                # the updated weights
         assert rel_l2(p.detach().cpu().float() - decayed, delta.float()) < 0.2    # the applied step
     assert 0 < opt.update_norm_ratio() < 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_native_muon_step_equals_the_operations_one_by_one(dtype):
+    """Several steps over stacks and a single matrix (whole and ragged tiles of the long side, all of it
+    on chip and streamed, one shape that the fused iteration declines) against the step in torch operations on copies: momentum bit for bit, weights and the
+    update / weight norm ratio within the iteration's bf16 noise."""
+    from nanospeaker_b200 import kernels, muon as MU
+    torch.manual_seed(3)
+    shapes = [(5, 576, 256), (2, 256, 256), (1, 288, 256), (2, 1056, 256), (5, 128, 576), (128, 128),
+              (2, 128, 768), (3, 128, 1056), (3, 96, 64)]
+    a = [torch.nn.Parameter((torch.randn(*s) * 0.05).to(dtype).cuda()) for s in shapes]
+    b = [torch.nn.Parameter(p.detach().clone()) for p in a]
+    oa, ob = MU.Muon(a, lr=0.02), MU.Muon(b, lr=0.02)
+    for step in range(3):
+        for p, q in zip(a, b):
+            p.grad = torch.randn_like(p)
+            q.grad = p.grad.clone()
+        version, before = a[0]._version, [p.detach().clone() for p in a]
+        oa.step()
+        assert a[0]._version > version
+        native = MU._native_ok
+        MU._native_ok = lambda p, buf: False
+        try:
+            ob.step()
+        finally:
+            MU._native_ok = native
+        for p, q, p0 in zip(a, b, before):
+            assert torch.equal(oa.state[p]["momentum"], ob.state[q]["momentum"])
+            assert rel_l2(p.detach(), q.detach()) < 2e-3
+            if dtype == torch.float32:
+                decayed = p0 * (1 - 0.02 * 0.1)
+                assert rel_l2(p.detach() - decayed, q.detach() - decayed) < 2e-2, tuple(p.shape)
+            q.data.copy_(p.data)
+        assert abs(oa.update_norm_ratio() / ob.update_norm_ratio() - 1) < 2e-2
+    kernels.check_status("cuda")

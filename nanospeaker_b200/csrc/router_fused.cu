@@ -176,12 +176,18 @@ __global__ void __launch_bounds__(WARPS * 32)
 }
 
 // ---------------------------------------------------------------- four lanes per token
-// The same routine for the common shapes (at most 96 experts, top_k <= 8), with four lanes per
+// The same routine for the common shapes (at most 128 experts, top_k <= 8), with four lanes per
 // token instead of a warp: lane q of a group holds experts [q * EPL, (q + 1) * EPL) in registers,
-// so a warp routes eight tokens at once and the cross-lane steps shrink to two shuffle rounds. The
-// warp-per-token kernel above spends 611 warp instructions per token on E = 76 (three values per
-// lane, every reduction five shuffles deep, most lanes idle in the top-k rounds) and is bound by
-// instruction issue; this one needs about a quarter of that.
+// so a warp routes eight tokens at once. Each lane keeps the KT largest keys of its experts as a
+// sorted list (a minimum and a maximum per entry and expert), two shuffle rounds merge the four
+// lists, and what is at or above the smallest key that is in belongs to the selection: a lane marks
+// its own, ties for the last place are trimmed from the highest index down, and the rest goes to
+// the token's list in shared memory in index order, from where each lane ranks two entries.
+// Bound by instruction issue (170 warp instructions per token on E = 76, top_k = 6; 370 with a search
+// over all registers per winner, 611 with a warp per token as above) and, below ~16k tokens, by its
+// latency. Against the search per winner: 131072 tokens 66 -> 48 us, 16384 tokens with column sums
+// 14.3 -> 12.3 us, 333 tokens 10.8 -> 8.7 us. A lane per token with rolled loops needs as many
+// instructions but a quarter of the warps, and a warp alone issues one in five cycles: 16 us at 333.
 // Selection rule, softmax arithmetic and outputs are those of router_fused_kernel; sums run in a
 // different order, so weights may differ in the last fp32 bit before they are rounded to bf16.
 constexpr int RF4_THREADS = 512;
@@ -192,7 +198,34 @@ __device__ __forceinline__ float key_float(uint32_t k) {   // inverse of float_k
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
 }
 
-template <int EPL, bool COLSUM>
+// a <- the KT largest of two descending lists of KT (max of one against the other reversed), sorted
+// again if asked: a bitonic merge, or the 12-comparator network for 6.
+template <int KT, bool SORT>
+__device__ __forceinline__ void merge_top(uint32_t (&a)[KT], const uint32_t (&b)[KT]) {
+#pragma unroll
+  for (int j = 0; j < KT; ++j) a[j] = max(a[j], b[KT - 1 - j]);
+  auto order = [&](int x, int y) {
+    const uint32_t hi = max(a[x], a[y]), lo = min(a[x], a[y]);
+    a[x] = hi;
+    a[y] = lo;
+  };
+  if constexpr (SORT && KT == 6) {
+    order(0, 5), order(1, 3), order(2, 4);
+    order(1, 2), order(3, 4);
+    order(0, 3), order(2, 5);
+    order(0, 1), order(2, 3), order(4, 5);
+    order(1, 2), order(3, 4);
+  } else if constexpr (SORT) {
+#pragma unroll
+    for (int d = KT / 2; d > 0; d >>= 1)
+#pragma unroll
+      for (int j = 0; j < KT; ++j)
+        if ((j & d) == 0) order(j, j + d);
+  }
+}
+
+// KT: the smallest of 2, 4, 6, 8 that holds top_k.
+template <int EPL, int KT, bool COLSUM>
 __global__ void __launch_bounds__(RF4_THREADS)
     router_fused4_kernel(const __nv_bfloat16* __restrict__ logits, int ld,
                          const float* __restrict__ bias, const float* __restrict__ noise, int64_t n_tokens, int n_experts, int top_k,
@@ -206,11 +239,11 @@ __global__ void __launch_bounds__(RF4_THREADS)
   // resident beside this kernel's blocks, which are short of issue slots as it is). A batch that
   // one block routes, plans and scatters (decode) keeps it: there the launch chain is what counts.
   if (sc.counts != nullptr) pdl_trigger();
-  pdl_wait();
-  static_assert(EPL % 8 == 0, "a lane loads its experts as 16-byte pieces");
+  static_assert(EPL % 4 == 0 && EPL <= 32, "a lane loads its experts as 8-byte pieces");
   static_assert(RF4_THREADS == DISPATCH_THREADS, "the scatter pass runs on this kernel's block");
-  __shared__ float cs[RF4_THREADS / 32][4 * EPL];
+  __shared__ float cs[COLSUM ? RF4_THREADS / 32 : 1][4 * EPL];
   __shared__ int32_t hist[MAX_EXPERTS];
+  __shared__ uint2 lists[RF4_TOKENS][KT + 1];   // (key, expert); an odd stride
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int q = lane & 3, sub = lane >> 2;
   const int e0 = q * EPL;
@@ -219,8 +252,10 @@ __global__ void __launch_bounds__(RF4_THREADS)
     for (int e = threadIdx.x; e < n_experts + n_shared; e += blockDim.x) hist[e] = 0;
     __syncthreads();
   }
+  pdl_wait();
   const int kS = top_k + n_shared;
   const bool need_full = full_softmax || !normalize;
+  uint2* const list = lists[warp * 8 + sub];
 
   float b[EPL];
   [[maybe_unused]] float csum[EPL];
@@ -243,25 +278,20 @@ __global__ void __launch_bounds__(RF4_THREADS)
     uint32_t key[EPL];   // first the values (as float bits), then the order-preserving keys
     float mx = -CUDART_INF_F;
     {
-      const uint4* rp = reinterpret_cast<const uint4*>(logits + tc * ld + e0);
+      const uint2* rp = reinterpret_cast<const uint2*>(logits + tc * ld + e0);
+      uint2 r[EPL / 4];
 #pragma unroll
-      for (int c = 0; c < EPL / 8; ++c) {
-        const uint4 r = __ldg(rp + c);
-        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+      for (int c = 0; c < EPL / 4; ++c)
+        r[c] = e0 + 4 * c < n_experts ? __ldg(rp + c) : make_uint2(0u, 0u);
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[h]));
-          const int i = c * 8 + 2 * h;
-          float v0 = (e0 + i < n_experts) ? f.x + b[i] : -CUDART_INF_F;
-          float v1 = (e0 + i + 1 < n_experts) ? f.y + b[i + 1] : -CUDART_INF_F;
-          if (noise != nullptr) {   // exploration noise, one value per (token, expert)
-            if (e0 + i < n_experts) v0 += __ldg(noise + tc * n_experts + e0 + i);
-            if (e0 + i + 1 < n_experts) v1 += __ldg(noise + tc * n_experts + e0 + i + 1);
-          }
-          key[i] = __float_as_uint(v0);
-          key[i + 1] = __float_as_uint(v1);
-          mx = fmaxf(mx, fmaxf(v0, v1));
-        }
+      for (int i = 0; i < EPL; ++i) {
+        const uint32_t w = (i & 2) ? r[i / 4].y : r[i / 4].x;
+        const float f = __uint_as_float((i & 1) ? w & 0xffff0000u : w << 16);
+        float v = e0 + i < n_experts ? f + b[i] : -CUDART_INF_F;
+        if (noise != nullptr && e0 + i < n_experts)   // exploration noise, one value per (token, expert)
+          v += __ldg(noise + tc * n_experts + e0 + i);
+        key[i] = __float_as_uint(v);
+        mx = fmaxf(mx, v);
       }
     }
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
@@ -283,76 +313,106 @@ __global__ void __launch_bounds__(RF4_THREADS)
         for (int i = 0; i < EPL; ++i) csum[i] += ex[i] * inv;
       }
     }
+    uint32_t top[KT];   // this lane's largest keys, descending
+#pragma unroll
+    for (int j = 0; j < KT; ++j) top[j] = 0u;
 #pragma unroll
     for (int i = 0; i < EPL; ++i) {
-      const uint32_t fk = float_key(__uint_as_float(key[i]));
-      key[i] = (e0 + i < n_experts) ? (fk == 0u ? 1u : fk) : 0u;
+      // (no key of a value is 0: that is what experts past the end get)
+      const uint32_t x = e0 + i < n_experts ? float_key(__uint_as_float(key[i])) : 0u;
+      key[i] = x;
+#pragma unroll
+      for (int j = KT - 1; j > 0; --j)
+        if (j <= i) top[j] = max(top[j], min(top[j - 1], x));
+      top[0] = max(top[0], x);
     }
-
-    // top-k: local best (lowest index among equal keys), then two rounds across the four lanes
-    float sv[RF4_MAX_TOPK];
-    int si[RF4_MAX_TOPK];
+    {
+      uint32_t other[KT];
 #pragma unroll
-    for (int j = 0; j < RF4_MAX_TOPK; ++j) {
-      sv[j] = 0.f;
-      si[j] = 0;
-      if (j < top_k) {
-        uint32_t bk = 0u;
-        int be = 0x7FFFFFFF;
+      for (int j = 0; j < KT; ++j) other[j] = __shfl_xor_sync(0xffffffffu, top[j], 1);
+      merge_top<KT, true>(top, other);
 #pragma unroll
-        for (int i = 0; i < EPL; ++i)
-          if (key[i] > bk) {
-            bk = key[i];
-            be = e0 + i;
-          }
-#pragma unroll
-        for (int o = 1; o <= 2; o <<= 1) {
-          const uint32_t ok = __shfl_xor_sync(0xffffffffu, bk, o);
-          const int oe = __shfl_xor_sync(0xffffffffu, be, o);
-          if (ok > bk || (ok == bk && oe < be)) {
-            bk = ok;
-            be = oe;
-          }
-        }
-        const int slot = be - e0;   // only the owner's slot is in range
-#pragma unroll
-        for (int i = 0; i < EPL; ++i)
-          if (i == slot) key[i] = 0u;
-        sv[j] = key_float(bk);
-        si[j] = be;
-      }
+      for (int j = 0; j < KT; ++j) other[j] = __shfl_xor_sync(0xffffffffu, top[j], 2);
+      merge_top<KT, true>(top, other);
     }
+    uint32_t last = 0xFFFFFFFFu;   // the smallest key that is in
+#pragma unroll
+    for (int j = 0; j < KT; ++j) last = min(last, j < top_k ? top[j] : 0xFFFFFFFFu);
 
-    // weights of the selected experts (every lane of the group computes all of them)
-    float p[RF4_MAX_TOPK];
-    if (need_full) {
-      float s = 0.f;
+    uint32_t in = 0u;   // this lane's experts that are in
 #pragma unroll
-      for (int j = 0; j < RF4_MAX_TOPK; ++j) {
-        p[j] = j < top_k ? expf(sv[j] - mx) / denom : 0.f;
-        s += p[j];
+    for (int i = 0; i < EPL; ++i)
+      if (key[i] >= last) in |= 1u << i;
+    int n = __popc(in);
+    int total = n + __shfl_xor_sync(0xffffffffu, n, 1);
+    total += __shfl_xor_sync(0xffffffffu, total, 2);
+    if (__any_sync(0xffffffffu, total > top_k)) {
+      // more ties for the last place than places: the highest experts among them are out
+      uint32_t tie = 0u;
+#pragma unroll
+      for (int i = 0; i < EPL; ++i)
+        if (key[i] == last) tie |= 1u << i;
+      const int nt = __popc(tie);
+      int over = total - top_k;
+#pragma unroll
+      for (int k = 3; k > 0; --k) {   // what the lanes above take
+        const int up = __shfl_sync(0xffffffffu, nt, (lane & ~3) + k);
+        if (k > q) over -= up;
       }
-      if (normalize && top_k > 1 && full_softmax) {
-#pragma unroll
-        for (int j = 0; j < RF4_MAX_TOPK; ++j) p[j] = p[j] / s;
+      for (over = min(over, nt); over > 0; --over) {
+        const uint32_t bit = 0x80000000u >> __clz(tie);
+        tie ^= bit;
+        in ^= bit;
       }
-    } else {
-      float s = 0.f;
+      n = __popc(in);
+    }
+    int pos = n;
+    {
+      const int u1 = __shfl_up_sync(0xffffffffu, pos, 1);
+      if (q >= 1) pos += u1;
+      const int u2 = __shfl_up_sync(0xffffffffu, pos, 2);
+      if (q >= 2) pos += u2;
+      pos -= n;
+    }
+    __syncwarp();   // the previous token's list has been read
 #pragma unroll
-      for (int j = 0; j < RF4_MAX_TOPK; ++j) {
-        p[j] = j < top_k ? expf(sv[j] - sv[0]) : 0.f;
-        s += p[j];
-      }
+    for (int i = 0; i < EPL; ++i)
+      if (in >> i & 1u) list[pos++] = make_uint2(key[i], uint32_t(e0 + i));
+    __syncwarp();
+
+    // lane q ranks entries q and q + 4: by value descending, then by index
+    uint2 cand[KT];
 #pragma unroll
-      for (int j = 0; j < RF4_MAX_TOPK; ++j) p[j] = p[j] / s;
+    for (int j = 0; j < KT; ++j) cand[j] = j < top_k ? list[j] : make_uint2(0u, 0u);
+    float p[2], s = 0.f;
+    int rank[2], ei[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int me = q + 4 * h;
+      const bool mine = me < top_k;
+      const uint2 c = mine ? list[me] : make_uint2(0u, 0u);
+      const float val = key_float(c.x);
+      p[h] = !mine ? 0.f : need_full ? expf(val - mx) / denom : expf(val - mx);
+      s += p[h];
+      ei[h] = int(c.y);
+      rank[h] = 0;
+#pragma unroll
+      for (int j = 0; j < KT; ++j)
+        if (cand[j].x > c.x || (cand[j].x == c.x && j < me)) ++rank[h];
+    }
+    if (!need_full || (normalize && top_k > 1 && full_softmax)) {
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      p[0] = p[0] / s;
+      p[1] = p[1] / s;
     }
     if (valid) {
 #pragma unroll
-      for (int j = 0; j < RF4_MAX_TOPK; ++j)
-        if (j < top_k && (j & 3) == q) {
-          w_all[t * kS + j] = __float2bfloat16(p[j]);
-          idx_all[t * kS + j] = si[j];
-          if (chunked) atomicAdd(&hist[si[j]], 1);
+      for (int h = 0; h < 2; ++h)
+        if (q + 4 * h < top_k) {
+          w_all[t * kS + rank[h]] = __float2bfloat16(p[h]);
+          idx_all[t * kS + rank[h]] = ei[h];
+          if (chunked) atomicAdd(&hist[ei[h]], 1);
         }
       for (int jj = top_k + q; jj < kS; jj += 4) {   // the shared experts: every token, weight 1
         w_all[t * kS + jj] = __float2bfloat16(1.f);
@@ -401,23 +461,36 @@ __global__ void __launch_bounds__(RF4_THREADS)
   }
 }
 
-// Whether the four-lane kernel covers a call, and with how many experts per lane (0 = no).
+// Whether the four-lane kernel covers a call, and with how many experts per lane (0 = no). Rows are
+// read as 8-byte pieces up to the one with the last expert.
 static int rf4_experts_per_lane(const void* logits, int ld, int n_experts, int top_k) {
-  if (top_k > RF4_MAX_TOPK || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(logits) & 15u) != 0) return 0;
-  if (n_experts <= 64 && ld >= 64) return 16;
-  if (n_experts <= 96 && ld >= 96) return 24;
-  return 0;
+  if (top_k > RF4_MAX_TOPK || ld % 4 != 0 || ld < (n_experts + 3) / 4 * 4 ||
+      (reinterpret_cast<uintptr_t>(logits) & 7u) != 0)
+    return 0;
+  return n_experts <= 32 ? 8 : n_experts <= 64 ? 16 : n_experts <= 80 ? 20 : n_experts <= 128 ? 32 : 0;
 }
 
+template <int EPL, int KT, typename... Args>
+static void launch_rf4_as(bool want_colsum, unsigned grid, cudaStream_t st, Args... args) {
+  if (want_colsum)
+    launch_pdl(router_fused4_kernel<EPL, KT, true>, dim3(grid), dim3(RF4_THREADS), 0, st, args...);
+  else
+    launch_pdl(router_fused4_kernel<EPL, KT, false>, dim3(grid), dim3(RF4_THREADS), 0, st, args...);
+}
+template <int EPL, typename... Args>
+static void launch_rf4_epl(int top_k, bool want_colsum, unsigned grid, cudaStream_t st, Args... args) {
+  if (top_k <= 2) launch_rf4_as<EPL, 2>(want_colsum, grid, st, args...);
+  else if (top_k <= 4) launch_rf4_as<EPL, 4>(want_colsum, grid, st, args...);
+  else if (top_k <= 6) launch_rf4_as<EPL, 6>(want_colsum, grid, st, args...);
+  else launch_rf4_as<EPL, 8>(want_colsum, grid, st, args...);
+}
 template <typename... Args>
-static void launch_rf4(int epl, bool want_colsum, unsigned grid, cudaStream_t st, Args... args) {
-  if (epl == 16) {
-    if (want_colsum) launch_pdl(router_fused4_kernel<16, true>, dim3(grid), dim3(RF4_THREADS), 0, st, args...);
-    else launch_pdl(router_fused4_kernel<16, false>, dim3(grid), dim3(RF4_THREADS), 0, st, args...);
-  } else {
-    if (want_colsum) launch_pdl(router_fused4_kernel<24, true>, dim3(grid), dim3(RF4_THREADS), 0, st, args...);
-    else launch_pdl(router_fused4_kernel<24, false>, dim3(grid), dim3(RF4_THREADS), 0, st, args...);
-  }
+static void launch_rf4(int epl, int top_k, bool want_colsum, unsigned grid, cudaStream_t st,
+                       Args... args) {
+  if (epl == 8) launch_rf4_epl<8>(top_k, want_colsum, grid, st, args...);
+  else if (epl == 16) launch_rf4_epl<16>(top_k, want_colsum, grid, st, args...);
+  else if (epl == 20) launch_rf4_epl<20>(top_k, want_colsum, grid, st, args...);
+  else launch_rf4_epl<32>(top_k, want_colsum, grid, st, args...);
 }
 
 // d(logits) as bf16 [T, ld_out] (columns >= n_experts zero) from d(w_all) (first top_k columns of
@@ -625,7 +698,7 @@ int launch_router_fused_chunked(const __nv_bfloat16* logits, int ld, const float
       fuse = *sc;
       if (did_scatter) *did_scatter = true;
     }
-    launch_rf4(epl, full_softmax && colsum != nullptr, unsigned(n_blocks), st, logits, ld, bias,
+    launch_rf4(epl, top_k, full_softmax && colsum != nullptr, unsigned(n_blocks), st, logits, ld, bias,
                noise, n_tokens, n_experts, top_k, n_shared, normalize, full_softmax, w_all, idx_all, colsum,
                tokens_per_block, block_hist, sorted_ids, l_cap, fuse);
     return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
@@ -705,7 +778,7 @@ int moe_b200_router_fused(const void* logits, int32_t ld, const float* bias, con
   if (const int epl = rf4_experts_per_lane(logits, ld, n_experts, top_k)) {
     int64_t blocks = (n_tokens + RF4_TOKENS - 1) / RF4_TOKENS;
     if (blocks > 148 * 2) blocks = 148 * 2;
-    launch_rf4(epl, full_softmax && colsum != nullptr, unsigned(blocks), st, lg, ld, bias, noise,
+    launch_rf4(epl, top_k, full_softmax && colsum != nullptr, unsigned(blocks), st, lg, ld, bias, noise,
                n_tokens,
                n_experts, top_k, n_shared, normalize, full_softmax, w, idx_all, colsum, 0,
                static_cast<int32_t*>(nullptr), static_cast<int32_t*>(nullptr), int64_t(0),

@@ -6,7 +6,7 @@ import torch
 from conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
-ATOMIC_TOL = 5e-3
+ATOMIC_TOL = 8e-3      # bf16 adds in no fixed order, on both sides
 
 
 def _block(bias, capacity, n_shared, combine, train=True, d=576, e=76, k=6):

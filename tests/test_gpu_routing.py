@@ -184,3 +184,27 @@ def test_router_dispatch_equals_router_fused_then_dispatch(T, E, k, S):
     for a, b in ((5, 2), (6, 3), (8, 5)):                             # pad_offsets, counts, inv_ids
         assert torch.equal(got[a], ref[b])
     K.check_status("cuda")
+
+
+@pytest.mark.parametrize("E,k,ld", [(8, 8, 8), (32, 1, 32), (33, 2, 36), (64, 3, 64), (76, 6, 76), (80, 5, 128),
+                                    (81, 4, 84), (128, 8, 128), (128, 7, 192)])
+def test_router_fused_selection_with_many_ties(E, k, ld):
+    """The four-lanes-per-token router at the edges of its experts per lane and list lengths, on logits of
+    few distinct values: every place of the selection is decided by the index order."""
+    from nanospeaker_b200 import kernels as K
+    torch.manual_seed(E * k)
+    T = 141
+    logits = torch.full((T, ld), 99.0, device="cuda", dtype=torch.bfloat16)     # padding is not read
+    logits[:, :E] = torch.randint(-2, 3, (T, E), device="cuda").bfloat16()
+    w_all, idx_all, colsum = K.router_fused(logits, None, E, k, 1, True, True)
+    lf = logits[:, :E].float().cpu()
+    order = torch.sort(lf, dim=1, descending=True, stable=True)[1][:, :k]
+    assert torch.equal(idx_all[:, :k].cpu(), order)
+    probs = lf.softmax(-1)
+    sel = probs.gather(1, order)
+    sel = sel / sel.sum(1, keepdim=True) if k > 1 else sel      # (one expert: its probability stays)
+    assert torch.allclose(w_all[:, :k].float().cpu(), sel, atol=4e-3, rtol=8e-3)
+    assert torch.allclose(colsum.cpu(), probs.sum(0), rtol=1e-4, atol=1e-4)
+    got = K.router_dispatch(logits, None, E, k, 1, True, False)
+    assert torch.equal(got[1][:, :k].cpu(), order)
+    K.check_status("cuda")

@@ -292,7 +292,7 @@ int moe_b200_rmsnorm_bwd(const void* dh, const void* x, const float* rstd, const
  * [g | u] ([rows, 2*d_hidden], kept for the backward). a is [rows, d_model] (shared by all fixed
  * groups) or gathered. Replaces _gemm1_kernel (src/model/moe_kernel.py:269-323).
  * d_hidden must be 128.
- * a_tokens (may be NULL; routed schedule with a second weight stack, no gather): the token-major
+ * a_tokens (may be NULL; routed schedule with a second weight stack): the token-major
  * matrix [n_tokens, d_model] the slot-ordered rows were copied from. The groups of the second stack
  * (shared experts: every token once, in token order) then read row `slot - pad_offsets[group]` of
  * a_tokens instead of row `slot` of a, so their rows of a need not have been written at all (see
@@ -345,7 +345,8 @@ int moe_b200_down_gemm_acc(const void* hid, int64_t rows, int32_t k_dim, const v
  * dOut gathered through sorted_ids; a1, da1, hidw are stacked per fixed group.
  * Replaces the dH use of _gemm2_kernel plus _glu_bwd_kernel
  * (src/model/moe_kernel.py:676-692, 510-553). dtw may be NULL.
- * dout_tokens / n_tokens / pad_offsets: as a_tokens of moe_b200_up_gemm, for the rows of douts. */
+ * dout_tokens / n_tokens / pad_offsets: as a_tokens of moe_b200_up_gemm, for the rows of douts; not
+ * with a gather. */
 int moe_b200_dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, const void* w_out,
                              int32_t n_groups, const void* w_extra, int32_t n_extra,
                              int32_t d_hidden, const int32_t* expert_ids,

@@ -377,7 +377,8 @@ int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
   } else {
     STEP(moe_b200_up_gemm(d.x, z.l_cap, D, d.w_in, E, d.w_sh_in, S, H, f.k.expert_ids,
                           f.k.n_post_pad, 0, f.k.sorted_ids, z.ks, z.m, d.activation, f.s.hid,
-                          nullptr, nullptr, 0, nullptr, f.k.bias_in, d.status, stream));
+                          nullptr, S ? d.x : nullptr, S ? T : 0, f.k.pad_offsets, f.k.bias_in,
+                          d.status, stream));
   }
   // down + combine
   if (d.store_combine) {

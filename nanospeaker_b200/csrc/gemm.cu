@@ -240,9 +240,9 @@ static RowsArgs base_args(const int32_t* expert_ids, const int32_t* n_post_pad,
 // a_tokens [n_tokens, k_dim] and the schedule fields that switch those groups over to it.
 static int use_token_rows(RowsArgs* g, CUtensorMap* tmA2, const void* a_tokens, int64_t n_tokens,
                           const int32_t* pad_offsets, int32_t n_groups, int32_t n_extra,
-                          int32_t n_fixed_groups, int32_t gather_top_k, int32_t k_dim) {
+                          int32_t n_fixed_groups, int32_t k_dim) {
   if (!a_tokens) return MOE_B200_OK;
-  if (n_extra < 1 || n_fixed_groups > 0 || gather_top_k > 0 || n_tokens < 1) return MOE_B200_ERR_SHAPE;
+  if (n_extra < 1 || n_fixed_groups > 0 || n_tokens < 1) return MOE_B200_ERR_SHAPE;
   if (!pad_offsets) return MOE_B200_ERR_NULL;
   if ((reinterpret_cast<uintptr_t>(a_tokens) & 15u) != 0) return MOE_B200_ERR_ALIGN;
   if (!map_rows_kmajor(tmA2, a_tokens, 1, n_tokens, k_dim)) return MOE_B200_ERR_TMA;
@@ -328,14 +328,12 @@ int moe_b200_up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w
   const int64_t tiles = max_tiles(rows, 1, n_fixed_groups);
   CUtensorMap tmA2 = tmA;
   const int rc2 = use_token_rows(&g, &tmA2, a_tokens, n_tokens, pad_offsets, n_groups, n_extra,
-                                 n_fixed_groups, gather_top_k, d_model);
+                                 n_fixed_groups, d_model);
   if (rc2 != MOE_B200_OK) return rc2;
-  if (gather_top_k > 0)
-    return launch_rows<256, 4, true, EPI_GLU, true>(tmA, tmB, tmB2, tmB, g, tiles, st);
 #ifndef MOE_NO_PAIR_UP
   // Routed schedule with the run table at hand: CTA pairs, each CTA loading half of the expert's
   // weight tile (the 4-D weight maps then bring 2 of the 4 64-column boxes per copy).
-  if (n_fixed_groups == 0 && pad_offsets != nullptr && fused) {
+  if (n_fixed_groups == 0 && pad_offsets != nullptr && fused && gather_top_k == 0) {
     int32_t f2 = 0;
     CUtensorMap hB, hB2;
     if (!map_weight_mnmajor(&hB, w_in, n_groups, d_model, 2 * d_hidden, 2, &f2)) return MOE_B200_ERR_TMA;
@@ -348,6 +346,8 @@ int moe_b200_up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w
         tmA, tmA2, hB, hB2, hB, g, max_pair_units(rows, n_groups + n_extra, 1), st);
   }
 #endif
+  if (gather_top_k > 0)
+    return launch_rows<256, 4, true, EPI_GLU, true>(tmA, tmB, tmB2, tmB, g, tiles, st, &tmA2);
   return launch_rows<256, 4, true, EPI_GLU>(tmA, tmB, tmB2, tmB, g, tiles, st, &tmA2);
 }
 
@@ -447,8 +447,9 @@ int moe_b200_dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, c
   if (!map_rows_kmajor(&tmAux, a1, n_fixed_groups > 0 ? n_fixed_groups : 1, rows, 2 * d_hidden))
     return MOE_B200_ERR_TMA;
   CUtensorMap tmA2 = tmA;
+  if (dout_tokens && gather_top_k > 0) return MOE_B200_ERR_SHAPE;
   const int rc2 = use_token_rows(&g, &tmA2, dout_tokens, n_tokens, pad_offsets, n_groups, n_extra,
-                                 n_fixed_groups, gather_top_k, d_model);
+                                 n_fixed_groups, d_model);
   if (rc2 != MOE_B200_OK) return rc2;
   if (gather_top_k > 0)
     return launch_rows<128, 3, false, EPI_GLUBWD, true>(tmA, tmB, tmB2, tmAux, g, tiles, st);

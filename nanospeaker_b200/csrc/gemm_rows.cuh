@@ -6,10 +6,10 @@ namespace moe {
 
 constexpr int ROWS_THREADS = 320;
 constexpr int EPI_WARPS = 8;
-// A gathered with cp.async needs many loads in flight, and a warp only keeps a few outstanding:
-// three more producer warps (10..12) join warp 0, each copying 32 of a stage's 128 rows.
+// A gathered with cp.async is bound by what the issuing warps do per stage:
+// four warps of their own (10..13), each copying 32 of a stage's 128 rows.
 constexpr int GATHER_WARPS = 4;
-constexpr int ROWS_THREADS_GATHER = ROWS_THREADS + (GATHER_WARPS - 1) * 32;
+constexpr int ROWS_THREADS_GATHER = ROWS_THREADS + GATHER_WARPS * 32;
 // The GLU-backward epilogue reads a tile of pre-activations [128 x 2 BN]: one more warp brings it
 // into shared memory by TMA one tile ahead (with per-thread global loads the epilogue waited for
 // them tile after tile: dHidden took 77 us with those loads, 50 us without).
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
   [[maybe_unused]] uint64_t* afull_bar = tempty_bar + 2;
   [[maybe_unused]] uint64_t* aempty_bar = afull_bar + 2;
   constexpr bool AUX_IN = epi_loads_aux(EPI);
-  constexpr int AUX_WARP = 2 + EPI_WARPS + (GATHER_A ? GATHER_WARPS - 1 : 0);
+  constexpr int AUX_WARP = 2 + EPI_WARPS + (GATHER_A ? GATHER_WARPS : 0);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::MISC_OFFSET);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* dtw_part = reinterpret_cast<float*>(smem + L::PART_OFFSET);
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
     tma_prefetch_desc(&tmB2);
     if constexpr (TMA_OUT) tma_prefetch_desc(&tmOut);
     for (int s = 0; s < STAGES; ++s) {
-      // gathered A: every lane of warp 0 arrives (through its cp.async) next to the TMA transaction
+      // gathered A: every lane of its warps arrives (through its cp.async) next to the TMA transaction
       mbar_init(full_bar + s, GATHER_A ? GATHER_WARPS * 32 + 1 : 1);
       mbar_init(empty_bar + s, 1);
     }
@@ -278,27 +278,44 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
           tma_load_3d(dst + i * OUT_BOX_BYTES, &tmOut, afull_bar + b, 64 * i, tc.m_tile * BM, tc.z);
       }
     }
-  } else if (GATHER_A && (warp == 0 || (warp >= 2 + EPI_WARPS && warp != AUX_WARP))) {
+  } else if (GATHER_A && warp >= 2 + EPI_WARPS && warp < 2 + EPI_WARPS + GATHER_WARPS) {
     // --------------------------------- producers, gathered A: four warps copy 32 rows each
     // Lane (r4 = lane / 8, c = lane % 8) moves 16-byte chunk c of rows r4, r4 + 4, ... of its
     // warp's 32 rows: eight lanes cover one row's 128-byte k slice, so global reads are whole
     // lines. The chunk lands at (c ^ (row & 7)), the 128-byte swizzle the UMMA descriptor expects.
-    // Warp 0's lane 0 also issues the TMA loads of B.
-    // Completion protocol: a lane's copies of stage i are known to have landed after
-    // cp.async.wait_group; the lane then makes them visible to the async proxy (the tensor core
-    // reads shared memory through it) with fence.proxy.async and arrives on the stage's barrier.
-    // That hand-over trails the issue loop by one stage so the wait is normally already over.
-    const int gw = warp == 0 ? 0 : warp - (1 + EPI_WARPS);
+    // Warp 0 issues the TMA loads: of B, and of the shared experts' rows (tokens in order), for which
+    // these warps only keep the count.
+    // Completion: a lane's arrive on the stage's barrier is itself asynchronous and fires when its
+    // copies have landed; the MMA warp, having seen the barrier, makes them visible to the async proxy
+    // (the tensor core reads shared memory through it). A fence.proxy.async of the lanes themselves
+    // waits for ALL their copies in flight, the later stages' too.
+    // What bounds it is the warps' own work per stage, not the ring (its stages are free when they get
+    // there). 131072 tokens: 417 us with that fence, one copy group ahead, and the loads of B and of the
+    // shared experts' rows in one of these warps; 371 with asynchronous arrives and those rows by TMA;
+    // 347 with the pairs fetched a tile ahead; 322 with B's loads in a warp of their own (16384: 67 ->
+    // 49). 2 or 8 warps, or one polling lane per warp, are slower (340, 340, 330).
+    const int gw = warp - (2 + EPI_WARPS);
     uint32_t it = 0;
-    int pending = -1;  // stage whose copies are issued but not yet handed over
     const int r4 = lane >> 3, c = lane & 7;
+    // the next tile's owner and pairs are fetched with the current tile
+    auto load_pair = [&](int t) {
+      return t < total_tiles
+                 ? __ldg(p.sorted_ids + int64_t((t / p.n_chunks) % m_tiles) * BM + gw * 32 + lane)
+                 : p.n_pairs;
+    };
     int group_next = tile_group(p, blockIdx.x, m_tiles, total_tiles);
+    int pair_next = load_pair(blockIdx.x);
     for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
-      TileCoord tc = decode_tile(p, t, m_tiles, BN);
-      tc.group = group_next;
+      const bool a_alt = group_next >= p.a2_first_group;
+      const int my_tok = pair_next < p.n_pairs ? pair_next / p.top_k : -1;  // of row gw * 32 + lane
       group_next = tile_group(p, t + gridDim.x, m_tiles, total_tiles);
-      const int pair = __ldg(p.sorted_ids + int64_t(tc.m_tile) * BM + gw * 32 + lane);
-      const int my_tok = pair < p.n_pairs ? pair / p.top_k : -1;  // token of row gw*32 + lane
+      pair_next = load_pair(t + gridDim.x);
+      const __nv_bfloat16* src[8];   // rows i * 4 + r4 of this warp's 32, null: zeros
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int tok = __shfl_sync(0xffffffffu, my_tok, i * 4 + r4);
+        src[i] = tok >= 0 ? p.a_src + int64_t(tok) * p.a_cols + c * 8 : nullptr;
+      }
       for (int kt = 0; kt < p.num_k; ++kt, ++it) {
         const int s = it % STAGES;
         const uint32_t use = it / STAGES;
@@ -307,53 +324,22 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
           atomicExch(p.status, ST_WAIT_TIMEOUT);
         }
         if (__any_sync(0xffffffffu, *abort_flag)) break;
-        uint8_t* sA = smem + s * L::STAGE_BYTES;
-        uint8_t* sB = sA + A_STAGE_BYTES;
-        const int k0 = kt * BK;
-        if (warp == 0 && lane == 0) {
-          mbar_expect_tx(full_bar + s, L::B_STAGE_BYTES);
-          // the tile's expert lives in the first weight stack or (shared experts) the second
-          const bool first = tc.group < p.n_groups_b1;
-          const CUtensorMap* mb = first ? &tmB : &tmB2;
-          const int gb = first ? tc.group : tc.group - p.n_groups_b1;
-          if constexpr (B_MN) {
-            if (p.b_fused) {
-              tma_load_4d(sB, mb, full_bar + s, 0, k0, tc.n0 / 64, gb);
-            } else {
+        if (!a_alt) {
+          const int k0 = kt * BK;
+          const bool col_ok = k0 + c * 8 < p.a_cols;
+          const uint32_t sA_u = smem_u32(smem + s * L::STAGE_BYTES) + uint32_t(gw * 32) * 128u;
 #pragma unroll
-              for (int j = 0; j < BN / 64; ++j)
-                tma_load_3d(sB + j * 8192, mb, full_bar + s, tc.n0 + 64 * j, k0, gb);
-            }
-          } else {
-            tma_load_3d(sB, mb, full_bar + s, k0, tc.n0, gb);
+          for (int i = 0; i < 8; ++i) {
+            const int row = i * 4 + r4;
+            const bool ok = src[i] != nullptr && col_ok;
+            cp_async_16(sA_u + row * 128 + ((c ^ (row & 7)) << 4), ok ? src[i] + k0 : p.a_src,
+                        ok ? 16u : 0u);
           }
         }
-        const int col = k0 + c * 8;
-        const bool col_ok = col < p.a_cols;
-        const uint32_t sA_u = smem_u32(sA);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int lrow = i * 4 + r4;
-          const int tok = __shfl_sync(0xffffffffu, my_tok, lrow);
-          const int row = gw * 32 + lrow;
-          const bool ok = tok >= 0 && col_ok;
-          const __nv_bfloat16* src = ok ? p.a_src + int64_t(tok) * p.a_cols + col : p.a_src;
-          cp_async_16(sA_u + row * 128 + ((c ^ (row & 7)) << 4), src, ok ? 16u : 0u);
-        }
-        cp_async_commit();
-        if (pending >= 0) {
-          cp_async_wait<1>();
-          fence_proxy_async();
-          mbar_arrive(full_bar + pending);
-        }
-        pending = s;
+        cp_async_arrive(full_bar + s);
       }
     }
-    if (pending >= 0) {
-      cp_async_wait<0>();
-      fence_proxy_async();
-      mbar_arrive(full_bar + pending);
-    }
+    cp_async_wait_all();   // (matters after an abort only)
   } else if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
@@ -384,7 +370,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
           }
           uint8_t* sA = smem + s * L::STAGE_BYTES;
           uint8_t* sB = sA + A_STAGE_BYTES;
-          mbar_expect_tx(full_bar + s, L::STAGE_BYTES);
+          mbar_expect_tx(full_bar + s, GATHER_A && !a_alt ? L::B_STAGE_BYTES : L::STAGE_BYTES);
           const int g_sum = p.sum_groups > 0 ? kt / p.num_k : 0;
           const int k0 = (kt - g_sum * p.num_k) * BK;
           if (p.sum_groups > 0)
@@ -392,7 +378,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
                         tc.m_tile * BM + __ldg(p.sum_offsets + g_sum), 0);
           else if (a_alt)
             tma_load_3d(sA, &tmA2, full_bar + s, k0, tc.m_tile * BM - a_start, 0);
-          else
+          else if (!GATHER_A)
             tma_load_3d(sA, &tmA, full_bar + s, k0, tc.m_tile * BM, p.a_grouped ? tc.z : 0);
           // the tile's expert lives in the first weight stack or (shared experts) the second
           const bool first = tc.group < p.n_groups_b1;
@@ -436,6 +422,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
             atomicExch(p.status, ST_WAIT_TIMEOUT);
             break;
           }
+          if constexpr (GATHER_A) fence_proxy_async();   // the producers' cp.async (see there)
           tc_fence_after();
           const uint32_t sA = smem_u32(smem + s * L::STAGE_BYTES);
           issue_stage_mmas<BN, false, B_MN>(sA, sA + A_STAGE_BYTES, d_tmem, kt == 0);

@@ -12,7 +12,8 @@
 namespace moe {
 
 constexpr int WGRAD_THREADS = 320;   // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
-constexpr int WGRAD_THREADS_GATHER = 320 + (GATHER_WARPS - 1) * 32;  // + producer warps 10..12
+constexpr int WGRAD_GATHER_WARPS = 4;
+constexpr int WGRAD_THREADS_GATHER = 320 + (WGRAD_GATHER_WARPS - 1) * 32;  // + producer warps 10..12
 constexpr int WGRAD_MAX_GROUPS = 256;
 // Work items are walked longest first (up to this many; beyond it, in list order): CTAs take items
 // round-robin, and with runs of very different lengths the list order left some CTAs with 1.6x the
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
     tma_prefetch_desc(&tmAlt);
     for (int s = 0; s < STAGES; ++s) {
       // a gathered operand: every lane of warp 0 arrives (through its cp.async) next to the TMA
-      mbar_init(full_bar + s, gather ? GATHER_WARPS * 32 + 1 : 1);
+      mbar_init(full_bar + s, gather ? WGRAD_GATHER_WARPS * 32 + 1 : 1);
       mbar_init(empty_bar + s, 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
         const int txy = t % tiles_xy;
         const int m0 = (txy / tiles_y) * BM, n0 = (txy % tiles_y) * BN;
         const int ga = p.a_grouped ? w.group : 0, gb = p.b_grouped ? w.group : 0;
-        constexpr int ROWS_PER_WARP = BK / GATHER_WARPS;  // 16 rows of a stage per producer warp
+        constexpr int ROWS_PER_WARP = BK / WGRAD_GATHER_WARPS;  // 16 rows of a stage per producer warp
         // token of row gw*16 + lane of the NEXT stage, fetched one stage ahead of its use
         int next_tok = -1;
         auto fetch_tok = [&](int kt) {

@@ -76,6 +76,14 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst_smem, const void* src, 
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+// This thread's arrive on an mbarrier (one of the count it was initialised with), made when all its
+// cp.async so far have landed; the thread itself does not wait.
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 // Wait until at most N of this thread's committed cp.async groups are still in flight.
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {

@@ -1,5 +1,5 @@
 // The whole block's forward and backward as ONE host call each: the stage sequence of
-// nanospeaker_b200/moe_kernel.py (router GEMM, routing + dispatch, permute, up/gate GEMM + GLU,
+// nanospeaker_b200/moe_kernel.py (router GEMM, routing + dispatch, gather + up/gate GEMM + GLU,
 // down GEMM, combine, balance loss; and the backward with its three independent
 // branches on three streams) issued from C++, for hosts that pay per call into this library -- a
 // Python caller's ~22 ctypes calls per step cost it more than the GPU needs for the work.
@@ -22,6 +22,7 @@
 #include "../../include/moe_b200.h"
 #include "pdl.cuh"
 #include "routing.cuh"
+#include "stages.cuh"
 
 namespace {
 
@@ -365,15 +366,12 @@ int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
                             f.k.inv_ids, f.s.block_hist, f.s.block_hist_bytes, d.capacity, d.status,
                             stream, &n_disp));
   launched += n_disp - 1;
-  // experts: up/gate + GLU over the permuted rows, which the backward needs again, or (nothing kept)
-  // gathering the token rows itself
+  // experts: up/gate + GLU, gathering the token rows itself; a training forward leaves them in slot
+  // order on the way, for the weight gradients
   if (f.train) {
-    STEP(moe_b200_permute(d.x, T, D, z.ks, f.k.sorted_ids, S ? first_shared : f.k.n_post_pad,
-                          z.l_cap, f.k.xs, stream));
-    STEP(moe_b200_up_gemm(f.k.xs, z.l_cap, D, d.w_in, E, d.w_sh_in, S, H, f.k.expert_ids,
-                          f.k.n_post_pad, 0, nullptr, 0, 0, d.activation, f.s.hid, f.k.a1,
-                          S ? d.x : nullptr, S ? T : 0, f.k.pad_offsets, f.k.bias_in, d.status,
-                          stream));
+    STEP(moe::up_gemm(d.x, z.l_cap, D, d.w_in, E, d.w_sh_in, S, H, f.k.expert_ids, f.k.n_post_pad, 0,
+                      f.k.sorted_ids, z.ks, z.m, d.activation, f.s.hid, f.k.a1, S ? d.x : nullptr,
+                      S ? T : 0, f.k.pad_offsets, f.k.bias_in, f.k.xs, d.status, stream));
   } else {
     STEP(moe_b200_up_gemm(d.x, z.l_cap, D, d.w_in, E, d.w_sh_in, S, H, f.k.expert_ids,
                           f.k.n_post_pad, 0, f.k.sorted_ids, z.ks, z.m, d.activation, f.s.hid,
@@ -478,12 +476,11 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
   const bool store = d.store_combine != 0;
   const int32_t* offs = S ? b.k.pad_offsets : nullptr;
 
-  STEP(moe_b200_permute(b.grad_out, T, D, z.ks, b.k.sorted_ids, live, z.l_cap, b.s.douts, stream));
-  STEP(moe_b200_dhidden_glu_bwd(b.s.douts, z.l_cap, D, d.w_out, E, d.w_sh_out, S, H,
-                                b.k.expert_ids, b.k.n_post_pad, 0, b.k.sorted_ids, 0, b.k.w_all,
-                                z.m, b.k.a1, d.activation, b.s.da1, b.s.hidw, b.s.dtw,
-                                S ? b.grad_out : nullptr, S ? T : 0, offs, d.status, stream));
-  // fork: everything below depends only on the two launches above
+  STEP(moe::dhidden_glu_bwd(b.grad_out, z.l_cap, D, d.w_out, E, d.w_sh_out, S, H, b.k.expert_ids,
+                            b.k.n_post_pad, 0, b.k.sorted_ids, z.ks, b.k.w_all, z.m, b.k.a1,
+                            d.activation, b.s.da1, b.s.hidw, b.s.dtw, S ? b.grad_out : nullptr,
+                            S ? T : 0, offs, b.s.douts, d.status, stream));
+  // fork: everything below depends only on the launch above
   const ForkEventsLease lease;
   if (!lease.ok) return MOE_B200_ERR_CUDA;
   const ForkEvents* ev = &lease.ev;

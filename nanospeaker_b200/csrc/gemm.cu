@@ -1,6 +1,7 @@
 // Host side of the grouped tcgen05 GEMMs: builds the TMA tensor maps for each stage's operands and
 // launches the matching instantiation of grouped_gemm_kernel (gemm.cuh).
 #include "gemm.cuh"
+#include "stages.cuh"
 #include "tma_map.cuh"
 
 #include <cuda.h>
@@ -88,11 +89,11 @@ static int sm_count() {
 }
 
 // Persistent launch: one CTA per SM (fewer if the tile list is shorter than that).
-template <int BN, int STAGES, bool B_MN, int EPI, bool GATHER_A = false, int OUT_BOXES = 4>
+template <int BN, int STAGES, bool B_MN, int EPI, int GATHER = GATHER_NO, int OUT_BOXES = 4>
 static int launch_rows(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmB2,
                        const CUtensorMap& tmOut, const RowsArgs& args, int64_t max_tiles,
                        cudaStream_t st, const CUtensorMap* tmA2 = nullptr) {
-  auto kern = rows_gemm_kernel<BN, STAGES, B_MN, EPI, GATHER_A, OUT_BOXES>;
+  auto kern = rows_gemm_kernel<BN, STAGES, B_MN, EPI, GATHER, OUT_BOXES>;
   constexpr int smem = RowsSmem<BN, STAGES, EPI, OUT_BOXES>::DYNAMIC;
   static_assert(smem <= 232448, "shared memory of a row GEMM exceeds the 227 KB per-CTA limit");
   static std::once_flag once;
@@ -103,7 +104,7 @@ static int launch_rows(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   if (attr_err != cudaSuccess) return MOE_B200_ERR_CUDA;
   const int64_t sms = sm_count();
   const unsigned grid = unsigned(max_tiles < sms ? max_tiles : sms);
-  const cudaError_t err = launch_pdl(kern, dim3(grid), dim3(rows_threads(EPI, GATHER_A)),
+  const cudaError_t err = launch_pdl(kern, dim3(grid), dim3(rows_threads(EPI, GATHER)),
                                      size_t(smem), st, tmA, tmA2 ? *tmA2 : tmA, tmB, tmB2, tmOut,
                                      args);
   return err == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
@@ -127,7 +128,7 @@ static int launch_rows2(const CUtensorMap& tmA, const CUtensorMap& tmA2, const C
     if (attr_err != cudaSuccess) return;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(unsigned(sm_count() / 2 * 2));
-    cfg.blockDim = dim3(rows_threads(EPI, false));
+    cfg.blockDim = dim3(rows_threads(EPI, GATHER_NO));
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -142,7 +143,7 @@ static int launch_rows2(const CUtensorMap& tmA, const CUtensorMap& tmA2, const C
   int64_t clusters = std::min<int64_t>(max_clusters, sm_count() / 2);
   if (max_units < clusters) clusters = max_units;
   const cudaError_t err = launch_pdl_pairs(kern, dim3(unsigned(2 * clusters)),
-                                           dim3(rows_threads(EPI, false)), size_t(smem), st, tmA,
+                                           dim3(rows_threads(EPI, GATHER_NO)), size_t(smem), st, tmA,
                                            tmA2, tmB, tmB2, tmOut, args);
   return err == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
 }
@@ -275,15 +276,14 @@ using namespace moe;
     return n_extra < 0 || n_fixed_groups > 0 ? MOE_B200_ERR_SHAPE : MOE_B200_ERR_NULL; \
   if (n_extra > 0 && !aligned16(w_extra)) return MOE_B200_ERR_ALIGN;
 
-extern "C" {
+namespace moe {
 
-int moe_b200_up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w_in,
-                     int32_t n_groups, const void* w_extra, int32_t n_extra, int32_t d_hidden, const int32_t* expert_ids,
-                     const int32_t* n_post_pad, int32_t n_fixed_groups,
-                     const int32_t* sorted_ids, int32_t gather_top_k, int64_t n_pairs,
-                     int32_t activation, void* hid, void* raw, const void* a_tokens,
-                     int64_t n_tokens, const int32_t* pad_offsets, const void* bias,
-                     int32_t* status, void* stream) {
+int up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w_in, int32_t n_groups,
+            const void* w_extra, int32_t n_extra, int32_t d_hidden, const int32_t* expert_ids,
+            const int32_t* n_post_pad, int32_t n_fixed_groups, const int32_t* sorted_ids,
+            int32_t gather_top_k, int64_t n_pairs, int32_t activation, void* hid, void* raw,
+            const void* a_tokens, int64_t n_tokens, const int32_t* pad_offsets, const void* bias,
+            void* rows_out, int32_t* status, void* stream) {
   CHECK_SCHED();
   if (bias && (n_fixed_groups > 0 || (reinterpret_cast<uintptr_t>(bias) & 15u) != 0))
     return n_fixed_groups > 0 ? MOE_B200_ERR_SHAPE : MOE_B200_ERR_ALIGN;
@@ -302,7 +302,11 @@ int moe_b200_up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w
   tmB2 = tmB;
   if (n_extra > 0 && !map_weight_mnmajor(&tmB2, w_extra, n_extra, d_model, 2 * d_hidden, 4, &fused))
     return MOE_B200_ERR_TMA;
-  if (gather_top_k > 0)
+  if (rows_out && (gather_top_k < 1 || !aligned16(rows_out)))
+    return gather_top_k < 1 ? MOE_B200_ERR_SHAPE : MOE_B200_ERR_ALIGN;
+  if (rows_out) {
+    if (!map_rows_kmajor(&tmA, rows_out, 1, rows, d_model)) return MOE_B200_ERR_TMA;
+  } else if (gather_top_k > 0)
     tmA = tmB;  // unused: A rows are gathered with cp.async
   else if (!map_rows_kmajor(&tmA, a, 1, rows, d_model))
     return MOE_B200_ERR_TMA;
@@ -346,9 +350,27 @@ int moe_b200_up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w
         tmA, tmA2, hB, hB2, hB, g, max_pair_units(rows, n_groups + n_extra, 1), st);
   }
 #endif
+  if (rows_out)
+    return launch_rows<256, 4, true, EPI_GLU, GATHER_KEEP>(tmA, tmB, tmB2, tmB, g, tiles, st, &tmA2);
   if (gather_top_k > 0)
-    return launch_rows<256, 4, true, EPI_GLU, true>(tmA, tmB, tmB2, tmB, g, tiles, st, &tmA2);
+    return launch_rows<256, 4, true, EPI_GLU, GATHER_ROWS>(tmA, tmB, tmB2, tmB, g, tiles, st, &tmA2);
   return launch_rows<256, 4, true, EPI_GLU>(tmA, tmB, tmB2, tmB, g, tiles, st, &tmA2);
+}
+
+}  // namespace moe
+
+extern "C" {
+
+int moe_b200_up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w_in,
+                     int32_t n_groups, const void* w_extra, int32_t n_extra, int32_t d_hidden, const int32_t* expert_ids,
+                     const int32_t* n_post_pad, int32_t n_fixed_groups,
+                     const int32_t* sorted_ids, int32_t gather_top_k, int64_t n_pairs,
+                     int32_t activation, void* hid, void* raw, const void* a_tokens,
+                     int64_t n_tokens, const int32_t* pad_offsets, const void* bias,
+                     int32_t* status, void* stream) {
+  return up_gemm(a, rows, d_model, w_in, n_groups, w_extra, n_extra, d_hidden, expert_ids,
+                 n_post_pad, n_fixed_groups, sorted_ids, gather_top_k, n_pairs, activation, hid, raw,
+                 a_tokens, n_tokens, pad_offsets, bias, nullptr, status, stream);
 }
 
 int moe_b200_down_gemm(const void* hid, int64_t rows, int32_t k_dim, const void* w_out,
@@ -388,18 +410,22 @@ int moe_b200_down_gemm(const void* hid, int64_t rows, int32_t k_dim, const void*
   g.ld_out = d_model;
   g.out_gstride = rows * int64_t(d_model);
   g.n_groups_b1 = n_extra > 0 ? n_groups : INT32_MAX;
-  return launch_rows<192, 4, true, EPI_SCALE, false, 4>(
+  return launch_rows<192, 4, true, EPI_SCALE, GATHER_NO, 4>(
       tmA, tmB, tmB2, tmOut, g, max_tiles(rows, g.n_chunks, n_fixed_groups), static_cast<cudaStream_t>(stream));
 }
 
-int moe_b200_dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, const void* w_out,
+}  // extern "C"
+
+namespace moe {
+
+int dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, const void* w_out,
                              int32_t n_groups, const void* w_extra, int32_t n_extra,
                              int32_t d_hidden, const int32_t* expert_ids,
                              const int32_t* n_post_pad, int32_t n_fixed_groups,
                              const int32_t* sorted_ids, int32_t gather_top_k, const void* pair_w,
                              int64_t n_pairs, const void* a1, int32_t activation, void* da1,
                              void* hidw, void* dtw, const void* dout_tokens, int64_t n_tokens,
-                             const int32_t* pad_offsets, int32_t* status, void* stream) {
+                             const int32_t* pad_offsets, void* rows_out, int32_t* status, void* stream) {
   CHECK_SCHED();
   if (gather_top_k < 0 || (gather_top_k > 0 && (n_fixed_groups > 0 || !sorted_ids)))
     return MOE_B200_ERR_SHAPE;
@@ -416,7 +442,11 @@ int moe_b200_dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, c
   tmB2 = tmB;
   if (n_extra > 0 && !map_weight_kmajor(&tmB2, w_extra, n_extra, d_hidden, d_model, 128))
     return MOE_B200_ERR_TMA;
-  if (gather_top_k > 0)
+  if (rows_out && (gather_top_k < 1 || !aligned16(rows_out)))
+    return gather_top_k < 1 ? MOE_B200_ERR_SHAPE : MOE_B200_ERR_ALIGN;
+  if (rows_out) {
+    if (!map_rows_kmajor(&tmA, rows_out, 1, rows, d_model)) return MOE_B200_ERR_TMA;
+  } else if (gather_top_k > 0)
     tmA = tmB;  // unused: dOut rows are gathered with cp.async
   else if (!map_rows_kmajor(&tmA, douts, 1, rows, d_model))
     return MOE_B200_ERR_TMA;
@@ -447,14 +477,32 @@ int moe_b200_dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, c
   if (!map_rows_kmajor(&tmAux, a1, n_fixed_groups > 0 ? n_fixed_groups : 1, rows, 2 * d_hidden))
     return MOE_B200_ERR_TMA;
   CUtensorMap tmA2 = tmA;
-  if (dout_tokens && gather_top_k > 0) return MOE_B200_ERR_SHAPE;
   const int rc2 = use_token_rows(&g, &tmA2, dout_tokens, n_tokens, pad_offsets, n_groups, n_extra,
                                  n_fixed_groups, d_model);
   if (rc2 != MOE_B200_OK) return rc2;
+  if (rows_out)
+    return launch_rows<128, MOE_DH_STAGES, false, EPI_GLUBWD, GATHER_KEEP, MOE_DH_AUX_BUFS>(
+        tmA, tmB, tmB2, tmAux, g, tiles, st, &tmA2);
   if (gather_top_k > 0)
-    return launch_rows<128, 3, false, EPI_GLUBWD, true>(tmA, tmB, tmB2, tmAux, g, tiles, st);
-  return launch_rows<128, MOE_DH_STAGES, false, EPI_GLUBWD, false, MOE_DH_AUX_BUFS>(
+    return launch_rows<128, MOE_DH_STAGES, false, EPI_GLUBWD, GATHER_ROWS, MOE_DH_AUX_BUFS>(
+        tmA, tmB, tmB2, tmAux, g, tiles, st, &tmA2);
+  return launch_rows<128, MOE_DH_STAGES, false, EPI_GLUBWD, GATHER_NO, MOE_DH_AUX_BUFS>(
       tmA, tmB, tmB2, tmAux, g, tiles, st, &tmA2);
+}
+
+}  // namespace moe
+
+extern "C" {
+
+int moe_b200_dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, const void* w_out,
+                             int32_t n_groups, const void* w_extra, int32_t n_extra,
+                             int32_t d_hidden, const int32_t* expert_ids,
+                             const int32_t* n_post_pad, int32_t n_fixed_groups,
+                             const int32_t* sorted_ids, int32_t gather_top_k, const void* pair_w,
+                             int64_t n_pairs, const void* a1, int32_t activation, void* da1,
+                             void* hidw, void* dtw, const void* dout_tokens, int64_t n_tokens,
+                             const int32_t* pad_offsets, int32_t* status, void* stream) {
+  return dhidden_glu_bwd(douts, rows, d_model, w_out, n_groups, w_extra, n_extra, d_hidden, expert_ids, n_post_pad, n_fixed_groups, sorted_ids, gather_top_k, pair_w, n_pairs, a1, activation, da1, hidw, dtw, dout_tokens, n_tokens, pad_offsets, nullptr, status, stream);
 }
 
 int moe_b200_dx_gemm(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in,
@@ -484,7 +532,7 @@ int moe_b200_dx_gemm(const void* da1, int64_t rows, int32_t d_hidden, const void
   g.ld_out = d_model;
   g.out_gstride = rows * int64_t(d_model);
   g.n_groups_b1 = n_extra > 0 ? n_groups : INT32_MAX;
-  return launch_rows<192, 4, false, EPI_RAW, false, 3>(
+  return launch_rows<192, 4, false, EPI_RAW, GATHER_NO, 3>(
       tmA, tmB, tmB2, tmOut, g, max_tiles(rows, g.n_chunks, n_fixed_groups), static_cast<cudaStream_t>(stream));
 }
 
@@ -523,7 +571,7 @@ int moe_b200_down_gemm_sum(const void* hid, int64_t rows, int32_t k_dim, const v
   g.out = static_cast<__nv_bfloat16*>(out);
   g.ld_out = d_model;
   g.n_groups_b1 = INT32_MAX;
-  return launch_rows<192, 4, true, EPI_SCALE, false, 4>(
+  return launch_rows<192, 4, true, EPI_SCALE, GATHER_NO, 4>(
       tmA, tmB, tmB, tmOut, g, max_tiles(n_tokens, g.n_chunks, 1), static_cast<cudaStream_t>(stream));
 }
 
@@ -547,7 +595,7 @@ int moe_b200_dx_gemm_sum(const void* da1, int64_t rows, int32_t d_hidden, const 
   g.out = static_cast<__nv_bfloat16*>(out);
   g.ld_out = d_model;
   g.n_groups_b1 = INT32_MAX;
-  return launch_rows<192, 4, false, EPI_RAW, false, 3>(
+  return launch_rows<192, 4, false, EPI_RAW, GATHER_NO, 3>(
       tmA, tmB, tmB, tmOut, g, max_tiles(n_tokens, g.n_chunks, 1), static_cast<cudaStream_t>(stream));
 }
 
@@ -617,7 +665,7 @@ int moe_b200_down_gemm_acc(const void* hid, int64_t rows, int32_t k_dim, const v
   g.out = static_cast<__nv_bfloat16*>(acc);
   g.ld_out = d_model;
   g.n_groups_b1 = n_extra > 0 ? n_groups : INT32_MAX;
-  return launch_rows<192, MOE_RED_DOWN_STAGES, true, EPI_SCALE_RED, false, MOE_RED_DOWN_BUFS>(
+  return launch_rows<192, MOE_RED_DOWN_STAGES, true, EPI_SCALE_RED, GATHER_NO, MOE_RED_DOWN_BUFS>(
       tmA, tmB, tmB2, tmB, g, max_tiles(rows, g.n_chunks, n_fixed_groups),
       static_cast<cudaStream_t>(stream));
 }
@@ -670,7 +718,7 @@ int moe_b200_dx_gemm_acc(const void* da1, int64_t rows, int32_t d_hidden, const 
         static_cast<cudaStream_t>(stream));
   }
 #endif
-  return launch_rows<192, MOE_RED_DX_STAGES, false, EPI_RAW_RED, false, MOE_RED_DX_BUFS>(
+  return launch_rows<192, MOE_RED_DX_STAGES, false, EPI_RAW_RED, GATHER_NO, MOE_RED_DX_BUFS>(
       tmA, tmB, tmB2, tmB, g, max_tiles(rows, g.n_chunks, n_fixed_groups),
       static_cast<cudaStream_t>(stream));
 }

@@ -21,9 +21,12 @@ constexpr int RED_WARPS = 4;
 __host__ __device__ constexpr bool epi_reduces(int epi) {
   return epi == EPI_RAW_RED || epi == EPI_SCALE_RED;
 }
-__host__ __device__ constexpr int rows_threads(int epi, bool gather) {
-  return (gather ? ROWS_THREADS_GATHER : ROWS_THREADS) + (epi_loads_aux(epi) ? 32 : 0) +
-         (epi_reduces(epi) ? RED_WARPS * 32 : 0);
+// What the A operand is: a buffer in slot order; token rows gathered by the producers; the same, and
+// written back in slot order from the stages (a training step's weight gradients read them).
+enum GatherMode { GATHER_NO = 0, GATHER_ROWS = 1, GATHER_KEEP = 2 };
+__host__ __device__ constexpr int rows_threads(int epi, int gather) {
+  return (gather ? ROWS_THREADS_GATHER : ROWS_THREADS) + (gather == GATHER_KEEP ? 32 : 0) +
+         (epi_loads_aux(epi) ? 32 : 0) + (epi_reduces(epi) ? RED_WARPS * 32 : 0);
 }
 
 // Epilogues that leave through TMA stage the tile in shared memory one 64-column box (128 rows x
@@ -183,8 +186,8 @@ __device__ __forceinline__ float epilogue_glubwd(uint32_t taddr, int c_lo, int c
   return part;
 }
 
-template <int BN, int STAGES, bool B_MN, int EPI, bool GATHER_A, int OUT_BOXES = 4>
-__global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
+template <int BN, int STAGES, bool B_MN, int EPI, int GATHER, int OUT_BOXES = 4>
+__global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
     rows_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
                      const __grid_constant__ CUtensorMap tmA2,
                      const __grid_constant__ CUtensorMap tmB,
@@ -195,6 +198,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
   // this CTA is resident while the previous grid's last CTAs still work.
   pdl_trigger();
   using L = RowsSmem<BN, STAGES, EPI, OUT_BOXES>;
+  constexpr bool GATHER_A = GATHER != GATHER_NO;
   constexpr bool TMA_OUT = epi_uses_tma_store(EPI);
   static_assert(BN % 64 == 0 && BN <= 256, "BN must be a multiple of 64 up to 256");
   constexpr uint32_t TMEM_BUF = BN <= 128 ? 128 : 256;  // columns per accumulator buffer
@@ -211,6 +215,8 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
   [[maybe_unused]] uint64_t* aempty_bar = afull_bar + 2;
   constexpr bool AUX_IN = epi_loads_aux(EPI);
   constexpr int AUX_WARP = 2 + EPI_WARPS + (GATHER_A ? GATHER_WARPS : 0);
+  constexpr int KEEP_WARP = AUX_WARP + (AUX_IN ? 1 : 0);
+  static_assert(GATHER != GATHER_KEEP || !epi_reduces(EPI), "the reducers' warps");
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::MISC_OFFSET);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* dtw_part = reinterpret_cast<float*>(smem + L::PART_OFFSET);
@@ -228,7 +234,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
     for (int s = 0; s < STAGES; ++s) {
       // gathered A: every lane of its warps arrives (through its cp.async) next to the TMA transaction
       mbar_init(full_bar + s, GATHER_A ? GATHER_WARPS * 32 + 1 : 1);
-      mbar_init(empty_bar + s, 1);
+      mbar_init(empty_bar + s, GATHER == GATHER_KEEP ? 2 : 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar + b, 1);
@@ -277,6 +283,38 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_A), 1)
         for (int i = 0; i < 2 * BN / 64; ++i)  // 64-column boxes of [gate | up], rows past the end read 0
           tma_load_3d(dst + i * OUT_BOX_BYTES, &tmOut, afull_bar + b, 64 * i, tc.m_tile * BM, tc.z);
       }
+    }
+  } else if (GATHER == GATHER_KEEP && warp == KEEP_WARP) {
+    // --------------------------- the gathered rows in slot order: a stage's A box through TMA
+    // (not the shared experts' tiles: whoever reads those rows finds them in token order). A stage is
+    // free when both the MMAs and this copy have read it; what it costs is that time in a ring of
+    // four (one stage's release held back: + 4 us, two: + 11). Against a pass of its own that makes
+    // the slot-ordered copy for a GEMM on CTA pairs: forward 82 -> 76 us at 16384 tokens, 37 -> 28 at
+    // 4096, 30 -> 20 at 512; the backward's dHidden 90 -> 83, 30 -> 27, 22 -> 15.
+    if (elect_one()) {
+      uint32_t it = 0;
+      int group_next = tile_group(p, blockIdx.x, m_tiles, total_tiles);
+      for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
+        const TileCoord tc = decode_tile(p, t, m_tiles, BN, false);
+        const bool a_alt = group_next >= p.a2_first_group;
+        group_next = tile_group(p, t + gridDim.x, m_tiles, total_tiles);
+        for (int kt = 0; kt < p.num_k; ++kt, ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait(full_bar + s, (it / STAGES) & 1, p.status)) {
+            *abort_flag = 1;
+            atomicExch(p.status, ST_WAIT_TIMEOUT);
+            break;
+          }
+          if (!a_alt) {
+            fence_proxy_async();
+            tma_store_3d(&tmA, smem + s * L::STAGE_BYTES, kt * BK, tc.m_tile * BM, 0);
+            bulk_commit();
+            bulk_wait_read<0>();
+          }
+          mbar_arrive(empty_bar + s);
+        }
+      }
+      bulk_wait_read<0>();
     }
   } else if (GATHER_A && warp >= 2 + EPI_WARPS && warp < 2 + EPI_WARPS + GATHER_WARPS) {
     // --------------------------------- producers, gathered A: four warps copy 32 rows each

@@ -125,7 +125,7 @@ struct Unit2 {
 };
 
 template <int BN, int STAGES, bool B_MN, int EPI>
-__global__ void __launch_bounds__(rows_threads(EPI, false), 1)
+__global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
     rows_gemm2_kernel(const __grid_constant__ CUtensorMap tmA,
                       const __grid_constant__ CUtensorMap tmA2,
                       const __grid_constant__ CUtensorMap tmB,

@@ -1,0 +1,23 @@
+// Stages of the block with options that the C entry points of the same names do not have (gemm.cu).
+#pragma once
+#include <stdint.h>
+
+namespace moe {
+// moe_b200_up_gemm / moe_b200_dhidden_glu_bwd with gathered rows (gather_top_k > 0) that are also written
+// in slot order to rows_out [rows, d_model] (null: not), the routed experts' runs only: what
+// moe_b200_permute up to the first shared run would have written.
+int up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w_in, int32_t n_groups,
+            const void* w_extra, int32_t n_extra, int32_t d_hidden, const int32_t* expert_ids,
+            const int32_t* n_post_pad, int32_t n_fixed_groups, const int32_t* sorted_ids,
+            int32_t gather_top_k, int64_t n_pairs, int32_t activation, void* hid, void* raw,
+            const void* a_tokens, int64_t n_tokens, const int32_t* pad_offsets, const void* bias,
+            void* rows_out, int32_t* status, void* stream);
+int dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, const void* w_out,
+                    int32_t n_groups, const void* w_extra, int32_t n_extra,
+                    int32_t d_hidden, const int32_t* expert_ids,
+                    const int32_t* n_post_pad, int32_t n_fixed_groups,
+                    const int32_t* sorted_ids, int32_t gather_top_k, const void* pair_w,
+                    int64_t n_pairs, const void* a1, int32_t activation, void* da1,
+                    void* hidw, void* dtw, const void* dout_tokens, int64_t n_tokens,
+                    const int32_t* pad_offsets, void* rows_out, int32_t* status, void* stream);
+}  // namespace moe

@@ -6,11 +6,10 @@
 // Everything here is host code over the other entry points of include/moe_b200.h, plus a few
 // trivial kernels: zero / copy a few words (memset and device-to-device copy nodes go to a copy
 // engine, where they queue behind a caller's large host-to-device copy in flight: the end-to-end
-// step lost 13 us to that), and the forward's first and last launch, which fold what would
-// otherwise be small launches of their own on the critical path (pad the router weight, stack the
-// biases, clear the column sums; counts for the caller, balance loss, dropped pairs). All of them wait for their
-// predecessors programmatically like the library's other kernels, so none of them breaks the
-// chain of early launches.
+// step lost 13 us to that), and the forward's first launch, which folds what would otherwise be small
+// launches of their own on the critical path (pad the router weight, stack the biases, clear the
+// column sums). All of them wait for their predecessors programmatically like the library's other
+// kernels, so none of them breaks the chain of early launches.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -106,56 +105,6 @@ inline int to_bf16(const float* src, void* dst, int32_t n, cudaStream_t st) {
   const int blocks = std::min((n + 255) / 256, 592);
   moe::launch_pdl(to_bf16_kernel, dim3(unsigned(blocks)), dim3(256), 0, st, src,
                   static_cast<__nv_bfloat16*>(dst), n);
-  return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
-}
-
-// The forward's last launch: the routed experts' counts for the caller and the balance loss
-// aux = coef * E * sum_e (counts[e] / sum counts) * (colsum[e] / T) -- the arithmetic of
-// moe_b200_balance_loss, same order -- or zero when the loss is off (colsum == nullptr); with a
-// capacity also the number of pairs over it. One warp.
-// It does not release its dependents early: when a backward follows in the same graph, letting
-// that backward's first kernel become resident under the down GEMM cost the step 2 us.
-__global__ void finish_fwd_kernel(const int32_t* __restrict__ counts_all,
-                                  int32_t* __restrict__ counts, const float* __restrict__ colsum,
-                                  int n_experts, int64_t n_tokens, float coef,
-                                  float* __restrict__ aux, int aux_is_16bit, int32_t capacity,
-                                  int64_t* __restrict__ dropped) {
-  moe::pdl_wait();
-  const int lane = threadIdx.x;
-  float dot = 0.f, tot = 0.f;
-  int over = 0;
-  for (int e = lane; e < n_experts; e += 32) {
-    const int32_t ci = counts_all[e];
-    counts[e] = ci;
-    if (capacity > 0) over += max(ci - capacity, 0);
-    if (colsum != nullptr) {
-      const float c = float(ci);
-      dot += c * colsum[e];
-      tot += c;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    dot += __shfl_xor_sync(0xffffffffu, dot, o);
-    tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    over += __shfl_xor_sync(0xffffffffu, over, o);
-  }
-  if (lane == 0) {
-    if (dropped != nullptr) *dropped = over;
-    if (aux_is_16bit)
-      *reinterpret_cast<uint16_t*>(aux) = 0;
-    else
-      aux[0] = colsum == nullptr ? 0.f
-                                 : coef * float(n_experts) * dot / fmaxf(tot, 1.f) /
-                                       float(n_tokens > 0 ? n_tokens : 1);
-  }
-}
-
-inline int finish_fwd(const int32_t* counts_all, int32_t* counts, const float* colsum,
-                      int n_experts, int64_t n_tokens, float coef, float* aux, int aux_is_16bit,
-                      int32_t capacity, int64_t* dropped, cudaStream_t st) {
-  moe::launch_pdl(finish_fwd_kernel, dim3(1), dim3(32), 0, st, counts_all, counts, colsum,
-                  n_experts, n_tokens, coef, aux, aux_is_16bit, capacity, dropped);
   return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
 }
 
@@ -359,11 +308,12 @@ int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
   if (!d.logits_in)
     STEP(moe_b200_down_gemm(d.x, T, D, f.k.router_wp, 1, nullptr, 0, z.ld, nullptr, nullptr, 1,
                             nullptr, nullptr, 0, f.k.logits, nullptr, d.status, stream));
+  const moe::FinishArgs fin{f.counts, colsum, f.aux, f.dropped, T, d.aux_coef, E, f.aux_is_16bit};
   int n_disp = 0;
   STEP(moe::router_dispatch(logits, ld, d.logit_bias, d.noise, T, E, d.top_k, S, d.normalize,
                             d.full_softmax, f.k.w_all, f.k.idx_all, colsum, f.k.sorted_ids,
                             f.k.expert_ids, f.k.pad_offsets, f.k.counts_all, f.k.n_post_pad,
-                            f.k.inv_ids, f.s.block_hist, f.s.block_hist_bytes, d.capacity, d.status,
+                            f.k.inv_ids, f.s.block_hist, f.s.block_hist_bytes, d.capacity, fin, d.status,
                             stream, &n_disp));
   launched += n_disp - 1;
   // experts: up/gate + GLU, gathering the token rows itself; a training forward leaves them in slot
@@ -398,9 +348,6 @@ int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
                                 f.k.expert_ids, f.k.n_post_pad, 0, f.k.sorted_ids, f.k.w_all, z.m,
                                 z.ks, f.out, T, f.k.bias_out, d.status, stream));
   }
-  if (f.counts)
-    STEP(finish_fwd(f.k.counts_all, f.counts, colsum, E, T, d.aux_coef, f.aux, f.aux_is_16bit,
-                    d.capacity, f.dropped, st));
   if (n_launches) *n_launches = launched;
   return MOE_B200_OK;
 }

@@ -26,6 +26,40 @@ __device__ __forceinline__ int64_t ld_i64(const int64_t* p) {
   return SAME_KERNEL ? int64_t(__ldcg(reinterpret_cast<const long long*>(p))) : *p;
 }
 
+// One warp; total = the experts' counts.
+template <bool SAME_KERNEL>
+__device__ __forceinline__ void finish_forward(const FinishArgs& f, const int32_t* total,
+                                               int32_t capacity) {
+  const int lane = threadIdx.x & 31;
+  float dot = 0.f, tot = 0.f;
+  int over = 0;
+  for (int e = lane; e < f.n_experts; e += 32) {
+    const int32_t ci = total[e];
+    f.counts[e] = ci;
+    if (capacity > 0) over += max(ci - capacity, 0);
+    if (f.colsum != nullptr) {
+      const float c = float(ci);
+      dot += c * (SAME_KERNEL ? __ldcg(f.colsum + e) : __ldg(f.colsum + e));
+      tot += c;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    dot += __shfl_xor_sync(0xffffffffu, dot, o);
+    tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    over += __shfl_xor_sync(0xffffffffu, over, o);
+  }
+  if (lane == 0) {
+    if (f.dropped != nullptr) *f.dropped = over;
+    if (f.aux_is_16bit)
+      *reinterpret_cast<uint16_t*>(f.aux) = 0;
+    else
+      f.aux[0] = f.colsum == nullptr ? 0.f
+                                     : f.coef * float(f.n_experts) * dot / fmaxf(tot, 1.f) /
+                                           float(f.n_tokens > 0 ? f.n_tokens : 1);
+  }
+}
+
 // Pass 2: plan + stable scatter. Every block first sums the histograms itself (n_blocks is at most
 // 128, the table sits in L2): per expert the total over all blocks and the share of the blocks
 // before this one; from the totals the 128-aligned run offsets. Each block writes its slice of the
@@ -41,7 +75,7 @@ __device__ __forceinline__ void dispatch_scatter_body(
     const int64_t* topk_idx, int64_t n_pairs, int n_experts, int chunk, int n_blocks,
     const int32_t* block_hist, int32_t* counts, int32_t* pad_offsets, int32_t* n_post_pad,
     int32_t* expert_ids, int64_t n_tiles_cap, int32_t* sorted_ids, int32_t* inv_ids,
-    int32_t capacity, int32_t n_capped, int blk, int nblk) {
+    int32_t capacity, int32_t n_capped, const FinishArgs& fin, int blk, int nblk) {
   // capacity > 0: an expert keeps the first `capacity` pairs of its run (lowest pair ids) and drops
   // the rest: a dropped pair gets no slot (inv_ids = -1) and the runs are laid out by the kept
   // counts, while counts[] still reports the routing decisions. Only experts below n_capped are
@@ -92,6 +126,8 @@ __device__ __forceinline__ void dispatch_scatter_body(
   for (int i = threadIdx.x; i < DISPATCH_WARPS * MAX_EXPERTS; i += blockDim.x)
     (&cursor[0][0])[i] = 0;
   __syncthreads();
+  if (fin.counts != nullptr && blk == 0 && warp == 1)
+    finish_forward<SAME_KERNEL>(fin, total, capacity);
   // exclusive scan of the padded run lengths (one warp, 8 consecutive experts per lane)
   if (warp == 0) {
     constexpr int PER = MAX_EXPERTS / 32;

@@ -41,10 +41,11 @@ static inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 blo
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
-// The same launch for kernels that run as clusters of two CTAs (grid.x a multiple of 2).
+// The same launch for kernels that run as clusters of CTAs (grid.x a multiple of the cluster).
 template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_pdl_pairs(void (*kern)(KArgs...), dim3 grid, dim3 block,
-                                           size_t smem, cudaStream_t st, Args&&... args) {
+static inline cudaError_t launch_pdl_cluster(void (*kern)(KArgs...), unsigned cluster, dim3 grid,
+                                             dim3 block, size_t smem, cudaStream_t st,
+                                             Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -52,7 +53,7 @@ static inline cudaError_t launch_pdl_pairs(void (*kern)(KArgs...), dim3 grid, di
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.x = cluster;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -64,6 +65,11 @@ static inline cudaError_t launch_pdl_pairs(void (*kern)(KArgs...), dim3 grid, di
   cfg.numAttrs = 2;
 #endif
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_pdl_pairs(void (*kern)(KArgs...), dim3 grid, dim3 block,
+                                           size_t smem, cudaStream_t st, Args&&... args) {
+  return launch_pdl_cluster(kern, 2u, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 }  // namespace moe

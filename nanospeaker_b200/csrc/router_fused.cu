@@ -8,6 +8,8 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include <mutex>
+
 #include "../../include/moe_b200.h"
 #include "pdl.cuh"
 #include "routing.cuh"
@@ -237,7 +239,7 @@ __global__ void __launch_bounds__(RF4_THREADS)
   // No early release of the next kernel when a scatter launch follows: with it the step measured
   // 4.5 us slower (the likely reason: the dispatch's scatter blocks, 512 threads each, become
   // resident beside this kernel's blocks, which are short of issue slots as it is). A batch that
-  // one block routes, plans and scatters (decode) keeps it: there the launch chain is what counts.
+  // one cluster routes, plans and scatters keeps it: there the launch chain is what counts.
   if (sc.counts != nullptr) pdl_trigger();
   static_assert(EPL % 4 == 0 && EPL <= 32, "a lane loads its experts as 8-byte pieces");
   static_assert(RF4_THREADS == DISPATCH_THREADS, "the scatter pass runs on this kernel's block");
@@ -450,13 +452,15 @@ __global__ void __launch_bounds__(RF4_THREADS)
     const int64_t hi = lo + per < l_cap ? lo + per : l_cap;
     for (int64_t sl = lo + threadIdx.x; sl < hi; sl += blockDim.x) sorted_ids[sl] = int32_t(n_pairs);
     if (sc.counts != nullptr) {
-      // one block holds the whole input: plan and scatter here instead of in a second launch (what
-      // this block wrote above is read back through L2 after the barrier)
-      __syncthreads();
-      dispatch_scatter_body<true>(idx_all, n_pairs, n_experts + n_shared, tokens_per_block * kS, 1,
-                                  block_hist, sc.counts, sc.pad_offsets, sc.n_post_pad,
-                                  sc.expert_ids, sc.n_tiles_cap, sorted_ids, sc.inv_ids,
-                                  sc.capacity, sc.n_capped, 0, 1);
+      // the blocks are one cluster: plan and scatter here instead of in a second launch (what they
+      // wrote above is read back through L2 after the cluster's barrier)
+      asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+      dispatch_scatter_body<true>(idx_all, n_pairs, n_experts + n_shared, tokens_per_block * kS,
+                                  int(gridDim.x), block_hist, sc.counts, sc.pad_offsets,
+                                  sc.n_post_pad, sc.expert_ids, sc.n_tiles_cap, sorted_ids,
+                                  sc.inv_ids, sc.capacity, sc.n_capped, sc.fin, int(blockIdx.x),
+                                  int(gridDim.x));
     }
   }
 }
@@ -470,27 +474,63 @@ static int rf4_experts_per_lane(const void* logits, int ld, int n_experts, int t
   return n_experts <= 32 ? 8 : n_experts <= 64 ? 16 : n_experts <= 80 ? 20 : n_experts <= 128 ? 32 : 0;
 }
 
-template <int EPL, int KT, typename... Args>
-static void launch_rf4_as(bool want_colsum, unsigned grid, cudaStream_t st, Args... args) {
-  if (want_colsum)
-    launch_pdl(router_fused4_kernel<EPL, KT, true>, dim3(grid), dim3(RF4_THREADS), 0, st, args...);
+// A cluster that routes and dispatches alone. 16 blocks (2048 tokens) are past the portable size and
+// need a cluster of SMs that has them; 8 (1024) always go.
+constexpr unsigned RF4_CLUSTER = 16, RF4_CLUSTER_PORTABLE = 8;
+
+template <int EPL, int KT, bool COLSUM, typename... Args>
+static void launch_rf4_kernel(unsigned grid, bool* one_cluster, cudaStream_t st, ScatterArgs sc,
+                              Args... args) {
+  auto kern = router_fused4_kernel<EPL, KT, COLSUM>;
+  if (*one_cluster && grid > RF4_CLUSTER_PORTABLE) {
+    static std::once_flag once;
+    static int fits = 0;
+    std::call_once(once, [&] {
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(RF4_CLUSTER);
+      cfg.blockDim = dim3(RF4_THREADS);
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = RF4_CLUSTER;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+              cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&fits, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        fits = 0;
+      }
+    });
+    *one_cluster = fits > 0;
+  }
+  if (!*one_cluster) sc = ScatterArgs{};
+  if (*one_cluster && grid > 1)
+    launch_pdl_cluster(kern, grid, dim3(grid), dim3(RF4_THREADS), 0, st, args..., sc);
   else
-    launch_pdl(router_fused4_kernel<EPL, KT, false>, dim3(grid), dim3(RF4_THREADS), 0, st, args...);
+    launch_pdl(kern, dim3(grid), dim3(RF4_THREADS), 0, st, args..., sc);
+}
+template <int EPL, int KT, typename... Args>
+static void launch_rf4_as(bool want_colsum, Args... args) {
+  if (want_colsum) launch_rf4_kernel<EPL, KT, true>(args...);
+  else launch_rf4_kernel<EPL, KT, false>(args...);
 }
 template <int EPL, typename... Args>
-static void launch_rf4_epl(int top_k, bool want_colsum, unsigned grid, cudaStream_t st, Args... args) {
-  if (top_k <= 2) launch_rf4_as<EPL, 2>(want_colsum, grid, st, args...);
-  else if (top_k <= 4) launch_rf4_as<EPL, 4>(want_colsum, grid, st, args...);
-  else if (top_k <= 6) launch_rf4_as<EPL, 6>(want_colsum, grid, st, args...);
-  else launch_rf4_as<EPL, 8>(want_colsum, grid, st, args...);
+static void launch_rf4_epl(int top_k, Args... args) {
+  if (top_k <= 2) launch_rf4_as<EPL, 2>(args...);
+  else if (top_k <= 4) launch_rf4_as<EPL, 4>(args...);
+  else if (top_k <= 6) launch_rf4_as<EPL, 6>(args...);
+  else launch_rf4_as<EPL, 8>(args...);
 }
+// *one_cluster: the blocks shall go on to the dispatch's second pass (sc); cleared if they cannot.
 template <typename... Args>
-static void launch_rf4(int epl, int top_k, bool want_colsum, unsigned grid, cudaStream_t st,
-                       Args... args) {
-  if (epl == 8) launch_rf4_epl<8>(top_k, want_colsum, grid, st, args...);
-  else if (epl == 16) launch_rf4_epl<16>(top_k, want_colsum, grid, st, args...);
-  else if (epl == 20) launch_rf4_epl<20>(top_k, want_colsum, grid, st, args...);
-  else launch_rf4_epl<32>(top_k, want_colsum, grid, st, args...);
+static void launch_rf4(int epl, int top_k, bool want_colsum, unsigned grid, bool* one_cluster,
+                       cudaStream_t st, const ScatterArgs& sc, Args... args) {
+  if (epl == 8) launch_rf4_epl<8>(top_k, want_colsum, grid, one_cluster, st, sc, args...);
+  else if (epl == 16) launch_rf4_epl<16>(top_k, want_colsum, grid, one_cluster, st, sc, args...);
+  else if (epl == 20) launch_rf4_epl<20>(top_k, want_colsum, grid, one_cluster, st, sc, args...);
+  else launch_rf4_epl<32>(top_k, want_colsum, grid, one_cluster, st, sc, args...);
 }
 
 // d(logits) as bf16 [T, ld_out] (columns >= n_experts zero) from d(w_all) (first top_k columns of
@@ -693,14 +733,12 @@ int launch_router_fused_chunked(const __nv_bfloat16* logits, int ld, const float
                                 cudaStream_t st, const ScatterArgs* sc, bool* did_scatter) {
   if (did_scatter) *did_scatter = false;
   if (const int epl = rf4_experts_per_lane(logits, ld, n_experts, top_k)) {
-    ScatterArgs fuse{};
-    if (sc != nullptr && n_blocks == 1) {
-      fuse = *sc;
-      if (did_scatter) *did_scatter = true;
-    }
-    launch_rf4(epl, top_k, full_softmax && colsum != nullptr, unsigned(n_blocks), st, logits, ld, bias,
-               noise, n_tokens, n_experts, top_k, n_shared, normalize, full_softmax, w_all, idx_all, colsum,
-               tokens_per_block, block_hist, sorted_ids, l_cap, fuse);
+    bool one_cluster = sc != nullptr && n_blocks <= int(RF4_CLUSTER);
+    launch_rf4(epl, top_k, full_softmax && colsum != nullptr, unsigned(n_blocks), &one_cluster, st,
+               sc != nullptr ? *sc : ScatterArgs{}, logits, ld, bias, noise, n_tokens, n_experts,
+               top_k, n_shared, normalize, full_softmax, w_all, idx_all, colsum, tokens_per_block,
+               block_hist, sorted_ids, l_cap);
+    if (did_scatter) *did_scatter = one_cluster;
     return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
   }
 #define LAUNCH(NS)                                                                              \
@@ -778,11 +816,11 @@ int moe_b200_router_fused(const void* logits, int32_t ld, const float* bias, con
   if (const int epl = rf4_experts_per_lane(logits, ld, n_experts, top_k)) {
     int64_t blocks = (n_tokens + RF4_TOKENS - 1) / RF4_TOKENS;
     if (blocks > 148 * 2) blocks = 148 * 2;
-    launch_rf4(epl, top_k, full_softmax && colsum != nullptr, unsigned(blocks), st, lg, ld, bias, noise,
-               n_tokens,
-               n_experts, top_k, n_shared, normalize, full_softmax, w, idx_all, colsum, 0,
-               static_cast<int32_t*>(nullptr), static_cast<int32_t*>(nullptr), int64_t(0),
-               ScatterArgs{});
+    bool one_cluster = false;
+    launch_rf4(epl, top_k, full_softmax && colsum != nullptr, unsigned(blocks), &one_cluster, st,
+               ScatterArgs{}, lg, ld, bias, noise, n_tokens, n_experts, top_k, n_shared, normalize,
+               full_softmax, w, idx_all, colsum, 0, static_cast<int32_t*>(nullptr),
+               static_cast<int32_t*>(nullptr), int64_t(0));
     return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
   }
 #define LAUNCH(NS)                                                                          \

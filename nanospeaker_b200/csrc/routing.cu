@@ -292,12 +292,13 @@ __global__ void __launch_bounds__(DISPATCH_THREADS)
                             int32_t* __restrict__ counts, int32_t* __restrict__ pad_offsets,
                             int32_t* __restrict__ n_post_pad, int32_t* __restrict__ expert_ids,
                             int64_t n_tiles_cap, int32_t* __restrict__ sorted_ids,
-                            int32_t* __restrict__ inv_ids, int32_t capacity, int32_t n_capped) {
+                            int32_t* __restrict__ inv_ids, int32_t capacity, int32_t n_capped,
+                            const FinishArgs fin) {
   pdl_trigger();
   pdl_wait();
   dispatch_scatter_body<false>(topk_idx, n_pairs, n_experts, chunk, n_blocks, block_hist, counts,
                                pad_offsets, n_post_pad, expert_ids, n_tiles_cap, sorted_ids, inv_ids,
-                               capacity, n_capped, int(blockIdx.x), int(gridDim.x));
+                               capacity, n_capped, fin, int(blockIdx.x), int(gridDim.x));
 }
 
 // Both dispatch entry points: histogram pass, then plan + scatter.
@@ -314,7 +315,8 @@ static int launch_dispatch(const int64_t* topk_idx, int64_t n_pairs, int32_t n_e
                n_experts, chunk, block_hist, sorted_ids, l_cap, status);
   launch_pdl(dispatch_scatter_kernel, dim3(blocks > 0 ? blocks : 1), dim3(DISPATCH_THREADS), 0, st,
              topk_idx, n_pairs, n_experts, chunk, blocks, block_hist, counts, pad_offsets,
-             n_post_pad, expert_ids, l_cap / ALIGN_M, sorted_ids, inv_ids, capacity, n_capped);
+             n_post_pad, expert_ids, l_cap / ALIGN_M, sorted_ids, inv_ids, capacity, n_capped,
+             FinishArgs{});
   return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
 }
 
@@ -434,7 +436,7 @@ int moe_b200_router_dispatch(const void* logits, int32_t ld, const float* bias,
                              size_t scratch_bytes, int32_t* status, void* stream) {
   return router_dispatch(logits, ld, bias, noise, n_tokens, n_experts, top_k, n_shared, normalize,
                          full_softmax, w_all, idx_all, colsum, sorted_ids, expert_ids, pad_offsets,
-                         counts, n_post_pad, inv_ids, scratch, scratch_bytes, 0, status, stream,
+                         counts, n_post_pad, inv_ids, scratch, scratch_bytes, 0, FinishArgs{}, status, stream,
                          nullptr);
 }
 
@@ -448,8 +450,8 @@ int router_dispatch(const void* logits, int32_t ld, const float* bias,
                     int64_t* idx_all, float* colsum, int32_t* sorted_ids,
                     int32_t* expert_ids, int32_t* pad_offsets, int32_t* counts,
                     int32_t* n_post_pad, int32_t* inv_ids, void* scratch,
-                    size_t scratch_bytes, int32_t capacity, int32_t* status, void* stream,
-                    int* launches) {
+                    size_t scratch_bytes, int32_t capacity, const FinishArgs& fin, int32_t* status,
+                    void* stream, int* launches) {
   const int32_t n_all = n_experts + n_shared;
   if (n_experts < 1 || n_all > MAX_EXPERTS || top_k < 1 || top_k > n_experts || n_shared < 0 ||
       top_k + n_shared > 32 || top_k > MAX_TOPK || n_tokens < 1 || ld < n_experts ||
@@ -467,9 +469,9 @@ int router_dispatch(const void* logits, int32_t ld, const float* bias,
   const int blocks = int((n_tokens + tpb - 1) / tpb);
   int32_t* block_hist = static_cast<int32_t*>(scratch);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // a batch that fits one block (128 tokens) is routed, planned and scattered by ONE launch
+  // a batch whose blocks fit one cluster is routed, planned and scattered by ONE launch
   const ScatterArgs sc{counts,  pad_offsets, n_post_pad, expert_ids, l_cap / ALIGN_M,
-                       inv_ids, capacity,    n_experts};
+                       inv_ids, capacity,    n_experts,  fin};
   bool did_scatter = false;
   const int rc = launch_router_fused_chunked(
       static_cast<const __nv_bfloat16*>(logits), ld, bias, noise, n_tokens, n_experts, top_k,
@@ -482,7 +484,7 @@ int router_dispatch(const void* logits, int32_t ld, const float* bias,
   launch_pdl(dispatch_scatter_kernel, dim3(blocks), dim3(DISPATCH_THREADS), 0, st,
              static_cast<const int64_t*>(idx_all), n_pairs, int(n_all), tpb * kS, blocks,
              static_cast<const int32_t*>(block_hist), counts, pad_offsets, n_post_pad, expert_ids,
-             l_cap / ALIGN_M, sorted_ids, inv_ids, capacity, n_experts);
+             l_cap / ALIGN_M, sorted_ids, inv_ids, capacity, n_experts, fin);
   return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
 }
 }  // namespace moe

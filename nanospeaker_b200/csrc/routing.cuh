@@ -26,8 +26,21 @@ namespace moe {
 // router_fused.cu: router top-k in chunked mode (block b owns tokens [b * tokens_per_block, ...))
 // that also leaves the dispatch's per-block histograms and the sentinel fill. Returns an error code
 // of include/moe_b200.h.
-// With `sc` given and the whole input in one block (n_blocks == 1), the four-lanes-per-token kernel
-// also runs the dispatch's second pass itself and *did_scatter is set: no further launch is needed.
+// With `sc` given and few enough blocks for one cluster, the four-lanes-per-token kernel also runs the
+// dispatch's second pass itself and *did_scatter is set: no further launch is needed.
+// What a forward reports besides its output, made where the counts are: the routed experts' counts for
+// the caller, the balance loss coef * E * sum_e (counts[e] / sum counts) * (colsum[e] / T) -- the
+// arithmetic of moe_b200_balance_loss, same order -- or zero when it is off (colsum null), and with a
+// capacity the number of pairs over it.
+struct FinishArgs {
+  int32_t* counts;        // null: nothing of this
+  const float* colsum;
+  float* aux;
+  int64_t* dropped;       // may be null
+  int64_t n_tokens;
+  float coef;
+  int32_t n_experts, aux_is_16bit;
+};
 struct ScatterArgs {
   int32_t* counts;
   int32_t* pad_offsets;
@@ -37,6 +50,7 @@ struct ScatterArgs {
   int32_t* inv_ids;
   int32_t capacity;   // > 0: experts below n_capped keep the first `capacity` pairs of their runs
   int32_t n_capped;
+  FinishArgs fin;
 };
 int launch_router_fused_chunked(const __nv_bfloat16* logits, int ld, const float* bias,
                                 const float* noise,
@@ -47,14 +61,14 @@ int launch_router_fused_chunked(const __nv_bfloat16* logits, int ld, const float
                                 cudaStream_t st, const ScatterArgs* sc = nullptr,
                                 bool* did_scatter = nullptr);
 // routing.cu: moe_b200_router_dispatch with an expert capacity (0 = dropless) on the first n_experts
-// experts; *launches (may be null) receives the number of kernels.
+// experts and the forward's reports; *launches (may be null) receives the number of kernels.
 int router_dispatch(const void* logits, int32_t ld, const float* bias, const float* noise,
                     int64_t n_tokens, int32_t n_experts, int32_t top_k, int32_t n_shared,
                     int32_t normalize, int32_t full_softmax, void* w_all, int64_t* idx_all,
                     float* colsum, int32_t* sorted_ids, int32_t* expert_ids, int32_t* pad_offsets,
                     int32_t* counts, int32_t* n_post_pad, int32_t* inv_ids, void* scratch,
-                    size_t scratch_bytes, int32_t capacity, int32_t* status, void* stream,
-                    int* launches);
+                    size_t scratch_bytes, int32_t capacity, const FinishArgs& fin, int32_t* status,
+                    void* stream, int* launches);
 // router_fused.cu: moe_b200_router_fused_bwd with two more inputs. extra_dw [T, extra_ld] bf16: what
 // d(topk_w) of a pair gains, read at its expert's column; inv_ids [T * (k + S)]: pairs without a slot
 // (dropped by a capacity) have no d(topk_w). Either may be null.

@@ -208,3 +208,24 @@ def test_router_fused_selection_with_many_ties(E, k, ld):
     got = K.router_dispatch(logits, None, E, k, 1, True, False)
     assert torch.equal(got[1][:, :k].cpu(), order)
     K.check_status("cuda")
+
+
+@pytest.mark.parametrize("T", [128, 257, 1024, 1025, 2048, 2049])
+def test_router_and_dispatch_in_one_cluster(T):
+    """The edges of the batches that one cluster routes, plans and scatters (portable size, the largest,
+    one past it) against the separate entry points."""
+    from nanospeaker_b200 import kernels as K
+    torch.manual_seed(T)
+    logits = torch.randn(T, 128, device="cuda").bfloat16()
+    w_all, idx_all, colsum = K.router_fused(logits, None, 76, 6, 2, True, True)
+    ref = K.dispatch(idx_all, 78)
+    for _ in range(3):
+        got = K.router_dispatch(logits, None, 76, 6, 2, True, True)
+        assert torch.equal(got[0], w_all) and torch.equal(got[1], idx_all)
+        assert torch.allclose(got[2], colsum, rtol=1e-5, atol=1e-4)
+        live = int(ref[4])
+        assert int(got[7]) == live and torch.equal(got[3][:live], ref[0][:live])
+        assert torch.equal(got[4][: live // 128], ref[1][: live // 128])
+        for a, b in ((5, 2), (6, 3), (8, 5)):
+            assert torch.equal(got[a], ref[b])
+    K.check_status("cuda")

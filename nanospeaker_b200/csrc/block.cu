@@ -334,10 +334,10 @@ int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
                             f.k.n_post_pad, 0, f.k.sorted_ids, f.k.w_all, z.m, f.s.y,
                             f.k.bias_out, d.status, stream));
     STEP(moe_b200_combine(f.s.y, f.k.inv_ids, T, z.ks, D, d.residual, nullptr, f.out, stream));
-  } else if (S && !d.residual && !f.k.bias_out) {
-    // the shared experts' share, stored, is the accumulator's first value
-    STEP(moe_b200_down_gemm_sum(f.s.hid, z.l_cap, H, d.w_sh_out, S, D, first_shared, T, f.out,
-                                d.status, stream));
+  } else if (S && !f.k.bias_out) {
+    // the shared experts' share, and the residual, stored, are the accumulator's first value
+    STEP(moe::down_gemm_sum(f.s.hid, z.l_cap, H, d.w_sh_out, S, D, first_shared, T, d.residual,
+                            f.out, d.status, stream));
     STEP(moe_b200_down_gemm_acc(f.s.hid, z.l_cap, H, d.w_out, E, nullptr, 0, D, f.k.expert_ids,
                                 first_shared, 0, f.k.sorted_ids, f.k.w_all, z.m, z.ks, f.out, T,
                                 nullptr, d.status, stream));
@@ -366,7 +366,7 @@ struct Bwd {
 // once, and live as long as the process (there is no point at which a static could destroy them:
 // the runtime may already be gone).
 struct ForkEvents {
-  cudaEvent_t fork = nullptr, dx = nullptr, a = nullptr, b = nullptr;
+  cudaEvent_t fork = nullptr, dl = nullptr, a = nullptr, b = nullptr;
 };
 class ForkEventsLease {
  public:
@@ -383,7 +383,7 @@ class ForkEventsLease {
       }
     }
     ok = true;
-    for (cudaEvent_t* p : {&ev.fork, &ev.dx, &ev.a, &ev.b})
+    for (cudaEvent_t* p : {&ev.fork, &ev.dl, &ev.a, &ev.b})
       ok = ok && cudaEventCreateWithFlags(p, cudaEventDisableTiming) == cudaSuccess;
   }
   ~ForkEventsLease() {
@@ -421,6 +421,8 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
   const int32_t* first_shared = b.k.pad_offsets + E;
   const int32_t* live = S ? first_shared : b.k.n_post_pad;
   const bool store = d.store_combine != 0;
+  // a token has a row in a run once at most; runs are padded to whole tiles
+  const int64_t longest_run = (T + 127) / 128 * 128;
   const int32_t* offs = S ? b.k.pad_offsets : nullptr;
 
   STEP(moe::dhidden_glu_bwd(b.grad_out, z.l_cap, D, d.w_out, E, d.w_sh_out, S, H, b.k.expert_ids,
@@ -437,33 +439,15 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
   if (sa != main_st) CU(cudaStreamWaitEvent(sa, ev->fork, 0));
   if (sb != main_st) CU(cudaStreamWaitEvent(sb, ev->fork, 0));
 
-  // main: dx's first value (the shared experts' share, stored), dW_in, the routed rows of dx
-  if (!store) {
-    if (S) {
-      STEP(moe_b200_dx_gemm_sum(b.s.da1, z.l_cap, H, d.w_sh_in, S, D, first_shared, T, b.dx,
-                                d.status, stream));
-    } else {
-      STEP(zero_words(b.dx, T * D / 2, main_st));
-    }
-    CU(cudaEventRecord(ev->dx, main_st));
-  }
-  STEP(moe_b200_wgrad(b.k.xs, 0, D, b.s.da1, 0, 2 * H, z.l_cap, b.k.pad_offsets, z.n_all, 0,
-                      nullptr, 0, 0, 0, b.dw_in, E, S ? b.dw_sh_in : nullptr, b.s.part_in,
-                      b.s.part_in_bytes, S ? d.x : nullptr, S ? T : 0, S ? 1 : 0, d.status,
-                      stream));
-  if (store) {
-    STEP(moe_b200_dx_gemm(b.s.da1, z.l_cap, H, d.w_in, E, d.w_sh_in, S, D, b.k.expert_ids,
-                          b.k.n_post_pad, 0, b.s.ydx, d.status, stream));
-  } else {
-    STEP(moe_b200_dx_gemm_acc(b.s.da1, z.l_cap, H, d.w_in, E, nullptr, 0, D, b.k.expert_ids, live,
-                              0, b.k.sorted_ids, z.m, z.ks, b.dx, T, b.k.pad_offsets, d.status,
-                              stream));
-  }
+  // main: dW_in, then dx: its first value (the shared experts' share and the router's, stored), the
+  // routed rows
+  STEP(moe::wgrad(b.k.xs, 0, D, b.s.da1, 0, 2 * H, z.l_cap, b.k.pad_offsets, z.n_all, 0, nullptr, 0,
+                  0, 0, b.dw_in, E, S ? b.dw_sh_in : nullptr, b.s.part_in, b.s.part_in_bytes,
+                  S ? d.x : nullptr, S ? T : 0, S ? 1 : 0, longest_run, 2 * H, d.status, stream));
   // side a: dW_out, then the bias gradients (column sums over the runs)
-  STEP(moe_b200_wgrad(b.s.hidw, 0, H, b.s.douts, 0, D, z.l_cap, b.k.pad_offsets, z.n_all, 0,
-                      nullptr, 0, 0, 0, b.dw_out, E, S ? b.dw_sh_out : nullptr, b.s.part_out,
-                      b.s.part_out_bytes, S ? b.grad_out : nullptr, S ? T : 0, S ? 2 : 0, d.status,
-                      sa));
+  STEP(moe::wgrad(b.s.hidw, 0, H, b.s.douts, 0, D, z.l_cap, b.k.pad_offsets, z.n_all, 0, nullptr, 0,
+                  0, 0, b.dw_out, E, S ? b.dw_sh_out : nullptr, b.s.part_out, b.s.part_out_bytes,
+                  S ? b.grad_out : nullptr, S ? T : 0, S ? 2 : 0, longest_run, D, d.status, sa));
   const int32_t n_bi = b.s.db_in ? z.n_all * 2 * H : 0, n_bo = b.s.db_out ? z.n_all * D : 0;
   if (n_bi) {
     STEP(zero_words(b.s.db_in, n_bi, sa));
@@ -489,17 +473,25 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
                              d.capacity > 0 ? b.k.inv_ids : nullptr, T, E, d.top_k, S,
                              d.normalize, d.full_softmax, b.grad_aux, b.k.counts_all, d.aux_coef,
                              b.s.dl, z.ld, sb));
-  STEP(moe_b200_wgrad(d.x, 0, D, b.s.dl, 0, z.ld, T, nullptr, 1, 0, nullptr, 0, 0, 0,
-                      b.s.d_router_padded, 1, nullptr, b.s.part_r, b.s.part_r_bytes, nullptr, 0, 0,
-                      d.status, sb));
-  STEP(moe_b200_copy_cols(b.s.d_router_padded, D, E, z.ld, b.d_router, E, sb));
+  CU(cudaEventRecord(ev->dl, sb));
+  // (a product of one chunk is stored with the padded width and copied)
+  const bool padded = E != z.ld && T <= moe::wgrad_chunk_rows(D, z.ld, T, 1, 0);
+  STEP(moe::wgrad(d.x, 0, D, b.s.dl, 0, z.ld, T, nullptr, 1, 0, nullptr, 0, 0, 0,
+                  padded ? b.s.d_router_padded : b.d_router, 1, nullptr, b.s.part_r,
+                  b.s.part_r_bytes, nullptr, 0, 0, T, padded ? z.ld : E, d.status, sb));
+  if (padded) STEP(moe_b200_copy_cols(b.s.d_router_padded, D, E, z.ld, b.d_router, E, sb));
   if (store) {
+    STEP(moe_b200_dx_gemm(b.s.da1, z.l_cap, H, d.w_in, E, d.w_sh_in, S, D, b.k.expert_ids,
+                          b.k.n_post_pad, 0, b.s.ydx, d.status, stream));
     STEP(moe_b200_dx_gemm(b.s.dl, T, z.ld / 2, b.k.router_wp, 1, nullptr, 0, D, nullptr, nullptr,
                           1, b.s.dx_router, d.status, sb));
   } else {
-    if (sb != main_st) CU(cudaStreamWaitEvent(sb, ev->dx, 0));
-    STEP(moe_b200_dx_gemm_acc(b.s.dl, T, z.ld / 2, b.k.router_wp, 1, nullptr, 0, D, nullptr,
-                              nullptr, 1, nullptr, 0, 1, b.dx, T, nullptr, d.status, sb));
+    if (sb != main_st) CU(cudaStreamWaitEvent(main_st, ev->dl, 0));
+    STEP(moe::dx_gemm_sum(b.s.da1, z.l_cap, H, d.w_sh_in, S, D, first_shared, T, b.s.dl,
+                          b.k.router_wp, z.ld, b.dx, d.status, stream));
+    STEP(moe_b200_dx_gemm_acc(b.s.da1, z.l_cap, H, d.w_in, E, nullptr, 0, D, b.k.expert_ids, live,
+                              0, b.k.sorted_ids, z.m, z.ks, b.dx, T, b.k.pad_offsets, d.status,
+                              stream));
   }
   // join
   if (sa != main_st) {

@@ -502,7 +502,10 @@ int moe_b200_dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, c
                              int64_t n_pairs, const void* a1, int32_t activation, void* da1,
                              void* hidw, void* dtw, const void* dout_tokens, int64_t n_tokens,
                              const int32_t* pad_offsets, int32_t* status, void* stream) {
-  return dhidden_glu_bwd(douts, rows, d_model, w_out, n_groups, w_extra, n_extra, d_hidden, expert_ids, n_post_pad, n_fixed_groups, sorted_ids, gather_top_k, pair_w, n_pairs, a1, activation, da1, hidw, dtw, dout_tokens, n_tokens, pad_offsets, nullptr, status, stream);
+  return dhidden_glu_bwd(douts, rows, d_model, w_out, n_groups, w_extra, n_extra, d_hidden, expert_ids,
+                         n_post_pad, n_fixed_groups, sorted_ids, gather_top_k, pair_w, n_pairs, a1,
+                         activation, da1, hidw, dtw, dout_tokens, n_tokens, pad_offsets, nullptr,
+                         status, stream);
 }
 
 int moe_b200_dx_gemm(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in,
@@ -549,11 +552,16 @@ static int sum_checks(const void* a, const void* w, const void* out, const int32
   return MOE_B200_OK;
 }
 
-int moe_b200_down_gemm_sum(const void* hid, int64_t rows, int32_t k_dim, const void* w_out,
-                           int32_t n_sum, int32_t d_model, const int32_t* run_offsets,
-                           int64_t n_tokens, void* out, int32_t* status, void* stream) {
+}  // extern "C"
+
+namespace moe {
+
+int down_gemm_sum(const void* hid, int64_t rows, int32_t k_dim, const void* w_out,
+                  int32_t n_sum, int32_t d_model, const int32_t* run_offsets,
+                  int64_t n_tokens, const void* addend, void* out, int32_t* status, void* stream) {
   const int rc = sum_checks(hid, w_out, out, run_offsets, rows, n_sum, n_tokens, status);
   if (rc != MOE_B200_OK) return rc;
+  if (addend && !aligned16(addend)) return MOE_B200_ERR_ALIGN;
   if (k_dim % 8 != 0 || k_dim < 64 || d_model % 32 != 0) return MOE_B200_ERR_UNSUPPORTED;
   CUtensorMap tmA, tmB, tmOut;
   int32_t fused = 0;
@@ -571,32 +579,79 @@ int moe_b200_down_gemm_sum(const void* hid, int64_t rows, int32_t k_dim, const v
   g.out = static_cast<__nv_bfloat16*>(out);
   g.ld_out = d_model;
   g.n_groups_b1 = INT32_MAX;
+  g.addend = static_cast<const __nv_bfloat16*>(addend);
   return launch_rows<192, 4, true, EPI_SCALE, GATHER_NO, 4>(
       tmA, tmB, tmB, tmOut, g, max_tiles(n_tokens, g.n_chunks, 1), static_cast<cudaStream_t>(stream));
 }
 
-int moe_b200_dx_gemm_sum(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in,
-                         int32_t n_sum, int32_t d_model, const int32_t* run_offsets,
-                         int64_t n_tokens, void* out, int32_t* status, void* stream) {
-  const int rc = sum_checks(da1, w_in, out, run_offsets, rows, n_sum, n_tokens, status);
-  if (rc != MOE_B200_OK) return rc;
+}  // namespace moe
+
+extern "C" {
+
+int moe_b200_down_gemm_sum(const void* hid, int64_t rows, int32_t k_dim, const void* w_out,
+                           int32_t n_sum, int32_t d_model, const int32_t* run_offsets,
+                           int64_t n_tokens, void* out, int32_t* status, void* stream) {
+  return down_gemm_sum(hid, rows, k_dim, w_out, n_sum, d_model, run_offsets, n_tokens, nullptr, out,
+                       status, stream);
+}
+
+}  // extern "C"
+
+namespace moe {
+
+int dx_gemm_sum(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in, int32_t n_sum,
+                int32_t d_model, const int32_t* run_offsets, int64_t n_tokens, const void* a_extra,
+                const void* w_extra, int32_t k_extra, void* out, int32_t* status, void* stream) {
+  if (n_sum > 0 || !a_extra) {
+    const int rc = sum_checks(da1, w_in, out, run_offsets, rows, n_sum, n_tokens, status);
+    if (rc != MOE_B200_OK) return rc;
+  } else if (n_tokens < 1 || n_sum < 0) {
+    return MOE_B200_ERR_SHAPE;
+  } else if (!out || !status) {
+    return MOE_B200_ERR_NULL;
+  } else if (!aligned16(out)) {
+    return MOE_B200_ERR_ALIGN;
+  }
   if (d_hidden % 4 != 0 || d_hidden < 32 || d_model % 32 != 0) return MOE_B200_ERR_UNSUPPORTED;
-  CUtensorMap tmA, tmB, tmOut;
-  if (!map_rows_kmajor(&tmA, da1, 1, rows, 2 * d_hidden) ||
-      !map_weight_kmajor(&tmB, w_in, n_sum, d_model, 2 * d_hidden, 192) ||
-      !map_rows_kmajor(&tmOut, out, 1, n_tokens, d_model))
+  CUtensorMap tmA, tmB, tmA2, tmB2, tmOut;
+  if (a_extra) {
+    if (!w_extra) return MOE_B200_ERR_NULL;
+    if (!aligned16(a_extra) || !aligned16(w_extra)) return MOE_B200_ERR_ALIGN;
+    if (k_extra < 64 || k_extra % 8 != 0) return MOE_B200_ERR_UNSUPPORTED;
+    if (!map_rows_kmajor(&tmA2, a_extra, 1, n_tokens, k_extra) ||
+        !map_weight_kmajor(&tmB2, w_extra, 1, d_model, k_extra, 192))
+      return MOE_B200_ERR_TMA;
+  }
+  if (n_sum > 0 && (!map_rows_kmajor(&tmA, da1, 1, rows, 2 * d_hidden) ||
+                    !map_weight_kmajor(&tmB, w_in, n_sum, d_model, 2 * d_hidden, 192)))
     return MOE_B200_ERR_TMA;
+  if (!map_rows_kmajor(&tmOut, out, 1, n_tokens, d_model)) return MOE_B200_ERR_TMA;
+  if (!a_extra) tmA2 = tmA, tmB2 = tmB;
+  if (n_sum == 0) tmA = tmA2, tmB = tmB2;
   RowsArgs g = base_args(nullptr, nullptr, 1, n_tokens, status);
   g.sum_groups = n_sum;
   g.sum_offsets = run_offsets;
   g.num_k = (2 * d_hidden + BK - 1) / BK;
+  g.extra_k = a_extra ? (k_extra + BK - 1) / BK : 0;
   g.n_dim = d_model;
   g.n_chunks = (d_model + 191) / 192;
   g.out = static_cast<__nv_bfloat16*>(out);
   g.ld_out = d_model;
   g.n_groups_b1 = INT32_MAX;
   return launch_rows<192, 4, false, EPI_RAW, GATHER_NO, 3>(
-      tmA, tmB, tmB, tmOut, g, max_tiles(n_tokens, g.n_chunks, 1), static_cast<cudaStream_t>(stream));
+      tmA, tmB, tmB2, tmOut, g, max_tiles(n_tokens, g.n_chunks, 1), static_cast<cudaStream_t>(stream),
+      &tmA2);
+}
+
+}  // namespace moe
+
+extern "C" {
+
+int moe_b200_dx_gemm_sum(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in,
+                         int32_t n_sum, int32_t d_model, const int32_t* run_offsets,
+                         int64_t n_tokens, void* out, int32_t* status, void* stream) {
+  return dx_gemm_sum(da1, rows, d_hidden, w_in, n_sum, d_model, run_offsets, n_tokens, nullptr,
+                     nullptr, 0, out, status, stream);
 }
 
 // Ring stages / staging buffers of the two accumulating row GEMMs (shared memory per CTA: stages x
@@ -747,6 +802,16 @@ static int auto_ks_rows(int32_t m_dim, int32_t n_dim, int64_t rows, int n_groups
   return int(ks);
 }
 
+}  // extern "C"
+
+namespace moe {
+int wgrad_chunk_rows(int32_t m_dim, int32_t n_dim, int64_t rows, int32_t n_groups, int32_t routed) {
+  return auto_ks_rows(m_dim, n_dim, rows, n_groups, routed);
+}
+}  // namespace moe
+
+extern "C" {
+
 int moe_b200_wgrad_scratch_bytes(int32_t m_dim, int32_t n_dim, int64_t rows, int32_t n_groups,
                                  int32_t routed, int32_t ks_rows, size_t* partial_bytes) {
   if (m_dim < 1 || n_dim < 1 || rows < 0 || n_groups < 1 || ks_rows < 0 || ks_rows % 64 != 0 ||
@@ -760,13 +825,17 @@ int moe_b200_wgrad_scratch_bytes(int32_t m_dim, int32_t n_dim, int64_t rows, int
   return MOE_B200_OK;
 }
 
-int moe_b200_wgrad(const void* a, int32_t a_grouped, int32_t m_dim, const void* b,
-                   int32_t b_grouped, int32_t n_dim, int64_t rows, const int32_t* pad_offsets,
-                   int32_t n_groups, int32_t ks_rows, const int32_t* sorted_ids,
-                   int32_t gather_top_k, int64_t n_pairs, int32_t gather_which, void* dw,
-                   int32_t n_first, void* dw_extra, void* partials, size_t partial_bytes,
-                   const void* alt, int64_t alt_rows, int32_t alt_which, int32_t* status,
-                   void* stream) {
+}  // extern "C"
+
+namespace moe {
+
+int wgrad(const void* a, int32_t a_grouped, int32_t m_dim, const void* b,
+          int32_t b_grouped, int32_t n_dim, int64_t rows, const int32_t* pad_offsets,
+          int32_t n_groups, int32_t ks_rows, const int32_t* sorted_ids,
+          int32_t gather_top_k, int64_t n_pairs, int32_t gather_which, void* dw,
+          int32_t n_first, void* dw_extra, void* partials, size_t partial_bytes,
+          const void* alt, int64_t alt_rows, int32_t alt_which, int64_t max_run, int32_t out_cols, int32_t* status,
+          void* stream) {
   if (rows < 0 || rows > (int64_t(1) << 30) || n_groups < 1 || n_groups > WGRAD_MAX_GROUPS ||
       m_dim < 1 || n_dim < 1)
     return MOE_B200_ERR_SHAPE;
@@ -856,7 +925,11 @@ int moe_b200_wgrad(const void* a, int32_t a_grouped, int32_t m_dim, const void* 
   g.n_pairs = int32_t(n_pairs);
   const unsigned items = unsigned(wgrad_items(rows, n_groups, routed, ks_rows));
   // the second pass can be skipped when no run can have more than one chunk
-  const bool may_split = rows > ks_rows;
+  if (max_run < 1 || max_run > rows) max_run = rows;
+  const bool may_split = max_run > ks_rows;
+  if (out_cols != n_dim && (out_cols > n_dim || routed || n_groups != 1 || !may_split))
+    return MOE_B200_ERR_UNSUPPORTED;
+  g.out_cols = out_cols;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned tx = unsigned((m_dim + BM - 1) / BM);
   // reduce CTAs per tile slice: they share the split runs (at most rows / ks_rows of them)
@@ -879,6 +952,22 @@ int moe_b200_wgrad(const void* a, int32_t a_grouped, int32_t m_dim, const void* 
   }
   if (rc != MOE_B200_OK) return rc;
   return cudaGetLastError() == cudaSuccess ? MOE_B200_OK : MOE_B200_ERR_CUDA;
+}
+
+}  // namespace moe
+
+extern "C" {
+
+int moe_b200_wgrad(const void* a, int32_t a_grouped, int32_t m_dim, const void* b,
+                   int32_t b_grouped, int32_t n_dim, int64_t rows, const int32_t* pad_offsets,
+                   int32_t n_groups, int32_t ks_rows, const int32_t* sorted_ids,
+                   int32_t gather_top_k, int64_t n_pairs, int32_t gather_which, void* dw,
+                   int32_t n_first, void* dw_extra, void* partials, size_t partial_bytes,
+                   const void* alt, int64_t alt_rows, int32_t alt_which, int32_t* status,
+                   void* stream) {
+  return wgrad(a, a_grouped, m_dim, b, b_grouped, n_dim, rows, pad_offsets, n_groups, ks_rows,
+               sorted_ids, gather_top_k, n_pairs, gather_which, dw, n_first, dw_extra, partials,
+               partial_bytes, alt, alt_rows, alt_which, rows, n_dim, status, stream);
 }
 
 }  // extern "C"

@@ -65,9 +65,11 @@ struct RowsArgs {
   // token rows, accumulated over sum_groups groups -- C = sum_g A_g @ B_g with A_g = rows
   // [sum_offsets[g], sum_offsets[g] + rows_host) of the slot-ordered buffer (device offsets: the
   // dispatch's run starts) and B_g = group g of the weight stack. The k loop simply runs over
-  // sum_groups * num_k stages.
-  int32_t sum_groups;
+  // sum_groups * num_k stages. extra_k > 0: and then over extra_k stages of one more product, of the
+  // second A map (token-major [rows_host, .]) and the second B map.
+  int32_t sum_groups, extra_k;
   const int32_t* sum_offsets;
+  const __nv_bfloat16* addend; // group-summed schedule, SCALE: [rows_host, ld_out] added to the result
   int32_t b_fused;             // MN-major B: the maps are 4-D (64 n, k, n / 64, group) and one copy
                                // brings all BN / 64 boxes of a stage (a TMA instruction costs the
                                // issuing thread about as much as a whole stage of MMAs)
@@ -103,6 +105,7 @@ struct WgradArgs {
   const int32_t* sorted_ids;
   int32_t top_k, n_pairs;
   int32_t m_dim, n_dim;        // rows / cols of one C[e]
+  int32_t out_cols;            // columns of `out` (n_dim, or the first out_cols of a split product)
   __nv_bfloat16* out;          // [n_out1, m_dim, n_dim]: groups [0, n_out1)
   __nv_bfloat16* out_extra;    // [G - n_out1, m_dim, n_dim]: the remaining groups (may be null)
   int32_t n_out1;

@@ -397,7 +397,8 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
         const bool a_alt = tc.group >= p.a2_first_group;
         group_next = tile_group(p, t + gridDim.x, m_tiles, total_tiles);
         start_next = run_start_of(group_next);
-        const int k_total = p.sum_groups > 0 ? p.sum_groups * p.num_k : p.num_k;
+        const bool summed = p.sum_groups > 0 || p.extra_k > 0;
+        const int k_sum = p.sum_groups * p.num_k, k_total = summed ? k_sum + p.extra_k : p.num_k;
         for (int kt = 0; kt < k_total; ++kt, ++it) {
           const int s = it % STAGES;
           const uint32_t use = it / STAGES;
@@ -409,9 +410,12 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
           uint8_t* sA = smem + s * L::STAGE_BYTES;
           uint8_t* sB = sA + A_STAGE_BYTES;
           mbar_expect_tx(full_bar + s, GATHER_A && !a_alt ? L::B_STAGE_BYTES : L::STAGE_BYTES);
-          const int g_sum = p.sum_groups > 0 ? kt / p.num_k : 0;
-          const int k0 = (kt - g_sum * p.num_k) * BK;
-          if (p.sum_groups > 0)
+          const bool extra = summed && kt >= k_sum;
+          const int g_sum = summed && !extra ? kt / p.num_k : 0;
+          const int k0 = (extra ? kt - k_sum : kt - g_sum * p.num_k) * BK;
+          if (extra)
+            tma_load_3d(sA, &tmA2, full_bar + s, k0, tc.m_tile * BM, 0);
+          else if (summed)
             tma_load_3d(sA, &tmA, full_bar + s, k0,
                         tc.m_tile * BM + __ldg(p.sum_offsets + g_sum), 0);
           else if (a_alt)
@@ -419,10 +423,9 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
           else if (!GATHER_A)
             tma_load_3d(sA, &tmA, full_bar + s, k0, tc.m_tile * BM, p.a_grouped ? tc.z : 0);
           // the tile's expert lives in the first weight stack or (shared experts) the second
-          const bool first = tc.group < p.n_groups_b1;
+          const bool first = tc.group < p.n_groups_b1 && !extra;
           const CUtensorMap* mb = first ? &tmB : &tmB2;
-          const int gb = p.sum_groups > 0 ? g_sum
-                                          : first ? tc.group : tc.group - p.n_groups_b1;
+          const int gb = summed ? g_sum : first ? tc.group : tc.group - p.n_groups_b1;
           if constexpr (B_MN) {
             if (p.b_fused) {
               tma_load_4d(sB, mb, full_bar + s, 0, k0, tc.n0 / 64, gb);
@@ -452,7 +455,9 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + b * TMEM_BUF;
-        const int k_total = p.sum_groups > 0 ? p.sum_groups * p.num_k : p.num_k;
+        const int k_total = p.sum_groups > 0 || p.extra_k > 0
+                                ? p.sum_groups * p.num_k + p.extra_k
+                                : p.num_k;
         for (int kt = 0; kt < k_total; ++kt, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait(full_bar + s, (it / STAGES) & 1, p.status)) {
@@ -563,6 +568,24 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
       const int b = j & 1;
       const float w_n = load_w(pair_n);                    // next tile's weight
       const int pair_nn = load_pair(t + 2 * gridDim.x);    // the pair id of the tile after that
+      // this row's part of the addend, fetched under the tile's MMAs
+      [[maybe_unused]] uint32_t add_w[EPI == EPI_SCALE ? BN / 64 : 1][16];
+      if constexpr (EPI == EPI_SCALE) {
+        if (p.addend != nullptr) {
+          const int64_t r = int64_t(tc.m_tile) * BM + row;
+#pragma unroll
+          for (int jb = 0; jb < BN / 64; ++jb) {
+            const int col = tc.n0 + jb * 64 + half * 32;
+            if (r < p.rows_host && col < p.n_dim) {
+              ld_global_nc_v8(p.addend + r * p.ld_out + col, add_w[jb]);
+              ld_global_nc_v8(p.addend + r * p.ld_out + col + 16, add_w[jb] + 8);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) add_w[jb][i] = 0u;
+            }
+          }
+        }
+      }
       // A wait that gives up (status already flagged) falls through: the epilogue keeps its
       // barrier protocol intact and the host sees the status word.
       if (!mbar_wait(tfull_bar + b, (uint32_t(j) >> 1) & 1, p.status))
@@ -616,6 +639,13 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
               add_bias32(cur, bias_row + tc.n0 + jb * 64 + half * 32);
 #pragma unroll
             for (int i = 0; i < 32; ++i) cur[i] *= w;
+            if (p.addend != nullptr) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                cur[2 * i] += __uint_as_float(add_w[jb][i] << 16);
+                cur[2 * i + 1] += __uint_as_float(add_w[jb][i] & 0xffff0000u);
+              }
+            }
           }
           const uint32_t buf = smem_u32(smem + L::STAGING_OFFSET + (box_count % OUT_BOXES) * OUT_BOX_BYTES);
 #pragma unroll

@@ -463,7 +463,14 @@ __global__ void __launch_bounds__(256)
       // partial layout [column chunk][row][32 floats]
       const int cc = f / (BM * 8), row = (f / 8) % BM, i4 = f % 8;
       const int m = tile_m * BM + row, n = n0 + cc * 32 + i4 * 4;
-      if (m < p.m_dim && n < p.n_dim) {
+      if (p.out_cols != p.n_dim) {   // one group, narrower rows of any alignment
+        if (m < p.m_dim) {
+          __nv_bfloat16* dst = p.out + int64_t(m) * p.out_cols + n;
+          const float a[4] = {acc.x, acc.y, acc.z, acc.w};
+          for (int u = 0; u < 4; ++u)
+            if (n + u < p.out_cols) dst[u] = __float2bfloat16(a[u]);
+        }
+      } else if (m < p.m_dim && n < p.n_dim) {
         const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y);
         const __nv_bfloat162 hi = __floats2bfloat162_rn(acc.z, acc.w);
         uint2 w;

@@ -20,4 +20,24 @@ int dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, const void
                     int64_t n_pairs, const void* a1, int32_t activation, void* da1,
                     void* hidw, void* dtw, const void* dout_tokens, int64_t n_tokens,
                     const int32_t* pad_offsets, void* rows_out, int32_t* status, void* stream);
+// moe_b200_down_gemm_sum with addend [n_tokens, d_model] (may be null) added to the sum.
+int down_gemm_sum(const void* hid, int64_t rows, int32_t k_dim, const void* w_out,
+                  int32_t n_sum, int32_t d_model, const int32_t* run_offsets,
+                  int64_t n_tokens, const void* addend, void* out, int32_t* status, void* stream);
+// moe_b200_dx_gemm_sum with one more product in the sum: a_extra [n_tokens, k_extra] @ w_extra
+// [d_model, k_extra]^T (a_extra may be null; with it n_sum may be 0).
+int dx_gemm_sum(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in, int32_t n_sum,
+                int32_t d_model, const int32_t* run_offsets, int64_t n_tokens, const void* a_extra,
+                const void* w_extra, int32_t k_extra, void* out, int32_t* status, void* stream);
+// moe_b200_wgrad with what the caller knows beside: no run is longer than max_run rows, and dw has
+// out_cols columns (other than n_dim: one fixed group of more than the rows of a chunk).
+int wgrad(const void* a, int32_t a_grouped, int32_t m_dim, const void* b,
+          int32_t b_grouped, int32_t n_dim, int64_t rows, const int32_t* pad_offsets,
+          int32_t n_groups, int32_t ks_rows, const int32_t* sorted_ids,
+          int32_t gather_top_k, int64_t n_pairs, int32_t gather_which, void* dw,
+          int32_t n_first, void* dw_extra, void* partials, size_t partial_bytes,
+          const void* alt, int64_t alt_rows, int32_t alt_which, int64_t max_run, int32_t out_cols, int32_t* status,
+          void* stream);
+// Rows per split-K chunk that moe_b200_wgrad picks.
+int wgrad_chunk_rows(int32_t m_dim, int32_t n_dim, int64_t rows, int32_t n_groups, int32_t routed);
 }  // namespace moe

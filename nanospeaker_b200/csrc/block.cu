@@ -366,7 +366,7 @@ struct Bwd {
 // once, and live as long as the process (there is no point at which a static could destroy them:
 // the runtime may already be gone).
 struct ForkEvents {
-  cudaEvent_t fork = nullptr, dl = nullptr, a = nullptr, b = nullptr;
+  cudaEvent_t fork = nullptr, dx = nullptr, a = nullptr, b = nullptr;
 };
 class ForkEventsLease {
  public:
@@ -383,7 +383,7 @@ class ForkEventsLease {
       }
     }
     ok = true;
-    for (cudaEvent_t* p : {&ev.fork, &ev.dl, &ev.a, &ev.b})
+    for (cudaEvent_t* p : {&ev.fork, &ev.dx, &ev.a, &ev.b})
       ok = ok && cudaEventCreateWithFlags(p, cudaEventDisableTiming) == cudaSuccess;
   }
   ~ForkEventsLease() {
@@ -439,11 +439,26 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
   if (sa != main_st) CU(cudaStreamWaitEvent(sa, ev->fork, 0));
   if (sb != main_st) CU(cudaStreamWaitEvent(sb, ev->fork, 0));
 
-  // main: dW_in, then dx: its first value (the shared experts' share and the router's, stored), the
-  // routed rows
+  // main: dx's first value (the shared experts' share, stored), dW_in, the routed rows of dx
+  if (!store) {
+    if (S)
+      STEP(moe_b200_dx_gemm_sum(b.s.da1, z.l_cap, H, d.w_sh_in, S, D, first_shared, T, b.dx,
+                                d.status, stream));
+    else
+      STEP(zero_words(b.dx, T * D / 2, main_st));
+    CU(cudaEventRecord(ev->dx, main_st));
+  }
   STEP(moe::wgrad(b.k.xs, 0, D, b.s.da1, 0, 2 * H, z.l_cap, b.k.pad_offsets, z.n_all, 0, nullptr, 0,
                   0, 0, b.dw_in, E, S ? b.dw_sh_in : nullptr, b.s.part_in, b.s.part_in_bytes,
                   S ? d.x : nullptr, S ? T : 0, S ? 1 : 0, longest_run, 2 * H, d.status, stream));
+  if (store) {
+    STEP(moe_b200_dx_gemm(b.s.da1, z.l_cap, H, d.w_in, E, d.w_sh_in, S, D, b.k.expert_ids,
+                          b.k.n_post_pad, 0, b.s.ydx, d.status, stream));
+  } else {
+    STEP(moe_b200_dx_gemm_acc(b.s.da1, z.l_cap, H, d.w_in, E, nullptr, 0, D, b.k.expert_ids, live,
+                              0, b.k.sorted_ids, z.m, z.ks, b.dx, T, b.k.pad_offsets, d.status,
+                              stream));
+  }
   // side a: dW_out, then the bias gradients (column sums over the runs)
   STEP(moe::wgrad(b.s.hidw, 0, H, b.s.douts, 0, D, z.l_cap, b.k.pad_offsets, z.n_all, 0, nullptr, 0,
                   0, 0, b.dw_out, E, S ? b.dw_sh_out : nullptr, b.s.part_out, b.s.part_out_bytes,
@@ -462,9 +477,10 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
                                  S ? b.grad_out : nullptr, S ? T : 0, E, b.s.db_out, sa));
     STEP(to_bf16(b.s.db_out, b.db_out, n_bo, sa));
   }
-  // side b: the router's backward, its weight gradient, its share of dx. With b_out a pair's
-  // d(topk_w) gains <dOut[t], b_out[e]>: one row GEMM dOut @ b_out^T over all experts, read at the
-  // pair's column by the router kernel.
+  // side b: the router's backward, its weight gradient, its share of dx (as one more product of the
+  // sum that gives dx its first value the step was 4 to 10 us slower: that sum then has to wait for
+  // it). With b_out a pair's d(topk_w) gains <dOut[t], b_out[e]>: one row GEMM dOut @ b_out^T over
+  // all experts, read at the pair's column by the router kernel.
   if (b.s.b_extra)
     STEP(moe_b200_dx_gemm(b.grad_out, T, D / 2, b.k.bias_out_k, 1, nullptr, 0, z.ld, nullptr,
                           nullptr, 1, b.s.b_extra, d.status, sb));
@@ -473,7 +489,6 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
                              d.capacity > 0 ? b.k.inv_ids : nullptr, T, E, d.top_k, S,
                              d.normalize, d.full_softmax, b.grad_aux, b.k.counts_all, d.aux_coef,
                              b.s.dl, z.ld, sb));
-  CU(cudaEventRecord(ev->dl, sb));
   // (a product of one chunk is stored with the padded width and copied)
   const bool padded = E != z.ld && T <= moe::wgrad_chunk_rows(D, z.ld, T, 1, 0);
   STEP(moe::wgrad(d.x, 0, D, b.s.dl, 0, z.ld, T, nullptr, 1, 0, nullptr, 0, 0, 0,
@@ -481,17 +496,12 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
                   b.s.part_r_bytes, nullptr, 0, 0, T, padded ? z.ld : E, d.status, sb));
   if (padded) STEP(moe_b200_copy_cols(b.s.d_router_padded, D, E, z.ld, b.d_router, E, sb));
   if (store) {
-    STEP(moe_b200_dx_gemm(b.s.da1, z.l_cap, H, d.w_in, E, d.w_sh_in, S, D, b.k.expert_ids,
-                          b.k.n_post_pad, 0, b.s.ydx, d.status, stream));
     STEP(moe_b200_dx_gemm(b.s.dl, T, z.ld / 2, b.k.router_wp, 1, nullptr, 0, D, nullptr, nullptr,
                           1, b.s.dx_router, d.status, sb));
   } else {
-    if (sb != main_st) CU(cudaStreamWaitEvent(main_st, ev->dl, 0));
-    STEP(moe::dx_gemm_sum(b.s.da1, z.l_cap, H, d.w_sh_in, S, D, first_shared, T, b.s.dl,
-                          b.k.router_wp, z.ld, b.dx, d.status, stream));
-    STEP(moe_b200_dx_gemm_acc(b.s.da1, z.l_cap, H, d.w_in, E, nullptr, 0, D, b.k.expert_ids, live,
-                              0, b.k.sorted_ids, z.m, z.ks, b.dx, T, b.k.pad_offsets, d.status,
-                              stream));
+    if (sb != main_st) CU(cudaStreamWaitEvent(sb, ev->dx, 0));
+    STEP(moe_b200_dx_gemm_acc(b.s.dl, T, z.ld / 2, b.k.router_wp, 1, nullptr, 0, D, nullptr,
+                              nullptr, 1, nullptr, 0, 1, b.dx, T, nullptr, d.status, sb));
   }
   // join
   if (sa != main_st) {
@@ -505,7 +515,11 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
 #undef CU
   if (store)
     STEP(moe_b200_combine(b.s.ydx, b.k.inv_ids, T, z.ks, D, b.s.dx_router, nullptr, b.dx, stream));
-  if (n_launches) *n_launches = launched + 3;   // the three weight gradients may add a reduction pass
+  // the weight gradients' reduction passes
+  launched += (longest_run > moe::wgrad_chunk_rows(D, 2 * H, z.l_cap, z.n_all, 1)) +
+              (longest_run > moe::wgrad_chunk_rows(H, D, z.l_cap, z.n_all, 1)) +
+              (T > moe::wgrad_chunk_rows(D, z.ld, T, 1, 0));
+  if (n_launches) *n_launches = launched;
   return MOE_B200_OK;
 }
 

@@ -595,63 +595,28 @@ int moe_b200_down_gemm_sum(const void* hid, int64_t rows, int32_t k_dim, const v
                        status, stream);
 }
 
-}  // extern "C"
-
-namespace moe {
-
-int dx_gemm_sum(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in, int32_t n_sum,
-                int32_t d_model, const int32_t* run_offsets, int64_t n_tokens, const void* a_extra,
-                const void* w_extra, int32_t k_extra, void* out, int32_t* status, void* stream) {
-  if (n_sum > 0 || !a_extra) {
-    const int rc = sum_checks(da1, w_in, out, run_offsets, rows, n_sum, n_tokens, status);
-    if (rc != MOE_B200_OK) return rc;
-  } else if (n_tokens < 1 || n_sum < 0) {
-    return MOE_B200_ERR_SHAPE;
-  } else if (!out || !status) {
-    return MOE_B200_ERR_NULL;
-  } else if (!aligned16(out)) {
-    return MOE_B200_ERR_ALIGN;
-  }
+int moe_b200_dx_gemm_sum(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in,
+                         int32_t n_sum, int32_t d_model, const int32_t* run_offsets,
+                         int64_t n_tokens, void* out, int32_t* status, void* stream) {
+  const int rc = sum_checks(da1, w_in, out, run_offsets, rows, n_sum, n_tokens, status);
+  if (rc != MOE_B200_OK) return rc;
   if (d_hidden % 4 != 0 || d_hidden < 32 || d_model % 32 != 0) return MOE_B200_ERR_UNSUPPORTED;
-  CUtensorMap tmA, tmB, tmA2, tmB2, tmOut;
-  if (a_extra) {
-    if (!w_extra) return MOE_B200_ERR_NULL;
-    if (!aligned16(a_extra) || !aligned16(w_extra)) return MOE_B200_ERR_ALIGN;
-    if (k_extra < 64 || k_extra % 8 != 0) return MOE_B200_ERR_UNSUPPORTED;
-    if (!map_rows_kmajor(&tmA2, a_extra, 1, n_tokens, k_extra) ||
-        !map_weight_kmajor(&tmB2, w_extra, 1, d_model, k_extra, 192))
-      return MOE_B200_ERR_TMA;
-  }
-  if (n_sum > 0 && (!map_rows_kmajor(&tmA, da1, 1, rows, 2 * d_hidden) ||
-                    !map_weight_kmajor(&tmB, w_in, n_sum, d_model, 2 * d_hidden, 192)))
+  CUtensorMap tmA, tmB, tmOut;
+  if (!map_rows_kmajor(&tmA, da1, 1, rows, 2 * d_hidden) ||
+      !map_weight_kmajor(&tmB, w_in, n_sum, d_model, 2 * d_hidden, 192) ||
+      !map_rows_kmajor(&tmOut, out, 1, n_tokens, d_model))
     return MOE_B200_ERR_TMA;
-  if (!map_rows_kmajor(&tmOut, out, 1, n_tokens, d_model)) return MOE_B200_ERR_TMA;
-  if (!a_extra) tmA2 = tmA, tmB2 = tmB;
-  if (n_sum == 0) tmA = tmA2, tmB = tmB2;
   RowsArgs g = base_args(nullptr, nullptr, 1, n_tokens, status);
   g.sum_groups = n_sum;
   g.sum_offsets = run_offsets;
   g.num_k = (2 * d_hidden + BK - 1) / BK;
-  g.extra_k = a_extra ? (k_extra + BK - 1) / BK : 0;
   g.n_dim = d_model;
   g.n_chunks = (d_model + 191) / 192;
   g.out = static_cast<__nv_bfloat16*>(out);
   g.ld_out = d_model;
   g.n_groups_b1 = INT32_MAX;
   return launch_rows<192, 4, false, EPI_RAW, GATHER_NO, 3>(
-      tmA, tmB, tmB2, tmOut, g, max_tiles(n_tokens, g.n_chunks, 1), static_cast<cudaStream_t>(stream),
-      &tmA2);
-}
-
-}  // namespace moe
-
-extern "C" {
-
-int moe_b200_dx_gemm_sum(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in,
-                         int32_t n_sum, int32_t d_model, const int32_t* run_offsets,
-                         int64_t n_tokens, void* out, int32_t* status, void* stream) {
-  return dx_gemm_sum(da1, rows, d_hidden, w_in, n_sum, d_model, run_offsets, n_tokens, nullptr,
-                     nullptr, 0, out, status, stream);
+      tmA, tmB, tmB, tmOut, g, max_tiles(n_tokens, g.n_chunks, 1), static_cast<cudaStream_t>(stream));
 }
 
 // Ring stages / staging buffers of the two accumulating row GEMMs (shared memory per CTA: stages x

@@ -65,9 +65,8 @@ struct RowsArgs {
   // token rows, accumulated over sum_groups groups -- C = sum_g A_g @ B_g with A_g = rows
   // [sum_offsets[g], sum_offsets[g] + rows_host) of the slot-ordered buffer (device offsets: the
   // dispatch's run starts) and B_g = group g of the weight stack. The k loop simply runs over
-  // sum_groups * num_k stages. extra_k > 0: and then over extra_k stages of one more product, of the
-  // second A map (token-major [rows_host, .]) and the second B map.
-  int32_t sum_groups, extra_k;
+  // sum_groups * num_k stages.
+  int32_t sum_groups;
   const int32_t* sum_offsets;
   const __nv_bfloat16* addend; // group-summed schedule, SCALE: [rows_host, ld_out] added to the result
   int32_t b_fused;             // MN-major B: the maps are 4-D (64 n, k, n / 64, group) and one copy

@@ -397,8 +397,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
         const bool a_alt = tc.group >= p.a2_first_group;
         group_next = tile_group(p, t + gridDim.x, m_tiles, total_tiles);
         start_next = run_start_of(group_next);
-        const bool summed = p.sum_groups > 0 || p.extra_k > 0;
-        const int k_sum = p.sum_groups * p.num_k, k_total = summed ? k_sum + p.extra_k : p.num_k;
+        const int k_total = p.sum_groups > 0 ? p.sum_groups * p.num_k : p.num_k;
         for (int kt = 0; kt < k_total; ++kt, ++it) {
           const int s = it % STAGES;
           const uint32_t use = it / STAGES;
@@ -410,12 +409,9 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
           uint8_t* sA = smem + s * L::STAGE_BYTES;
           uint8_t* sB = sA + A_STAGE_BYTES;
           mbar_expect_tx(full_bar + s, GATHER_A && !a_alt ? L::B_STAGE_BYTES : L::STAGE_BYTES);
-          const bool extra = summed && kt >= k_sum;
-          const int g_sum = summed && !extra ? kt / p.num_k : 0;
-          const int k0 = (extra ? kt - k_sum : kt - g_sum * p.num_k) * BK;
-          if (extra)
-            tma_load_3d(sA, &tmA2, full_bar + s, k0, tc.m_tile * BM, 0);
-          else if (summed)
+          const int g_sum = p.sum_groups > 0 ? kt / p.num_k : 0;
+          const int k0 = (kt - g_sum * p.num_k) * BK;
+          if (p.sum_groups > 0)
             tma_load_3d(sA, &tmA, full_bar + s, k0,
                         tc.m_tile * BM + __ldg(p.sum_offsets + g_sum), 0);
           else if (a_alt)
@@ -423,9 +419,10 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
           else if (!GATHER_A)
             tma_load_3d(sA, &tmA, full_bar + s, k0, tc.m_tile * BM, p.a_grouped ? tc.z : 0);
           // the tile's expert lives in the first weight stack or (shared experts) the second
-          const bool first = tc.group < p.n_groups_b1 && !extra;
+          const bool first = tc.group < p.n_groups_b1;
           const CUtensorMap* mb = first ? &tmB : &tmB2;
-          const int gb = summed ? g_sum : first ? tc.group : tc.group - p.n_groups_b1;
+          const int gb = p.sum_groups > 0 ? g_sum
+                                          : first ? tc.group : tc.group - p.n_groups_b1;
           if constexpr (B_MN) {
             if (p.b_fused) {
               tma_load_4d(sB, mb, full_bar + s, 0, k0, tc.n0 / 64, gb);
@@ -455,9 +452,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + b * TMEM_BUF;
-        const int k_total = p.sum_groups > 0 || p.extra_k > 0
-                                ? p.sum_groups * p.num_k + p.extra_k
-                                : p.num_k;
+        const int k_total = p.sum_groups > 0 ? p.sum_groups * p.num_k : p.num_k;
         for (int kt = 0; kt < k_total; ++kt, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait(full_bar + s, (it / STAGES) & 1, p.status)) {

@@ -24,11 +24,6 @@ int dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, const void
 int down_gemm_sum(const void* hid, int64_t rows, int32_t k_dim, const void* w_out,
                   int32_t n_sum, int32_t d_model, const int32_t* run_offsets,
                   int64_t n_tokens, const void* addend, void* out, int32_t* status, void* stream);
-// moe_b200_dx_gemm_sum with one more product in the sum: a_extra [n_tokens, k_extra] @ w_extra
-// [d_model, k_extra]^T (a_extra may be null; with it n_sum may be 0).
-int dx_gemm_sum(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in, int32_t n_sum,
-                int32_t d_model, const int32_t* run_offsets, int64_t n_tokens, const void* a_extra,
-                const void* w_extra, int32_t k_extra, void* out, int32_t* status, void* stream);
 // moe_b200_wgrad with what the caller knows beside: no run is longer than max_run rows, and dw has
 // out_cols columns (other than n_dim: one fixed group of more than the rows of a chunk).
 int wgrad(const void* a, int32_t a_grouped, int32_t m_dim, const void* b,

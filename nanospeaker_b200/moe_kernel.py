@@ -704,14 +704,18 @@ def moe_block_bwd(
     side_out.wait_stream(main)
     side_router.wait_stream(main)
     if atomic_combine:
-        # dx gets its first value by plain stores (the shared experts' share, or zeros); the router's
-        # share on the third stream is added once that has happened, the routed rows after it (the
-        # order of the one-call backward, which stores both shares as one)
+        # dx gets its first value by plain stores (the shared experts' share, or zeros); the
+        # router's share on the third stream is added once that has happened
         dx = _dx_first_value(da1, w_sh_in, pad_offsets, e_n, x)
         dx_ready = torch.cuda.Event()
         dx_ready.record(main)
     g_in = K.wgrad(xs, da1, pad_offsets, e_n + s_n, n_extra=s_n,
                    token_rows=("a", x) if s_n else None)
+    if atomic_combine:
+        _dx_add_routed(da1, w_in, w_sh_in is not None, expert_ids, n_post_pad, pad_offsets,
+                       sorted_ids, m, ks, dx)
+    else:
+        ydx = K.dx_gemm(da1, w_in, expert_ids, n_post_pad, 0, w_extra=w_sh_in)
     with torch.cuda.stream(side_out):
         g_out = K.wgrad(hidw, douts, pad_offsets, e_n + s_n, n_extra=s_n,
                         token_rows=("b", grad_out) if s_n else None)
@@ -721,19 +725,12 @@ def moe_block_bwd(
         dl = K.router_fused_bwd(logits, logit_bias, idx_all, dtw.view(n, ks), e_n, top_k, s_n,
                                 normalize, full_softmax, d_aux, counts_all, aux_coef,
                                 logits.shape[1], noise)
+        d_router = K.copy_cols(K.wgrad(x, dl, None, 1)[0], e_n)   # pad columns dropped
         if atomic_combine:   # the router's share of dx joins the same accumulator
             side_router.wait_event(dx_ready)
             K.dx_gemm_acc(dl.unsqueeze(0), router_w_padded, None, None, 1, None, 0, 1, dx)
-            dx_ready.record(side_router)
         else:
             dx_router = K.dx_gemm(dl, router_w_padded, None, None, 1)[0]
-        d_router = K.copy_cols(K.wgrad(x, dl, None, 1)[0], e_n)   # pad columns dropped
-    if atomic_combine:
-        main.wait_event(dx_ready)
-        _dx_add_routed(da1, w_in, w_sh_in is not None, expert_ids, n_post_pad, pad_offsets,
-                       sorted_ids, m, ks, dx)
-    else:
-        ydx = K.dx_gemm(da1, w_in, expert_ids, n_post_pad, 0, w_extra=w_sh_in)
     main.wait_stream(side_out)
     main.wait_stream(side_router)
     if s_n:

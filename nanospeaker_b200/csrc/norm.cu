@@ -83,7 +83,10 @@ __global__ void __launch_bounds__(NORM_WARPS * 32)
 
 // dx[t] = rstd * (gamma * dh) - x * rstd^3 / D * <gamma * dh, x>  (+ add[t], the residual branch)
 // dgamma += sum_t dh[t] * x[t] * rstd[t]   (fp32; per-block partial sums in shared memory, then
-// one atomic per block and column)
+// one atomic per block and column). HBM-bound: three rows read, one written. All of a row's loads are
+// in flight before the first is used, and the shared-memory sums are laid out by column / 8 so that a
+// warp's atomics hit different banks (as column * 8 they were 8-way conflicts): 16384 x 576 with a
+// residual 27 -> 18 us behind the block's backward. Blocks per SM: as many as are resident.
 template <int NCH>
 __global__ void __launch_bounds__(NORM_WARPS * 32)
     rmsnorm_bwd_kernel(const uint4* __restrict__ dh, const uint4* __restrict__ x,
@@ -105,15 +108,22 @@ __global__ void __launch_bounds__(NORM_WARPS * 32)
 
   const int64_t warps = int64_t(gridDim.x) * NORM_WARPS;
   for (int64_t t = int64_t(blockIdx.x) * NORM_WARPS + (threadIdx.x >> 5); t < n_rows; t += warps) {
-    uint4 vd[NCH], vx[NCH];
+    uint4 vd[NCH], vx[NCH], va[NCH];
     const float r = rstd[t];
     float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < NCH; ++i) {   // all of a row's loads at once
+      const int c = i * 32 + lane;
+      if (c < chunks_per_row) {
+        vd[i] = __ldcs(dh + t * chunks_per_row + c);
+        vx[i] = __ldcs(x + t * chunks_per_row + c);
+        va[i] = add != nullptr ? __ldcs(add + t * chunks_per_row + c) : make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
 #pragma unroll
     for (int i = 0; i < NCH; ++i) {
       const int c = i * 32 + lane;
       if (c < chunks_per_row) {
-        vd[i] = dh[t * chunks_per_row + c];
-        vx[i] = x[t * chunks_per_row + c];
         float d[8], xx[8], g[8];
         unpack8(vd[i], d);
         unpack8(vx[i], xx);
@@ -138,7 +148,7 @@ __global__ void __launch_bounds__(NORM_WARPS * 32)
         for (int k = 0; k < 8; ++k) o[k] = r * g[k] * d[k] - xx[k] * coef;
         if (add != nullptr) {
           float a[8];
-          unpack8(add[t * chunks_per_row + c], a);
+          unpack8(va[i], a);
 #pragma unroll
           for (int k = 0; k < 8; ++k) o[k] += a[k];
         }
@@ -151,11 +161,12 @@ __global__ void __launch_bounds__(NORM_WARPS * 32)
     const int c = i * 32 + lane;
     if (c < chunks_per_row) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) atomicAdd(&dg_s[c * 8 + k], dg[i][k]);
+      for (int k = 0; k < 8; ++k) atomicAdd(&dg_s[k * chunks_per_row + c], dg[i][k]);
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n_cols; i += blockDim.x) atomicAdd(dgamma + i, dg_s[i]);
+  for (int i = threadIdx.x; i < n_cols; i += blockDim.x)
+    atomicAdd(dgamma + i, dg_s[(i & 7) * chunks_per_row + (i >> 3)]);
 }
 
 static unsigned norm_grid(int64_t n_rows, int blocks_per_sm) {
@@ -203,10 +214,10 @@ int moe_b200_rmsnorm_bwd(const void* dh, const void* x, const float* rstd, const
   if (!dh || !x || !rstd || !gamma || !dx || !dgamma) return MOE_B200_ERR_NULL;
   if (!aligned16(dh) || !aligned16(x) || !aligned16(gamma) || !aligned16(add) || !aligned16(dx))
     return MOE_B200_ERR_ALIGN;
-  // few blocks: every block ends with one atomic per column on dgamma
+  // few blocks (the resident ones): every block ends with one atomic per column on dgamma
   const int nch = (d_model / 8 + 31) / 32;
 #define LAUNCH(N)                                                                              \
-  launch_pdl(rmsnorm_bwd_kernel<N>, dim3(norm_grid(n_rows, 3)), dim3(NORM_WARPS * 32),            \
+  launch_pdl(rmsnorm_bwd_kernel<N>, dim3(norm_grid(n_rows, N <= 2 ? 3 : 2)), dim3(NORM_WARPS * 32),            \
              size_t(d_model) * sizeof(float), static_cast<cudaStream_t>(stream),                  \
              static_cast<const uint4*>(dh), static_cast<const uint4*>(x), rstd,                   \
              static_cast<const uint4*>(gamma), static_cast<const uint4*>(add), n_rows,            \

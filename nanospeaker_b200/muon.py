@@ -152,5 +152,6 @@ class Muon(torch.optim.Optimizer):
                 params, grads, bufs = (list(t) for t in zip(*members))
                 norms = K.shim().muon_step(params, grads, bufs, lr, mom, wd, group["ns_steps"],
                                            *NS_COEFFS, 1e-7)
-                self._update_sq = self._update_sq + norms[0]
-                self._param_sq = self._param_sq + norms[1]
+                if torch.is_tensor(self._update_sq):
+                    norms = norms + torch.stack((self._update_sq, self._param_sq))
+                self._update_sq, self._param_sq = norms

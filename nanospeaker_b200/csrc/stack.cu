@@ -36,6 +36,7 @@
 
 #include "../../include/moe_b200.h"
 #include "act.cuh"
+#include "agree.cuh"
 #include "pdl.cuh"
 #include "ptx.cuh"
 #include "routing.cuh"
@@ -201,7 +202,7 @@ __host__ __device__ inline StackSmem stack_smem(int T, int D, int n_stages, int 
   s.tokw = take(ST_MAX_SLOTS * 16 * 4);                // their pairs' weights
   s.lg = take(2 * MAX_EXPERTS * 4);                    // logits, their sort keys
   s.bars = take(2 * ST_PARTS * 8);
-  s.misc = take(16 + ST_MAX_ITEMS * 4 + ST_MAX_ITEMS * 16);   // abort flag, token counts, items
+  s.misc = take(16 + ST_MAX_ITEMS * 4 + ST_MAX_ITEMS * 16);   // flags, token counts, items
   s.total = at;
   return s;
 }
@@ -260,6 +261,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.bars);   // [ST_PARTS] up / down weights of an item
   uint64_t* empty = full + ST_PARTS;                             // [ST_PARTS] their stages are free again
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.misc);
+  volatile int* go_on = abort_flag + 1;   // written by compute thread 0 alone
   int* cnt = reinterpret_cast<int*>(smem + L.misc + 16);
   StackItem* items = reinterpret_cast<StackItem*>(smem + L.misc + 16 + ST_MAX_ITEMS * 4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -347,9 +349,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   const bool has_token = cta < p.T;
   const int kpad = 1 << p.kshift;
 
-  // One thread looks at the counter, the CTA follows. False: given up.
+  // One thread looks at the counter and at the abort flag (which the TMA warp, outside the compute
+  // warps' barrier, sets at any time), the CTA follows. False: given up.
   auto grid_wait = [&](const uint32_t* ctr, uint32_t target) {
-    if (tid == 0) {
+    const bool go = agree(tid == 0, go_on, [&] {
       uint32_t n = 0;
 #pragma unroll 1
       while (load_gpu(ctr) < target) {
@@ -359,9 +362,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
           break;
         }
       }
-    }
-    ct_sync();
-    return *abort_flag == 0;
+      return *abort_flag == 0;
+    }, ct_sync);
+    if (!go && tid == 0) __nanosleep(1000000);   // let the loads in flight land before the CTA leaves
+    return go;
   };
   int ring_s = 0, part = 0;   // the ring as the consumers see it: the current item's first stage, its part
   auto part_wait = [&](int q) {

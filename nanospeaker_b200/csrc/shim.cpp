@@ -17,9 +17,13 @@
 #include <torch/csrc/autograd/variable.h>
 #include <torch/extension.h>
 
+#include <algorithm>
+#include <array>
 #include <atomic>
+#include <memory>
 #include <mutex>
 #include <optional>
+#include <vector>
 
 #include "../../include/moe_b200.h"
 
@@ -215,10 +219,7 @@ struct Grads {
   Tensor dx, d_router, dw_in, dw_out, dw_sh_in, dw_sh_out, db_in, db_out, db_sh_in, db_sh_out;
 };
 
-Grads launch_backward(const Operands& p, const Options& o, const Tensor& kept,
-                      const Tensor& grad_out, const Tensor& grad_aux) {
-  const c10::cuda::CUDAGuard on(p.x.device());
-  const moe_b200_block_desc d = describe(p, o);
+Grads empty_grads(const Operands& p) {
   Grads g;
   g.dx = at::empty_like(p.x);
   g.d_router = at::empty_like(p.router_w);
@@ -228,6 +229,14 @@ Grads launch_backward(const Operands& p, const Options& o, const Tensor& kept,
     g.dw_sh_in = at::empty_like(p.w_sh_in);
     g.dw_sh_out = at::empty_like(p.w_sh_out);
   }
+  return g;
+}
+
+// Fills g (empty_grads); the biases' gradients come with it.
+void launch_backward(const Operands& p, const Options& o, const Tensor& kept,
+                     const Tensor& grad_out, const Tensor& grad_aux, Grads& g) {
+  const c10::cuda::CUDAGuard on(p.x.device());
+  const moe_b200_block_desc d = describe(p, o);
   const int64_t e = d.n_experts, s = d.n_shared;
   Tensor db_in, db_out;   // one row per group of both weight stacks
   if (p.b_in.defined() || p.b_sh_in.defined())
@@ -258,6 +267,12 @@ Grads launch_backward(const Operands& p, const Options& o, const Tensor& kept,
   if (p.b_sh_in.defined()) g.db_sh_in = db_in.narrow(0, e, s);
   if (p.b_out.defined()) g.db_out = db_out.narrow(0, 0, e);
   if (p.b_sh_out.defined()) g.db_sh_out = db_out.narrow(0, e, s);
+}
+Grads launch_backward(const Operands& p, const Options& o, const Tensor& kept,
+                      const Tensor& grad_out, const Tensor& grad_aux) {
+  const c10::cuda::CUDAGuard on(p.x.device());
+  Grads g = empty_grads(p);
+  launch_backward(p, o, kept, grad_out, grad_aux, g);
   return g;
 }
 
@@ -504,7 +519,11 @@ std::tuple<Tensor, Tensor, Tensor> sublayer(
 // --------------------------------------------------------------------- replay from graphs
 // The block's training step for one input shape, forward and backward each captured in a CUDA graph
 // and replayed behind an autograd node. Inputs and incoming gradients are copied into the graphs'
-// own buffers; results are those buffers (overwritten by the next call).
+// own buffers. The forward's results are those buffers (overwritten by the next call); a gradient is
+// whoever's it has become: autograd takes it as p.grad without a copy, and a second micro-step adds to
+// it. So the backward replays into buffers that nobody else holds: a trainer that clears its gradients
+// always meets the first set, one that accumulates has the first set as p.grad and the second on the
+// way, and where those two are both held the last set's results leave as copies.
 class GraphedBlock : public std::enable_shared_from_this<GraphedBlock> {
  public:
   GraphedBlock(const Tensor& x, const Tensor& router_w, const OptTensor& logit_bias,
@@ -537,12 +556,8 @@ class GraphedBlock : public std::enable_shared_from_this<GraphedBlock> {
       fwd_.capture_begin();
       r_ = launch_forward(p_, opt_, true);
       fwd_.capture_end();
-      const int64_t l1 = n_launched;
-      bwd_.capture_begin(fwd_.pool());
-      g_ = launch_backward(p_, opt_, r_.kept, grad_out_, grad_aux_);
-      bwd_.capture_end();
-      n_fwd_ = l1 - l0;
-      n_bwd_ = n_launched - l1;
+      n_fwd_ = n_launched - l0;
+      capture_backward(cudaStreamCaptureModeGlobal);
     }
   }
 
@@ -559,18 +574,58 @@ class GraphedBlock : public std::enable_shared_from_this<GraphedBlock> {
       grad_aux_.copy_(grad_aux.reshape({1}), true);
     else if (opt_.full_softmax)
       grad_aux_.zero_();
-    bwd_.replay();
+    size_t i = 0;
+    while (i < bwd_.size() && held(bwd_[i]->grads)) ++i;
+    if (i == bwd_.size()) {
+      const c10::cuda::CUDAStreamGuard work(
+          c10::cuda::getStreamFromPool(false, p_.x.get_device()));
+      capture_backward(cudaStreamCaptureModeThreadLocal);   // (other threads may be at work by now)
+    }
+    bwd_[i]->graph.replay();
     n_launched += n_bwd_;
-    return g_;
+    Grads g = bwd_[i]->grads;
+    for (Tensor* t : all(g))
+      if (t->defined()) *t = i < SETS_GIVEN_OUT ? t->detach() : t->clone();
+    return g;
   }
 
  private:
+  // A capture of the backward and the gradients it leaves.
+  struct BackwardGraph {
+    at::cuda::CUDAGraph graph;
+    Grads grads;
+  };
+  static constexpr size_t SETS_GIVEN_OUT = 2;
+
+  static std::array<Tensor*, 6> all(Grads& g) {
+    return {&g.dx, &g.d_router, &g.dw_in, &g.dw_out, &g.dw_sh_in, &g.dw_sh_out};
+  }
+  // Whether anybody else refers to these buffers.
+  static bool held(Grads& g) {
+    for (const Tensor* t : all(g))
+      if (t->defined() && t->storage().use_count() > 1) return true;
+    return false;
+  }
+  // On the current stream. The gradients are allocated ahead of the capture: its pool is scratch that
+  // the other graphs use as well, one after the other.
+  void capture_backward(cudaStreamCaptureMode mode) {
+    auto b = std::make_unique<BackwardGraph>();
+    b->grads = empty_grads(p_);
+    const int64_t l0 = n_launched;
+    b->graph.capture_begin(fwd_.pool(), mode);
+    launch_backward(p_, opt_, r_.kept, grad_out_, grad_aux_, b->grads);
+    b->graph.capture_end();
+    n_bwd_ = n_launched - l0;
+    n_launched -= n_bwd_;   // (a capture launches nothing)
+    bwd_.push_back(std::move(b));
+  }
+
   Options opt_;
   Operands p_;
   Results r_;
-  Grads g_;
   Tensor grad_out_, grad_aux_;
-  at::cuda::CUDAGraph fwd_, bwd_;
+  at::cuda::CUDAGraph fwd_;
+  std::vector<std::unique_ptr<BackwardGraph>> bwd_;
   int64_t n_fwd_ = 0, n_bwd_ = 0;
 };
 
@@ -582,10 +637,8 @@ struct MoEGraphedBackward : public torch::autograd::Node {
     std::lock_guard<std::mutex> lock(mutex_);
     if (!grads[0].defined() && !grads[1].defined()) return variable_list(6);
     at::NoGradGuard no_grad;
-    const Grads g = graphs->backward(grads[0], grads[1]);
-    auto out = [](const Tensor& t) { return t.defined() ? t.detach() : t; };
-    return {out(g.dx), out(g.d_router), out(g.dw_in), out(g.dw_out), out(g.dw_sh_in),
-            out(g.dw_sh_out)};
+    Grads g = graphs->backward(grads[0], grads[1]);
+    return {g.dx, g.d_router, g.dw_in, g.dw_out, g.dw_sh_in, g.dw_sh_out};
   }
 };
 

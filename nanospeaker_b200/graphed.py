@@ -35,14 +35,29 @@ class _BlockWithAux(nn.Module):
         return out, aux, self.block.expert_counts.to(torch.float32)
 
 
+class _OwnGradient(torch.autograd.Function):
+    """The tensor itself, with a gradient of its own: torch's graphed callables hand back their own
+    buffers, autograd takes such a buffer as p.grad without a copy, and the next replay overwrites it."""
+
+    @staticmethod
+    def forward(ctx, t):
+        return t.view_as(t)
+
+    @staticmethod
+    def backward(ctx, grad):
+        return grad.clone()
+
+
 class GraphedMoEBlock(nn.Module):
     """`block(x)` replayed from CUDA graphs, one forward/backward pair per (input shape, dtype,
     training mode), captured on first use. Inputs the kernels decline (CPU tensors, other dtypes,
     exploration noise: anything `block._whole_block_ok` turns down) go through the block itself.
 
     The captured graphs hold the parameters by address: change them in place (an optimizer step
-    does), do not replace them. A capture costs a few warm-up steps; do the first call of every
-    shape outside any timed region."""
+    does), do not replace them. The output, `aux_loss` and what the backward needs lie in the
+    graphs' buffers: the next call of the same shape overwrites them. Gradients do not: any number
+    of micro-steps may add up before they are cleared. A capture costs a few warm-up steps;
+    do the first call of every shape outside any timed region."""
 
     def __init__(self, block: MoEBlock, warmup_iters: int = 3):
         super().__init__()
@@ -95,14 +110,20 @@ class GraphedMoEBlock(nn.Module):
 
     def _callable_for(self, x: torch.Tensor):
         key = (tuple(x.shape), x.dtype, x.device, self.block.training, x.requires_grad)
+        names, params = zip(*self._pair.named_parameters())
         fn = self._graphed.get(key)
         if fn is None:
             sample = torch.zeros_like(x).normal_().requires_grad_(x.requires_grad)
+
+            def step(x, *weights):
+                return torch.func.functional_call(self._pair, dict(zip(names, weights)), (x,))
+            weights = (p.detach().requires_grad_(p.requires_grad) for p in params)
             fn = torch.cuda.make_graphed_callables(
-                self._pair, (sample,), num_warmup_iters=self.warmup_iters,
+                step, (sample, *weights), num_warmup_iters=self.warmup_iters,
                 allow_unused_input=True)
             self._graphed[key] = fn
-        return fn
+        return lambda x: fn(*(_OwnGradient.apply(t) if t.requires_grad else t
+                              for t in (x, *params)))
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         b = self.block

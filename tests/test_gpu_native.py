@@ -105,3 +105,35 @@ def test_native_sublayer_equals_the_python_node(combine, n_shared, T):
         res.append(dict(out=out.detach(), dx=xc.grad, **{n: p.grad for n, p in sub.named_parameters()}))
     for n in res[0]:
         assert rel_l2(res[0][n], res[1][n]) < ATOMIC_TOL, n
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])   # (fp32: torch's graphed callable)
+def test_graphed_gradients_stay_when_the_next_backward_replays(dtype):
+    """Micro-steps that add up without clearing, against the block called directly; then gradients kept
+    by the caller over more steps than the graphs have sets of buffers."""
+    from nanospeaker_b200 import GraphedMoEBlock, kernels
+    T = 200
+    m = _block(False, None, 2, "store").to(dtype)
+    g = GraphedMoEBlock(m)
+    params = list(m.parameters())
+    gouts = [torch.randn(T, 576, device="cuda").bfloat16() for _ in range(5)]
+    xs = [torch.randn(T, 576, device="cuda").bfloat16() for _ in range(5)]
+
+    def grads(call, i):
+        x = xs[i].clone().requires_grad_(True)
+        return torch.autograd.grad([call(x)], [x, *params], [gouts[i]])
+    want = [grads(m, i) for i in range(5)]
+    for _ in range(2):                                   # twice: cleared in between
+        for p in params:
+            p.grad = None
+        total = [torch.zeros_like(p) for p in params]
+        for i in range(4):
+            g(xs[i].clone().requires_grad_(True)).backward(gouts[i])
+            for t, w in zip(total, want[i][1:]):
+                t.add_(w)
+            for p, t in zip(params, total):
+                assert torch.equal(p.grad, t), i
+    kept = [grads(g, i) for i in range(5)]
+    for a, b in zip(kept, want):
+        assert all(torch.equal(u, v) for u, v in zip(a, b))
+    kernels.check_status("cuda")

@@ -529,7 +529,7 @@ class GraphedBlock : public std::enable_shared_from_this<GraphedBlock> {
   GraphedBlock(const Tensor& x, const Tensor& router_w, const OptTensor& logit_bias,
                const Tensor& w_in, const Tensor& w_out, const OptTensor& w_sh_in,
                const OptTensor& w_sh_out, int64_t top_k, bool normalize, bool full_softmax,
-               double aux_coef, int64_t activation, bool store)
+               double aux_coef, int64_t activation, bool store, int64_t warmup_iters)
       : opt_{top_k, activation, 0, normalize, full_softmax, store, false, false, aux_coef} {
     at::NoGradGuard no_grad;
     const c10::cuda::CUDAGuard on(x.device());
@@ -541,13 +541,13 @@ class GraphedBlock : public std::enable_shared_from_this<GraphedBlock> {
     check_operands(p_, opt_);
     grad_out_ = at::zeros_like(p_.x);
     grad_aux_ = at::zeros({1}, p_.x.options().dtype(at::kFloat));
-    // once outside the capture: lazy initialisations, the status word, the side streams
+    // at least once outside the capture: lazy initialisations, the status word, the side streams
     const auto main = c10::cuda::getCurrentCUDAStream();
     const auto side = c10::cuda::getStreamFromPool(false, p_.x.get_device());
     C10_CUDA_CHECK(cudaStreamSynchronize(main.stream()));
     {
       const c10::cuda::CUDAStreamGuard work(side);
-      {
+      for (int64_t i = 0; i < std::max<int64_t>(1, warmup_iters); ++i) {
         Results r = launch_forward(p_, opt_, true);
         launch_backward(p_, opt_, r.kept, grad_out_, grad_aux_);
       }
@@ -735,7 +735,7 @@ PYBIND11_MODULE(_moe_shim, m) {
   m.def("muon_step", &muon_step);
   py::class_<GraphedBlock, std::shared_ptr<GraphedBlock>>(m, "GraphedBlock")
       .def(py::init<const Tensor&, const Tensor&, const OptTensor&, const Tensor&, const Tensor&,
-                    const OptTensor&, const OptTensor&, int64_t, bool, bool, double, int64_t,
-                    bool>())
+                    const OptTensor&, const OptTensor&, int64_t, bool, bool, double, int64_t, bool,
+                    int64_t>())
       .def("run", &GraphedBlock::run);
 }

@@ -56,8 +56,8 @@ class GraphedMoEBlock(nn.Module):
     The captured graphs hold the parameters by address: change them in place (an optimizer step
     does), do not replace them. The output, `aux_loss` and what the backward needs lie in the
     graphs' buffers: the next call of the same shape overwrites them. Gradients do not: any number
-    of micro-steps may add up before they are cleared. A capture costs a few warm-up steps;
-    do the first call of every shape outside any timed region."""
+    of micro-steps may add up before they are cleared. A capture costs `warmup_iters` steps (at least
+    one); do the first call of every shape outside any timed region."""
 
     def __init__(self, block: MoEBlock, warmup_iters: int = 3):
         super().__init__()
@@ -104,7 +104,8 @@ class GraphedMoEBlock(nn.Module):
             g = MK.K.shim().GraphedBlock(
                 torch.randn_like(x2), rw, bias, w_in, w_out, sh_in, sh_out,
                 b.router.top_k, bool(b.router.normalize_weights), b.router.wants_probs(),
-                b.router.aux_loss_coef, MK._act_id(b._kernel_act), not MK._atomic(b.combine_mode))
+                b.router.aux_loss_coef, MK._act_id(b._kernel_act), not MK._atomic(b.combine_mode),
+                self.warmup_iters)
             self._graphed[key] = g
         return g
 

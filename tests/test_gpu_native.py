@@ -137,3 +137,18 @@ def test_graphed_gradients_stay_when_the_next_backward_replays(dtype):
     for a, b in zip(kept, want):
         assert all(torch.equal(u, v) for u, v in zip(a, b))
     kernels.check_status("cuda")
+
+
+def test_graphed_block_runs_the_warm_up_it_is_asked_for():
+    from nanospeaker_b200 import GraphedMoEBlock, kernels
+    m = _block(False, None, 2, "store")
+    x = torch.randn(64, 576, device="cuda").bfloat16().requires_grad_(True)
+    launches = []
+    for n in (1, 4):
+        before = kernels.LAUNCHES
+        g = GraphedMoEBlock(m, warmup_iters=n)
+        g(x)
+        launches.append(kernels.LAUNCHES - before)
+    before = kernels.LAUNCHES
+    g(x).float().sum().backward()
+    assert launches[1] - launches[0] == 3 * (kernels.LAUNCHES - before)

@@ -608,8 +608,8 @@ int moe_b200_block_backward(const moe_b200_block_desc* desc, const void* grad_ou
  * x <- x + block_l(x) for n_layers blocks of one shape on up to 256 tokens (the decode loop of
  * src/model/nanospeaker.py:254-269 without attention and norms): one persistent kernel, launched
  * cooperatively, per-pair rows summed in fp32 in a fixed order (bit-reproducible).
- * moe_b200_stack_supported: 1 where the shape is covered, 0 where the layers are called one by one
- * (moe_b200_block_infer). moe_b200_stack_plan fills layer `layer` of a host buffer of
+ * moe_b200_stack_supported: 1 where the shape is covered and the current device holds the whole grid
+ * at once, 0 where the layers are called one by one (moe_b200_block_infer). moe_b200_stack_plan fills layer `layer` of a host buffer of
  * moe_b200_stack_plan_bytes bytes with the addresses of that layer's tensors (router_w [D, E]
  * unpadded, weights as for moe_b200_block_fwd, all 16-byte aligned); the caller copies the whole
  * buffer to the device once (64-byte aligned) and keeps it as long as the weights stay where they are.

@@ -30,9 +30,7 @@
 #include <math_constants.h>
 #include <stdint.h>
 
-#include <algorithm>
 #include <cstring>
-#include <mutex>
 
 #include "../../include/moe_b200.h"
 #include "act.cuh"
@@ -40,41 +38,12 @@
 #include "pdl.cuh"
 #include "ptx.cuh"
 #include "routing.cuh"
+#include "stack_shape.cuh"
 #include "tma_map.cuh"
 
 namespace moe {
 
-constexpr int ST_H = 128;                  // hidden units per expert
-constexpr int ST_SLICE = 32;               // of them in one work item
-constexpr int ST_SLICES = ST_H / ST_SLICE;
-constexpr int ST_STAGE = 8192;             // ring stage: [gate | up][64 d][32 units] or [2][32 units][64 d]
-constexpr int ST_HALF = ST_STAGE / 2;
-// 16 compute warps: the phases are chains of dependent instructions, so what counts is how few of them a
-// warp has. One more warp issues the TMA loads: a box of 64-byte rows occupies the TMA unit for some
-// 200 cycles, and whoever issues a part's loads stands in that queue for a microsecond. (It leaves a
-// thread 96 registers; a spill would cost more, it finds no room in the L1 beside the shared memory.)
-constexpr int ST_WARPS = 16;
-constexpr int ST_CT = ST_WARPS * 32;       // compute threads
-constexpr int ST_THREADS = ST_CT + 32;
-constexpr int ST_PASS = 16;                // tokens per pass over an item (two mma column tiles)
-constexpr int ST_ACC_LD = 68;              // floats between tokens of the up accumulators
-constexpr int ST_ACC_BYTES = 4 * ST_PASS * ST_ACC_LD * 4;
-constexpr int ST_HID_LD = 40;              // bf16 between tokens of the hidden rows (80 B: no conflicts)
-constexpr int ST_MAX_T = 256;
-constexpr int ST_MAX_ITEMS = 8;            // items of one CTA and layer
-constexpr int ST_MAX_STAGES = 24;
-constexpr int ST_PARTS = 32;               // barriers for the two parts of an item; more than stages
-constexpr int ST_MAX_SLOTS = 4;            // tokens of one CTA
-constexpr int ST_RED_BYTES = 16 * ST_CT;   // token phase: partial sums, then the router's
-static_assert(ST_RED_BYTES <= ST_ACC_BYTES, "they share the accumulators' place");
-// Router weight chunks (four columns of a row; a thread has 23 at 76 experts and d_model 576): the
-// first ST_ROUTER_PRE are held in registers across the hand-over, the next are copied to the row
-// buffer and the accumulators, which are free then, and ST_ROUTER_EXTRA bytes beside them, and
-// ST_ROUTER_LATE more are fetched when the partial rows are in. Chunks loaded at their use cost an L2
-// latency a batch.
-constexpr int ST_ROUTER_PRE = 5, ST_ROUTER_LATE = 10, ST_ROUTER_EXTRA = 8192;
-static_assert(ST_PASS == ST_WARPS, "a warp has one token of a pass");
-static_assert(ST_MAX_ITEMS <= ST_WARPS, "a warp lists one item's tokens");
+static_assert(ST_MAX_GROUPS == MAX_EXPERTS, "the routing kernels take as many");
 
 struct alignas(64) StackLayer {
   CUtensorMap in, out, sh_in, sh_out;
@@ -177,34 +146,6 @@ __device__ __forceinline__ float stack_act(int act, float g) {
 __device__ __forceinline__ int opaque(int v) {
   asm volatile("" : "+r"(v));
   return v;
-}
-
-// Shared memory behind the ring, in order.
-struct StackSmem {
-  int xs, acc, hid, list, xrow, res, tokw, lg, bars, misc, total;
-};
-__host__ __device__ inline StackSmem stack_smem(int T, int D, int n_stages, int extra) {
-  const int dpad = (D + 63) / 64 * 64;
-  StackSmem s;
-  int at = n_stages * ST_STAGE;
-  auto take = [&](int bytes) {
-    const int r = at;
-    at += (bytes + 15) / 16 * 16;
-    return r;
-  };
-  take(extra);                                         // router weight chunks, with xs and acc
-  s.xs = take(ST_PASS * (dpad * 2 + 16));              // token rows of a pass
-  s.acc = take(ST_ACC_BYTES);                          // up accumulators; token phase: partial sums
-  s.hid = take((T + ST_PASS - 1) / ST_PASS * ST_PASS * ST_HID_LD * 2);
-  s.list = take(2 * ST_MAX_ITEMS * T * 2);             // an item's tokens, and their pairs
-  s.xrow = take(dpad * 4);                             // token phase: the row, fp32
-  s.res = take(ST_MAX_SLOTS * D * 2);                  // residual rows of this CTA's tokens
-  s.tokw = take(ST_MAX_SLOTS * 16 * 4);                // their pairs' weights
-  s.lg = take(2 * MAX_EXPERTS * 4);                    // logits, their sort keys
-  s.bars = take(2 * ST_PARTS * 8);
-  s.misc = take(16 + ST_MAX_ITEMS * 4 + ST_MAX_ITEMS * 16);   // flags, token counts, items
-  s.total = at;
-  return s;
 }
 
 // One warp: the k largest of lg[0, E) (value descending, ties to the lowest index; keys[e] is
@@ -714,48 +655,39 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
 }
 
 // ---------------------------------------------------------------------------------- host
-static int stack_grid() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-      n = 148;
+static StackDevice look_at(int device) {
+  StackDevice d;
+  int coop = 0;
+  auto ready = [&](const void* kern) {   // its CTAs per SM, with all the shared memory it may ask for
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_MAX_SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, ST_THREADS, ST_MAX_SMEM) != cudaSuccess)
+      return 0;
+    return n;
+  };
+  if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess)
+    d.blocks_per_sm = std::min(ready(reinterpret_cast<const void*>(stack_kernel<3>)),
+                               ready(reinterpret_cast<const void*>(stack_kernel<8>)));
+  d.cooperative = coop != 0;
+  cudaGetLastError();
+  return d;
+}
+static const StackDevice& stack_device() {
+  static const StackDevice none = {148, 1, true};   // without a device: the shape alone decides
+  static PerDevice<StackDevice> devices;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return none;
   }
-  return n;
+  const StackDevice* d = devices.get(dev, look_at);
+  return d != nullptr ? *d : none;
 }
 
 __global__ void stack_reset_kernel(uint32_t* ctr) {
   pdl_wait();
   if (threadIdx.x < 2) ctr[threadIdx.x] = 0u;
-}
-
-// The shape side of a launch; false: the layer-by-layer path is the one that takes it.
-struct StackShape {
-  int sh_tokens, sh_blocks, n_items, n_stages, router_extra, smem;
-};
-static bool stack_shape(int64_t T, int D, int H, int E, int S, int k, StackShape* o) {
-  if (T < 1 || T > ST_MAX_T || H != ST_H || D < 64 || D % 32 != 0 || D > 1024 || E < 4 ||
-      E % 4 != 0 || S < 0 || E + S > MAX_EXPERTS || k < 1 || k > E || k + S > 16)
-    return false;
-  const int grid = stack_grid();
-  if (T > int64_t(ST_MAX_SLOTS) * grid) return false;
-  // a shared expert sees every token: one pass's worth of them per work item keeps it in the range of
-  // the others, as long as that does not give every CTA more items
-  o->sh_tokens = int(std::min<int64_t>(T, T > 128 ? 2 * ST_PASS : ST_PASS));
-  o->sh_blocks = int((T + o->sh_tokens - 1) / o->sh_tokens);
-  o->n_items = ST_SLICES * (E + S * o->sh_blocks);
-  if (o->n_items > ST_MAX_ITEMS * grid) return false;
-  const int limit = 232448 - 1024, n_in = (D + 63) / 64;
-  for (int extra : {ST_ROUTER_EXTRA, 0}) {
-    const int rest = stack_smem(int(T), D, 0, extra).total;
-    o->router_extra = extra;
-    o->n_stages = std::min((limit - rest) / ST_STAGE, ST_MAX_STAGES);
-    if (limit > rest && o->n_stages >= n_in) break;   // an item's up weights are there at once
-  }
-  if (o->n_stages < n_in) return false;
-  o->smem = stack_smem(int(T), D, o->n_stages, o->router_extra).total + 1024;
-  return true;
 }
 
 struct StackScratch {
@@ -790,7 +722,7 @@ extern "C" {
 int moe_b200_stack_supported(int64_t n_tokens, int32_t d_model, int32_t d_hidden,
                              int32_t n_experts, int32_t n_shared, int32_t top_k) {
   StackShape o;
-  return stack_shape(n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, &o) ? 1 : 0;
+  return stack_shape(stack_device(), n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, &o) ? 1 : 0;
 }
 
 size_t moe_b200_stack_plan_bytes(int32_t n_layers) {
@@ -851,7 +783,8 @@ int moe_b200_stack_infer(const void* plan, int32_t n_layers, const void* x, void
                          void* stream) {
   StackShape o;
   if (n_layers < 1 || activation < 0 || activation > 4) return MOE_B200_ERR_SHAPE;
-  if (!stack_shape(n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, &o))
+  const StackDevice& dev = stack_device();
+  if (!stack_shape(dev, n_tokens, d_model, d_hidden, n_experts, n_shared, top_k, &o))
     return MOE_B200_ERR_UNSUPPORTED;
   if (!plan || !x || !out || !scratch || !status) return MOE_B200_ERR_NULL;
   if ((reinterpret_cast<uintptr_t>(plan) & 63u) != 0 ||
@@ -860,14 +793,6 @@ int moe_b200_stack_infer(const void* plan, int32_t n_layers, const void* x, void
     return MOE_B200_ERR_ALIGN;
   const StackScratch s = stack_scratch(scratch, n_tokens, d_model, n_shared, top_k);
   if (scratch_bytes < s.total) return MOE_B200_ERR_SCRATCH;
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(stack_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-    if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(stack_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-  });
-  if (attr_err != cudaSuccess) return MOE_B200_ERR_CUDA;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   launch_pdl(stack_reset_kernel, dim3(1), dim3(32), 0, st, s.ctr);
   StackArgs a{};
@@ -895,7 +820,7 @@ int moe_b200_stack_infer(const void* plan, int32_t n_layers, const void* x, void
   a.ctr = s.ctr;
   a.status = status;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(unsigned(stack_grid()));
+  cfg.gridDim = dim3(unsigned(dev.grid()));
   cfg.blockDim = dim3(ST_THREADS);
   cfg.dynamicSmemBytes = size_t(o.smem);
   cfg.stream = st;

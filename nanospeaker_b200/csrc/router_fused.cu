@@ -466,12 +466,16 @@ __global__ void __launch_bounds__(RF4_THREADS)
 }
 
 // Whether the four-lane kernel covers a call, and with how many experts per lane (0 = no). Rows are
-// read as 8-byte pieces up to the one with the last expert.
+// read as 8-byte pieces up to the one with the last expert. Every expert of a lane costs about as much
+// whether it exists or not, so a count takes the next larger tier of these; with the balance loss, 16384
+// and 131072 tokens, us: 64 / top 4 6.8 and 30, 76 / top 6 8.8 and 43, 96 / top 8 9.9 and 50 (in the tier
+// of 32: 13.3 and 67), 128 / top 8 12.9 and 63.
 static int rf4_experts_per_lane(const void* logits, int ld, int n_experts, int top_k) {
   if (top_k > RF4_MAX_TOPK || ld % 4 != 0 || ld < (n_experts + 3) / 4 * 4 ||
       (reinterpret_cast<uintptr_t>(logits) & 7u) != 0)
     return 0;
-  return n_experts <= 32 ? 8 : n_experts <= 64 ? 16 : n_experts <= 80 ? 20 : n_experts <= 128 ? 32 : 0;
+  return n_experts <= 32 ? 8 : n_experts <= 64 ? 16 : n_experts <= 80 ? 20 : n_experts <= 96 ? 24
+         : n_experts <= 128 ? 32 : 0;
 }
 
 // A cluster that routes and dispatches alone. 16 blocks (2048 tokens) are past the portable size and
@@ -530,6 +534,7 @@ static void launch_rf4(int epl, int top_k, bool want_colsum, unsigned grid, bool
   if (epl == 8) launch_rf4_epl<8>(top_k, want_colsum, grid, one_cluster, st, sc, args...);
   else if (epl == 16) launch_rf4_epl<16>(top_k, want_colsum, grid, one_cluster, st, sc, args...);
   else if (epl == 20) launch_rf4_epl<20>(top_k, want_colsum, grid, one_cluster, st, sc, args...);
+  else if (epl == 24) launch_rf4_epl<24>(top_k, want_colsum, grid, one_cluster, st, sc, args...);
   else launch_rf4_epl<32>(top_k, want_colsum, grid, one_cluster, st, sc, args...);
 }
 

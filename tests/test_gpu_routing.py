@@ -187,7 +187,8 @@ def test_router_dispatch_equals_router_fused_then_dispatch(T, E, k, S):
 
 
 @pytest.mark.parametrize("E,k,ld", [(8, 8, 8), (32, 1, 32), (33, 2, 36), (64, 3, 64), (76, 6, 76), (80, 5, 128),
-                                    (81, 4, 84), (128, 8, 128), (128, 7, 192)])
+                                    (81, 4, 84), (81, 8, 96), (95, 1, 96), (96, 6, 96), (97, 3, 100),
+                                    (128, 8, 128), (128, 7, 192)])
 def test_router_fused_selection_with_many_ties(E, k, ld):
     """The four-lanes-per-token router at the edges of its experts per lane and list lengths, on logits of
     few distinct values: every place of the selection is decided by the index order."""

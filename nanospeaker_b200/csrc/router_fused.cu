@@ -818,7 +818,13 @@ int moe_b200_router_fused(const void* logits, int32_t ld, const float* bias, con
   const unsigned grid = rf_grid(n_tokens, (full_softmax && colsum) ? 4 : 16);
   const __nv_bfloat16* lg = static_cast<const __nv_bfloat16*>(logits);
   __nv_bfloat16* w = static_cast<__nv_bfloat16*>(w_all);
-  if (const int epl = rf4_experts_per_lane(logits, ld, n_experts, top_k)) {
+  // A token alone has the shorter chain with a warp to itself, as long as there are warps for all: past 96
+  // experts and up to 8192 tokens that wins (128 / top 8 with the balance loss, us: 2048 tokens 5.4
+  // against 12.7 with four lanes, 8192 11.3 against 12.8, 12288 13.5 against 12.8; without it 7.9 against
+  // 8.3 and 11.3 against 8.3). The block's form of this, with the dispatch in it, is the faster one with
+  // four lanes at every size.
+  const bool warp_per_token = n_experts > 96 && n_tokens <= 8192;
+  if (const int epl = warp_per_token ? 0 : rf4_experts_per_lane(logits, ld, n_experts, top_k)) {
     int64_t blocks = (n_tokens + RF4_TOKENS - 1) / RF4_TOKENS;
     if (blocks > 148 * 2) blocks = 148 * 2;
     bool one_cluster = false;

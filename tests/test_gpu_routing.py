@@ -211,6 +211,20 @@ def test_router_fused_selection_with_many_ties(E, k, ld):
     K.check_status("cuda")
 
 
+@pytest.mark.parametrize("E,T", [(96, 300), (97, 300), (128, 8192), (128, 8193)])
+def test_router_fused_on_both_sides_of_the_warp_per_token_rule(E, T):
+    """A warp per token or four lanes: the same selection, weights within a bf16 step."""
+    from nanospeaker_b200 import kernels as K
+    torch.manual_seed(E + T)
+    logits = torch.randn(T, 128, device="cuda").bfloat16()
+    w_all, idx_all, colsum = K.router_fused(logits, None, E, 8, 1, True, True)
+    got = K.router_dispatch(logits, None, E, 8, 1, True, True)        # (four lanes, always)
+    assert torch.equal(got[1], idx_all)
+    assert torch.allclose(got[0].float(), w_all.float(), rtol=2 ** -7, atol=0)
+    assert torch.allclose(got[2], colsum, rtol=1e-5, atol=1e-4)
+    K.check_status("cuda")
+
+
 @pytest.mark.parametrize("T", [128, 257, 1024, 1025, 2048, 2049])
 def test_router_and_dispatch_in_one_cluster(T):
     """The edges of the batches that one cluster routes, plans and scatters (portable size, the largest,

@@ -36,25 +36,35 @@ class StackedMoEDecoder:
             b.eval()
         self._graphs = {}
         self._consts = {}
+        self._padded = {}
         self._plans = {}
 
-    def _fast_args(self, b: MoEBlock, x: torch.Tensor):
-        """Per-block constants of the kernel path (weights are fixed while decoding): the padded
-        router weight and the weights in x.dtype, built on first use. None when the block's
-        kernels decline this input (then the block's own forward runs)."""
+    def _block_args(self, b: MoEBlock, x: torch.Tensor):
+        """Per-block constants of the kernel path (weights are fixed while decoding): the weights in
+        x.dtype and the options, built on first use. None when the block's kernels decline this
+        input (then the block's own forward runs)."""
         if not b._whole_block_ok(x):      # biases, a capacity, ...: the block's own forward
             return None
         key = (id(b), x.dtype, x.device)
         if key not in self._consts:
-            from . import moe_kernel as MK
             cast = lambda t: None if t is None else t.detach().to(x.dtype).contiguous()
             bias = b.router.logit_bias
             self._consts[key] = (
-                MK.pad_router_weight(b.router.W.detach(), x.dtype),
-                None if bias is None else bias.detach().to(torch.float32).contiguous(),
+                cast(b.router.W), None if bias is None else bias.detach().to(torch.float32).contiguous(),
                 cast(b.W_in), cast(b.W_out), cast(b.W_sh_in), cast(b.W_sh_out),
                 b.n_experts, b.router.top_k, bool(b.router.normalize_weights), b._kernel_act)
         return self._consts[key]
+
+    def _fast_args(self, b: MoEBlock, x: torch.Tensor):
+        """The same for the layer-by-layer path, which reads a padded router weight."""
+        args = self._block_args(b, x)
+        if args is None:
+            return None
+        key = (id(b), x.dtype, x.device)
+        if key not in self._padded:
+            from . import moe_kernel as MK
+            self._padded[key] = MK.pad_router_weight(args[0], x.dtype)
+        return (self._padded[key],) + args[1:]
 
     def _stack_plan(self, x: torch.Tensor):
         """(plan, shape arguments) of the one-kernel stack, or None where it does not apply: blocks
@@ -64,18 +74,15 @@ class StackedMoEDecoder:
         key = (x.dtype, x.device)
         if key not in self._plans:
             plan = None
-            args = [self._fast_args(b, x) for b in self.blocks]
+            args = [self._block_args(b, x) for b in self.blocks]
             if all(a is not None for a in args):
                 shapes = {(b.d_model, b.d_hidden, b.n_experts, b.n_shared) + a[7:]
                           for b, a in zip(self.blocks, args)}
                 if len(shapes) == 1:
                     d, h, e, s, k, normalize, act = shapes.pop()
                     if K.stack_supported(1, d, h, e, s, k):
-                        routers = [b.router.W.detach().to(x.dtype).contiguous()
-                                   for b in self.blocks]
-                        plan = (K.stack_plan([(w,) + a[1:6] for w, a in zip(routers, args)], s),
-                                (d, h, e, s, k), (h, e, s, k, normalize, K.KERNEL_ACTIVATIONS[act]),
-                                routers)
+                        plan = (K.stack_plan([a[:6] for a in args], s), (d, h, e, s, k),
+                                (h, e, s, k, normalize, K.KERNEL_ACTIVATIONS[act]))
             self._plans[key] = plan
         plan = self._plans[key]
         if plan is None or x.shape[0] < 1 or not K.stack_supported(x.shape[0], *plan[1]):

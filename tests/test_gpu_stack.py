@@ -151,3 +151,22 @@ def test_stack_runs_all_layers_and_in_a_graph():
         y = torch.randn(T, 576, device="cuda").bfloat16()
         assert torch.equal(stack.step(y), stack.eager(y))
     kernels.check_status("cuda")
+
+
+def test_the_one_kernel_stack_needs_no_padded_router_weights():
+    from nanospeaker_b200 import kernels
+    from nanospeaker_b200.decode import StackedMoEDecoder
+    blocks = _blocks(2)
+    stack = StackedMoEDecoder(blocks)
+    x = torch.randn(3, 576, device="cuda").bfloat16()
+    before = kernels.LAUNCHES
+    assert stack._stack_plan(x) is not None and kernels.LAUNCHES == before
+    want = _layer(blocks[1], _layer(blocks[0], x))              # layer by layer they are made, and kept
+    kept = [stack._fast_args(b, x)[0] for b in blocks]
+    assert all(stack._fast_args(b, x)[0] is w for b, w in zip(blocks, kept))
+    from nanospeaker_b200 import moe_kernel as MK
+    MK._ONE_CALL = False
+    try:
+        assert rel_l2(stack.eager(x), want) < 1e-6
+    finally:
+        MK._ONE_CALL = True

@@ -309,6 +309,17 @@ int moe_b200_up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w
                      int64_t n_tokens, const int32_t* pad_offsets, const void* bias,
                      int32_t* status, void* stream);
 
+/* The same with gathered rows that are also left in slot order in rows_out [rows, d_model], the routed
+ * experts' runs only: what moe_b200_permute up to the first shared run writes, pad rows (zeros)
+ * included. The block's training forward runs this one; the weight-gradient GEMM reads rows_out. */
+int moe_b200_up_gemm_keep(const void* a, int64_t rows, int32_t d_model, const void* w_in,
+                          int32_t n_groups, const void* w_extra, int32_t n_extra, int32_t d_hidden,
+                          const int32_t* expert_ids, const int32_t* n_post_pad,
+                          const int32_t* sorted_ids, int32_t gather_top_k, int64_t n_pairs,
+                          int32_t activation, void* hid, void* raw, const void* a_tokens,
+                          int64_t n_tokens, const int32_t* pad_offsets, const void* bias,
+                          void* rows_out, int32_t* status, void* stream);
+
 /* Down GEMM with the router weight fused: y[row] = (hid[row] @ w_out[e]) * pair_w[sorted_ids[row]]
  * (w_out [n_groups, k_dim, d_model]; weight 1 when pair_w is NULL). With fixed groups hid is
  * [S, rows, k_dim]. Replaces the forward use of _gemm2_kernel
@@ -355,6 +366,18 @@ int moe_b200_dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, c
                              int64_t n_pairs, const void* a1, int32_t activation, void* da1,
                              void* hidw, void* dtw, const void* dout_tokens, int64_t n_tokens,
                              const int32_t* pad_offsets, int32_t* status, void* stream);
+
+/* The same with gathered rows that are also left in slot order in rows_out, as moe_b200_up_gemm_keep
+ * does (the block's backward). */
+int moe_b200_dhidden_glu_bwd_keep(const void* douts, int64_t rows, int32_t d_model, const void* w_out,
+                                  int32_t n_groups, const void* w_extra, int32_t n_extra,
+                                  int32_t d_hidden, const int32_t* expert_ids,
+                                  const int32_t* n_post_pad, const int32_t* sorted_ids,
+                                  int32_t gather_top_k, const void* pair_w, int64_t n_pairs,
+                                  const void* a1, int32_t activation, void* da1, void* hidw, void* dtw,
+                                  const void* dout_tokens, int64_t n_tokens,
+                                  const int32_t* pad_offsets, void* rows_out, int32_t* status,
+                                  void* stream);
 
 /* dX GEMM: ydx[row] = da1[row] @ w_in[e]^T, reading w_in [n_groups, d_model, 2*d_hidden] in place
  * (no transposed copy). With fixed groups da1 and ydx are stacked [S, rows, .]. Replaces the dX use

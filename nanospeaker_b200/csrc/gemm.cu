@@ -373,6 +373,20 @@ int moe_b200_up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w
                  a_tokens, n_tokens, pad_offsets, bias, nullptr, status, stream);
 }
 
+int moe_b200_up_gemm_keep(const void* a, int64_t rows, int32_t d_model, const void* w_in,
+                          int32_t n_groups, const void* w_extra, int32_t n_extra, int32_t d_hidden,
+                          const int32_t* expert_ids, const int32_t* n_post_pad,
+                          const int32_t* sorted_ids, int32_t gather_top_k, int64_t n_pairs,
+                          int32_t activation, void* hid, void* raw, const void* a_tokens,
+                          int64_t n_tokens, const int32_t* pad_offsets, const void* bias,
+                          void* rows_out, int32_t* status, void* stream) {
+  if (!rows_out) return MOE_B200_ERR_NULL;
+  if (gather_top_k < 1) return MOE_B200_ERR_SHAPE;
+  return up_gemm(a, rows, d_model, w_in, n_groups, w_extra, n_extra, d_hidden, expert_ids,
+                 n_post_pad, 0, sorted_ids, gather_top_k, n_pairs, activation, hid, raw, a_tokens,
+                 n_tokens, pad_offsets, bias, rows_out, status, stream);
+}
+
 int moe_b200_down_gemm(const void* hid, int64_t rows, int32_t k_dim, const void* w_out,
                        int32_t n_groups, const void* w_extra, int32_t n_extra, int32_t d_model, const int32_t* expert_ids,
                        const int32_t* n_post_pad, int32_t n_fixed_groups,
@@ -506,6 +520,22 @@ int moe_b200_dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, c
                          n_post_pad, n_fixed_groups, sorted_ids, gather_top_k, pair_w, n_pairs, a1,
                          activation, da1, hidw, dtw, dout_tokens, n_tokens, pad_offsets, nullptr,
                          status, stream);
+}
+
+int moe_b200_dhidden_glu_bwd_keep(const void* douts, int64_t rows, int32_t d_model, const void* w_out,
+                                  int32_t n_groups, const void* w_extra, int32_t n_extra,
+                                  int32_t d_hidden, const int32_t* expert_ids,
+                                  const int32_t* n_post_pad, const int32_t* sorted_ids,
+                                  int32_t gather_top_k, const void* pair_w, int64_t n_pairs,
+                                  const void* a1, int32_t activation, void* da1, void* hidw, void* dtw,
+                                  const void* dout_tokens, int64_t n_tokens,
+                                  const int32_t* pad_offsets, void* rows_out, int32_t* status,
+                                  void* stream) {
+  if (!rows_out) return MOE_B200_ERR_NULL;
+  if (gather_top_k < 1) return MOE_B200_ERR_SHAPE;
+  return dhidden_glu_bwd(douts, rows, d_model, w_out, n_groups, w_extra, n_extra, d_hidden, expert_ids,
+                         n_post_pad, 0, sorted_ids, gather_top_k, pair_w, n_pairs, a1, activation, da1,
+                         hidw, dtw, dout_tokens, n_tokens, pad_offsets, rows_out, status, stream);
 }
 
 int moe_b200_dx_gemm(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in,

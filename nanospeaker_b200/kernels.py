@@ -368,7 +368,7 @@ def copy_cols(src: torch.Tensor, dst_ld: int) -> torch.Tensor:
 
 
 def up_gemm(a, w_in, expert_ids, n_post_pad, n_fixed: int, act: int, want_raw: bool,
-            gather=None, w_extra=None, token_rows=None, bias=None, pad_offsets=None):
+            gather=None, w_extra=None, token_rows=None, bias=None, pad_offsets=None, rows_out=None):
     """a x w_in [G, D, 2H] -> (act(g)*u [rows, H], raw [g|u] [rows, 2H] | None).
     a is slot-ordered [rows, D]; or, with gather=(sorted_ids, top_k), the token-major x [T, D] whose
     rows the kernel gathers itself (rows = len(sorted_ids)). n_fixed = S > 0 applies weight
@@ -378,7 +378,9 @@ def up_gemm(a, w_in, expert_ids, n_post_pad, n_fixed: int, act: int, want_raw: b
     x [T, D] (row = slot - start of the expert's run) instead of from a, whose rows in those runs
     need not have been written.
     pad_offsets (the dispatch's run starts; implied by token_rows): lets the routed schedule run on
-    CTA pairs that share each weight tile."""
+    CTA pairs that share each weight tile.
+    rows_out [rows, D] (with gather): receives the gathered rows of the routed experts' runs in slot
+    order."""
     _need_cuda(a, w_in)
     tok, offs = token_rows if token_rows is not None else (None, pad_offsets)
     d = a.shape[1]
@@ -390,11 +392,18 @@ def up_gemm(a, w_in, expert_ids, n_post_pad, n_fixed: int, act: int, want_raw: b
     h = h2 // 2
     hid = _stack(n_fixed, rows, h, a)
     raw = _stack(n_fixed, rows, h2, a) if want_raw else None
-    _lib.check(_lib.load().moe_b200_up_gemm(
-        a.data_ptr(), rows, d, w_in.data_ptr(), g, xp, xn, h, _lib.ptr(expert_ids),
-        _lib.ptr(n_post_pad), n_fixed, _lib.ptr(sids), top_k, n_pairs, act, hid.data_ptr(), _lib.ptr(raw),
-        _lib.ptr(tok), tok.shape[0] if tok is not None else 0, _lib.ptr(offs), _lib.ptr(bias),
-        status_word(a.device).data_ptr(), _stream(a)), "moe_b200_up_gemm")
+    head = (a.data_ptr(), rows, d, w_in.data_ptr(), g, xp, xn, h, _lib.ptr(expert_ids),
+            _lib.ptr(n_post_pad))
+    body = (_lib.ptr(sids), top_k, n_pairs, act, hid.data_ptr(), _lib.ptr(raw), _lib.ptr(tok),
+            tok.shape[0] if tok is not None else 0, _lib.ptr(offs), _lib.ptr(bias))
+    tail = (status_word(a.device).data_ptr(), _stream(a))
+    if rows_out is not None:
+        assert n_fixed == 0 and rows_out.shape == (rows, d) and rows_out.is_contiguous()
+        _need_cuda(rows_out)
+        _lib.check(_lib.load().moe_b200_up_gemm_keep(*head, *body, rows_out.data_ptr(), *tail),
+                   "moe_b200_up_gemm_keep")
+    else:
+        _lib.check(_lib.load().moe_b200_up_gemm(*head, n_fixed, *body, *tail), "moe_b200_up_gemm")
     _count(1 if rows else 0)
     return hid, raw
 
@@ -490,10 +499,10 @@ def dx_gemm_acc(da1, w_in, expert_ids, n_post_pad, n_fixed: int, sorted_ids, n_p
 
 def dhidden_glu_bwd(douts, w_out, expert_ids, n_post_pad, n_fixed: int, sorted_ids, pair_w,
                     n_pairs: int, a1, act: int, want_dtw: bool, gather_top_k: int = 0,
-                    w_extra=None, token_rows=None, dtw_out=None):
+                    w_extra=None, token_rows=None, dtw_out=None, rows_out=None):
     """-> (da1 [.., rows, 2H], hidw [.., rows, H], dtw [n_pairs] | None). douts is slot-ordered
     [rows, D], or with gather_top_k > 0 the token-major dOut [T, D] gathered through sorted_ids.
-    token_rows=(dout, pad_offsets): as for up_gemm, for the rows of douts."""
+    token_rows=(dout, pad_offsets): as for up_gemm, for the rows of douts; rows_out as there."""
     _need_cuda(douts, w_out, a1)
     tok, offs = token_rows if token_rows is not None else (None, None)
     d = douts.shape[1]
@@ -506,12 +515,20 @@ def dhidden_glu_bwd(douts, w_out, expert_ids, n_post_pad, n_fixed: int, sorted_i
         dtw = dtw_out if dtw_out is not None else torch.empty(n_pairs, dtype=douts.dtype,
                                                               device=douts.device)
     xp, xn = _extra(w_extra)
-    _lib.check(_lib.load().moe_b200_dhidden_glu_bwd(
-        douts.data_ptr(), rows, d, w_out.data_ptr(), g, xp, xn, h, _lib.ptr(expert_ids),
-        _lib.ptr(n_post_pad), n_fixed, _lib.ptr(sorted_ids), gather_top_k, _lib.ptr(pair_w),
-        n_pairs, a1.data_ptr(), act, da1.data_ptr(), hidw.data_ptr(), _lib.ptr(dtw),
-        _lib.ptr(tok), tok.shape[0] if tok is not None else 0, _lib.ptr(offs),
-        status_word(douts.device).data_ptr(), _stream(douts)), "moe_b200_dhidden_glu_bwd")
+    head = (douts.data_ptr(), rows, d, w_out.data_ptr(), g, xp, xn, h, _lib.ptr(expert_ids),
+            _lib.ptr(n_post_pad))
+    body = (_lib.ptr(sorted_ids), gather_top_k, _lib.ptr(pair_w), n_pairs, a1.data_ptr(), act,
+            da1.data_ptr(), hidw.data_ptr(), _lib.ptr(dtw), _lib.ptr(tok),
+            tok.shape[0] if tok is not None else 0, _lib.ptr(offs))
+    tail = (status_word(douts.device).data_ptr(), _stream(douts))
+    if rows_out is not None:
+        assert n_fixed == 0 and rows_out.shape == (rows, d) and rows_out.is_contiguous()
+        _need_cuda(rows_out)
+        _lib.check(_lib.load().moe_b200_dhidden_glu_bwd_keep(*head, *body, rows_out.data_ptr(), *tail),
+                   "moe_b200_dhidden_glu_bwd_keep")
+    else:
+        _lib.check(_lib.load().moe_b200_dhidden_glu_bwd(*head, n_fixed, *body, *tail),
+                   "moe_b200_dhidden_glu_bwd")
     _count(1 if rows else 0)
     return da1, hidw, dtw
 

@@ -91,6 +91,13 @@ def test_arguments_are_validated_before_any_launch(lib):
     assert up(128, 128, 5, 0) == -1     # more fixed groups than weight matrices
     assert up(128, 128, 1, 2) == -1     # gathered A only on the routed schedule
     assert up(128, 128, 1, 0, 2) == -1  # a second weight stack only on the routed schedule
+    upk = lambda topk, rows_out: lib.moe_b200_up_gemm_keep(
+        p, 128, 64, p, 4, p, 0, 128, p, p, p, topk, 8, 0, p, null, null, 0, null, null, rows_out, p, null)
+    dhk = lambda topk, rows_out: lib.moe_b200_dhidden_glu_bwd_keep(
+        p, 128, 64, p, 4, p, 0, 128, p, p, p, topk, p, 8, p, 0, p, p, p, null, 0, null, rows_out, p, null)
+    for keep in (upk, dhk):
+        assert keep(2, null) == -2      # nowhere to leave the rows
+        assert keep(0, p) == -1         # rows to leave, but none gathered
     # the accumulating GEMMs: the token-major accumulator and the slot -> token map are checked too
     dacc = lambda rows, fixed, sid, topk, acc, n_tok=4, n_pairs=8: lib.moe_b200_down_gemm_acc(
         p, rows, 128, p, 4, null, 0, 64, p, p, fixed, sid, p, n_pairs, topk, acc, n_tok, null, p,

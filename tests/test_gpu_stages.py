@@ -313,6 +313,39 @@ def test_shared_experts_read_token_rows_in_place(T, E, S, k, D):
     K().check_status("cuda")
 
 
+@pytest.mark.parametrize("T,E,S,k,D", [(300, 8, 2, 2, 576), (1, 4, 0, 1, 96), (129, 4, 1, 2, 96),
+                                       (2048, 76, 2, 6, 576)])
+def test_gathering_gemms_leave_the_rows_in_slot_order(T, E, S, k, D):
+    """The forms of the up GEMM and of dHidden that the block's training step runs: the outputs of the
+    gathering forms bit for bit, and the rows that the permute up to the first shared run writes."""
+    H, ks = 128, k + S
+    torch.manual_seed(T + S)
+    idx = torch.cat([torch.randn(T, E).topk(k, -1).indices,
+                     torch.arange(E, E + S).expand(T, S)], 1)
+    sids, eids, offs, counts, npp, inv = [t.cuda() for t in O.dispatch(idx, E + S)]
+    g = lambda *shape, s=1.0: (torch.randn(*shape, device="cuda") * s).bfloat16()
+    x, dout = g(T, D), g(T, D)
+    w_in, w_out = g(E, D, 2 * H, s=D ** -0.5), g(E, H, D, s=H ** -0.5)
+    extra_in = dict(w_extra=g(S, D, 2 * H, s=D ** -0.5), token_rows=(x, offs)) if S else {}
+    extra_out = dict(w_extra=g(S, H, D, s=H ** -0.5), token_rows=(dout, offs)) if S else {}
+    tw = torch.rand(T * ks, device="cuda").bfloat16()
+    nl, M, routed = int(npp), T * ks, int(offs[E])
+    rows = [torch.full((sids.numel(), D), float("nan"), device="cuda", dtype=torch.bfloat16)
+            for _ in range(2)]
+    up = lambda **kw: K().up_gemm(x, w_in, eids, npp, 0, 0, True, gather=(sids, ks), **extra_in, **kw)
+    ref, got = up(), up(rows_out=rows[0])
+    dh = lambda **kw: K().dhidden_glu_bwd(dout, w_out, eids, npp, 0, sids, tw, M, ref[1], 0, True,
+                                          gather_top_k=ks, **extra_out, **kw)
+    ref_b, got_b = dh(), dh(rows_out=rows[1])
+    for a, b in zip(ref + ref_b[:2], got + got_b[:2]):
+        assert torch.equal(a[:nl], b[:nl])
+    assert torch.equal(ref_b[2], got_b[2])
+    for src, out in ((x, rows[0]), (dout, rows[1])):
+        assert torch.equal(out[:routed], K().permute(src, ks, sids, offs[E:E + 1])[:routed])
+        assert torch.isnan(out[routed:].float()).all()
+    K().check_status("cuda")
+
+
 @pytest.mark.parametrize("T,E,k,D,skew", CASES)
 def test_accumulating_down_and_dx_gemms_match_store_then_combine(T, E, k, D, skew):
     """The GEMMs that add their rows straight into the token-major result (bf16 atomics) against

@@ -268,11 +268,11 @@ def build_stages(m, x):
         copies = lambda t: [t.clone() for _ in range(3)]
         xr = copies(x)
         gather = (sids, ka)
-        # as in the block op: the permute stops at the first shared run, the shared experts read
-        # their rows from the token-major matrix itself
+        # as in the block op: the shared experts read their rows from the token-major matrix itself
         live = offs[E:E + 1]
         Mr = T * k                                   # routed pairs: the rows the permute copies
         xs = copies(K.permute(x, ka, sids, npp))
+        kept = [torch.empty_like(xs[0]) for _ in range(3)]
         hid0, a1 = K.up_gemm(xs[0], m.W_in, eids, npp, 0, 0, True, w_extra=m.W_sh_in)
         hid = copies(hid0)
         y = copies(K.down_gemm(hid[0], m.W_out, eids, npp, 0, sids, tw, M, w_extra=m.W_sh_out))
@@ -307,19 +307,24 @@ def build_stages(m, x):
              lambda i: K.router_fused(logits_p, bias, E, k, S, True, True)),
             ("dispatch alone (histogram, plan + scatter)", GE, M * 8 * 2 + M * 4 * 3, 0,
              lambda i: K.dispatch(idx_all, Ea)),
+            # the up GEMM gathers its rows from x and leaves the routed ones in slot order for dW_in
+            ("up_gemm+glu (gathers, keeps rows and a1)", TF, 2.0 * M * D * 2 * H, 1,
+             lambda i: K.up_gemm(xr[i % 3], m.W_in, eids, npp, 0, 0, True, gather=gather,
+                                 w_extra=m.W_sh_in, token_rows=(xr[i % 3], offs),
+                                 rows_out=kept[i % 3])),
+            ("up_gemm+glu (gathered rows, inference)", TF, 2.0 * M * D * 2 * H, 0,
+             lambda i: K.up_gemm(xr[i % 3], m.W_in, eids, npp, 0, 0, False, gather=gather,
+                                 w_extra=m.W_sh_in, token_rows=(xr[i % 3], offs))),
+            ("up_gemm+glu (slot-ordered rows, +a1 saved)", TF, 2.0 * M * D * 2 * H, 0,
+             lambda i: K.up_gemm(xs[i % 3], m.W_in, eids, npp, 0, 0, True, w_extra=m.W_sh_in,
+                                 token_rows=(xr[i % 3], offs))),
             # compulsory traffic: x read once (its k + S re-reads hit L2), every slot row written
             ("permute (routed rows; shared experts read x in place)", GE,
-             T * D * 2 + Mr * D * 2 + Mr * 4, 2,
+             T * D * 2 + Mr * D * 2 + Mr * 4, 0,
              lambda i: K.permute(xr[i % 3], ka, sids, live)),
             ("permute, every row (without the shared-row shortcut)", GE,
              T * D * 2 + M * D * 2 + M * 4, 0,
              lambda i: K.permute(xr[i % 3], ka, sids, npp)),
-            ("up_gemm+glu (+a1 saved)", TF, 2.0 * M * D * 2 * H, 1,
-             lambda i: K.up_gemm(xs[i % 3], m.W_in, eids, npp, 0, 0, True, w_extra=m.W_sh_in,
-                                 token_rows=(xr[i % 3], offs))),
-            ("up_gemm+glu (gathered rows, inference)", TF, 2.0 * M * D * 2 * H, 0,
-             lambda i: K.up_gemm(xr[i % 3], m.W_in, eids, npp, 0, 0, False, gather=gather,
-                                 w_extra=m.W_sh_in)),
             # the step's default: the shared experts' rows (token-ordered, weight 1) are summed by a
             # plain-store GEMM that gives the token-major result its first value; the routed
             # experts' rows are then added to it in the down / dX GEMMs' epilogues (bf16 atomics in L2)
@@ -335,14 +340,19 @@ def build_stages(m, x):
                                    w_extra=m.W_sh_out)),
             ("combine (store mode)", GE, M * D * 2 + M * 4 + T * D * 2, 0,
              lambda i: K.combine(y[i % 3], inv, T, ka)),
-            ("balance_loss", GE, E * 8, 1, lambda i: K.balance_loss(colsum, counts, E, T, 1e-2)),
-            ("dhidden+glu_bwd", TF, 2.0 * M * D * H, 1,
+            ("balance_loss (in the block: part of the dispatch)", GE, E * 8, 0, lambda i: K.balance_loss(colsum, counts, E, T, 1e-2)),
+            ("dhidden+glu_bwd (gathers, keeps rows)", TF, 2.0 * M * D * H, 1,
+             lambda i: K.dhidden_glu_bwd(xr[i % 3], m.W_out, eids, npp, 0, sids, tw, M, a1, 0,
+                                         True, gather_top_k=ka, w_extra=m.W_sh_out,
+                                         token_rows=(xr[i % 3], offs), rows_out=kept[i % 3])),
+            ("dhidden+glu_bwd (gathered rows)", TF, 2.0 * M * D * H, 0,
+             lambda i: K.dhidden_glu_bwd(xr[i % 3], m.W_out, eids, npp, 0, sids, tw, M, a1, 0,
+                                         True, gather_top_k=ka, w_extra=m.W_sh_out,
+                                         token_rows=(xr[i % 3], offs))),
+            ("dhidden+glu_bwd (slot-ordered rows)", TF, 2.0 * M * D * H, 0,
              lambda i: K.dhidden_glu_bwd(xs[i % 3], m.W_out, eids, npp, 0, sids, tw, M, a1, 0,
                                          True, w_extra=m.W_sh_out,
                                          token_rows=(xr[i % 3], offs))),
-            ("dhidden+glu_bwd (gathered rows)", TF, 2.0 * M * D * H, 0,
-             lambda i: K.dhidden_glu_bwd(xr[i % 3], m.W_out, eids, npp, 0, sids, tw, M, a1, 0,
-                                         True, gather_top_k=ka, w_extra=m.W_sh_out)),
             ("dx_gemm shared experts (stores; first value of dx)", TF, 2.0 * T * S * 2 * H * D, 1,
              lambda i: K.dx_gemm_sum(da1[i % 3], m.W_sh_in, offs[E:], T, out=acc[i % 3])),
             ("dx_gemm+combine (routed rows, atomic adds into dx)", TF, 2.0 * T * k * 2 * H * D, 1,
@@ -383,20 +393,26 @@ def gemm_stage_bytes(T, ld):
     D, H, k, S = D_MODEL, D_HIDDEN, TOP_K, N_SHARED
     M, G = T * (k + S), N_EXPERTS + S
     w_in, w_out = G * D * 2 * H * 2, G * H * D * 2
+    dh = M * 2 * H * 2 + w_out + M * 3 * H * 2 + M * 2
     return {
         "router GEMM": T * D * 2 + D * ld * 2 + T * ld * 2,
-        "up_gemm+glu (+a1 saved)": M * D * 2 + w_in + M * 3 * H * 2,
+        # (gathering forms: the token-major matrix once; the kept copy has the routed rows)
+        "up_gemm+glu (gathers, keeps": T * D * 2 + w_in + M * 3 * H * 2 + T * k * D * 2,
         "up_gemm+glu (gathered rows, inference)": T * D * 2 + w_in + M * H * 2,
+        "up_gemm+glu (slot-ordered": T * k * D * 2 + T * D * 2 + w_in + M * 3 * H * 2,
         "down_gemm+scale (stores": M * H * 2 + w_out + M * D * 2,
         # atomic variants: no per-pair rows; the token-major result is read and written once in HBM
         "down_gemm+scale+combine": T * k * H * 2 + N_EXPERTS * H * D * 2 + 2 * T * D * 2,
         "dx_gemm+combine": T * k * 2 * H * 2 + N_EXPERTS * D * 2 * H * 2 + 2 * T * D * 2,
         "down_gemm shared experts": T * S * H * 2 + S * H * D * 2 + T * D * 2,
         "dx_gemm shared experts": T * S * 2 * H * 2 + S * D * 2 * H * 2 + T * D * 2,
-        "dhidden+glu_bwd": M * D * 2 + M * 2 * H * 2 + w_out + M * 3 * H * 2 + M * 2,
+        "dhidden+glu_bwd (gathers, keeps": T * D * 2 + dh + T * k * D * 2,
+        "dhidden+glu_bwd (gathered": T * D * 2 + dh,
+        "dhidden+glu_bwd (slot-ordered": T * k * D * 2 + T * D * 2 + dh,
         "dx_gemm (stores": M * 2 * H * 2 + w_in + M * D * 2,
-        "wgrad_in (gemm + reduce)": M * D * 2 + M * 2 * H * 2 + w_in,
-        "wgrad_out (gemm + reduce)": M * H * 2 + M * D * 2 + w_out,
+        # (the shared experts' rows are read from the token-major matrix)
+        "wgrad_in (gemm + reduce)": T * k * D * 2 + T * D * 2 + M * 2 * H * 2 + w_in,
+        "wgrad_out (gemm + reduce)": M * H * 2 + T * k * D * 2 + T * D * 2 + w_out,
     }
 
 

@@ -439,6 +439,10 @@ struct Ns {
     const float inv = 1.f / (sqrtf(ss) + js.eps);
     uint32_t loads = 0;
     bool ok = true;
+    // (a warp gives up as one: the loads from TMEM and the arrives below take all its lanes)
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, js.status)) != 0;
+    };
     auto arrive = [&](uint64_t* bar) {
       fence_proxy_async();
       tc_fence_before();
@@ -450,7 +454,7 @@ struct Ns {
       for (int t = 0; t < nt; ++t)
         if (i == 0 || t >= SLOTS) loads ^= 1u << (t % SLOTS);
       const float s = i == 0 ? inv : 1.f, s2 = s * s;
-      ok = mbar_wait(&bars->acc_full, 0, js.status);
+      ok = wait(&bars->acc_full, 0);
       if (!ok) break;
       tc_fence_after();
 #pragma unroll 1
@@ -459,7 +463,7 @@ struct Ns {
                          poly + uint32_t((c & ~1) + side) * NS_BOX, row, c & 1,
                          [&](float, float g) { return s2 * g; });
       arrive(&bars->conv_done);
-      ok = mbar_wait(&bars->acc_full, 1, js.status);
+      ok = wait(&bars->acc_full, 1);
       if (!ok) break;
       tc_fence_after();
 #pragma unroll 1
@@ -471,8 +475,8 @@ struct Ns {
       for (int j = 0; j < nt; ++j) {
         const int t = nt - 1 - j, v = i * nt + j, sl = t % SLOTS;
         if (j >= SLOTS) loads ^= 1u << sl;
-        ok = mbar_wait(bars->upd_full + (v & 1), uint32_t(v >> 1) & 1u, js.status) &&
-             mbar_wait(bars->full + sl, (loads >> sl & 1u) ^ 1u, js.status);
+        ok = wait(bars->upd_full + (v & 1), uint32_t(v >> 1) & 1u) &&
+             wait(bars->full + sl, (loads >> sl & 1u) ^ 1u);
         if (!ok) break;
         tc_fence_after();
         const int live = min(128, job.length - 128 * t);

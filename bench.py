@@ -47,10 +47,11 @@ N_INPUT_SETS = 8         # x / dOut pairs cycled through so successive steps do 
 METRIC = "MoE-block tokens/s (fwd+bwd)"
 
 # DRAM traffic per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the kernels that have
-# been captured with ncu on this workload; see profiles/ncu_block_kernels_T16384.md and
-# profiles/ncu_dW_in_dHidden_permute_T16384.md.
+# been captured with ncu on this workload; see profiles/ncu_block_kernels_T16384.md.
 NCU_TRAFFIC_BYTES = {"permute (routed rows; shared experts read x in place)": 82.0e6,
-                     "wgrad_in (gemm + reduce)": 243.2e6, "dhidden+glu_bwd": 285.7e6}
+                     "up_gemm+glu (gathers, keeps rows and a1)": 234.7e6,
+                     "dhidden+glu_bwd (gathers, keeps rows)": 312.4e6,
+                     "wgrad_in (gemm + reduce)": 242.6e6, "wgrad_out (gemm + reduce)": 185.7e6}
 # (filled from the ncu summaries under profiles/; a kernel without a capture reports null)
 
 FLOP_PER_TOKEN_FWD_BWD = 10_879_488   # 3 * (routed up 1 769 472 + down 884 736 + shared 884 736 + router 87 552)
@@ -509,8 +510,7 @@ def run_ours(args):
             all_reduce_gradients(params)
 
     # The step has no host sync and no data-dependent shape, so the whole forward+backward is
-    # captured once into a CUDA graph and replayed: the ~60 launches of a step then cost one
-    # submission instead of ~1 ms of Python and launch overhead.
+    # captured once into a CUDA graph and replayed: the launches of a step then cost one submission.
     static_x = dev_x[0].clone().requires_grad_(True)
     static_dout = dev_dout[0].clone()
 
@@ -1243,20 +1243,15 @@ def run_side_workload(args):
         layers, T = 20, 64
         stack = StackedMoEDecoder([make_block(1000 + i) for i in range(layers)])
         xs = [torch.randn(T, D_MODEL, generator=g).bfloat16().to(dev) for _ in range(8)]
-        stack.eager(xs[0])        # (the first step also pads every block's router weight, once)
+        stack.eager(xs[0])        # (the first step also lays out the plan)
         l0 = K.LAUNCHES
         stack.eager(xs[0])
         launches = K.LAUNCHES - l0
         eager_ms = time_loop(lambda i: stack.eager(xs[i % 8]))
         ms = time_loop(lambda i: stack.step(xs[i % 8]))
-        # the same stack with the combine in the down GEMM's epilogue (one launch fewer per block;
-        # bf16 atomics, so not bit-reproducible from run to run: not the decoder's default)
-        stack_atomic = StackedMoEDecoder(stack.blocks, combine="atomic")
-        ms_atomic = time_loop(lambda i: stack_atomic.step(xs[i % 8]))
         line = {"metric": "MoE decode stack latency (20 blocks, forward)", "value": ms,
                 "unit": "ms", "higher_is_better": False, "tokens_per_s": T / (ms / 1e3),
                 "eager_ms": eager_ms, "gpu_launches_per_step": launches,
-                "atomic_combine_ms": ms_atomic,
                 "config": {"workload": "BASELINE config 3: 20 stacked MoE blocks (independent "
                                        "weights), T=64 tokens, bf16, forward, one CUDA graph"}}
     else:

@@ -83,10 +83,13 @@ __global__ void __launch_bounds__(NORM_WARPS * 32)
 
 // dx[t] = rstd * (gamma * dh) - x * rstd^3 / D * <gamma * dh, x>  (+ add[t], the residual branch)
 // dgamma += sum_t dh[t] * x[t] * rstd[t]   (fp32; per-block partial sums in shared memory, then
-// one atomic per block and column). HBM-bound: three rows read, one written. All of a row's loads are
-// in flight before the first is used, and the shared-memory sums are laid out by column / 8 so that a
-// warp's atomics hit different banks (as column * 8 they were 8-way conflicts): 16384 x 576 with a
-// residual 27 -> 18 us behind the block's backward. Blocks per SM: as many as are resident.
+// one atomic per block and column). Three rows read, one written; 16384 x 576 with a residual: 19.5 us
+// alone, 0.59 of the copy rate, 18 behind the block's backward (27 before what follows). All of a row's
+// loads are in flight before the first is used, and the shared-memory sums are laid out by column / 8 so
+// that a warp's atomics hit different banks (as column * 8 they were 8-way conflicts). It is not HBM that
+// bounds it (DRAM 41 % busy) but what a warp does between two rows: 112 registers leave an SM 16 warps,
+// each loads a row, waits and computes in turn (a third of the stalls are those loads, issue slots 54 %
+// busy). Blocks per SM: as many as are resident.
 template <int NCH>
 __global__ void __launch_bounds__(NORM_WARPS * 32)
     rmsnorm_bwd_kernel(const uint4* __restrict__ dh, const uint4* __restrict__ x,

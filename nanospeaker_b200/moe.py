@@ -8,9 +8,10 @@ src/train/metrics.py:84-97) and its checkpoints work unchanged.
 
 Paths, in the order `forward` tries them:
   1. kernel    CUDA + bf16 + a named activation + shapes the tiles cover: router top-k, dispatch,
-               permute, grouped GEMMs, combine and the shared experts all run as the `moe_b200`
-               ops (one whole-block op when there are no biases and no capacity; router +
-               dispatch + experts ops otherwise). No host sync. A missing or
+               grouped GEMMs, combine and the shared experts, all issued by one native call per
+               direction (csrc/shim.cpp). Under tracing or interception the same as `moe_b200` ops
+               (one whole-block op when there are no biases and no capacity; router + dispatch +
+               experts ops otherwise). No host sync. A missing or
                failing library raises; nothing is silently rerouted. An explicit capacity_factor
                (the reference's padded path, src/model/moe.py:225-283) runs on the same kernels:
                the dispatch drops the pairs over capacity instead of padding a batch.
@@ -122,8 +123,8 @@ class MoEBlock(nn.Module):
         return self._kernel_config_ok() and kernel_supported(x)
 
     def _whole_block_ok(self, x: torch.Tensor) -> bool:
-        """Can `forward` hand x to the single whole-block op? It has no bias operands and knows no
-        capacity, so those cases take router + fused_moe_forward."""
+        """Can x go to the forms without biases or a capacity: the whole-block op of traced calls, the
+        graph pair, the decode stack?"""
         return self._use_kernel(x) and self.b_in is None and self.b_sh_in is None
 
     # ---------------------------------------------------------------------------- bookkeeping

@@ -393,6 +393,12 @@ template <typename... T>
 bool any_grad(const T&... t) {
   return at::GradMode::is_enabled() && ((t.defined() && t.requires_grad()) || ...);
 }
+// The nodes here have no forward-mode derivative; an operand's would be dropped without a word.
+template <typename... T>
+void refuse_forward_mode(const T&... t) {
+  TORCH_CHECK_NOT_IMPLEMENTED(!((t.defined() && t._fw_grad(0).defined()) || ...),
+                              "the MoE block does not support forward mode AD");
+}
 template <typename N>
 std::shared_ptr<N> new_node() {
   return std::shared_ptr<N>(new N(), torch::autograd::deleteNode);
@@ -444,6 +450,8 @@ std::tuple<Tensor, Tensor, Tensor, OptTensor> block(
   std::shared_ptr<MoEBlockBackward> node;
   if (any_grad(p.x, p.router_w, p.w_in, p.w_out, p.w_sh_in, p.w_sh_out, p.b_in, p.b_out, p.b_sh_in,
                p.b_sh_out, p.residual)) {
+    refuse_forward_mode(p.x, p.router_w, p.w_in, p.w_out, p.w_sh_in, p.w_sh_out, p.b_in, p.b_out,
+                        p.b_sh_in, p.b_sh_out, p.residual);
     node = new_node<MoEBlockBackward>();
     node->set_next_edges(torch::autograd::collect_next_edges(
         p.x, p.router_w, p.w_in, p.w_out, p.w_sh_in, p.w_sh_out, p.b_in, p.b_out, p.b_sh_in,
@@ -479,6 +487,7 @@ std::tuple<Tensor, Tensor, Tensor> sublayer(
                   aux_coef};
   check_operands(p, o);
   TORCH_CHECK(gamma.dim() == 1 && gamma.size(0) == x.size(1), "gamma: expected [", x.size(1), "]");
+  refuse_forward_mode(x, gamma, p.router_w, p.w_in, p.w_out, p.w_sh_in, p.w_sh_out);
   std::shared_ptr<MoESublayerBackward> node;
   if (any_grad(x, gamma, p.router_w, p.w_in, p.w_out, p.w_sh_in, p.w_sh_out)) {
     node = new_node<MoESublayerBackward>();
@@ -650,6 +659,7 @@ std::tuple<Tensor, Tensor, Tensor> GraphedBlock::run(const Tensor& x_in, const T
                   x_in.device() == p_.x.device(),
               "the graphs were captured for another input shape");
   const Tensor si = w_sh_in.value_or(Tensor()), so = w_sh_out.value_or(Tensor());
+  refuse_forward_mode(x_in, router_w, w_in, w_out, si, so);
   std::shared_ptr<MoEGraphedBackward> node;
   if (any_grad(x_in, router_w, w_in, w_out, si, so)) {
     node = new_node<MoEGraphedBackward>();

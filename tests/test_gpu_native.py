@@ -152,3 +152,15 @@ def test_graphed_block_runs_the_warm_up_it_is_asked_for():
     before = kernels.LAUNCHES
     g(x).float().sum().backward()
     assert launches[1] - launches[0] == 3 * (kernels.LAUNCHES - before)
+
+
+@pytest.mark.parametrize("kind", ["plain", "bias", "capacity", "sublayer", "graphed"])
+def test_forward_mode_is_refused(kind):
+    import torch.autograd.forward_ad as fwad
+    from nanospeaker_b200 import GraphedMoEBlock, MoEFFNSublayer
+    m = _block(kind == "bias", 1.25 if kind == "capacity" else None, 2, "store")
+    call = (MoEFFNSublayer(m).to(torch.bfloat16).cuda() if kind == "sublayer" else
+            GraphedMoEBlock(m) if kind == "graphed" else m)
+    x = torch.randn(16, 576, device="cuda").bfloat16()
+    with fwad.dual_level(), pytest.raises(NotImplementedError, match="forward mode"):
+        call(fwad.make_dual(x, torch.ones_like(x)))

@@ -12,6 +12,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
@@ -330,6 +331,17 @@ Tensor as_grad_aux(const Tensor& g) {
   return g.defined() ? g.to(at::kFloat).reshape({1}) : Tensor();
 }
 
+// What a backward returns. It is made without grad mode, so that under create_graph the gradients would
+// pass for constants; differentiating them again is an error.
+variable_list once(variable_list grads) {
+  if (!at::GradMode::is_enabled()) return grads;
+  for (Tensor& g : grads)
+    if (g.defined()) g = g.detach().set_requires_grad(true);
+  auto error = std::make_shared<torch::autograd::DelayedError>(
+      "the MoE block's backward cannot be differentiated again", int64_t(grads.size()));
+  return (*error)(std::move(grads));
+}
+
 // Edges, in order: x, router_w, w_in, w_out, w_sh_in, w_sh_out, b_in, b_out, b_sh_in, b_sh_out,
 // residual.
 struct MoEBlockBackward : public torch::autograd::Node {
@@ -344,6 +356,11 @@ struct MoEBlockBackward : public torch::autograd::Node {
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     if (!grads[0].defined() && !grads[1].defined()) return variable_list(11);
+    return once(gradients(grads));
+  }
+
+ private:
+  variable_list gradients(const variable_list& grads) {
     const Operands p = saved.unpack();
     const Tensor kept = saved.kept.unpack();
     at::NoGradGuard no_grad;
@@ -368,6 +385,11 @@ struct MoESublayerBackward : public torch::autograd::Node {
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     if (!grads[0].defined() && !grads[1].defined()) return variable_list(7);
+    return once(gradients(grads));
+  }
+
+ private:
+  variable_list gradients(const variable_list& grads) {
     const Operands p = saved.unpack();
     const Tensor kept = saved.kept.unpack();
     const Tensor xx = x.unpack(), gm = gamma.unpack(), rs = rstd.unpack();
@@ -645,9 +667,12 @@ struct MoEGraphedBackward : public torch::autograd::Node {
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     if (!grads[0].defined() && !grads[1].defined()) return variable_list(6);
-    at::NoGradGuard no_grad;
-    Grads g = graphs->backward(grads[0], grads[1]);
-    return {g.dx, g.d_router, g.dw_in, g.dw_out, g.dw_sh_in, g.dw_sh_out};
+    Grads g;
+    {
+      at::NoGradGuard no_grad;
+      g = graphs->backward(grads[0], grads[1]);
+    }
+    return once({g.dx, g.d_router, g.dw_in, g.dw_out, g.dw_sh_in, g.dw_sh_out});
   }
 };
 

@@ -164,3 +164,24 @@ def test_forward_mode_is_refused(kind):
     x = torch.randn(16, 576, device="cuda").bfloat16()
     with fwad.dual_level(), pytest.raises(NotImplementedError, match="forward mode"):
         call(fwad.make_dual(x, torch.ones_like(x)))
+
+
+@pytest.mark.parametrize("kind", ["plain", "bias", "capacity", "sublayer", "graphed"])
+def test_gradients_are_not_differentiated_again(kind):
+    """create_graph gives the same gradients, and an error where they would be differentiated (made without
+    grad mode, they would pass for constants)."""
+    from nanospeaker_b200 import GraphedMoEBlock, MoEFFNSublayer
+    m = _block(kind == "bias", 1.25 if kind == "capacity" else None, 2, "store")
+    call = (MoEFFNSublayer(m).to(torch.bfloat16).cuda() if kind == "sublayer" else
+            GraphedMoEBlock(m) if kind == "graphed" else m)
+    x = torch.randn(16, 576, device="cuda").bfloat16().requires_grad_(True)
+    first = lambda: call(x)[0] if kind == "sublayer" else call(x)
+    params = list(call.parameters())
+    for loss in (lambda o: o.float().sum(), lambda o: o.float().square().sum()):
+        want = torch.autograd.grad(loss(first()), [x, *params], allow_unused=True)
+        got = torch.autograd.grad(loss(first()), [x, *params], create_graph=True, allow_unused=True)
+        assert all((a is None) == (b is None) for a, b in zip(got, want))
+        if kind != "sublayer":      # (there the bf16 sums of the norm's weight come in any order)
+            assert all(torch.equal(a, b) for a, b in zip(got, want) if a is not None)
+        with pytest.raises(RuntimeError, match="differentiated again"):
+            (got[0].float().sum() + x.float().sum()).backward()

@@ -49,8 +49,11 @@ class StackedMoEDecoder:
         if key not in self._consts:
             cast = lambda t: None if t is None else t.detach().to(x.dtype).contiguous()
             bias = b.router.logit_bias
+            router = cast(b.router.W)
+            if router.data_ptr() % 16:    # (a view into a flat buffer, say: the stack reads 16-byte pieces)
+                router = router.clone()
             self._consts[key] = (
-                cast(b.router.W), None if bias is None else bias.detach().to(torch.float32).contiguous(),
+                router, None if bias is None else bias.detach().to(torch.float32).contiguous(),
                 cast(b.W_in), cast(b.W_out), cast(b.W_sh_in), cast(b.W_sh_out),
                 b.n_experts, b.router.top_k, bool(b.router.normalize_weights), b._kernel_act)
         return self._consts[key]

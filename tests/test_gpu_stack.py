@@ -170,3 +170,17 @@ def test_the_one_kernel_stack_needs_no_padded_router_weights():
         assert rel_l2(stack.eager(x), want) < 1e-6
     finally:
         MK._ONE_CALL = True
+
+
+def test_a_router_weight_at_any_address():
+    from nanospeaker_b200.decode import StackedMoEDecoder
+    b, = _blocks(1)
+    x = torch.randn(5, 576, device="cuda").bfloat16()
+    want = StackedMoEDecoder([b]).eager(x)
+    flat = torch.zeros(576 * 76 + 8, device="cuda", dtype=torch.bfloat16)
+    w = flat[3:3 + 576 * 76].view(576, 76)
+    w.copy_(b.router.W.detach())
+    b.router.W = torch.nn.Parameter(w)
+    assert b.router.W.data_ptr() % 16
+    stack = StackedMoEDecoder([b])
+    assert stack._stack_plan(x) is not None and torch.equal(stack.eager(x), want)

@@ -438,10 +438,10 @@ struct Ns {
     for (int k = 0; k < job.parts; ++k) ss += __ldcg(job.sumsq + int64_t(group) * job.parts + k);
     const float inv = 1.f / (sqrtf(ss) + js.eps);
     uint32_t loads = 0;
-    bool ok = true;
-    // (a warp gives up as one: the loads from TMEM and the arrives below take all its lanes)
+    // (nobody leaves after a wait that gave up: the loads from TMEM and the arrives below take all lanes of
+    // a warp. With the status flagged the other waits give up soon, too, and the host sees it.)
     auto wait = [&](uint64_t* bar, uint32_t parity) {
-      return __all_sync(0xffffffffu, mbar_wait(bar, parity, js.status)) != 0;
+      if (!mbar_wait(bar, parity, js.status)) atomicExch(js.status, ST_WAIT_TIMEOUT);
     };
     auto arrive = [&](uint64_t* bar) {
       fence_proxy_async();
@@ -449,13 +449,12 @@ struct Ns {
       __syncwarp();
       if (lane == 0) mbar_arrive(bar);
     };
-    for (int i = 0; i < js.steps && ok; ++i) {
+    for (int i = 0; i < js.steps; ++i) {
       // the parity bits of loads during the Gram pass
       for (int t = 0; t < nt; ++t)
         if (i == 0 || t >= SLOTS) loads ^= 1u << (t % SLOTS);
       const float s = i == 0 ? inv : 1.f, s2 = s * s;
-      ok = wait(&bars->acc_full, 0);
-      if (!ok) break;
+      wait(&bars->acc_full, 0);
       tc_fence_after();
 #pragma unroll 1
       for (int c = 0; c < 2 * BLOCKS; ++c)
@@ -463,8 +462,7 @@ struct Ns {
                          poly + uint32_t((c & ~1) + side) * NS_BOX, row, c & 1,
                          [&](float, float g) { return s2 * g; });
       arrive(&bars->conv_done);
-      ok = wait(&bars->acc_full, 1);
-      if (!ok) break;
+      wait(&bars->acc_full, 1);
       tc_fence_after();
 #pragma unroll 1
       for (int c = 0; c < 2 * BLOCKS; ++c)
@@ -475,9 +473,8 @@ struct Ns {
       for (int j = 0; j < nt; ++j) {
         const int t = nt - 1 - j, v = i * nt + j, sl = t % SLOTS;
         if (j >= SLOTS) loads ^= 1u << sl;
-        ok = wait(bars->upd_full + (v & 1), uint32_t(v >> 1) & 1u) &&
-             wait(bars->full + sl, (loads >> sl & 1u) ^ 1u);
-        if (!ok) break;
+        wait(bars->upd_full + (v & 1), uint32_t(v >> 1) & 1u);
+        wait(bars->full + sl, (loads >> sl & 1u) ^ 1u);
         tc_fence_after();
         const int live = min(128, job.length - 128 * t);
         const uint32_t d = lanes + uint32_t(v & 1) * UPD_COLS;
@@ -495,7 +492,6 @@ struct Ns {
         arrive(bars->upd_done + (v & 1));
       }
     }
-    if (!ok) atomicExch(js.status, ST_WAIT_TIMEOUT);
   }
 };
 

@@ -456,8 +456,13 @@ struct Ns {
       const float s = i == 0 ? inv : 1.f, s2 = s * s;
       wait(&bars->acc_full, 0);
       tc_fence_after();
+      if (!(s2 > 0.f))   // a norm that overflows: the direction is zero, its products may be infinite
 #pragma unroll 1
-      for (int c = 0; c < 2 * BLOCKS; ++c)
+        for (int c = 0; c < 8 * BLOCKS; ++c)
+          st_shared_v4(poly + uint32_t(2 * (c >> 3) + side) * NS_BOX + uint32_t(row) * 128u + (c & 7) * 16,
+                       0u, 0u, 0u, 0u);
+#pragma unroll 1
+      for (int c = s2 > 0.f ? 0 : 2 * BLOCKS; c < 2 * BLOCKS; ++c)
         convert32<false>(lanes + uint32_t(c >> 1) * 128u + uint32_t(side) * 64u + uint32_t(c & 1) * 32u,
                          poly + uint32_t((c & ~1) + side) * NS_BOX, row, c & 1,
                          [&](float, float g) { return s2 * g; });

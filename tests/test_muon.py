@@ -119,3 +119,42 @@ def test_native_muon_step_equals_the_operations_one_by_one(dtype):
             q.data.copy_(p.data)
         assert abs(oa.update_norm_ratio() / ob.update_norm_ratio() - 1) < 2e-2
     kernels.check_status("cuda")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [0.0, 1e-30, 1e25, float("inf"), float("nan")])
+def test_native_muon_step_with_extreme_gradients(value):
+    """Directions whose norm vanishes, overflows or is no number, beside ordinary ones, against the step in
+    torch operations: where that leaves numbers the same numbers, where it leaves none, none."""
+    from nanospeaker_b200 import kernels, muon as MU
+    torch.manual_seed(4)
+    shapes = [(3, 576, 256), (3, 128, 576)]
+    res = []
+    start = [(torch.randn(*s) * 0.05).bfloat16().cuda() for s in shapes]
+    grads = [torch.randn_like(p) for p in start]
+    finite = value == value and abs(value) != float("inf")
+    for g in grads:
+        if finite:
+            g[1].sign_().mul_(value)
+        else:
+            g[1, 5, 7] = value
+    for native in (True, False):
+        params = [torch.nn.Parameter(p.clone()) for p in start]
+        opt = MU.Muon(params, lr=0.02)
+        for p, g in zip(params, grads):
+            p.grad = g.clone()
+        keep = MU._native_ok
+        if not native:
+            MU._native_ok = lambda p, buf: False
+        try:
+            opt.step()
+        finally:
+            MU._native_ok = keep
+        res.append([p.detach() for p in params])
+    for a, b in zip(*res):
+        assert torch.equal(torch.isfinite(a), torch.isfinite(b))
+        assert bool(torch.isfinite(b[1]).all()) == finite
+        if finite:
+            assert rel_l2(a[1], b[1]) < 2e-3
+        assert rel_l2(a[[0, 2]], b[[0, 2]]) < 2e-3
+    kernels.check_status("cuda")

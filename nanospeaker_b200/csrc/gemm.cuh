@@ -130,38 +130,47 @@ __device__ __forceinline__ void ld_global_nc_v8(const void* p, uint32_t* w) {
                : "l"(p));
 }
 
-// 32 fp32 -> 32 bf16 = 64 bytes, stored as two 32-byte vectors (dst 32-byte aligned).
-__device__ __forceinline__ void store_bf16x32(__nv_bfloat16* dst, const float* v) {
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    uint32_t w[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      __nv_bfloat162 h = __floats2bfloat162_rn(v[q * 16 + 2 * i], v[q * 16 + 2 * i + 1]);
-      w[i] = *reinterpret_cast<uint32_t*>(&h);
-    }
-    st_global_v8(dst + q * 16, w);
-  }
+// Where a lane's stores of a pair of rows go: lanes 2i and 2i + 1 own rows r and r + 1, and both write
+// both of them, the even lane the first 32 bytes of every 64, the odd lane the second.
+struct RowPair {
+  __nv_bfloat16 *even, *odd;   // 32-byte aligned; null: not stored
+};
+__device__ __forceinline__ RowPair row_pair(__nv_bfloat16* row, int64_t ld, bool row_ok) {
+  const bool odd = threadIdx.x & 1;
+  const bool other_ok = __shfl_xor_sync(0xffffffffu, row_ok, 1);
+  RowPair r;
+  r.even = (odd ? other_ok : row_ok) ? row - (odd ? ld - 16 : 0) : nullptr;
+  r.odd = (odd ? row_ok : other_ok) ? row + (odd ? 16 : ld) : nullptr;
+  return r;
 }
-__device__ __forceinline__ void load_bf16x32(const __nv_bfloat16* src, float* v) {
+// This lane's 32 fp32 -> 32 bf16 = 64 bytes at column `col` of its row of the pair. An instruction covers
+// 64 bytes of 16 rows: with a row's 32 bytes per lane a store touches 32 lines and an SM's load/store
+// unit writes 32 GB/s, with 16 lines 50 (7.3 TB/s over the chip); the price is eight shuffles.
+__device__ __forceinline__ void store_bf16x32(const RowPair& r, int col, const float* v) {
+  const bool odd = threadIdx.x & 1;
+  uint32_t w[16], x[8];
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    uint32_t w[8];
-    ld_global_nc_v8(src + q * 16, w);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      __nv_bfloat162 h = *reinterpret_cast<__nv_bfloat162*>(&w[i]);
-      float2 f = __bfloat1622float2(h);
-      v[q * 16 + 2 * i] = f.x;
-      v[q * 16 + 2 * i + 1] = f.y;
-    }
+  for (int i = 0; i < 16; ++i) {
+    __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    w[i] = *reinterpret_cast<uint32_t*>(&h);
   }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) x[i] = __shfl_xor_sync(0xffffffffu, odd ? w[i] : w[8 + i], 1);
+  uint32_t a[8], b[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    a[i] = odd ? x[i] : w[i];
+    b[i] = odd ? w[8 + i] : x[i];
+  }
+  if (r.even != nullptr) st_global_v8(r.even + col, a);
+  if (r.odd != nullptr) st_global_v8(r.odd + col, b);
 }
-// 32 fp32 stored as four 32-byte vectors (dst 32-byte aligned).
-__device__ __forceinline__ void store_f32x32(float* dst, const float* v) {
+// A row's 32 fp32 of a partial tile's column chunk, laid out [8 columns][row][8]: a warp's store is
+// 1 KB in one piece.
+__device__ __forceinline__ void store_partial32(float* chunk, int row, const float* v) {
 #pragma unroll
   for (int q = 0; q < 4; ++q)
-    st_global_v8(dst + q * 8, reinterpret_cast<const uint32_t*>(v) + q * 8);
+    st_global_v8(chunk + (q * BM + row) * 8, reinterpret_cast<const uint32_t*>(v) + q * 8);
 }
 
 __device__ __forceinline__ void epi_bar_sync(int nthreads) {

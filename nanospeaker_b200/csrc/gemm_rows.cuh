@@ -110,10 +110,10 @@ __device__ __forceinline__ void add_bias32(float* v, const __nv_bfloat16* bias) 
 }
 
 template <int ACT, int BN>
-__device__ __forceinline__ void epilogue_glu(uint32_t taddr, int c_lo, int c_hi, bool row_ok,
-                                             __nv_bfloat16* out_row, __nv_bfloat16* raw_row,
-                                             const __nv_bfloat16* bias) {
+__device__ __forceinline__ void epilogue_glu(uint32_t taddr, int c_lo, int c_hi, const RowPair& out,
+                                             const RowPair& raw, const __nv_bfloat16* bias) {
   constexpr int HALF = BN / 2;  // gate = accumulator cols [0, HALF), up = [HALF, BN)
+  const bool keep_raw = __any_sync(0xffffffffu, raw.even != nullptr || raw.odd != nullptr);
 #pragma unroll 1
   for (int c = c_lo; c < c_hi; ++c) {
     float g[32], u[32];
@@ -124,13 +124,13 @@ __device__ __forceinline__ void epilogue_glu(uint32_t taddr, int c_lo, int c_hi,
       add_bias32(g, bias + c * 32);
       add_bias32(u, bias + HALF + c * 32);
     }
-    if (raw_row != nullptr && row_ok) {
-      store_bf16x32(raw_row + c * 32, g);
-      store_bf16x32(raw_row + HALF + c * 32, u);
+    if (keep_raw) {
+      store_bf16x32(raw, c * 32, g);
+      store_bf16x32(raw, HALF + c * 32, u);
     }
 #pragma unroll
     for (int i = 0; i < 32; ++i) g[i] = act_f<ACT>(g[i]) * u[i];
-    if (row_ok) store_bf16x32(out_row + c * 32, g);
+    store_bf16x32(out, c * 32, g);
   }
 }
 
@@ -155,9 +155,9 @@ __device__ __forceinline__ void load_tile_bf16x32(uint32_t tile, int row, int co
 // acc = G = dOut @ W_out^T for this row; a1_tile = the tile's [gate | up] pre-activations in shared
 // memory; H = BN. Returns this thread's share of <G, hidden>.
 template <int ACT, int BN>
-__device__ __forceinline__ float epilogue_glubwd(uint32_t taddr, int c_lo, int c_hi, bool row_ok,
-                                                 float w, uint32_t a1_tile, int row,
-                                                 __nv_bfloat16* da1, __nv_bfloat16* hw) {
+__device__ __forceinline__ float epilogue_glubwd(uint32_t taddr, int c_lo, int c_hi, float w,
+                                                 uint32_t a1_tile, int row, const RowPair& da1,
+                                                 const RowPair& hw) {
   float part = 0.f;
 #pragma unroll 1
   for (int c = c_lo; c < c_hi; ++c) {
@@ -177,11 +177,9 @@ __device__ __forceinline__ float epilogue_glubwd(uint32_t taddr, int c_lo, int c
       u[i] = dh * a;         // d up
       G[i] = w * hid;        // weighted hidden, the A operand of dW_out
     }
-    if (row_ok) {
-      store_bf16x32(da1 + c * 32, g);
-      store_bf16x32(da1 + BN + c * 32, u);
-      store_bf16x32(hw + c * 32, G);
-    }
+    store_bf16x32(da1, c * 32, g);
+    store_bf16x32(da1, BN + c * 32, u);
+    store_bf16x32(hw, c * 32, G);
   }
   return part;
 }
@@ -603,14 +601,15 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
         }
       }
       if constexpr (EPI == EPI_GLU) {
-        __nv_bfloat16* raw_row =
-            p.out2 ? p.out2 + tc.z * p.out2_gstride + grow * BN : nullptr;
+        const RowPair out = row_pair(out_row, p.ld_out, row_ok);
+        const RowPair raw = row_pair(p.out2 + tc.z * p.out2_gstride + grow * BN, BN,
+                                     row_ok && p.out2 != nullptr);
         switch (p.act) {
-          case ACT_SILU: epilogue_glu<ACT_SILU, BN>(taddr, c_lo, c_hi, row_ok, out_row, raw_row, bias_row); break;
-          case ACT_GELU: epilogue_glu<ACT_GELU, BN>(taddr, c_lo, c_hi, row_ok, out_row, raw_row, bias_row); break;
-          case ACT_RELU: epilogue_glu<ACT_RELU, BN>(taddr, c_lo, c_hi, row_ok, out_row, raw_row, bias_row); break;
-          case ACT_SIGMOID: epilogue_glu<ACT_SIGMOID, BN>(taddr, c_lo, c_hi, row_ok, out_row, raw_row, bias_row); break;
-          default: epilogue_glu<ACT_TANH, BN>(taddr, c_lo, c_hi, row_ok, out_row, raw_row, bias_row); break;
+          case ACT_SILU: epilogue_glu<ACT_SILU, BN>(taddr, c_lo, c_hi, out, raw, bias_row); break;
+          case ACT_GELU: epilogue_glu<ACT_GELU, BN>(taddr, c_lo, c_hi, out, raw, bias_row); break;
+          case ACT_RELU: epilogue_glu<ACT_RELU, BN>(taddr, c_lo, c_hi, out, raw, bias_row); break;
+          case ACT_SIGMOID: epilogue_glu<ACT_SIGMOID, BN>(taddr, c_lo, c_hi, out, raw, bias_row); break;
+          default: epilogue_glu<ACT_TANH, BN>(taddr, c_lo, c_hi, out, raw, bias_row); break;
         }
       } else if constexpr (EPI == EPI_RAW || EPI == EPI_SCALE) {
         // The tile leaves as 64-column boxes: the eight warps fill one box in shared memory (warp
@@ -706,8 +705,8 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(afull_bar + b);   // (release: the staged rows are visible)
       } else {  // EPI_GLUBWD
-        __nv_bfloat16* da1 = out_row;  // ld_out == 2 * BN
-        __nv_bfloat16* hw = p.out2 + tc.z * p.out2_gstride + grow * BN;
+        const RowPair da1 = row_pair(out_row, 2 * BN, row_ok);   // ld_out == 2 * BN
+        const RowPair hw = row_pair(p.out2 + tc.z * p.out2_gstride + grow * BN, BN, row_ok);
         // this tile's pre-activations were brought in by the aux warp
         const int ab = j % L::AUX_BUFS;
         if (!mbar_wait(afull_bar + ab, (uint32_t(j) / L::AUX_BUFS) & 1, p.status))
@@ -715,11 +714,11 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
         const uint32_t a1_tile = smem_u32(smem + L::AUX_OFFSET + ab * L::AUX_TILE_BYTES);
         float part;
         switch (p.act) {
-          case ACT_SILU: part = epilogue_glubwd<ACT_SILU, BN>(taddr, c_lo, c_hi, row_ok, w, a1_tile, row, da1, hw); break;
-          case ACT_GELU: part = epilogue_glubwd<ACT_GELU, BN>(taddr, c_lo, c_hi, row_ok, w, a1_tile, row, da1, hw); break;
-          case ACT_RELU: part = epilogue_glubwd<ACT_RELU, BN>(taddr, c_lo, c_hi, row_ok, w, a1_tile, row, da1, hw); break;
-          case ACT_SIGMOID: part = epilogue_glubwd<ACT_SIGMOID, BN>(taddr, c_lo, c_hi, row_ok, w, a1_tile, row, da1, hw); break;
-          default: part = epilogue_glubwd<ACT_TANH, BN>(taddr, c_lo, c_hi, row_ok, w, a1_tile, row, da1, hw); break;
+          case ACT_SILU: part = epilogue_glubwd<ACT_SILU, BN>(taddr, c_lo, c_hi, w, a1_tile, row, da1, hw); break;
+          case ACT_GELU: part = epilogue_glubwd<ACT_GELU, BN>(taddr, c_lo, c_hi, w, a1_tile, row, da1, hw); break;
+          case ACT_RELU: part = epilogue_glubwd<ACT_RELU, BN>(taddr, c_lo, c_hi, w, a1_tile, row, da1, hw); break;
+          case ACT_SIGMOID: part = epilogue_glubwd<ACT_SIGMOID, BN>(taddr, c_lo, c_hi, w, a1_tile, row, da1, hw); break;
+          default: part = epilogue_glubwd<ACT_TANH, BN>(taddr, c_lo, c_hi, w, a1_tile, row, da1, hw); break;
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(aempty_bar + ab);  // this warp is done with the tile's buffer

@@ -428,13 +428,14 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
         if (p.bias != nullptr) bias_row = p.bias + int64_t(tc.group) * p.n_dim;
       }
       if constexpr (EPI == EPI_GLU) {
-        __nv_bfloat16* raw_row = p.out2 ? p.out2 + grow * BN : nullptr;
+        const RowPair out = row_pair(out_row, p.ld_out, row_ok);
+        const RowPair raw = row_pair(p.out2 + grow * BN, BN, row_ok && p.out2 != nullptr);
         switch (p.act) {
-          case ACT_SILU: epilogue_glu<ACT_SILU, BN>(taddr, c_lo, c_hi, row_ok, out_row, raw_row, bias_row); break;
-          case ACT_GELU: epilogue_glu<ACT_GELU, BN>(taddr, c_lo, c_hi, row_ok, out_row, raw_row, bias_row); break;
-          case ACT_RELU: epilogue_glu<ACT_RELU, BN>(taddr, c_lo, c_hi, row_ok, out_row, raw_row, bias_row); break;
-          case ACT_SIGMOID: epilogue_glu<ACT_SIGMOID, BN>(taddr, c_lo, c_hi, row_ok, out_row, raw_row, bias_row); break;
-          default: epilogue_glu<ACT_TANH, BN>(taddr, c_lo, c_hi, row_ok, out_row, raw_row, bias_row); break;
+          case ACT_SILU: epilogue_glu<ACT_SILU, BN>(taddr, c_lo, c_hi, out, raw, bias_row); break;
+          case ACT_GELU: epilogue_glu<ACT_GELU, BN>(taddr, c_lo, c_hi, out, raw, bias_row); break;
+          case ACT_RELU: epilogue_glu<ACT_RELU, BN>(taddr, c_lo, c_hi, out, raw, bias_row); break;
+          case ACT_SIGMOID: epilogue_glu<ACT_SIGMOID, BN>(taddr, c_lo, c_hi, out, raw, bias_row); break;
+          default: epilogue_glu<ACT_TANH, BN>(taddr, c_lo, c_hi, out, raw, bias_row); break;
         }
       } else if constexpr (EPI == EPI_RAW_RED || EPI == EPI_SCALE_RED) {
         constexpr int NB = BN / 64;
@@ -473,18 +474,18 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(afull_bar + b);
       } else {  // EPI_GLUBWD
-        __nv_bfloat16* da1 = out_row;  // ld_out == 2 * BN
-        __nv_bfloat16* hw = p.out2 + grow * BN;
+        const RowPair da1 = row_pair(out_row, 2 * BN, row_ok);   // ld_out == 2 * BN
+        const RowPair hw = row_pair(p.out2 + grow * BN, BN, row_ok);
         if (!mbar_wait(afull_bar + b, (uint32_t(j) >> 1) & 1, p.status))
           atomicExch(p.status, ST_WAIT_TIMEOUT);
         const uint32_t a1_tile = smem_u32(smem + L::AUX_OFFSET + b * L::AUX_TILE_BYTES);
         float part;
         switch (p.act) {
-          case ACT_SILU: part = epilogue_glubwd<ACT_SILU, BN>(taddr, c_lo, c_hi, row_ok, w, a1_tile, row, da1, hw); break;
-          case ACT_GELU: part = epilogue_glubwd<ACT_GELU, BN>(taddr, c_lo, c_hi, row_ok, w, a1_tile, row, da1, hw); break;
-          case ACT_RELU: part = epilogue_glubwd<ACT_RELU, BN>(taddr, c_lo, c_hi, row_ok, w, a1_tile, row, da1, hw); break;
-          case ACT_SIGMOID: part = epilogue_glubwd<ACT_SIGMOID, BN>(taddr, c_lo, c_hi, row_ok, w, a1_tile, row, da1, hw); break;
-          default: part = epilogue_glubwd<ACT_TANH, BN>(taddr, c_lo, c_hi, row_ok, w, a1_tile, row, da1, hw); break;
+          case ACT_SILU: part = epilogue_glubwd<ACT_SILU, BN>(taddr, c_lo, c_hi, w, a1_tile, row, da1, hw); break;
+          case ACT_GELU: part = epilogue_glubwd<ACT_GELU, BN>(taddr, c_lo, c_hi, w, a1_tile, row, da1, hw); break;
+          case ACT_RELU: part = epilogue_glubwd<ACT_RELU, BN>(taddr, c_lo, c_hi, w, a1_tile, row, da1, hw); break;
+          case ACT_SIGMOID: part = epilogue_glubwd<ACT_SIGMOID, BN>(taddr, c_lo, c_hi, w, a1_tile, row, da1, hw); break;
+          default: part = epilogue_glubwd<ACT_TANH, BN>(taddr, c_lo, c_hi, w, a1_tile, row, da1, hw); break;
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(aempty_bar + b);

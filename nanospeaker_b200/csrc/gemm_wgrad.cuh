@@ -370,6 +370,7 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
                                                : p.out_extra + int64_t(w.group - p.n_out1) *
                                                                    p.m_dim * p.n_dim) +
                            int64_t(m) * p.n_dim + n0;
+      const RowPair rows = row_pair(dst, p.n_dim, m_ok);
       float* mine = p.partials + (int64_t(j) * tiles_xy + txy) * (int64_t(BM) * BN);
 #pragma unroll 1
       for (int c = c_lo; c < c_hi; ++c) {
@@ -382,9 +383,9 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
           for (int i = 0; i < 32; ++i) v[i] = 0.f;
         }
         if (w.n_c == 1) {
-          if (m_ok && n0 + c * 32 < p.n_dim) store_bf16x32(dst + c * 32, v);
+          if (n0 + c * 32 < p.n_dim) store_bf16x32(rows, c * 32, v);
         } else {
-          store_f32x32(mine + (int64_t(c) * BM + row) * 32, v);  // [column chunk][row][32]
+          store_partial32(mine + int64_t(c) * (BM * 32), row, v);
         }
       }
       if (have_acc) {
@@ -460,9 +461,9 @@ __global__ void __launch_bounds__(256)
         const float4 v = __ldcs(src + c2 * stride4);
         acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
       }
-      // partial layout [column chunk][row][32 floats]
-      const int cc = f / (BM * 8), row = (f / 8) % BM, i4 = f % 8;
-      const int m = tile_m * BM + row, n = n0 + cc * 32 + i4 * 4;
+      // partial layout [8 columns][row][8]: a float4 is half of a row's 8
+      const int c8 = f / (BM * 2), row = (f / 2) % BM, i4 = f % 2;
+      const int m = tile_m * BM + row, n = n0 + c8 * 8 + i4 * 4;
       if (p.out_cols != p.n_dim) {   // one group, narrower rows of any alignment
         if (m < p.m_dim) {
           __nv_bfloat16* dst = p.out + int64_t(m) * p.out_cols + n;

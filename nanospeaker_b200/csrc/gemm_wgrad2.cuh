@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(WGRAD_THREADS, 1)
                                                : p.out_extra + int64_t(w.group - p.n_out1) *
                                                                    p.m_dim * p.n_dim) +
                            int64_t(m) * p.n_dim + n0;
+      const RowPair rows = row_pair(dst, p.n_dim, m_ok);
       const int txy = tile_m * tiles_y + (uxy % tiles_y);
       float* mine = p.partials + (int64_t(j) * tiles_xy + txy) * (int64_t(BM) * BN);
       if (tile_ok) {
@@ -239,9 +240,9 @@ __global__ void __launch_bounds__(WGRAD_THREADS, 1)
             for (int i = 0; i < 32; ++i) v[i] = 0.f;
           }
           if (w.n_c == 1) {
-            if (m_ok && n0 + c * 32 < p.n_dim) store_bf16x32(dst + c * 32, v);
+            if (n0 + c * 32 < p.n_dim) store_bf16x32(rows, c * 32, v);
           } else {
-            store_f32x32(mine + (int64_t(c) * BM + row) * 32, v);
+            store_partial32(mine + int64_t(c) * (BM * 32), row, v);
           }
         }
       }

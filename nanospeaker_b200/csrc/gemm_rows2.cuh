@@ -97,7 +97,7 @@ __device__ __forceinline__ void tma_load_4d_2cta(void* dst, const CUtensorMap* m
       : "memory");
 }
 
-constexpr int ROWS2_MAX_GROUPS = 256;
+constexpr int ROWS2_MAX_GROUPS = WGRAD_MAX_GROUPS;
 
 template <int BN, int STAGES, int EPI>
 struct Rows2Smem {
@@ -114,7 +114,8 @@ struct Rows2Smem {
   static constexpr int PART_OFFSET = MISC_OFFSET + 16;
   static constexpr int RED_TOK_OFFSET = PART_OFFSET + 128 * 4;
   static constexpr int TABLE_OFFSET = RED_TOK_OFFSET + 2 * 128 * 4;   // pair_first, run_start
-  static constexpr int TOTAL = TABLE_OFFSET + 2 * (ROWS2_MAX_GROUPS + 1) * 4;
+  static constexpr int WALK_OFFSET = TABLE_OFFSET + 2 * (ROWS2_MAX_GROUPS + 1) * 4;   // the first unit
+  static constexpr int TOTAL = WALK_OFFSET + 32;
   static constexpr int DYNAMIC = TOTAL + 1024;
   static_assert(STAGE_BYTES % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
 };
@@ -124,15 +125,23 @@ struct Unit2 {
   bool valid;   // false: this CTA's half of the pair is past the end of the run
 };
 
+// Threads in the launch bound, for the registers it leaves a thread. dX is held to 96: its four warps per
+// scheduler at 114 leave no room for two warps of the router's weight gradient sums, which run beside it on
+// another stream and then came after it (training step of 16384 tokens + 15 us, 2048 graphed + 7).
+__host__ __device__ constexpr int rows2_bound(int epi) {
+  return epi == EPI_RAW_RED ? 672 : rows_threads(epi, GATHER_NO);
+}
+
 template <int BN, int STAGES, bool B_MN, int EPI>
-__global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
+__global__ void __launch_bounds__(rows2_bound(EPI), 1)
     rows_gemm2_kernel(const __grid_constant__ CUtensorMap tmA,
                       const __grid_constant__ CUtensorMap tmA2,
                       const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmB2,
                       const __grid_constant__ CUtensorMap tmOut, const RowsArgs p) {
+  // (the prologue up to the wait touches nothing an earlier kernel wrote: barriers, TMEM and the
+  // pair's meeting take 1.8 us)
   pdl_trigger();
-  pdl_wait();
   using L = Rows2Smem<BN, STAGES, EPI>;
   static_assert(BN % 32 == 0 && BN <= 256, "BN must be a multiple of 32 up to 256");
   static_assert(!B_MN || BN % 128 == 0, "an MN-major weight half must be whole 64-column boxes");
@@ -163,35 +172,6 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
   const int cluster = int(blockIdx.x) >> 1;
   const int n_groups = p.n_groups_total;
 
-  // ------------------------------------------------------------------------- pair table
-  // pair_first[g] = number of block pairs of the runs before g (a run of t blocks has ceil(t / 2))
-  if (warp == 2) {
-    int running = 0;
-    for (int base = 0; base < n_groups; base += 32) {
-      const int g = base + lane;
-      int lo = 0, hi = 0;
-      if (g < n_groups) {
-        lo = __ldg(p.a2_offsets + g);
-        hi = __ldg(p.a2_offsets + g + 1);
-      }
-      const int mine = (((hi - lo) >> 7) + 1) >> 1;
-      int incl = mine;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      if (g < n_groups) {
-        pair_first[g] = running + incl - mine;
-        run_start[g] = lo;
-      }
-      running += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) {
-      pair_first[n_groups] = running;
-      run_start[n_groups] = __ldg(p.a2_offsets + n_groups);
-    }
-  }
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmA2);
@@ -211,10 +191,6 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
     *abort_flag = 0;
     fence_mbar_init();
   }
-  __syncthreads();
-  const int total_units = pair_first[n_groups] * p.n_chunks;
-  if (cluster >= total_units) return;            // the same decision in both CTAs of the pair
-
   if (warp == 1) {
     tmem_alloc2(tmem_slot, TMEM_COLS);
     tmem_relinquish2();
@@ -223,21 +199,50 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
   cluster_sync_all();     // both CTAs' barriers are initialised and both have their TMEM
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
-  auto decode = [&](int u) {
-    Unit2 c;
-    const int nc = u % p.n_chunks;
-    const int pr = u / p.n_chunks;
-    int lo = 0, hi = n_groups;      // pair_first[lo] <= pr < pair_first[hi]
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (pair_first[mid] <= pr) lo = mid; else hi = mid;
+  // ------------------------------------------------------------------------- pair table
+  // pair_first[g] = number of block pairs of the runs before g (a run of t blocks has ceil(t / 2))
+  // A cluster takes consecutive units (the N chunks of a pair of blocks, then the next pair), so that the
+  // walk is an increment: finding a unit in the table took 0.7 us, once or twice per unit and role.
+  struct Walk {
+    int left, nc, pr, g;     // units left; N chunk, pair of blocks, its run
+  };
+  Walk* const first_unit = reinterpret_cast<Walk*>(smem + L::WALK_OFFSET);
+  if (warp == 2) {
+    const int pairs = prefix_runs(load_run_ends(p.a2_offsets, n_groups, lane), n_groups, lane, pair_first,
+                                  run_start, [](int rows) { return ((rows >> 7) + 1) >> 1; });
+    Walk w;
+    const int total = pairs * p.n_chunks, each = total / n_clusters, more = total - each * n_clusters;
+    const int first = each * cluster + min(cluster, more);
+    w.left = each + (cluster < more ? 1 : 0);
+    w.pr = first / p.n_chunks;
+    w.nc = first - w.pr * p.n_chunks;
+    __syncwarp();
+    int at_or_before = 0;
+    for (int base = 0; base < n_groups; base += 32)
+      at_or_before += __popc(__ballot_sync(0xffffffffu, base + lane < n_groups && pair_first[base + lane] <= w.pr));
+    w.g = at_or_before - 1;   // the last run that starts there or before
+    if (lane == 0) *first_unit = w;
+  }
+  __syncthreads();
+
+  auto walk = [&]() { return *first_unit; };
+  auto advance = [&](Walk& w) {
+    --w.left;
+    if (++w.nc == p.n_chunks) {
+      w.nc = 0;
+      ++w.pr;
+      while (w.g + 1 < n_groups && pair_first[w.g + 1] <= w.pr) ++w.g;
     }
-    const int blk = 2 * (pr - pair_first[lo]) + int(rank);
-    c.group = lo;
-    c.m_tile = (run_start[lo] >> 7) + blk;
-    c.valid = blk < ((run_start[lo + 1] - run_start[lo]) >> 7);
-    c.n0 = nc * BN;
+  };
+  auto unit_of = [&](const Walk& w) {
+    Unit2 c;
+    const int blk = 2 * (w.pr - pair_first[w.g]) + int(rank);
+    c.group = w.g;
+    c.m_tile = (run_start[w.g] >> 7) + blk;
+    c.valid = blk < ((run_start[w.g + 1] - run_start[w.g]) >> 7);
+    c.n0 = w.nc * BN;
     return c;
   };
 
@@ -245,8 +250,8 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
     // ------------------------------------------------ pre-activation tiles for the epilogue
     if (elect_one()) {
       int j = 0;
-      for (int u = cluster; u < total_units && !*abort_flag; u += n_clusters, ++j) {
-        const Unit2 tc = decode(u);
+      for (Walk u = walk(); u.left > 0 && !*abort_flag; advance(u), ++j) {
+        const Unit2 tc = unit_of(u);
         const int b = j & 1;
         const uint32_t use = uint32_t(j) >> 1;
         if (use > 0 && !mbar_wait(aempty_bar + b, (use - 1) & 1, p.status)) {
@@ -265,8 +270,8 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
     // ------------------------------------------------------------------ TMA producer (both CTAs)
     if (elect_one()) {
       uint32_t it = 0;
-      for (int u = cluster; u < total_units && !*abort_flag; u += n_clusters) {
-        const Unit2 tc = decode(u);
+      for (Walk u = walk(); u.left > 0 && !*abort_flag; advance(u)) {
+        const Unit2 tc = unit_of(u);
         const bool a_alt = tc.group >= p.a2_first_group;
         const int a_start = a_alt ? run_start[tc.group] : 0;
         const bool first = tc.group < p.n_groups_b1;
@@ -302,7 +307,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
       constexpr uint32_t idesc = umma_idesc(2 * BM, BN, false, B_MN);
       uint32_t it = 0;
       int j = 0;
-      for (int u = cluster; u < total_units && !*abort_flag; u += n_clusters, ++j) {
+      for (Walk u = walk(); u.left > 0 && !*abort_flag; --u.left, ++j) {
         const int b = j & 1;
         const uint32_t use = uint32_t(j) >> 1;
         if (use > 0 && !mbar_wait(tempty_bar + b, (use - 1) & 1, p.status)) {
@@ -341,8 +346,8 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
       int* tok_all = reinterpret_cast<int*>(smem + L::RED_TOK_OFFSET);
       const uint64_t keep = l2_policy_evict_last();
       int j = 0;
-      for (int u = cluster; u < total_units; u += n_clusters, ++j) {
-        const Unit2 tc = decode(u);
+      for (Walk u = walk(); u.left > 0; advance(u), ++j) {
+        const Unit2 tc = unit_of(u);
         const int b = j & 1;
         if (!mbar_wait(afull_bar + b, (uint32_t(j) >> 1) & 1, p.status))
           atomicExch(p.status, ST_WAIT_TIMEOUT);
@@ -396,25 +401,29 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
     // the leader's "accumulator empty" barriers, as cluster addresses
     const uint32_t tempty_leader = mapa_u32(smem_u32(tempty_bar), 0);
 
-    auto load_pair = [&](int u) {
-      if (u >= total_units || p.sorted_ids == nullptr) return p.n_pairs;
-      const Unit2 c = decode(u);
+    auto load_pair = [&](const Walk& u) {
+      if (u.left <= 0 || p.sorted_ids == nullptr) return p.n_pairs;
+      const Unit2 c = unit_of(u);
       return c.valid ? __ldg(p.sorted_ids + int64_t(c.m_tile) * BM + row) : p.n_pairs;
     };
     auto load_w = [&](int pr) {
       if (p.pair_w == nullptr) return 1.f;
       return pr < p.n_pairs ? __bfloat162float(__ldg(p.pair_w + pr)) : 0.f;
     };
-    int pair = load_pair(cluster);
-    int pair_n = load_pair(cluster + n_clusters);
+    Walk ahead = walk();
+    int pair = load_pair(ahead);
+    advance(ahead);
+    int pair_n = load_pair(ahead);
+    advance(ahead);
     float w = load_w(pair);
 
     int j = 0;
-    for (int u = cluster; u < total_units; u += n_clusters, ++j) {
-      const Unit2 tc = decode(u);
+    for (Walk u = walk(); u.left > 0; advance(u), ++j) {
+      const Unit2 tc = unit_of(u);
       const int b = j & 1;
       const float w_n = load_w(pair_n);
-      const int pair_nn = load_pair(u + 2 * n_clusters);
+      const int pair_nn = load_pair(ahead);
+      advance(ahead);
       if (!mbar_wait(tfull_bar + b, (uint32_t(j) >> 1) & 1, p.status))
         atomicExch(p.status, ST_WAIT_TIMEOUT);
       tc_fence_after();
@@ -497,7 +506,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER_NO), 1)
           } else {
             named_bar_sync(1, EPI_WARPS * 32);
             if (row_ok && pair < p.n_pairs) p.dtw[pair] = __float2bfloat16(part + dtw_part[row]);
-            if (u + n_clusters < total_units) named_bar_arrive(2, EPI_WARPS * 32);
+            if (u.left > 1) named_bar_arrive(2, EPI_WARPS * 32);
           }
         }
       }

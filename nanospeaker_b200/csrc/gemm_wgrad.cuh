@@ -19,6 +19,26 @@ constexpr int WGRAD_MAX_GROUPS = 256;
 // round-robin, and with runs of very different lengths the list order left some CTAs with 1.6x the
 // mean work at the bench's skew, the sorted order with 1.2x.
 constexpr int WGRAD_SORT_MAX = 1024;
+// A CTA's (a pair's) first units, found by all threads at once before the roles begin: searching them
+// out one by one costs each role 0.7 us per unit.
+constexpr int WGRAD_UNITS = 64;
+
+struct alignas(16) WgradUnit {
+  int row0, num_k, group, txy;   // rows [row0, row0 + 64 num_k) of a run (num_k < 0: no unit), tile of C
+  int item, n_c, pad[2];         // its work item, the chunks of its run
+};
+// The work list in shared memory (kept small: what a CTA leaves of an SM's shared memory is room for the
+// small kernels of the backward's other streams).
+struct WgradTable {
+  int first_item[WGRAD_MAX_GROUPS + 1], run_start[WGRAD_MAX_GROUPS + 1];
+  uint16_t order[WGRAD_SORT_MAX];
+  uint8_t group[WGRAD_SORT_MAX];
+  union alignas(16) {
+    int size[WGRAD_SORT_MAX];        // until the order is made
+    WgradUnit unit[WGRAD_UNITS];
+  };
+};
+static_assert(WGRAD_MAX_GROUPS <= 256 && WGRAD_SORT_MAX <= 65536, "the table's types");
 
 template <int BN, int STAGES>
 struct WgradSmem {
@@ -27,78 +47,183 @@ struct WgradSmem {
   static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
   static constexpr int N_BARS = 2 * STAGES + 4;  // full, empty, tmem_full[2], tmem_empty[2]
   static constexpr int MISC_OFFSET = BAR_OFFSET + 8 * N_BARS;
-  static constexpr int TABLE_OFFSET = MISC_OFFSET + 16;  // int first_item[G+1], int run_start[G+1]
-  static constexpr int TOK_OFFSET = TABLE_OFFSET + 2 * (WGRAD_MAX_GROUPS + 1) * 4;  // int[64]
-  static constexpr int ORDER_OFFSET = TOK_OFFSET + 64 * 4;  // int order[SORT_MAX], int size[SORT_MAX]
-  static constexpr int TOTAL = ORDER_OFFSET + 2 * WGRAD_SORT_MAX * 4;
+  static constexpr int TABLE_OFFSET = (MISC_OFFSET + 16 + 15) / 16 * 16;
+  static constexpr int TOTAL = TABLE_OFFSET + int(sizeof(WgradTable));
   static constexpr int DYNAMIC = TOTAL + 1024;
+  static_assert(DYNAMIC <= 232448, "one CTA's shared memory");
 };
 
 // Number of split-K work items of a run of `rows` rows.
 __host__ __device__ __forceinline__ int wgrad_chunks(int rows, int ks_rows) {
-  const int c = (rows + ks_rows - 1) / ks_rows;
-  return c > 0 ? c : 1;
+  return rows <= ks_rows ? 1 : (rows + ks_rows - 1) / ks_rows;
 }
 
-// Exclusive prefix of the per-run work-item counts into first_item[0..G] and the run starts into
-// run_start[0..G]; executed by one full warp.
-__device__ __forceinline__ void wgrad_build_table(const WgradArgs& p, int lane, int* first_item,
-                                                  int* run_start) {
-  int running = 0;
-  for (int base = 0; base < p.n_groups; base += 32) {
-    const int g = base + lane;
-    int lo = 0, hi = 0;
-    if (g < p.n_groups) {
-      if (p.pad_offsets != nullptr) {
-        lo = __ldg(p.pad_offsets + g);
-        hi = __ldg(p.pad_offsets + g + 1);
-      } else {
-        hi = p.rows_host;
-      }
+// Run g's start and end for g = 32 i + lane, i < 8 (one warp); every load is on its way before the first
+// is used.
+struct RunEnds {
+  int lo[WGRAD_MAX_GROUPS / 32], hi[WGRAD_MAX_GROUPS / 32];
+};
+__device__ __forceinline__ RunEnds load_run_ends(const int32_t* offsets, int n_groups, int lane) {
+  RunEnds r;
+#pragma unroll
+  for (int i = 0; i < WGRAD_MAX_GROUPS / 32; ++i) {
+    r.lo[i] = r.hi[i] = 0;
+    if (32 * i < n_groups) {
+      const int g = 32 * i + lane;
+      r.lo[i] = __ldg(offsets + min(g, n_groups));
+      r.hi[i] = __ldg(offsets + min(g + 1, n_groups));
     }
-    const int mine = g < p.n_groups ? wgrad_chunks(hi - lo, p.ks_rows) : 0;
+  }
+  return r;
+}
+// Exclusive prefix over the runs of what f makes of a run's length (one warp): sum[0..n_groups], and the
+// total.
+template <typename F>
+__device__ __forceinline__ int prefix_runs(const RunEnds& r, int n_groups, int lane, int* sum, int* start,
+                                           F f) {
+  int running = 0;
+#pragma unroll
+  for (int i = 0; i < WGRAD_MAX_GROUPS / 32; ++i) {
+    if (32 * i >= n_groups) break;
+    const int g = 32 * i + lane;
+    const int mine = g < n_groups ? f(r.hi[i] - r.lo[i]) : 0;
     int incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int v = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += v;
     }
-    if (g < p.n_groups) {
-      first_item[g] = running + incl - mine;
-      run_start[g] = lo;
+    if (g < n_groups) {
+      sum[g] = running + incl - mine;
+      start[g] = r.lo[i];
+      if (g == n_groups - 1) {
+        sum[n_groups] = running + incl;
+        start[n_groups] = r.hi[i];
+      }
     }
     running += __shfl_sync(0xffffffffu, incl, 31);
   }
-  if (lane == 0) {
-    first_item[p.n_groups] = running;
-    run_start[p.n_groups] = p.pad_offsets != nullptr ? __ldg(p.pad_offsets + p.n_groups)
-                                                     : p.rows_host;
+  return running;
+}
+
+// The work items before every run and the run starts, into table.first_item and table.run_start (one warp).
+__device__ __forceinline__ void wgrad_build_table(const WgradArgs& p, int lane, int* first_item,
+                                                  int* run_start) {
+  if (p.pad_offsets != nullptr) {
+    prefix_runs(load_run_ends(p.pad_offsets, p.n_groups, lane), p.n_groups, lane, first_item, run_start,
+                [&](int rows) { return wgrad_chunks(rows, p.ks_rows); });
+  } else {
+    const int per = wgrad_chunks(p.rows_host, p.ks_rows);
+    for (int g = lane; g <= p.n_groups; g += 32) {
+      first_item[g] = g * per;
+      run_start[g] = g < p.n_groups ? 0 : p.rows_host;
+    }
   }
 }
 
-struct WgradItem {
-  int group, first, n_c, row0, num_k;
-};
-
-// Work item j -> its run, its chunk and the rows it contracts over (binary search in the table).
-__device__ __forceinline__ WgradItem wgrad_item(const WgradArgs& p, const int* first_item,
-                                                const int* run_start, int j) {
-  int lo = 0, hi = p.n_groups;  // first_item[lo] <= j < first_item[hi]
+// Work item j of the list -> the rows it contracts over.
+__device__ __forceinline__ WgradUnit wgrad_item(const WgradArgs& p, const WgradTable& t, int group, int j) {
+  WgradUnit u{};
+  u.group = group;
+  u.item = j;
+  u.n_c = t.first_item[group + 1] - t.first_item[group];
+  const int start = t.run_start[group];
+  const int end = p.pad_offsets != nullptr ? t.run_start[group + 1] : p.rows_host;
+  u.row0 = start + (j - t.first_item[group]) * p.ks_rows;
+  int rows = end - u.row0;
+  rows = rows < 0 ? 0 : (rows > p.ks_rows ? p.ks_rows : rows);
+  u.num_k = (rows + BK - 1) / BK;
+  return u;
+}
+__device__ __forceinline__ int wgrad_group_of(const WgradTable& t, int n_groups, int j) {
+  int lo = 0, hi = n_groups;  // first_item[lo] <= j < first_item[hi]
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (first_item[mid] <= j) lo = mid; else hi = mid;
+    if (t.first_item[mid] <= j) lo = mid; else hi = mid;
   }
-  WgradItem it;
-  it.group = lo;
-  it.first = first_item[lo];
-  it.n_c = first_item[lo + 1] - it.first;
-  const int start = run_start[lo];
-  const int end = p.pad_offsets != nullptr ? run_start[lo + 1] : p.rows_host;
-  it.row0 = start + (j - it.first) * p.ks_rows;
-  int rows = end - it.row0;
-  rows = rows < 0 ? 0 : (rows > p.ks_rows ? p.ks_rows : rows);
-  it.num_k = (rows + BK - 1) / BK;
-  return it;
+  return lo;
+}
+
+// The walk over the units (positions in the walk order x tiles of C), dealt to `n` CTAs or pairs of which
+// this is `mine`. The order: items by decreasing length, ties by index (the same permutation in every
+// CTA). A round's units run alternately up and down the CTAs (0..n-1, then n-1..0): in decreasing length,
+// plain round-robin gave CTA 0 the longest unit of every round (busiest CTA 1.28 x the mean at the
+// bench's skew); the serpentine order gives 1.09 x.
+struct WgradWalk {
+  const WgradArgs& p;
+  const WgradTable& t;
+  int n, mine, tiles, total;
+  bool sorted;
+  __device__ __forceinline__ int rounds() const { return (total + n - 1) / n; }
+  __device__ __forceinline__ WgradUnit find(int rnd) const {
+    const int u = rnd * n + ((rnd & 1) ? n - 1 - mine : mine);
+    if (u >= total) {
+      WgradUnit none{};
+      none.num_k = -1;
+      return none;
+    }
+    const int pos = u / tiles, j = sorted ? int(t.order[pos]) : pos;
+    WgradUnit w = wgrad_item(p, t, sorted ? int(t.group[j]) : wgrad_group_of(t, p.n_groups, j), j);
+    w.txy = u - pos * tiles;
+    return w;
+  }
+  __device__ __forceinline__ WgradUnit unit(int rnd) const {
+    return rnd < WGRAD_UNITS ? t.unit[rnd] : find(rnd);
+  }
+};
+// Fills the table; all threads of the CTA, behind the wait for the earlier kernels.
+__device__ __forceinline__ WgradWalk wgrad_plan(const WgradArgs& p, WgradTable& t, int n, int mine,
+                                                int tiles) {
+  if (threadIdx.x < 32) {
+    wgrad_build_table(p, threadIdx.x, t.first_item, t.run_start);
+    // the reduction pass reads the item counts from global memory instead of rebuilding them
+    if (blockIdx.x == 0) {
+      __syncwarp();
+      for (int g = threadIdx.x; g <= p.n_groups; g += 32) p.item_table[g] = t.first_item[g];
+    }
+  }
+  __syncthreads();
+  const int n_items = t.first_item[p.n_groups];
+  const WgradWalk walk{p, t, n, mine, tiles, n_items * tiles, n_items <= WGRAD_SORT_MAX};
+  if (walk.sorted) {
+    if (p.n_groups > 8) {          // a thread per run
+      for (int g = threadIdx.x; g < p.n_groups; g += blockDim.x) {
+        WgradUnit u = wgrad_item(p, t, g, t.first_item[g]);
+        const int end = t.run_start[g + 1];
+        for (int j = u.item; j < u.item + u.n_c; ++j, u.row0 += p.ks_rows) {
+          t.size[j] = (min(end - u.row0, p.ks_rows) + BK - 1) / BK;
+          t.group[j] = uint8_t(g);
+        }
+      }
+    } else {
+      for (int j = threadIdx.x; j < n_items; j += blockDim.x) {
+        const int g = wgrad_group_of(t, p.n_groups, j);
+        t.size[j] = wgrad_item(p, t, g, j).num_k;
+        t.group[j] = uint8_t(g);
+      }
+    }
+    if (threadIdx.x < 16 && n_items + threadIdx.x < WGRAD_SORT_MAX) t.size[n_items + threadIdx.x] = -1;
+    __syncthreads();
+    // four lanes per item, four others at a time
+    for (int base = 0; base < n_items; base += blockDim.x / 4) {
+      const int i = base + int(threadIdx.x >> 2);
+      const int size = t.size[min(i, n_items - 1)];
+      int rank = 0;
+#pragma unroll 2
+      for (int k = 4 * (threadIdx.x & 3); k < n_items; k += 16) {
+        const int4 o = *reinterpret_cast<const int4*>(t.size + k);
+        rank += (o.x > size || (o.x == size && k < i)) + (o.y > size || (o.y == size && k + 1 < i)) +
+                (o.z > size || (o.z == size && k + 2 < i)) + (o.w > size || (o.w == size && k + 3 < i));
+      }
+      rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+      rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+      if (i < n_items && (threadIdx.x & 3) == 0) t.order[rank] = uint16_t(i);
+    }
+    __syncthreads();
+  }
+  for (int r = threadIdx.x; r < min(WGRAD_UNITS, walk.rounds()); r += blockDim.x) t.unit[r] = walk.find(r);
+  __syncthreads();
+  return walk;
 }
 
 // Persistent: one CTA per SM walks the list of (work item, m tile, n chunk); the accumulator is
@@ -125,22 +250,12 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
   uint64_t* tempty_bar = tfull_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::MISC_OFFSET);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* first_item = reinterpret_cast<int*>(smem + L::TABLE_OFFSET);
-  int* run_start = first_item + WGRAD_MAX_GROUPS + 1;
+  WgradTable& table = *reinterpret_cast<WgradTable*>(smem + L::TABLE_OFFSET);
   constexpr bool gather = GATHER != 0;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  if (warp == 2) {
-    pdl_wait();   // the run table is the dispatch's
-    wgrad_build_table(p, lane, first_item, run_start);
-    // the reduction pass reads the item counts from global memory instead of rebuilding them
-    if (blockIdx.x == 0) {
-      __syncwarp();
-      for (int g = lane; g <= p.n_groups; g += 32) p.item_table[g] = first_item[g];
-    }
-  }
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -164,38 +279,10 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_wait();      // every thread, before its first read of an earlier kernel's data
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();      // every thread, before its first read of an earlier kernel's data
   const int tiles_xy = tiles_x * tiles_y;
-  const int n_items = first_item[p.n_groups];
-  const int total = n_items * tiles_xy;  // t = position in the walk order * tiles_xy + tile
-  // walk order: items by decreasing length, ties by index (the same permutation in every CTA)
-  int* order = reinterpret_cast<int*>(smem + L::ORDER_OFFSET);
-  int* isize = order + WGRAD_SORT_MAX;
-  const bool sorted = n_items <= WGRAD_SORT_MAX;
-  if (sorted) {
-    for (int i = threadIdx.x; i < n_items; i += blockDim.x)
-      isize[i] = wgrad_item(p, first_item, run_start, i).num_k;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n_items; i += blockDim.x) {
-      const int mine = isize[i];
-      int rank = 0;
-      for (int k = 0; k < n_items; ++k) {
-        const int other = isize[k];
-        rank += (other > mine || (other == mine && k < i)) ? 1 : 0;
-      }
-      order[rank] = i;
-    }
-    __syncthreads();
-  }
-  auto item_at = [&](int pos) { return sorted ? order[pos] : pos; };
-  // A CTA's unit of round r: rounds run alternately up and down the CTAs (0..G-1, then G-1..0).
-  // The units are in decreasing length, so plain round-robin gave CTA 0 the longest unit of every
-  // round (busiest CTA 1.28 x the mean at the bench's skew); the serpentine order gives 1.09 x.
-  auto unit_of_round = [&](int rnd) {
-    const int g = int(gridDim.x), b = int(blockIdx.x);
-    return rnd * g + ((rnd & 1) ? g - 1 - b : b);
-  };
+  const WgradWalk walk = wgrad_plan(p, table, int(gridDim.x), int(blockIdx.x), tiles_xy);
 
   if (warp == 0 || warp >= 2 + EPI_WARPS) {
     // Producers. Plain operands arrive by TMA (warp 0, lane 0). A gathered operand is copied with
@@ -206,12 +293,9 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
     if (gather || (warp == 0 && lane == 0)) {
       uint32_t it = 0;
       int pending = -1;  // stage whose cp.async copies are issued but not yet handed over
-      for (int rnd = 0; rnd * int(gridDim.x) < total && !*abort_flag; ++rnd) {
-        const int t = unit_of_round(rnd);
-        if (t >= total) continue;
-        const WgradItem w = wgrad_item(p, first_item, run_start, item_at(t / tiles_xy));
-        const int txy = t % tiles_xy;
-        const int m0 = (txy / tiles_y) * BM, n0 = (txy % tiles_y) * BN;
+      for (int rnd = 0; rnd < walk.rounds() && !*abort_flag; ++rnd) {
+        const WgradUnit w = walk.unit(rnd);
+        const int m0 = (w.txy / tiles_y) * BM, n0 = (w.txy % tiles_y) * BN;
         const int ga = p.a_grouped ? w.group : 0, gb = p.b_grouped ? w.group : 0;
         constexpr int ROWS_PER_WARP = BK / WGRAD_GATHER_WARPS;  // 16 rows of a stage per producer warp
         // token of row gw*16 + lane of the NEXT stage, fetched one stage ahead of its use
@@ -244,7 +328,7 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
             // runs from alt_first_group on (the shared experts) take one operand from the
             // token-major matrix: its row is the slot row minus the start of the run
             const bool alt = p.alt_which != 0 && w.group >= p.alt_first_group;
-            const int r_alt = r - run_start[w.group];
+            const int r_alt = r - table.run_start[w.group];
             const bool a_alt = alt && p.alt_which == 1, b_alt = alt && p.alt_which == 2;
             const CUtensorMap* ma = a_alt ? &tmAlt : &tmA;
             const CUtensorMap* mb = b_alt ? &tmAlt : &tmB;
@@ -307,11 +391,9 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
     if (elect_one()) {
       uint32_t it = 0;
       int ju = 0;  // tiles that really used an accumulator buffer so far
-      for (int rnd = 0; rnd * int(gridDim.x) < total && !*abort_flag; ++rnd) {
-        const int t = unit_of_round(rnd);
-        if (t >= total) continue;
-        const WgradItem w = wgrad_item(p, first_item, run_start, item_at(t / tiles_xy));
-        if (w.num_k == 0) continue;  // empty run: the epilogue writes zeros, no accumulator used
+      for (int rnd = 0; rnd < walk.rounds() && !*abort_flag; ++rnd) {
+        const WgradUnit w = walk.unit(rnd);
+        if (w.num_k <= 0) continue;  // empty run: the epilogue writes zeros, no accumulator used
         const int b = ju & 1;
         const uint32_t use = uint32_t(ju) >> 1;
         ++ju;
@@ -347,11 +429,10 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
     const int c_lo = half * (NCH / 2), c_hi = c_lo + NCH / 2;
 
     int ju = 0;  // tiles that really used an accumulator buffer so far (same count as the MMA warp)
-    for (int rnd = 0; rnd * int(gridDim.x) < total; ++rnd) {
-      const int t = unit_of_round(rnd);
-      if (t >= total) continue;
-      const int j = item_at(t / tiles_xy), txy = t % tiles_xy;
-      const WgradItem w = wgrad_item(p, first_item, run_start, j);
+    for (int rnd = 0; rnd < walk.rounds(); ++rnd) {
+      const WgradUnit w = walk.unit(rnd);
+      if (w.num_k < 0) continue;
+      const int j = w.item, txy = w.txy;
       const int m0 = (txy / tiles_y) * BM, n0 = (txy % tiles_y) * BN;
       const bool have_acc = w.num_k > 0;
       // The MMA warp skips empty runs without touching a buffer, so the epilogue neither waits

@@ -19,9 +19,8 @@ struct Wgrad2Smem {
   static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
   static constexpr int N_BARS = 2 * STAGES + 4;
   static constexpr int MISC_OFFSET = BAR_OFFSET + 8 * N_BARS;
-  static constexpr int TABLE_OFFSET = MISC_OFFSET + 16;
-  static constexpr int ORDER_OFFSET = TABLE_OFFSET + 2 * (WGRAD_MAX_GROUPS + 1) * 4;
-  static constexpr int TOTAL = ORDER_OFFSET + 2 * WGRAD_SORT_MAX * 4;
+  static constexpr int TABLE_OFFSET = (MISC_OFFSET + 16 + 15) / 16 * 16;
+  static constexpr int TOTAL = TABLE_OFFSET + int(sizeof(WgradTable));
   static constexpr int DYNAMIC = TOTAL + 1024;
   static_assert(STAGE_BYTES % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
   static_assert(BN % 128 == 0, "a B half must be whole 64-column boxes");
@@ -35,8 +34,7 @@ __global__ void __launch_bounds__(WGRAD_THREADS, 1)
                        const __grid_constant__ CUtensorMap tmB,
                        const __grid_constant__ CUtensorMap tmAlt, const WgradArgs p, int tiles_x,
                        int tiles_y) {
-  pdl_trigger();
-  pdl_wait();
+  pdl_trigger();   // (the prologue up to the wait touches nothing an earlier kernel wrote)
   using L = Wgrad2Smem<BN, STAGES>;
   constexpr uint32_t TMEM_BUF = BN <= 128 ? 128 : 256;
   constexpr uint32_t TMEM_COLS = 2 * TMEM_BUF;
@@ -50,8 +48,7 @@ __global__ void __launch_bounds__(WGRAD_THREADS, 1)
   uint64_t* tempty_bar = tfull_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::MISC_OFFSET);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* first_item = reinterpret_cast<int*>(smem + L::TABLE_OFFSET);
-  int* run_start = first_item + WGRAD_MAX_GROUPS + 1;
+  WgradTable& table = *reinterpret_cast<WgradTable*>(smem + L::TABLE_OFFSET);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -59,13 +56,6 @@ __global__ void __launch_bounds__(WGRAD_THREADS, 1)
   const int n_clusters = int(gridDim.x) >> 1;
   const int cluster = int(blockIdx.x) >> 1;
 
-  if (warp == 2) {
-    wgrad_build_table(p, lane, first_item, run_start);
-    if (blockIdx.x == 0) {
-      __syncwarp();
-      for (int g = lane; g <= p.n_groups; g += 32) p.item_table[g] = first_item[g];
-    }
-  }
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -86,46 +76,21 @@ __global__ void __launch_bounds__(WGRAD_THREADS, 1)
     tmem_relinquish2();
   }
   tc_fence_before();
-  __syncthreads();
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
   const int pairs_x = (tiles_x + 1) >> 1;
   const int units_xy = pairs_x * tiles_y;      // pair tiles per work item
   const int tiles_xy = tiles_x * tiles_y;      // single tiles per work item (partial layout)
-  const int n_items = first_item[p.n_groups];
-  const int total = n_items * units_xy;
-  int* order = reinterpret_cast<int*>(smem + L::ORDER_OFFSET);
-  int* isize = order + WGRAD_SORT_MAX;
-  const bool sorted = n_items <= WGRAD_SORT_MAX;
-  if (sorted) {
-    for (int i = threadIdx.x; i < n_items; i += blockDim.x)
-      isize[i] = wgrad_item(p, first_item, run_start, i).num_k;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n_items; i += blockDim.x) {
-      const int mine = isize[i];
-      int rk = 0;
-      for (int k = 0; k < n_items; ++k) {
-        const int other = isize[k];
-        rk += (other > mine || (other == mine && k < i)) ? 1 : 0;
-      }
-      order[rk] = i;
-    }
-    __syncthreads();
-  }
-  auto item_at = [&](int pos) { return sorted ? order[pos] : pos; };
-  auto unit_of_round = [&](int rnd) {   // serpentine over the clusters
-    return rnd * n_clusters + ((rnd & 1) ? n_clusters - 1 - cluster : cluster);
-  };
+  const WgradWalk walk = wgrad_plan(p, table, n_clusters, cluster, units_xy);
 
   if (warp == 0) {
     if (lane == 0) {
       uint32_t it = 0;
-      for (int rnd = 0; rnd * n_clusters < total && !*abort_flag; ++rnd) {
-        const int t = unit_of_round(rnd);
-        if (t >= total) continue;
-        const WgradItem w = wgrad_item(p, first_item, run_start, item_at(t / units_xy));
-        const int uxy = t % units_xy;
+      for (int rnd = 0; rnd < walk.rounds() && !*abort_flag; ++rnd) {
+        const WgradUnit w = walk.unit(rnd);
+        const int uxy = w.txy;
         const int m0 = ((uxy / tiles_y) * 2 + int(rank)) * BM;       // this CTA's rows of C
         const int n0 = (uxy % tiles_y) * BN + int(rank) * (BN / 2);  // this CTA's half of B
         const int ga = p.a_grouped ? w.group : 0, gb = p.b_grouped ? w.group : 0;
@@ -145,7 +110,7 @@ __global__ void __launch_bounds__(WGRAD_THREADS, 1)
           uint8_t* sB = sA + A_STAGE_BYTES;
           if (rank == 0) mbar_expect_tx(full_bar + s, 2 * L::STAGE_BYTES);
           const int r = w.row0 + kt * BK;
-          const int r_alt = r - run_start[w.group];
+          const int r_alt = r - table.run_start[w.group];
           // 4-D maps (64 cols, row, col / 64, group); a box group past the last column is zero fill
           tma_load_4d_2cta(sA, ma, full_bar + s, 0, a_alt ? r_alt : r, m0 / 64, a_alt ? 0 : ga);
           tma_load_4d_2cta(sB, mb, full_bar + s, 0, b_alt ? r_alt : r, n0 / 64, b_alt ? 0 : gb);
@@ -157,11 +122,9 @@ __global__ void __launch_bounds__(WGRAD_THREADS, 1)
       constexpr uint32_t idesc = umma_idesc(2 * BM, BN, true, true);
       uint32_t it = 0;
       int ju = 0;
-      for (int rnd = 0; rnd * n_clusters < total && !*abort_flag; ++rnd) {
-        const int t = unit_of_round(rnd);
-        if (t >= total) continue;
-        const WgradItem w = wgrad_item(p, first_item, run_start, item_at(t / units_xy));
-        if (w.num_k == 0) continue;
+      for (int rnd = 0; rnd < walk.rounds() && !*abort_flag; ++rnd) {
+        const WgradUnit w = walk.unit(rnd);
+        if (w.num_k <= 0) continue;
         const int b = ju & 1;
         const uint32_t use = uint32_t(ju) >> 1;
         ++ju;
@@ -202,11 +165,10 @@ __global__ void __launch_bounds__(WGRAD_THREADS, 1)
     const uint32_t tempty_leader = mapa_u32(smem_u32(tempty_bar), 0);
 
     int ju = 0;
-    for (int rnd = 0; rnd * n_clusters < total; ++rnd) {
-      const int t = unit_of_round(rnd);
-      if (t >= total) continue;
-      const int j = item_at(t / units_xy), uxy = t % units_xy;
-      const WgradItem w = wgrad_item(p, first_item, run_start, j);
+    for (int rnd = 0; rnd < walk.rounds(); ++rnd) {
+      const WgradUnit w = walk.unit(rnd);
+      if (w.num_k < 0) continue;
+      const int j = w.item, uxy = w.txy;
       const int tile_m = (uxy / tiles_y) * 2 + int(rank);     // this CTA's 128-row tile of C
       const int m0 = tile_m * BM, n0 = (uxy % tiles_y) * BN;
       const bool tile_ok = tile_m < tiles_x;

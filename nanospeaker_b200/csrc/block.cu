@@ -408,6 +408,12 @@ class ForkEventsLease {
   int dev_ = -1;
 };
 
+// From more tokens than this, dX adds the router's share itself (its weights' tiles as one more run). As a
+// launch of its own on a side stream it finds no room beside dX's CTAs and comes after them: 16384 tokens
+// 419 against 405 us with it in dX, 5000 graphed 231 against 229. But then dX has to wait for another
+// stream and loses its early launch: 2048 graphed 163 against 168, 300 the same.
+constexpr int64_t DX_WITH_ROUTER_TOKENS = 4096;
+
 int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
   const moe_b200_block_desc& d = b.d;
   const Sizes z = sizes(d.n_tokens, d.n_experts, d.n_shared, d.top_k);
@@ -439,30 +445,44 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
   if (sa != main_st) CU(cudaStreamWaitEvent(sa, ev->fork, 0));
   if (sb != main_st) CU(cudaStreamWaitEvent(sb, ev->fork, 0));
 
-  // main: dx's first value (the shared experts' share, stored), dW_in, the routed rows of dx
+  // main: dx's first value (the shared experts' share, stored), dW_in, the routed rows of dx. The router's
+  // share of dx comes with those (dx_with_router) or by a launch of its own on side b.
+  const bool dx_with_router = !store && T > DX_WITH_ROUTER_TOKENS;
   if (!store) {
     if (S)
       STEP(moe_b200_dx_gemm_sum(b.s.da1, z.l_cap, H, d.w_sh_in, S, D, first_shared, T, b.dx,
                                 d.status, stream));
     else
       STEP(zero_words(b.dx, T * D / 2, main_st));
-    CU(cudaEventRecord(ev->dx, main_st));
+    if (!dx_with_router) CU(cudaEventRecord(ev->dx, main_st));
   }
   STEP(moe::wgrad(b.k.xs, 0, D, b.s.da1, 0, 2 * H, z.l_cap, b.k.pad_offsets, z.n_all, 0, nullptr, 0,
                   0, 0, b.dw_in, E, S ? b.dw_sh_in : nullptr, b.s.part_in, b.s.part_in_bytes,
                   S ? d.x : nullptr, S ? T : 0, S ? 1 : 0, longest_run, 2 * H, d.status, stream));
-  if (store) {
-    STEP(moe_b200_dx_gemm(b.s.da1, z.l_cap, H, d.w_in, E, d.w_sh_in, S, D, b.k.expert_ids,
-                          b.k.n_post_pad, 0, b.s.ydx, d.status, stream));
-  } else {
-    STEP(moe_b200_dx_gemm_acc(b.s.da1, z.l_cap, H, d.w_in, E, nullptr, 0, D, b.k.expert_ids, live,
-                              0, b.k.sorted_ids, z.m, z.ks, b.dx, T, b.k.pad_offsets, d.status,
-                              stream));
-  }
   // side a: dW_out, then the bias gradients (column sums over the runs)
   STEP(moe::wgrad(b.s.hidw, 0, H, b.s.douts, 0, D, z.l_cap, b.k.pad_offsets, z.n_all, 0, nullptr, 0,
                   0, 0, b.dw_out, E, S ? b.dw_sh_out : nullptr, b.s.part_out, b.s.part_out_bytes,
                   S ? b.grad_out : nullptr, S ? T : 0, S ? 2 : 0, longest_run, D, d.status, sa));
+  // side b: the router's backward. With b_out a pair's d(topk_w) gains <dOut[t], b_out[e]>: one row GEMM
+  // dOut @ b_out^T over all experts, read at the pair's column by the router kernel.
+  if (b.s.b_extra)
+    STEP(moe_b200_dx_gemm(b.grad_out, T, D / 2, b.k.bias_out_k, 1, nullptr, 0, z.ld, nullptr,
+                          nullptr, 1, b.s.b_extra, d.status, sb));
+  STEP(moe::router_fused_bwd(d.logits_in ? d.logits_in : b.k.logits, d.logits_in ? E : z.ld,
+                             d.logit_bias, d.noise, b.k.idx_all, b.s.dtw, b.s.b_extra, z.ld,
+                             d.capacity > 0 ? b.k.inv_ids : nullptr, T, E, d.top_k, S,
+                             d.normalize, d.full_softmax, b.grad_aux, b.k.counts_all, d.aux_coef,
+                             b.s.dl, z.ld, sb));
+  if (dx_with_router && sb != main_st) CU(cudaEventRecord(ev->dx, sb));
+  if (store) {
+    STEP(moe_b200_dx_gemm(b.s.da1, z.l_cap, H, d.w_in, E, d.w_sh_in, S, D, b.k.expert_ids,
+                          b.k.n_post_pad, 0, b.s.ydx, d.status, stream));
+  } else {
+    if (dx_with_router && sb != main_st) CU(cudaStreamWaitEvent(main_st, ev->dx, 0));
+    STEP(moe::dx_gemm_acc(b.s.da1, z.l_cap, H, d.w_in, E, nullptr, 0, D, b.k.expert_ids, live, 0,
+                          b.k.sorted_ids, z.m, z.ks, b.dx, T, b.k.pad_offsets,
+                          dx_with_router ? b.s.dl : nullptr, b.k.router_wp, z.ld, d.status, stream));
+  }
   const int32_t n_bi = b.s.db_in ? z.n_all * 2 * H : 0, n_bo = b.s.db_out ? z.n_all * D : 0;
   if (n_bi) {
     STEP(zero_words(b.s.db_in, n_bi, sa));
@@ -477,19 +497,8 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
                                  S ? b.grad_out : nullptr, S ? T : 0, E, b.s.db_out, sa));
     STEP(to_bf16(b.s.db_out, b.db_out, n_bo, sa));
   }
-  // side b: the router's backward, its weight gradient, its share of dx (as one more product of the
-  // sum that gives dx its first value the step was 4 to 10 us slower: that sum then has to wait for
-  // it). With b_out a pair's d(topk_w) gains <dOut[t], b_out[e]>: one row GEMM dOut @ b_out^T over
-  // all experts, read at the pair's column by the router kernel.
-  if (b.s.b_extra)
-    STEP(moe_b200_dx_gemm(b.grad_out, T, D / 2, b.k.bias_out_k, 1, nullptr, 0, z.ld, nullptr,
-                          nullptr, 1, b.s.b_extra, d.status, sb));
-  STEP(moe::router_fused_bwd(d.logits_in ? d.logits_in : b.k.logits, d.logits_in ? E : z.ld,
-                             d.logit_bias, d.noise, b.k.idx_all, b.s.dtw, b.s.b_extra, z.ld,
-                             d.capacity > 0 ? b.k.inv_ids : nullptr, T, E, d.top_k, S,
-                             d.normalize, d.full_softmax, b.grad_aux, b.k.counts_all, d.aux_coef,
-                             b.s.dl, z.ld, sb));
-  // (a product of one chunk is stored with the padded width and copied)
+  // side b: the router's weight gradient (a product of one chunk is stored with the padded width and
+  // copied), and its share of dx: as rows of their own with a stored combine, or added
   const bool padded = E != z.ld && T <= moe::wgrad_chunk_rows(D, z.ld, T, 1, 0);
   STEP(moe::wgrad(d.x, 0, D, b.s.dl, 0, z.ld, T, nullptr, 1, 0, nullptr, 0, 0, 0,
                   padded ? b.s.d_router_padded : b.d_router, 1, nullptr, b.s.part_r,
@@ -498,7 +507,7 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
   if (store) {
     STEP(moe_b200_dx_gemm(b.s.dl, T, z.ld / 2, b.k.router_wp, 1, nullptr, 0, D, nullptr, nullptr,
                           1, b.s.dx_router, d.status, sb));
-  } else {
+  } else if (!dx_with_router) {
     if (sb != main_st) CU(cudaStreamWaitEvent(sb, ev->dx, 0));
     STEP(moe_b200_dx_gemm_acc(b.s.dl, T, z.ld / 2, b.k.router_wp, 1, nullptr, 0, D, nullptr,
                               nullptr, 1, nullptr, 0, 1, b.dx, T, nullptr, d.status, sb));

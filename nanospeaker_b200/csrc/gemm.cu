@@ -720,12 +720,16 @@ int moe_b200_down_gemm_acc(const void* hid, int64_t rows, int32_t k_dim, const v
       static_cast<cudaStream_t>(stream));
 }
 
-int moe_b200_dx_gemm_acc(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in,
+}  // extern "C"
+
+namespace moe {
+
+int dx_gemm_acc(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in,
                          int32_t n_groups, const void* w_extra, int32_t n_extra, int32_t d_model,
                          const int32_t* expert_ids, const int32_t* n_post_pad,
                          int32_t n_fixed_groups, const int32_t* sorted_ids, int64_t n_pairs,
-                         int32_t top_k, void* acc, int64_t n_tokens, const int32_t* pad_offsets,
-                         int32_t* status, void* stream) {
+                         int32_t top_k, void* acc, int64_t n_tokens, const int32_t* pad_offsets, const void* dl,
+                const void* router_w, int32_t ld, int32_t* status, void* stream) {
   CHECK_SCHED();
   if (d_hidden % 4 != 0 || d_hidden < 32 || d_model % 32 != 0) return MOE_B200_ERR_UNSUPPORTED;
   if (!da1 || !w_in) return MOE_B200_ERR_NULL;
@@ -733,6 +737,12 @@ int moe_b200_dx_gemm_acc(const void* da1, int64_t rows, int32_t d_hidden, const 
   const int rca = check_acc(n_fixed_groups, rows, sorted_ids, top_k, n_pairs, acc, n_tokens, d_model);
   if (rca != MOE_B200_OK) return rca;
   CHECK_EXTRA();
+  if (dl) {
+    if (!router_w) return MOE_B200_ERR_NULL;
+    if (!aligned16(dl) || !aligned16(router_w)) return MOE_B200_ERR_ALIGN;
+    if (n_fixed_groups > 0 || !pad_offsets || n_extra > 0 || ld < 64 || ld % 64 != 0)
+      return MOE_B200_ERR_UNSUPPORTED;
+  }
   const int gdim = n_fixed_groups > 0 ? n_fixed_groups : 1;
   CUtensorMap tmA, tmB, tmB2;
   if (!map_rows_kmajor(&tmA, da1, gdim, rows, 2 * d_hidden) ||
@@ -752,25 +762,47 @@ int moe_b200_dx_gemm_acc(const void* da1, int64_t rows, int32_t d_hidden, const 
   g.out = static_cast<__nv_bfloat16*>(acc);
   g.ld_out = d_model;
   g.n_groups_b1 = n_extra > 0 ? n_groups : INT32_MAX;
-#ifndef MOE_NO_PAIR_DX
   // Routed schedule with the run table at hand: CTA pairs, each CTA loading 96 of the 192 weight
   // rows of the tile.
   if (n_fixed_groups == 0 && pad_offsets != nullptr) {
     CUtensorMap hB, hB2;
     if (!map_weight_kmajor(&hB, w_in, n_groups, d_model, 2 * d_hidden, 96)) return MOE_B200_ERR_TMA;
     hB2 = hB;
+    CUtensorMap tmA2 = tmA;
+    int64_t units = max_pair_units(rows, n_groups + n_extra, g.n_chunks);
+    if (dl) {
+      if (!map_rows_kmajor(&tmA2, dl, 1, n_tokens, ld) ||
+          !map_weight_kmajor(&hB2, router_w, 1, d_model, ld, 96))
+        return MOE_B200_ERR_TMA;
+      g.beside_rows = int32_t(n_tokens);
+      g.beside_k = ld / BK;
+      units += (n_tokens + 2 * BM - 1) / (2 * BM) * g.n_chunks;
+    }
     if (n_extra > 0 && !map_weight_kmajor(&hB2, w_extra, n_extra, d_model, 2 * d_hidden, 96))
       return MOE_B200_ERR_TMA;
     g.a2_offsets = pad_offsets;
     g.n_groups_total = n_groups + n_extra;
     return launch_rows2<192, MOE_PAIR_DX_STAGES, false, EPI_RAW_RED>(
-        tmA, tmA, hB, hB2, hB, g, max_pair_units(rows, n_groups + n_extra, g.n_chunks),
-        static_cast<cudaStream_t>(stream));
+        tmA, tmA2, hB, hB2, hB, g, units, static_cast<cudaStream_t>(stream));
   }
-#endif
   return launch_rows<192, MOE_RED_DX_STAGES, false, EPI_RAW_RED, GATHER_NO, MOE_RED_DX_BUFS>(
       tmA, tmB, tmB2, tmB, g, max_tiles(rows, g.n_chunks, n_fixed_groups),
       static_cast<cudaStream_t>(stream));
+}
+
+}  // namespace moe
+
+extern "C" {
+
+int moe_b200_dx_gemm_acc(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in,
+                         int32_t n_groups, const void* w_extra, int32_t n_extra, int32_t d_model,
+                         const int32_t* expert_ids, const int32_t* n_post_pad,
+                         int32_t n_fixed_groups, const int32_t* sorted_ids, int64_t n_pairs,
+                         int32_t top_k, void* acc, int64_t n_tokens, const int32_t* pad_offsets,
+                         int32_t* status, void* stream) {
+  return dx_gemm_acc(da1, rows, d_hidden, w_in, n_groups, w_extra, n_extra, d_model, expert_ids,
+                     n_post_pad, n_fixed_groups, sorted_ids, n_pairs, top_k, acc, n_tokens, pad_offsets,
+                     nullptr, nullptr, 0, status, stream);
 }
 
 // The scratch buffer starts with the item table ([G + 1] int32), the partial tiles follow.

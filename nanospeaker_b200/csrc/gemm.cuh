@@ -68,6 +68,9 @@ struct RowsArgs {
   // sum_groups * num_k stages.
   int32_t sum_groups;
   const int32_t* sum_offsets;
+  int32_t beside_rows;         // CTA-pair kernel with an adding epilogue: after the routed runs, one more
+  int32_t beside_k;            // product of beside_k stages over beside_rows token rows in order (the
+                               // second A and B maps; 0 rows = none), added like the rest
   const __nv_bfloat16* addend; // group-summed schedule, SCALE: [rows_host, ld_out] added to the result
   int32_t b_fused;             // MN-major B: the maps are 4-D (64 n, k, n / 64, group) and one copy
                                // brings all BN / 64 boxes of a stage (a TMA instruction costs the

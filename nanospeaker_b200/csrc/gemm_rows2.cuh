@@ -114,7 +114,7 @@ struct Rows2Smem {
   static constexpr int PART_OFFSET = MISC_OFFSET + 16;
   static constexpr int RED_TOK_OFFSET = PART_OFFSET + 128 * 4;
   static constexpr int TABLE_OFFSET = RED_TOK_OFFSET + 2 * 128 * 4;   // pair_first, run_start
-  static constexpr int WALK_OFFSET = TABLE_OFFSET + 2 * (ROWS2_MAX_GROUPS + 1) * 4;   // the first unit
+  static constexpr int WALK_OFFSET = TABLE_OFFSET + 2 * (ROWS2_MAX_GROUPS + 2) * 4;   // the first unit
   static constexpr int TOTAL = WALK_OFFSET + 32;
   static constexpr int DYNAMIC = TOTAL + 1024;
   static_assert(STAGE_BYTES % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
@@ -123,6 +123,7 @@ struct Rows2Smem {
 struct Unit2 {
   int group, m_tile, n0;
   bool valid;   // false: this CTA's half of the pair is past the end of the run
+  bool beside;  // rows of the second product
 };
 
 // Threads in the launch bound, for the registers it leaves a thread. dX is held to 96: its four warps per
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   [[maybe_unused]] float* dtw_part = reinterpret_cast<float*>(smem + L::PART_OFFSET);
   int* pair_first = reinterpret_cast<int*>(smem + L::TABLE_OFFSET);
-  int* run_start = pair_first + ROWS2_MAX_GROUPS + 1;
+  int* run_start = pair_first + ROWS2_MAX_GROUPS + 2;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -171,6 +172,8 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
   const int n_clusters = int(gridDim.x) >> 1;
   const int cluster = int(blockIdx.x) >> 1;
   const int n_groups = p.n_groups_total;
+  constexpr bool BESIDE = EPI == EPI_RAW_RED;   // token rows of a second product as run n_groups
+  const int n_runs = n_groups + (BESIDE && p.beside_rows > 0 ? 1 : 0);
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
@@ -210,8 +213,12 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
   };
   Walk* const first_unit = reinterpret_cast<Walk*>(smem + L::WALK_OFFSET);
   if (warp == 2) {
-    const int pairs = prefix_runs(load_run_ends(p.a2_offsets, n_groups, lane), n_groups, lane, pair_first,
+    int pairs = prefix_runs(load_run_ends(p.a2_offsets, n_groups, lane), n_groups, lane, pair_first,
                                   run_start, [](int rows) { return ((rows >> 7) + 1) >> 1; });
+    if (n_runs > n_groups) {
+      pairs += (p.beside_rows + 2 * BM - 1) / (2 * BM);
+      if (lane == 0) pair_first[n_runs] = pairs;
+    }
     Walk w;
     const int total = pairs * p.n_chunks, each = total / n_clusters, more = total - each * n_clusters;
     const int first = each * cluster + min(cluster, more);
@@ -220,8 +227,8 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
     w.nc = first - w.pr * p.n_chunks;
     __syncwarp();
     int at_or_before = 0;
-    for (int base = 0; base < n_groups; base += 32)
-      at_or_before += __popc(__ballot_sync(0xffffffffu, base + lane < n_groups && pair_first[base + lane] <= w.pr));
+    for (int base = 0; base < n_runs; base += 32)
+      at_or_before += __popc(__ballot_sync(0xffffffffu, base + lane < n_runs && pair_first[base + lane] <= w.pr));
     w.g = at_or_before - 1;   // the last run that starts there or before
     if (lane == 0) *first_unit = w;
   }
@@ -233,15 +240,16 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
     if (++w.nc == p.n_chunks) {
       w.nc = 0;
       ++w.pr;
-      while (w.g + 1 < n_groups && pair_first[w.g + 1] <= w.pr) ++w.g;
+      while (w.g + 1 < n_runs && pair_first[w.g + 1] <= w.pr) ++w.g;
     }
   };
   auto unit_of = [&](const Walk& w) {
     Unit2 c;
     const int blk = 2 * (w.pr - pair_first[w.g]) + int(rank);
     c.group = w.g;
-    c.m_tile = (run_start[w.g] >> 7) + blk;
-    c.valid = blk < ((run_start[w.g + 1] - run_start[w.g]) >> 7);
+    c.beside = BESIDE && w.g == n_groups;
+    c.m_tile = (c.beside ? 0 : run_start[w.g] >> 7) + blk;
+    c.valid = c.beside || blk < ((run_start[w.g + 1] - run_start[w.g]) >> 7);
     c.n0 = w.nc * BN;
     return c;
   };
@@ -272,12 +280,13 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
       uint32_t it = 0;
       for (Walk u = walk(); u.left > 0 && !*abort_flag; advance(u)) {
         const Unit2 tc = unit_of(u);
-        const bool a_alt = tc.group >= p.a2_first_group;
-        const int a_start = a_alt ? run_start[tc.group] : 0;
-        const bool first = tc.group < p.n_groups_b1;
+        const bool a_alt = tc.beside || tc.group >= p.a2_first_group;
+        const int a_start = a_alt && !tc.beside ? run_start[tc.group] : 0;
+        const bool first = tc.group < p.n_groups_b1 && !tc.beside;
         const CUtensorMap* mb = first ? &tmB : &tmB2;
-        const int gb = first ? tc.group : tc.group - p.n_groups_b1;
-        for (int kt = 0; kt < p.num_k; ++kt, ++it) {
+        const int gb = tc.beside ? 0 : first ? tc.group : tc.group - p.n_groups_b1;
+        const int num_k = tc.beside ? p.beside_k : p.num_k;
+        for (int kt = 0; kt < num_k; ++kt, ++it) {
           const int s = it % STAGES;
           const uint32_t use = it / STAGES;
           if (use > 0 && !mbar_wait(empty_bar + s, (use - 1) & 1, p.status)) {
@@ -307,7 +316,8 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
       constexpr uint32_t idesc = umma_idesc(2 * BM, BN, false, B_MN);
       uint32_t it = 0;
       int j = 0;
-      for (Walk u = walk(); u.left > 0 && !*abort_flag; --u.left, ++j) {
+      for (Walk u = walk(); u.left > 0 && !*abort_flag; advance(u), ++j) {
+        const int num_k = BESIDE && u.g == n_groups ? p.beside_k : p.num_k;
         const int b = j & 1;
         const uint32_t use = uint32_t(j) >> 1;
         if (use > 0 && !mbar_wait(tempty_bar + b, (use - 1) & 1, p.status)) {
@@ -317,7 +327,7 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + b * TMEM_BUF;
-        for (int kt = 0; kt < p.num_k; ++kt, ++it) {
+        for (int kt = 0; kt < num_k; ++kt, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait(full_bar + s, (it / STAGES) & 1, p.status)) {
             *abort_flag = 1;
@@ -404,6 +414,7 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
     auto load_pair = [&](const Walk& u) {
       if (u.left <= 0 || p.sorted_ids == nullptr) return p.n_pairs;
       const Unit2 c = unit_of(u);
+      if (c.beside) return c.m_tile * BM + row;   // a token
       return c.valid ? __ldg(p.sorted_ids + int64_t(c.m_tile) * BM + row) : p.n_pairs;
     };
     auto load_w = [&](int pr) {
@@ -449,7 +460,9 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
       } else if constexpr (EPI == EPI_RAW_RED || EPI == EPI_SCALE_RED) {
         constexpr int NB = BN / 64;
         constexpr int ROWB = red_row_bytes(BN);
-        const int tok = (row_ok && pair < p.n_pairs) ? pair / p.top_k : -1;
+        const int tok = tc.beside                          ? (pair < p.beside_rows ? pair : -1)
+                        : row_ok && pair < p.n_pairs ? pair / p.top_k
+                                                           : -1;
         if (j >= 2 && !mbar_wait(aempty_bar + b, ((uint32_t(j) >> 1) - 1) & 1, p.status))
           atomicExch(p.status, ST_WAIT_TIMEOUT);
         uint8_t* stg = smem + L::STAGING_OFFSET + b * L::RED_TILE_BYTES;

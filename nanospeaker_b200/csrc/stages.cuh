@@ -24,6 +24,14 @@ int dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, const void
 int down_gemm_sum(const void* hid, int64_t rows, int32_t k_dim, const void* w_out,
                   int32_t n_sum, int32_t d_model, const int32_t* run_offsets,
                   int64_t n_tokens, const void* addend, void* out, int32_t* status, void* stream);
+// moe_b200_dx_gemm_acc, on the routed schedule with pad_offsets also adding the router's share, dl
+// [n_tokens, ld] @ router_w^T (router_w [d_model, ld], ld a multiple of 64; dl may be null).
+int dx_gemm_acc(const void* da1, int64_t rows, int32_t d_hidden, const void* w_in,
+                int32_t n_groups, const void* w_extra, int32_t n_extra, int32_t d_model,
+                const int32_t* expert_ids, const int32_t* n_post_pad, int32_t n_fixed_groups,
+                const int32_t* sorted_ids, int64_t n_pairs, int32_t top_k, void* acc, int64_t n_tokens,
+                const int32_t* pad_offsets, const void* dl, const void* router_w, int32_t ld,
+                int32_t* status, void* stream);
 // moe_b200_wgrad with what the caller knows beside: no run is longer than max_run rows, and dw has
 // out_cols columns (other than n_dim: one fixed group of more than the rows of a chunk).
 int wgrad(const void* a, int32_t a_grouped, int32_t m_dim, const void* b,

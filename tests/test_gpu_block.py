@@ -735,3 +735,30 @@ def test_global_balance_loss_shares_sum_to_the_loss_of_the_whole_batch():
     assert torch.equal((local[0] + local[1]).cpu().long(), o.expert_counts)
     assert abs(float(shares[0] + shares[1]) - float(o.aux_loss)) < 1e-5
     assert rel_l2(torch.cat(grads), xo.grad.float()) < 2e-2
+
+
+@pytest.mark.parametrize("E,n_shared,T", [(76, 2, 4096), (76, 2, 4097), (64, 0, 4353), (8, 1, 4609)])
+def test_dx_with_the_routers_share_inside(E, n_shared, T):
+    """Past 4096 tokens dX adds the router's share as one more run of its tiles: pairs of blocks with one
+    row, a whole block and a half, and an empty second block at the end of the tokens. Against the
+    deterministic combine, which sums the same rows in fp32: each of the top_k + 2 bf16 additions rounds a
+    partial sum by at most 2^-9 of it."""
+    from nanospeaker_b200 import MoEBlock, kernels
+    torch.manual_seed(T)
+    m = MoEBlock(512, E, d_ff=192, top_k=4, n_shared=n_shared, capacity_factor=None)
+    with torch.no_grad():
+        for p_ in m.parameters():
+            p_.copy_(torch.randn_like(p_) * (p_.shape[1] ** -0.5 if p_.dim() == 3 else 0.02))
+    m = m.to(torch.bfloat16).cuda().train()
+    x, dout = (torch.randn(T, 512, device="cuda").bfloat16() for _ in range(2))
+    dx = {}
+    for mode in ("atomic", "store"):
+        m.combine_mode = mode
+        xc = x.clone().requires_grad_(True)
+        out = m(xc)
+        torch.autograd.backward([out, m.aux_loss], [dout, torch.ones_like(m.aux_loss)])
+        dx[mode] = xc.grad
+    kernels.check_status("cuda")
+    assert rel_l2(dx["atomic"], dx["store"]) < 6 * 2.0 ** -9
+    rows = (dx["atomic"].float() - dx["store"].float()).norm(dim=1) / dx["store"].float().norm(dim=1)
+    assert float(rows.max()) < 12 * 2.0 ** -9      # no row misses a share

@@ -813,13 +813,25 @@ static int64_t wgrad_items(int64_t rows, int n_groups, int routed, int ks_rows) 
   return routed ? rows / ks_rows + n_groups : int64_t(n_groups) * wgrad_chunks(int(rows), ks_rows);
 }
 
-// Rows per split-K chunk when the caller leaves the choice to the library: expert runs are cut at
-// 3072 rows (measured at T=16384, 78 experts: dW_in 98 / 82 / 78 / 72 / 75 / 89 us for chunks of
-// 1024 / 1536 / 2048 / 3072 / 4096 / 8192 rows -- shorter chunks mean more fp32 partial tiles,
-// longer ones a longer tail); on the fixed schedule (few groups, every row) the chunks are sized so that the
-// work items fill the SMs about once.
+// Rows per split-K chunk when the caller leaves the choice to the library. Expert runs are cut so that a
+// chunk is about a CTA's share of the work, which grows with the slot rows: shorter chunks mean more fp32
+// partial tiles, longer ones a longer tail behind the longest run (a shared expert's: every token). 78
+// experts, dW_in / dW_out, us:
+//   tokens (slot rows)     1024         1536         2048         3072         4096 rows a chunk
+//   2048  (26 K)       20.9 / 16.5  23.0 / 18.6  21.4 / 17.7  21.4 / 17.7  21.5 / 17.9
+//   4096  (43 K)       29.3 / 22.0  26.6 / 21.9  27.5 / 22.8  31.7 / 27.2  32.5 / 28.9
+//   8192  (75 K)       46.0 / 31.3  38.2 / 29.6  38.6 / 31.0  38.9 / 32.4  41.3 / 35.8
+//   16384 (141 K)      86.6 / 60.3  73.1 / 51.7  64.5 / 44.6  57.2 / 43.6  57.2 / 45.2
+// Below 36 K rows the pass that sums the partial tiles costs the step more (2048 graphed 159 against 164),
+// and so it does where every run would be cut (10000 tokens, 8 experts: 207 against 212): not below twice
+// the mean run.
+// On the fixed schedule (few groups, every row) the chunks are sized so that the work items fill the SMs
+// about once.
 static int auto_ks_rows(int32_t m_dim, int32_t n_dim, int64_t rows, int n_groups, int routed) {
-  if (routed) return 3072;
+  if (routed) {
+    const int64_t share = std::max<int64_t>(rows / 28, 2 * rows / n_groups);
+    return rows < 36864 ? 3072 : int(std::min<int64_t>(3072, (share + 256) / 512 * 512));
+  }
   const int bn = n_dim % 256 == 0 ? 256 : 192;
   const int64_t tiles = int64_t((m_dim + BM - 1) / BM) * ((n_dim + bn - 1) / bn) * n_groups;
   int64_t splits = sm_count() / (tiles > 0 ? tiles : 1);

@@ -184,6 +184,7 @@ struct FwdScratch {
   void *hid, *y;                  // [L, H]; [L, D] (store combine only)
   void* block_hist;
   size_t block_hist_bytes;
+  void* front;                    // of the router's front of a small batch
   float* colsum;
   size_t total;
 };
@@ -195,6 +196,7 @@ FwdScratch carve_fwd(void* p, int64_t n_tokens, int32_t d_model, int32_t d_hidde
   f.hid = c.take(size_t(z.l_cap) * d_hidden * 2);
   f.block_hist_bytes = moe_b200_router_dispatch_scratch_bytes(n_tokens, z.n_all);
   f.block_hist = c.take(f.block_hist_bytes);
+  f.front = c.take(moe::router_front_scratch_bytes(n_tokens, n_experts, n_shared));
   f.colsum = static_cast<float*>(c.take(size_t(n_experts) * 4));
   if (store) f.y = c.take(size_t(z.l_cap) * d_model * 2);
   f.total = c.used;
@@ -276,7 +278,10 @@ int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
   void* stream = st;
   int launched = 0;
   const int32_t* first_shared = f.k.pad_offsets + E;   // start of the first shared run
-  float* colsum = d.full_softmax ? f.s.colsum : nullptr;
+  // a small batch's front end reads the router weight as it is and needs nothing prepared
+  const bool front = !d.logits_in && d.router_w &&
+                     moe::router_front_covers(T, D, E, S, d.top_k, d.x, d.router_w);
+  float* colsum = d.full_softmax && !front ? f.s.colsum : nullptr;
 
   PrepArgs pa{};
   auto job = [&](const void* src, int32_t rows, int32_t cols, void* dst, int32_t dst_rows,
@@ -285,7 +290,7 @@ int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
                                   src ? rows : 0, cols, dst_rows, dst_ld};
   };
   auto below = [](void* p, int64_t values) { return static_cast<uint16_t*>(p) + values; };
-  if (d.router_w) job(d.router_w, D, E, f.k.router_wp, D, z.ld);
+  if (d.router_w && !front) job(d.router_w, D, E, f.k.router_wp, D, z.ld);
   if (f.k.bias_in) {
     job(d.b_in, E, 2 * H, f.k.bias_in, E, 2 * H);
     if (S) job(d.b_sh_in, S, 2 * H, below(f.k.bias_in, int64_t(E) * 2 * H), S, 2 * H);
@@ -301,21 +306,32 @@ int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
   }
   if (pa.n_jobs || pa.n_clear) STEP(prep(pa, st));
 
-  // router: logits GEMM against the padded weight (one fixed group, no pair weights), then
-  // routing + dispatch
-  const void* logits = d.logits_in ? d.logits_in : f.k.logits;
-  const int32_t ld = d.logits_in ? E : z.ld;
-  if (!d.logits_in)
-    STEP(moe_b200_down_gemm(d.x, T, D, f.k.router_wp, 1, nullptr, 0, z.ld, nullptr, nullptr, 1,
-                            nullptr, nullptr, 0, f.k.logits, nullptr, d.status, stream));
   const moe::FinishArgs fin{f.counts, colsum, f.aux, f.dropped, T, d.aux_coef, E, f.aux_is_16bit};
-  int n_disp = 0;
-  STEP(moe::router_dispatch(logits, ld, d.logit_bias, d.noise, T, E, d.top_k, S, d.normalize,
-                            d.full_softmax, f.k.w_all, f.k.idx_all, colsum, f.k.sorted_ids,
-                            f.k.expert_ids, f.k.pad_offsets, f.k.counts_all, f.k.n_post_pad,
-                            f.k.inv_ids, f.s.block_hist, f.s.block_hist_bytes, d.capacity, fin, d.status,
-                            stream, &n_disp));
-  launched += n_disp - 1;
+  if (front) {
+    const moe::ScatterArgs sc{f.k.counts_all, f.k.pad_offsets, f.k.n_post_pad, f.k.expert_ids,
+                              z.l_cap / 128, f.k.inv_ids, d.capacity, E, fin};
+    const moe::FrontCall fc{d.x, d.router_w, d.logit_bias, d.noise, T, D, E, S, d.top_k, d.normalize,
+                            d.full_softmax, f.k.w_all, f.k.idx_all, f.train ? f.k.logits : nullptr,
+                            f.train ? f.k.router_wp : nullptr, z.ld, f.k.sorted_ids, sc, f.s.front,
+                            d.status};
+    STEP(moe::router_front(fc, st));
+    ++launched;
+  } else {
+    // router: logits GEMM against the padded weight (one fixed group, no pair weights), then
+    // routing + dispatch
+    const void* logits = d.logits_in ? d.logits_in : f.k.logits;
+    const int32_t ld = d.logits_in ? E : z.ld;
+    if (!d.logits_in)
+      STEP(moe_b200_down_gemm(d.x, T, D, f.k.router_wp, 1, nullptr, 0, z.ld, nullptr, nullptr, 1,
+                              nullptr, nullptr, 0, f.k.logits, nullptr, d.status, stream));
+    int n_disp = 0;
+    STEP(moe::router_dispatch(logits, ld, d.logit_bias, d.noise, T, E, d.top_k, S, d.normalize,
+                              d.full_softmax, f.k.w_all, f.k.idx_all, colsum, f.k.sorted_ids,
+                              f.k.expert_ids, f.k.pad_offsets, f.k.counts_all, f.k.n_post_pad,
+                              f.k.inv_ids, f.s.block_hist, f.s.block_hist_bytes, d.capacity, fin, d.status,
+                              stream, &n_disp));
+    launched += n_disp - 1;
+  }
   // experts: up/gate + GLU, gathering the token rows itself; a training forward leaves them in slot
   // order on the way, for the weight gradients
   if (f.train) {

@@ -26,8 +26,23 @@ __device__ __forceinline__ int64_t ld_i64(const int64_t* p) {
   return SAME_KERNEL ? int64_t(__ldcg(reinterpret_cast<const long long*>(p))) : *p;
 }
 
-// One warp; total = the experts' counts.
-template <bool SAME_KERNEL>
+// The run that the 128-row tile `tile` belongs to (0 past the live rows): the last expert whose run starts
+// at or before it and is not empty there.
+__device__ __forceinline__ int32_t tile_owner(const int32_t* off, int n_experts, int32_t live, int64_t tile) {
+  const int64_t row = tile * ALIGN_M;
+  if (row >= live) return 0;
+  int lo = 0, hi = n_experts;  // invariant: off[lo] <= row < off[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (off[mid] <= row) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// One warp; total = the experts' counts. Where the column sums are: written by an earlier kernel, earlier
+// in this kernel, or in shared memory.
+enum FinishFrom { FINISH_EARLIER = 0, FINISH_SAME_KERNEL = 1, FINISH_SHARED = 2 };
+template <int FROM>
 __device__ __forceinline__ void finish_forward(const FinishArgs& f, const int32_t* total,
                                                int32_t capacity) {
   const int lane = threadIdx.x & 31;
@@ -39,7 +54,9 @@ __device__ __forceinline__ void finish_forward(const FinishArgs& f, const int32_
     if (capacity > 0) over += max(ci - capacity, 0);
     if (f.colsum != nullptr) {
       const float c = float(ci);
-      dot += c * (SAME_KERNEL ? __ldcg(f.colsum + e) : __ldg(f.colsum + e));
+      dot += c * (FROM == FINISH_SHARED        ? f.colsum[e]
+                  : FROM == FINISH_SAME_KERNEL ? __ldcg(f.colsum + e)
+                                               : __ldg(f.colsum + e));
       tot += c;
     }
   }
@@ -127,7 +144,7 @@ __device__ __forceinline__ void dispatch_scatter_body(
     (&cursor[0][0])[i] = 0;
   __syncthreads();
   if (fin.counts != nullptr && blk == 0 && warp == 1)
-    finish_forward<SAME_KERNEL>(fin, total, capacity);
+    finish_forward<SAME_KERNEL ? FINISH_SAME_KERNEL : FINISH_EARLIER>(fin, total, capacity);
   // exclusive scan of the padded run lengths (one warp, 8 consecutive experts per lane)
   if (warp == 0) {
     constexpr int PER = MAX_EXPERTS / 32;
@@ -165,18 +182,7 @@ __device__ __forceinline__ void dispatch_scatter_body(
     const int64_t per = (n_tiles_cap + nblk - 1) / nblk;
     const int64_t t_hi = per * (blk + 1) < n_tiles_cap ? per * (blk + 1) : n_tiles_cap;
     for (int64_t tile = per * blk + threadIdx.x; tile < t_hi; tile += blockDim.x) {
-      int32_t owner = 0;
-      const int64_t row = tile * ALIGN_M;
-      if (row < live) {
-        // last expert whose run starts at or before this row and is non-empty there
-        int lo = 0, hi = n_experts;  // invariant: off[lo] <= row < off[hi]
-        while (hi - lo > 1) {
-          const int mid = (lo + hi) >> 1;
-          if (off[mid] <= row) lo = mid; else hi = mid;
-        }
-        owner = lo;
-      }
-      expert_ids[tile] = owner;
+      expert_ids[tile] = tile_owner(off, n_experts, live, tile);
     }
   }
   if (n_blocks == 0) return;

@@ -73,6 +73,9 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst_smem, const void* src, 
                "r"(src_bytes)
                : "memory");
 }
+__device__ __forceinline__ void cp_async_8(uint32_t dst_smem, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst_smem), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
 }

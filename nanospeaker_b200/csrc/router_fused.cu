@@ -13,6 +13,7 @@
 #include "../../include/moe_b200.h"
 #include "pdl.cuh"
 #include "routing.cuh"
+#include "route_token.cuh"
 #include "dispatch_scatter.cuh"
 
 namespace moe {
@@ -194,38 +195,6 @@ __global__ void __launch_bounds__(WARPS * 32)
 // different order, so weights may differ in the last fp32 bit before they are rounded to bf16.
 constexpr int RF4_THREADS = 512;
 constexpr int RF4_TOKENS = RF4_THREADS / 4;   // tokens per block and pass
-constexpr int RF4_MAX_TOPK = 8;
-
-__device__ __forceinline__ float key_float(uint32_t k) {   // inverse of float_key
-  return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-}
-
-// a <- the KT largest of two descending lists of KT (max of one against the other reversed), sorted
-// again if asked: a bitonic merge, or the 12-comparator network for 6.
-template <int KT, bool SORT>
-__device__ __forceinline__ void merge_top(uint32_t (&a)[KT], const uint32_t (&b)[KT]) {
-#pragma unroll
-  for (int j = 0; j < KT; ++j) a[j] = max(a[j], b[KT - 1 - j]);
-  auto order = [&](int x, int y) {
-    const uint32_t hi = max(a[x], a[y]), lo = min(a[x], a[y]);
-    a[x] = hi;
-    a[y] = lo;
-  };
-  if constexpr (SORT && KT == 6) {
-    order(0, 5), order(1, 3), order(2, 4);
-    order(1, 2), order(3, 4);
-    order(0, 3), order(2, 5);
-    order(0, 1), order(2, 3), order(4, 5);
-    order(1, 2), order(3, 4);
-  } else if constexpr (SORT) {
-#pragma unroll
-    for (int d = KT / 2; d > 0; d >>= 1)
-#pragma unroll
-      for (int j = 0; j < KT; ++j)
-        if ((j & d) == 0) order(j, j + d);
-  }
-}
-
 // KT: the smallest of 2, 4, 6, 8 that holds top_k.
 template <int EPL, int KT, bool COLSUM>
 __global__ void __launch_bounds__(RF4_THREADS)
@@ -256,11 +225,11 @@ __global__ void __launch_bounds__(RF4_THREADS)
   }
   pdl_wait();
   const int kS = top_k + n_shared;
-  const bool need_full = full_softmax || !normalize;
+  const RouteArgs args{noise, w_all, idx_all, n_experts, top_k, n_shared, normalize, full_softmax};
   uint2* const list = lists[warp * 8 + sub];
 
   float b[EPL];
-  [[maybe_unused]] float csum[EPL];
+  float csum[COLSUM ? EPL : 1];
 #pragma unroll
   for (int i = 0; i < EPL; ++i) {
     const int e = e0 + i;
@@ -277,150 +246,9 @@ __global__ void __launch_bounds__(RF4_THREADS)
     const int64_t t = base + warp * 8 + sub;
     const bool valid = t < t_hi;
     const int64_t tc = valid ? t : t_hi - 1;   // lanes past the end repeat the last token, write nothing
-    uint32_t key[EPL];   // first the values (as float bits), then the order-preserving keys
-    float mx = -CUDART_INF_F;
-    {
-      const uint2* rp = reinterpret_cast<const uint2*>(logits + tc * ld + e0);
-      uint2 r[EPL / 4];
-#pragma unroll
-      for (int c = 0; c < EPL / 4; ++c)
-        r[c] = e0 + 4 * c < n_experts ? __ldg(rp + c) : make_uint2(0u, 0u);
-#pragma unroll
-      for (int i = 0; i < EPL; ++i) {
-        const uint32_t w = (i & 2) ? r[i / 4].y : r[i / 4].x;
-        const float f = __uint_as_float((i & 1) ? w & 0xffff0000u : w << 16);
-        float v = e0 + i < n_experts ? f + b[i] : -CUDART_INF_F;
-        if (noise != nullptr && e0 + i < n_experts)   // exploration noise, one value per (token, expert)
-          v += __ldg(noise + tc * n_experts + e0 + i);
-        key[i] = __float_as_uint(v);
-        mx = fmaxf(mx, v);
-      }
-    }
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-
-    float denom = 0.f;
-    if (need_full) {
-      float ex[EPL];
-#pragma unroll
-      for (int i = 0; i < EPL; ++i) {
-        ex[i] = (e0 + i < n_experts) ? expf(__uint_as_float(key[i]) - mx) : 0.f;
-        denom += ex[i];
-      }
-      denom += __shfl_xor_sync(0xffffffffu, denom, 1);
-      denom += __shfl_xor_sync(0xffffffffu, denom, 2);
-      if constexpr (COLSUM) {
-        const float inv = valid ? 1.f / denom : 0.f;
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) csum[i] += ex[i] * inv;
-      }
-    }
-    uint32_t top[KT];   // this lane's largest keys, descending
-#pragma unroll
-    for (int j = 0; j < KT; ++j) top[j] = 0u;
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) {
-      // (no key of a value is 0: that is what experts past the end get)
-      const uint32_t x = e0 + i < n_experts ? float_key(__uint_as_float(key[i])) : 0u;
-      key[i] = x;
-#pragma unroll
-      for (int j = KT - 1; j > 0; --j)
-        if (j <= i) top[j] = max(top[j], min(top[j - 1], x));
-      top[0] = max(top[0], x);
-    }
-    {
-      uint32_t other[KT];
-#pragma unroll
-      for (int j = 0; j < KT; ++j) other[j] = __shfl_xor_sync(0xffffffffu, top[j], 1);
-      merge_top<KT, true>(top, other);
-#pragma unroll
-      for (int j = 0; j < KT; ++j) other[j] = __shfl_xor_sync(0xffffffffu, top[j], 2);
-      merge_top<KT, true>(top, other);
-    }
-    uint32_t last = 0xFFFFFFFFu;   // the smallest key that is in
-#pragma unroll
-    for (int j = 0; j < KT; ++j) last = min(last, j < top_k ? top[j] : 0xFFFFFFFFu);
-
-    uint32_t in = 0u;   // this lane's experts that are in
-#pragma unroll
-    for (int i = 0; i < EPL; ++i)
-      if (key[i] >= last) in |= 1u << i;
-    int n = __popc(in);
-    int total = n + __shfl_xor_sync(0xffffffffu, n, 1);
-    total += __shfl_xor_sync(0xffffffffu, total, 2);
-    if (__any_sync(0xffffffffu, total > top_k)) {
-      // more ties for the last place than places: the highest experts among them are out
-      uint32_t tie = 0u;
-#pragma unroll
-      for (int i = 0; i < EPL; ++i)
-        if (key[i] == last) tie |= 1u << i;
-      const int nt = __popc(tie);
-      int over = total - top_k;
-#pragma unroll
-      for (int k = 3; k > 0; --k) {   // what the lanes above take
-        const int up = __shfl_sync(0xffffffffu, nt, (lane & ~3) + k);
-        if (k > q) over -= up;
-      }
-      for (over = min(over, nt); over > 0; --over) {
-        const uint32_t bit = 0x80000000u >> __clz(tie);
-        tie ^= bit;
-        in ^= bit;
-      }
-      n = __popc(in);
-    }
-    int pos = n;
-    {
-      const int u1 = __shfl_up_sync(0xffffffffu, pos, 1);
-      if (q >= 1) pos += u1;
-      const int u2 = __shfl_up_sync(0xffffffffu, pos, 2);
-      if (q >= 2) pos += u2;
-      pos -= n;
-    }
-    __syncwarp();   // the previous token's list has been read
-#pragma unroll
-    for (int i = 0; i < EPL; ++i)
-      if (in >> i & 1u) list[pos++] = make_uint2(key[i], uint32_t(e0 + i));
-    __syncwarp();
-
-    // lane q ranks entries q and q + 4: by value descending, then by index
-    uint2 cand[KT];
-#pragma unroll
-    for (int j = 0; j < KT; ++j) cand[j] = j < top_k ? list[j] : make_uint2(0u, 0u);
-    float p[2], s = 0.f;
-    int rank[2], ei[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int me = q + 4 * h;
-      const bool mine = me < top_k;
-      const uint2 c = mine ? list[me] : make_uint2(0u, 0u);
-      const float val = key_float(c.x);
-      p[h] = !mine ? 0.f : need_full ? expf(val - mx) / denom : expf(val - mx);
-      s += p[h];
-      ei[h] = int(c.y);
-      rank[h] = 0;
-#pragma unroll
-      for (int j = 0; j < KT; ++j)
-        if (cand[j].x > c.x || (cand[j].x == c.x && j < me)) ++rank[h];
-    }
-    if (!need_full || (normalize && top_k > 1 && full_softmax)) {
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      s += __shfl_xor_sync(0xffffffffu, s, 2);
-      p[0] = p[0] / s;
-      p[1] = p[1] / s;
-    }
-    if (valid) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-        if (q + 4 * h < top_k) {
-          w_all[t * kS + rank[h]] = __float2bfloat16(p[h]);
-          idx_all[t * kS + rank[h]] = ei[h];
-          if (chunked) atomicAdd(&hist[ei[h]], 1);
-        }
-      for (int jj = top_k + q; jj < kS; jj += 4) {   // the shared experts: every token, weight 1
-        w_all[t * kS + jj] = __float2bfloat16(1.f);
-        idx_all[t * kS + jj] = n_experts + (jj - top_k);
-      }
-    }
+    route_token<EPL, KT, COLSUM>(
+        args, [&](int e) { return __ldg(reinterpret_cast<const uint2*>(logits + tc * ld + e)); }, t, tc,
+        valid, b, csum, list, chunked ? hist : nullptr);
   }
 
   if constexpr (COLSUM) {
@@ -474,8 +302,7 @@ static int rf4_experts_per_lane(const void* logits, int ld, int n_experts, int t
   if (top_k > RF4_MAX_TOPK || ld % 4 != 0 || ld < (n_experts + 3) / 4 * 4 ||
       (reinterpret_cast<uintptr_t>(logits) & 7u) != 0)
     return 0;
-  return n_experts <= 32 ? 8 : n_experts <= 64 ? 16 : n_experts <= 80 ? 20 : n_experts <= 96 ? 24
-         : n_experts <= 128 ? 32 : 0;
+  return rf4_lane_experts(n_experts);
 }
 
 // A cluster that routes and dispatches alone. 16 blocks (2048 tokens) are past the portable size and

@@ -69,6 +69,26 @@ int router_dispatch(const void* logits, int32_t ld, const float* bias, const flo
                     int32_t* counts, int32_t* n_post_pad, int32_t* inv_ids, void* scratch,
                     size_t scratch_bytes, int32_t capacity, const FinishArgs& fin, int32_t* status,
                     void* stream, int* launches);
+// router_front.cu: everything up to the plan for a small batch, from the token rows and the router weight
+// [D, E] as it is. Two launches; results as of the logits GEMM and router_dispatch.
+struct FrontCall {
+  const void *x, *router_w;
+  const float *bias, *noise;
+  int64_t n_tokens;
+  int32_t d_model, n_experts, n_shared, top_k, normalize, full_softmax;
+  void* w_all;
+  int64_t* idx_all;
+  void *logits, *w_padded;   // [T, ld], [D, ld] with zeros past E: for a backward; null: not written
+  int32_t ld;
+  int32_t* sorted_ids;
+  ScatterArgs scatter;       // its n_tiles_cap tells l_cap
+  void* scratch;
+  int32_t* status;
+};
+bool router_front_covers(int64_t n_tokens, int32_t d_model, int32_t n_experts, int32_t n_shared,
+                         int32_t top_k, const void* x, const void* router_w);
+size_t router_front_scratch_bytes(int64_t n_tokens, int32_t n_experts, int32_t n_shared);
+int router_front(const FrontCall& c, cudaStream_t st);
 // router_fused.cu: moe_b200_router_fused_bwd with two more inputs. extra_dw [T, extra_ld] bf16: what
 // d(topk_w) of a pair gains, read at its expert's column; inv_ids [T * (k + S)]: pairs without a slot
 // (dropped by a capacity) have no d(topk_w). Either may be null.

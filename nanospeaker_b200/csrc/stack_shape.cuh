@@ -4,7 +4,8 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <mutex>
+
+#include "per_device.cuh"
 
 #ifdef __CUDACC__
 #define MOE_STACK_FN __host__ __device__ inline
@@ -82,23 +83,6 @@ struct StackDevice {
   int sms = 0, blocks_per_sm = 0;
   bool cooperative = false;
   int grid() const { return cooperative && blocks_per_sm > 0 ? sms : 0; }   // 0: cannot be launched
-};
-
-// One value per device, made on first use.
-template <typename T>
-class PerDevice {
- public:
-  template <typename Make>
-  const T* get(int device, Make make) {   // null: no such device
-    if (device < 0 || device >= MAX) return nullptr;
-    std::call_once(once_[device], [&] { value_[device] = make(device); });
-    return value_ + device;
-  }
-
- private:
-  static constexpr int MAX = 64;
-  std::once_flag once_[MAX];
-  T value_[MAX];
 };
 
 // The shape side of a launch; false: the layer-by-layer path is the one that takes it.

@@ -762,3 +762,48 @@ def test_dx_with_the_routers_share_inside(E, n_shared, T):
     assert rel_l2(dx["atomic"], dx["store"]) < 6 * 2.0 ** -9
     rows = (dx["atomic"].float() - dx["store"].float()).norm(dim=1) / dx["store"].float().norm(dim=1)
     assert float(rows.max()) < 12 * 2.0 ** -9      # no row misses a share
+
+
+@pytest.mark.parametrize("T,D,E,k,S,norm,full,noise", [
+    (1, 576, 76, 6, 2, True, True, False),       # one token: a block with 15 empty rows
+    (15, 64, 4, 4, 0, True, False, False),       # the smallest shape, every expert chosen
+    (16, 576, 80, 8, 1, False, False, True),     # a full block; softmax over all experts without the loss
+    (17, 1024, 64, 1, 2, True, True, True),      # a second block with one token
+    (300, 256, 36, 3, 3, True, True, True),
+    (2047, 512, 96, 5, 0, False, True, False),
+    (2048, 576, 128, 8, 2, True, True, False),   # as many blocks as the plan takes
+])
+def test_small_front_equals_the_general_path(T, D, E, k, S, norm, full, noise):
+    """Up to 2048 tokens the block forms its logits, routes and dispatches in two launches of their own.
+    Against the stage sequence (padded weight, logits GEMM, router and dispatch): every tensor of the plan,
+    the logits and the weights bit-equal, ties (repeated expert columns, a token of zeros) included; the
+    balance loss sums the same probabilities in another order."""
+    from nanospeaker_b200 import moe_kernel as MK, kernels
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    w = (rnd(D, E) * 0.05).bfloat16()
+    w[:, E // 2] = w[:, 0]
+    x = rnd(T, D).bfloat16()
+    x[0] = 0
+    wi, wo = (rnd(E, D, 256) * D ** -0.5).bfloat16(), (rnd(E, 128, D) * 0.09).bfloat16()
+    si, so = ((rnd(S, D, 256) * D ** -0.5).bfloat16(), (rnd(S, 128, D) * 0.09).bfloat16()) if S else (None, None)
+    args = (x, w, rnd(E) * 0.3, wi, wo, si, so, k, norm, full, 0.01, "silu", True,
+            None, True, rnd(T, E) * 0.1 if noise else None, False)
+    res = {}
+    with torch.no_grad():
+        for one in (True, False):
+            MK._ONE_CALL = one
+            try:
+                res[one] = torch.ops.moe_b200.moe_block(*args)
+            finally:
+                MK._ONE_CALL = True
+    kernels.check_status("cuda")
+    a, b = res[True], res[False]
+    live = int(a[12].item())
+    assert live == int(b[12].item())
+    for i in (2, 5, 6, 7, 10, 11, 13):   # counts, logits, weights, experts, offsets, counts of all, inverse
+        assert torch.equal(a[i], b[i]), i
+    assert torch.equal(a[8][:live], b[8][:live]) and torch.equal(a[9][: live // 128], b[9][: live // 128])
+    # |sum of T fp32 terms in another order| <= T 2^-24 of the sum
+    assert abs(float(a[1]) - float(b[1])) <= max(T, 64) * 2.0 ** -23 * abs(float(b[1]))
+    assert rel_l2(a[0], b[0]) < ATOMIC_TOL * (k + S) / 3

@@ -179,12 +179,23 @@ Kept carve_kept(void* p, int64_t n_tokens, int32_t d_model, int32_t d_hidden, in
   return k;
 }
 
+// From this many tokens on the inference forward's GEMMs walk the tiles token window by token window instead
+// of expert by expert (FinishArgs::order): a token's k rows are then gathered, and added to, while the token's
+// row is in L2. 2048 tokens to a window.
+constexpr int64_t ORDERED_TOKENS = 32768;
+inline int32_t order_windows(int64_t n_tokens) {
+  int32_t w = 1;
+  while (w < 4096 && int64_t(w) * 2 * 2048 <= n_tokens) w *= 2;
+  return w;
+}
+
 // Scratch of the forward: dead when it returns.
 struct FwdScratch {
   void *hid, *y;                  // [L, H]; [L, D] (store combine only)
   void* block_hist;
   size_t block_hist_bytes;
   void* front;                    // of the router's front of a small batch
+  int2* order;                    // [L / 128] the tiles' order (large batches only)
   float* colsum;
   size_t total;
 };
@@ -197,6 +208,7 @@ FwdScratch carve_fwd(void* p, int64_t n_tokens, int32_t d_model, int32_t d_hidde
   f.block_hist_bytes = moe_b200_router_dispatch_scratch_bytes(n_tokens, z.n_all);
   f.block_hist = c.take(f.block_hist_bytes);
   f.front = c.take(moe::router_front_scratch_bytes(n_tokens, n_experts, n_shared));
+  if (n_tokens >= ORDERED_TOKENS) f.order = static_cast<int2*>(c.take(size_t(z.l_cap / 128 + 1) * 8));
   f.colsum = static_cast<float*>(c.take(size_t(n_experts) * 4));
   if (store) f.y = c.take(size_t(z.l_cap) * d_model * 2);
   f.total = c.used;
@@ -306,7 +318,9 @@ int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
   }
   if (pa.n_jobs || pa.n_clear) STEP(prep(pa, st));
 
-  const moe::FinishArgs fin{f.counts, colsum, f.aux, f.dropped, T, d.aux_coef, E, f.aux_is_16bit};
+  int2* const order = f.train || !f.counts ? nullptr : f.s.order;
+  const moe::FinishArgs fin{f.counts, colsum, f.aux, f.dropped, T, d.aux_coef, E, f.aux_is_16bit,
+                            order, order_windows(T)};
   if (front) {
     const moe::ScatterArgs sc{f.k.counts_all, f.k.pad_offsets, f.k.n_post_pad, f.k.expert_ids,
                               z.l_cap / 128, f.k.inv_ids, d.capacity, E, fin};
@@ -337,12 +351,11 @@ int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
   if (f.train) {
     STEP(moe::up_gemm(d.x, z.l_cap, D, d.w_in, E, d.w_sh_in, S, H, f.k.expert_ids, f.k.n_post_pad, 0,
                       f.k.sorted_ids, z.ks, z.m, d.activation, f.s.hid, f.k.a1, S ? d.x : nullptr,
-                      S ? T : 0, f.k.pad_offsets, f.k.bias_in, f.k.xs, d.status, stream));
+                      S ? T : 0, f.k.pad_offsets, f.k.bias_in, f.k.xs, nullptr, d.status, stream));
   } else {
-    STEP(moe_b200_up_gemm(d.x, z.l_cap, D, d.w_in, E, d.w_sh_in, S, H, f.k.expert_ids,
-                          f.k.n_post_pad, 0, f.k.sorted_ids, z.ks, z.m, d.activation, f.s.hid,
-                          nullptr, S ? d.x : nullptr, S ? T : 0, f.k.pad_offsets, f.k.bias_in,
-                          d.status, stream));
+    STEP(moe::up_gemm(d.x, z.l_cap, D, d.w_in, E, d.w_sh_in, S, H, f.k.expert_ids, f.k.n_post_pad, 0,
+                      f.k.sorted_ids, z.ks, z.m, d.activation, f.s.hid, nullptr, S ? d.x : nullptr,
+                      S ? T : 0, f.k.pad_offsets, f.k.bias_in, nullptr, order, d.status, stream));
   }
   // down + combine
   if (d.store_combine) {
@@ -354,15 +367,15 @@ int run_forward(const Fwd& f, int32_t* n_launches, cudaStream_t st) {
     // the shared experts' share, and the residual, stored, are the accumulator's first value
     STEP(moe::down_gemm_sum(f.s.hid, z.l_cap, H, d.w_sh_out, S, D, first_shared, T, d.residual,
                             f.out, d.status, stream));
-    STEP(moe_b200_down_gemm_acc(f.s.hid, z.l_cap, H, d.w_out, E, nullptr, 0, D, f.k.expert_ids,
-                                first_shared, 0, f.k.sorted_ids, f.k.w_all, z.m, z.ks, f.out, T,
-                                nullptr, d.status, stream));
+    STEP(moe::down_gemm_acc(f.s.hid, z.l_cap, H, d.w_out, E, nullptr, 0, D, f.k.expert_ids, first_shared, 0,
+                            f.k.sorted_ids, f.k.w_all, z.m, z.ks, f.out, T, nullptr, order, d.status,
+                            stream));
   } else {
     if (d.residual) STEP(copy_words(d.residual, f.out, T * D / 2, st));
     else STEP(zero_words(f.out, T * D / 2, st));
-    STEP(moe_b200_down_gemm_acc(f.s.hid, z.l_cap, H, d.w_out, E, d.w_sh_out, S, D,
-                                f.k.expert_ids, f.k.n_post_pad, 0, f.k.sorted_ids, f.k.w_all, z.m,
-                                z.ks, f.out, T, f.k.bias_out, d.status, stream));
+    STEP(moe::down_gemm_acc(f.s.hid, z.l_cap, H, d.w_out, E, d.w_sh_out, S, D, f.k.expert_ids,
+                            f.k.n_post_pad, 0, f.k.sorted_ids, f.k.w_all, z.m, z.ks, f.out, T,
+                            f.k.bias_out, order, d.status, stream));
   }
   if (n_launches) *n_launches = launched;
   return MOE_B200_OK;

@@ -182,7 +182,26 @@ __device__ __forceinline__ void dispatch_scatter_body(
     const int64_t per = (n_tiles_cap + nblk - 1) / nblk;
     const int64_t t_hi = per * (blk + 1) < n_tiles_cap ? per * (blk + 1) : n_tiles_cap;
     for (int64_t tile = per * blk + threadIdx.x; tile < t_hi; tile += blockDim.x) {
-      expert_ids[tile] = tile_owner(off, n_experts, live, tile);
+      const int32_t owner = tile_owner(off, n_experts, live, tile);
+      expert_ids[tile] = owner;
+      if (fin.order != nullptr && tile * ALIGN_M < live) {
+        // tiles of expert e before window w: ceil(w * n_e / windows)
+        int32_t pos = int32_t(tile);
+        if (owner < fin.n_experts) {
+          const int sh = __ffs(fin.windows) - 1;
+          auto tiles_of = [&](int e) { return (off[e + 1] - off[e]) / ALIGN_M; };
+          auto up_to = [&](int n, int w) { return int32_t((int64_t(w) * n + fin.windows - 1) >> sh); };
+          const int i = int(tile) - off[owner] / ALIGN_M, n_mine = tiles_of(owner);
+          const int w = int((int64_t(i) << sh) / n_mine);
+          pos = i - up_to(n_mine, w);
+          for (int e = 0; e < fin.n_experts; ++e) {
+            const int n = tiles_of(e);
+            pos += up_to(n, w);
+            if (e < owner) pos += up_to(n, w + 1) - up_to(n, w);
+          }
+        }
+        fin.order[pos] = make_int2(int(tile), owner);
+      }
     }
   }
   if (n_blocks == 0) return;

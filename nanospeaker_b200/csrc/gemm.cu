@@ -283,7 +283,7 @@ int up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w_in, int3
             const int32_t* n_post_pad, int32_t n_fixed_groups, const int32_t* sorted_ids,
             int32_t gather_top_k, int64_t n_pairs, int32_t activation, void* hid, void* raw,
             const void* a_tokens, int64_t n_tokens, const int32_t* pad_offsets, const void* bias,
-            void* rows_out, int32_t* status, void* stream) {
+            void* rows_out, const int2* order, int32_t* status, void* stream) {
   CHECK_SCHED();
   if (bias && (n_fixed_groups > 0 || (reinterpret_cast<uintptr_t>(bias) & 15u) != 0))
     return n_fixed_groups > 0 ? MOE_B200_ERR_SHAPE : MOE_B200_ERR_ALIGN;
@@ -321,6 +321,7 @@ int up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w_in, int3
   g.out2 = static_cast<__nv_bfloat16*>(raw);
   g.out2_gstride = rows * int64_t(2 * d_hidden);
   g.act = activation;
+  g.order = n_fixed_groups == 0 ? order : nullptr;
   g.bias = static_cast<const __nv_bfloat16*>(bias);
   g.n_groups_b1 = n_extra > 0 ? n_groups : INT32_MAX;
   g.sorted_ids = sorted_ids;
@@ -370,7 +371,7 @@ int moe_b200_up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w
                      int32_t* status, void* stream) {
   return up_gemm(a, rows, d_model, w_in, n_groups, w_extra, n_extra, d_hidden, expert_ids,
                  n_post_pad, n_fixed_groups, sorted_ids, gather_top_k, n_pairs, activation, hid, raw,
-                 a_tokens, n_tokens, pad_offsets, bias, nullptr, status, stream);
+                 a_tokens, n_tokens, pad_offsets, bias, nullptr, nullptr, status, stream);
 }
 
 int moe_b200_up_gemm_keep(const void* a, int64_t rows, int32_t d_model, const void* w_in,
@@ -384,7 +385,7 @@ int moe_b200_up_gemm_keep(const void* a, int64_t rows, int32_t d_model, const vo
   if (gather_top_k < 1) return MOE_B200_ERR_SHAPE;
   return up_gemm(a, rows, d_model, w_in, n_groups, w_extra, n_extra, d_hidden, expert_ids,
                  n_post_pad, 0, sorted_ids, gather_top_k, n_pairs, activation, hid, raw, a_tokens,
-                 n_tokens, pad_offsets, bias, rows_out, status, stream);
+                 n_tokens, pad_offsets, bias, rows_out, nullptr, status, stream);
 }
 
 int moe_b200_down_gemm(const void* hid, int64_t rows, int32_t k_dim, const void* w_out,
@@ -677,12 +678,15 @@ static int check_acc(int32_t n_fixed_groups, int64_t rows, const int32_t* sorted
   return MOE_B200_OK;
 }
 
-int moe_b200_down_gemm_acc(const void* hid, int64_t rows, int32_t k_dim, const void* w_out,
-                           int32_t n_groups, const void* w_extra, int32_t n_extra, int32_t d_model,
-                           const int32_t* expert_ids, const int32_t* n_post_pad,
-                           int32_t n_fixed_groups, const int32_t* sorted_ids, const void* pair_w,
-                           int64_t n_pairs, int32_t top_k, void* acc, int64_t n_tokens,
-                           const void* bias, int32_t* status, void* stream) {
+}  // extern "C"
+
+namespace moe {
+
+int down_gemm_acc(const void* hid, int64_t rows, int32_t k_dim, const void* w_out, int32_t n_groups,
+                  const void* w_extra, int32_t n_extra, int32_t d_model, const int32_t* expert_ids,
+                  const int32_t* n_post_pad, int32_t n_fixed_groups, const int32_t* sorted_ids,
+                  const void* pair_w, int64_t n_pairs, int32_t top_k, void* acc, int64_t n_tokens,
+                  const void* bias, const int2* order, int32_t* status, void* stream) {
   CHECK_SCHED();
   if (bias && (n_fixed_groups > 0 || (reinterpret_cast<uintptr_t>(bias) & 15u) != 0))
     return n_fixed_groups > 0 ? MOE_B200_ERR_SHAPE : MOE_B200_ERR_ALIGN;
@@ -714,10 +718,26 @@ int moe_b200_down_gemm_acc(const void* hid, int64_t rows, int32_t k_dim, const v
   g.bias = static_cast<const __nv_bfloat16*>(bias);
   g.out = static_cast<__nv_bfloat16*>(acc);
   g.ld_out = d_model;
+  g.order = n_fixed_groups == 0 ? order : nullptr;
   g.n_groups_b1 = n_extra > 0 ? n_groups : INT32_MAX;
   return launch_rows<192, MOE_RED_DOWN_STAGES, true, EPI_SCALE_RED, GATHER_NO, MOE_RED_DOWN_BUFS>(
       tmA, tmB, tmB2, tmB, g, max_tiles(rows, g.n_chunks, n_fixed_groups),
       static_cast<cudaStream_t>(stream));
+}
+
+}  // namespace moe
+
+extern "C" {
+
+int moe_b200_down_gemm_acc(const void* hid, int64_t rows, int32_t k_dim, const void* w_out,
+                           int32_t n_groups, const void* w_extra, int32_t n_extra, int32_t d_model,
+                           const int32_t* expert_ids, const int32_t* n_post_pad,
+                           int32_t n_fixed_groups, const int32_t* sorted_ids, const void* pair_w,
+                           int64_t n_pairs, int32_t top_k, void* acc, int64_t n_tokens,
+                           const void* bias, int32_t* status, void* stream) {
+  return down_gemm_acc(hid, rows, k_dim, w_out, n_groups, w_extra, n_extra, d_model, expert_ids, n_post_pad,
+                       n_fixed_groups, sorted_ids, pair_w, n_pairs, top_k, acc, n_tokens, bias, nullptr,
+                       status, stream);
 }
 
 }  // extern "C"

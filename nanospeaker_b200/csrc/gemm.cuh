@@ -40,6 +40,8 @@ constexpr uint32_t MN_LBO = 8192u, MN_SBO = 1024u, MN_KADV = 2048u;
 struct RowsArgs {
   // schedule
   const int32_t* expert_ids;   // routed: [tiles] owner of each 128-row block
+  const int2* order;           // routed: [tiles] (128-row block, owner) in the order to be walked; null: as
+                               // they lie
   const int32_t* n_post_pad;   // routed: device scalar, live padded rows
   const int32_t* sorted_ids;   // routed: slot -> pair id, sentinel n_pairs in pad slots (may be null)
   int32_t n_fixed_groups;      // 0 = routed schedule; > 0 = groups 0..n-1, each over rows_host rows in

@@ -72,26 +72,32 @@ struct TileCoord {
   int m_tile, n0, group, z;
 };
 
-// t -> (group slice z, 128-row block, N chunk); N chunks of one row block are adjacent so its A
-// tile is still in L2 for the next chunk.
-__device__ __forceinline__ TileCoord decode_tile(const RowsArgs& p, int t, int m_tiles, int bn,
-                                                 bool want_group = true) {
-  TileCoord c;
-  const int nc = t % p.n_chunks;
+// The row block of tile t and its owner (or fixed group); N chunks of one row block are adjacent so its A
+// tile is still in L2 for the next chunk. Owner -1 past the end of the list. The producers ask for the tiles
+// after the next while they work on the current one: this is a global load, and what it leads to another,
+// whose latencies would otherwise sit at the head of every tile.
+struct TileRef {
+  int m_tile, group;
+};
+__device__ __forceinline__ TileRef tile_ref(const RowsArgs& p, int t, int m_tiles, int total_tiles) {
+  if (t >= total_tiles) return TileRef{0, -1};
   const int rest = t / p.n_chunks;
-  c.m_tile = rest % m_tiles;
-  c.z = rest / m_tiles;
-  c.n0 = nc * bn;
-  c.group = !want_group ? -1 : p.n_fixed_groups > 0 ? c.z : __ldg(p.expert_ids + c.m_tile);
-  return c;
+  if (p.n_fixed_groups > 0) return TileRef{rest % m_tiles, rest / m_tiles};
+  if (p.order != nullptr) {
+    const int2 r = __ldg(p.order + rest);
+    return TileRef{r.x, r.y};
+  }
+  return TileRef{rest, __ldg(p.expert_ids + rest)};
 }
-// The owner of tile t alone (-1 past the end of the list). The producers ask for the next tile's
-// owner while they work on the current one: the lookup is a global load whose latency would
-// otherwise sit at the head of every tile.
-__device__ __forceinline__ int tile_group(const RowsArgs& p, int t, int m_tiles, int total_tiles) {
-  if (t >= total_tiles) return -1;
+// t -> (group slice z, 128-row block, N chunk), without the owner of a routed tile.
+__device__ __forceinline__ TileCoord decode_tile(const RowsArgs& p, int t, int m_tiles, int bn) {
+  TileCoord c;
   const int rest = t / p.n_chunks;
-  return p.n_fixed_groups > 0 ? rest / m_tiles : __ldg(p.expert_ids + rest % m_tiles);
+  c.z = p.n_fixed_groups > 0 ? rest / m_tiles : 0;
+  c.m_tile = p.n_fixed_groups > 0 ? rest - c.z * m_tiles : p.order != nullptr ? __ldg(&p.order[rest].x) : rest;
+  c.n0 = (t - rest * p.n_chunks) * bn;
+  c.group = -1;
+  return c;
 }
 
 // v[0..31] += bias[0..31] (bf16, 16-byte aligned; the same address in every lane: a broadcast load)
@@ -291,11 +297,11 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
     // 4096, 30 -> 20 at 512; the backward's dHidden 90 -> 83, 30 -> 27, 22 -> 15.
     if (elect_one()) {
       uint32_t it = 0;
-      int group_next = tile_group(p, blockIdx.x, m_tiles, total_tiles);
+      TileRef next = tile_ref(p, blockIdx.x, m_tiles, total_tiles);
       for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
-        const TileCoord tc = decode_tile(p, t, m_tiles, BN, false);
-        const bool a_alt = group_next >= p.a2_first_group;
-        group_next = tile_group(p, t + gridDim.x, m_tiles, total_tiles);
+        const TileRef tc = next;
+        const bool a_alt = tc.group >= p.a2_first_group;
+        next = tile_ref(p, t + gridDim.x, m_tiles, total_tiles);
         for (int kt = 0; kt < p.num_k; ++kt, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait(full_bar + s, (it / STAGES) & 1, p.status)) {
@@ -333,19 +339,19 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
     const int gw = warp - (2 + EPI_WARPS);
     uint32_t it = 0;
     const int r4 = lane >> 3, c = lane & 7;
-    // the next tile's owner and pairs are fetched with the current tile
-    auto load_pair = [&](int t) {
-      return t < total_tiles
-                 ? __ldg(p.sorted_ids + int64_t((t / p.n_chunks) % m_tiles) * BM + gw * 32 + lane)
-                 : p.n_pairs;
+    // the next tile's pairs are fetched with the current tile, the place of the one after that, too
+    auto load_pair = [&](const TileRef& r) {
+      return r.group >= 0 ? __ldg(p.sorted_ids + int64_t(r.m_tile) * BM + gw * 32 + lane) : p.n_pairs;
     };
-    int group_next = tile_group(p, blockIdx.x, m_tiles, total_tiles);
-    int pair_next = load_pair(blockIdx.x);
+    TileRef next = tile_ref(p, blockIdx.x, m_tiles, total_tiles);
+    TileRef after = tile_ref(p, blockIdx.x + gridDim.x, m_tiles, total_tiles);
+    int pair_next = load_pair(next);
     for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
-      const bool a_alt = group_next >= p.a2_first_group;
+      const bool a_alt = next.group >= p.a2_first_group;
       const int my_tok = pair_next < p.n_pairs ? pair_next / p.top_k : -1;  // of row gw * 32 + lane
-      group_next = tile_group(p, t + gridDim.x, m_tiles, total_tiles);
-      pair_next = load_pair(t + gridDim.x);
+      next = after;
+      pair_next = load_pair(next);
+      after = tile_ref(p, t + 2 * gridDim.x, m_tiles, total_tiles);
       const __nv_bfloat16* src[8];   // rows i * 4 + r4 of this warp's 32, null: zeros
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -386,15 +392,20 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
       auto run_start_of = [&](int group) {
         return (group >= p.a2_first_group && group >= 0) ? __ldg(p.a2_offsets + group) : 0;
       };
-      int group_next = tile_group(p, blockIdx.x, m_tiles, total_tiles);
-      int start_next = run_start_of(group_next);
+      TileRef next = tile_ref(p, blockIdx.x, m_tiles, total_tiles);
+      TileRef after = tile_ref(p, blockIdx.x + gridDim.x, m_tiles, total_tiles);
+      int start_next = run_start_of(next.group);
       for (int t = blockIdx.x; t < total_tiles && !*abort_flag; t += gridDim.x) {
-        TileCoord tc = decode_tile(p, t, m_tiles, BN);
-        tc.group = group_next;
+        TileCoord tc;
+        tc.m_tile = next.m_tile;
+        tc.group = next.group;
+        tc.z = p.n_fixed_groups > 0 ? next.group : 0;
+        tc.n0 = (t % p.n_chunks) * BN;
         const int a_start = start_next;
         const bool a_alt = tc.group >= p.a2_first_group;
-        group_next = tile_group(p, t + gridDim.x, m_tiles, total_tiles);
-        start_next = run_start_of(group_next);
+        next = after;
+        start_next = run_start_of(next.group);
+        after = tile_ref(p, t + 2 * gridDim.x, m_tiles, total_tiles);
         const int k_total = p.sum_groups > 0 ? p.sum_groups * p.num_k : p.num_k;
         for (int kt = 0; kt < k_total; ++kt, ++it) {
           const int s = it % STAGES;
@@ -479,7 +490,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
       const uint64_t keep = l2_policy_evict_last();
       int j = 0;
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++j) {
-        const TileCoord tc = decode_tile(p, t, m_tiles, BN, false);
+        const TileCoord tc = decode_tile(p, t, m_tiles, BN);
         const int b = j & 1;
         if (!mbar_wait(afull_bar + b, (uint32_t(j) >> 1) & 1, p.status))
           atomicExch(p.status, ST_WAIT_TIMEOUT);
@@ -544,7 +555,8 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
     const bool fixed = p.n_fixed_groups > 0;
     auto load_pair = [&](int t) {
       if (t >= total_tiles || fixed || p.sorted_ids == nullptr) return p.n_pairs;
-      return __ldg(p.sorted_ids + int64_t((t / p.n_chunks) % m_tiles) * BM + row);
+      const int rest = t / p.n_chunks;
+      return __ldg(p.sorted_ids + int64_t(p.order != nullptr ? __ldg(&p.order[rest].x) : rest) * BM + row);
     };
     auto load_w = [&](int pr) {
       if (p.pair_w == nullptr) return 1.f;
@@ -557,7 +569,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
     int j = 0;
     [[maybe_unused]] uint32_t box_count = 0;
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++j) {
-      const TileCoord tc = decode_tile(p, t, m_tiles, BN, false);
+      const TileCoord tc = decode_tile(p, t, m_tiles, BN);
       const int b = j & 1;
       const float w_n = load_w(pair_n);                    // next tile's weight
       const int pair_nn = load_pair(t + 2 * gridDim.x);    // the pair id of the tile after that

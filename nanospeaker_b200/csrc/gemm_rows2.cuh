@@ -126,9 +126,10 @@ struct Unit2 {
   bool beside;  // rows of the second product
 };
 
-// Threads in the launch bound, for the registers it leaves a thread. dX is held to 96: its four warps per
+// Threads in the launch bound, for the registers it leaves a thread. dX is held to 80: its four warps per
 // scheduler at 114 leave no room for two warps of the router's weight gradient sums, which run beside it on
-// another stream and then came after it (training step of 16384 tokens + 15 us, 2048 graphed + 7).
+// another stream and then came after it (training step of 16384 tokens + 15 us, 2048 graphed + 7; at 96
+// registers 16384 tokens + 8).
 __host__ __device__ constexpr int rows2_bound(int epi) {
   return epi == EPI_RAW_RED ? 672 : rows_threads(epi, GATHER_NO);
 }

@@ -40,6 +40,11 @@ struct FinishArgs {
   int64_t n_tokens;
   float coef;
   int32_t n_experts, aux_is_16bit;
+  // The 128-row tiles in an order that keeps together what belongs to neighbouring tokens: a run's rows are
+  // in token order, so its tiles are cut into `windows` (a power of two) equal parts, and window by window
+  // come every routed expert's; the shared experts' tiles follow. (tile, owner); null: not made.
+  int2* order;
+  int32_t windows;
 };
 struct ScatterArgs {
   int32_t* counts;

@@ -1,6 +1,7 @@
 // Stages of the block with options that the C entry points of the same names do not have (gemm.cu).
 #pragma once
 #include <stdint.h>
+#include <vector_types.h>
 
 namespace moe {
 // moe_b200_up_gemm / moe_b200_dhidden_glu_bwd with gathered rows (gather_top_k > 0) that are also written
@@ -11,7 +12,13 @@ int up_gemm(const void* a, int64_t rows, int32_t d_model, const void* w_in, int3
             const int32_t* n_post_pad, int32_t n_fixed_groups, const int32_t* sorted_ids,
             int32_t gather_top_k, int64_t n_pairs, int32_t activation, void* hid, void* raw,
             const void* a_tokens, int64_t n_tokens, const int32_t* pad_offsets, const void* bias,
-            void* rows_out, int32_t* status, void* stream);
+            void* rows_out, const int2* order, int32_t* status, void* stream);
+// (order: FinishArgs::order, or null; moe_b200_down_gemm_acc with it:)
+int down_gemm_acc(const void* hid, int64_t rows, int32_t k_dim, const void* w_out, int32_t n_groups,
+                  const void* w_extra, int32_t n_extra, int32_t d_model, const int32_t* expert_ids,
+                  const int32_t* n_post_pad, int32_t n_fixed_groups, const int32_t* sorted_ids,
+                  const void* pair_w, int64_t n_pairs, int32_t top_k, void* acc, int64_t n_tokens,
+                  const void* bias, const int2* order, int32_t* status, void* stream);
 int dhidden_glu_bwd(const void* douts, int64_t rows, int32_t d_model, const void* w_out,
                     int32_t n_groups, const void* w_extra, int32_t n_extra,
                     int32_t d_hidden, const int32_t* expert_ids,

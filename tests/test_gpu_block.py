@@ -807,3 +807,30 @@ def test_small_front_equals_the_general_path(T, D, E, k, S, norm, full, noise):
     # |sum of T fp32 terms in another order| <= T 2^-24 of the sum
     assert abs(float(a[1]) - float(b[1])) <= max(T, 64) * 2.0 ** -23 * abs(float(b[1]))
     assert rel_l2(a[0], b[0]) < ATOMIC_TOL * (k + S) / 3
+
+
+@pytest.mark.parametrize("T,E,k,S,skew", [(32768, 8, 2, 2, 0.0), (33001, 76, 1, 0, 2.0), (40000, 5, 5, 1, 0.3)])
+def test_large_inference_walks_every_tile_once(T, E, k, S, skew):
+    """From 32768 tokens on the inference forward walks its tiles window by window: runs of unequal length,
+    empty ones, one expert with most of the tokens. Against the training forward, which walks them as they
+    lie: hidden rows and weights are the same bits, so with the deterministic combine the outputs are, and
+    with additions in L2 they differ by the order of k + 1 bf16 sums (2^-9 of the partial sum each)."""
+    from nanospeaker_b200 import MoEBlock, kernels
+    torch.manual_seed(T)
+    m = MoEBlock(256, E, d_ff=192, top_k=k, n_shared=S, capacity_factor=None)
+    with torch.no_grad():
+        for p_ in m.parameters():
+            p_.copy_(torch.randn_like(p_) * (p_.shape[1] ** -0.5 if p_.dim() == 3 else 0.02))
+    m = m.to(torch.bfloat16).cuda().eval()
+    m.router.logit_bias = torch.randn(E, device="cuda") * skew
+    x = torch.randn(T, 256, device="cuda").bfloat16()
+    for mode in ("store", "atomic"):
+        m.combine_mode = mode
+        with torch.no_grad():
+            a = m(x)
+        b = m(x).detach()      # parameters require gradients: the form that keeps its activations
+        if mode == "store":
+            assert torch.equal(a, b)
+        else:
+            assert rel_l2(a, b) < (k + 1) * 2.0 ** -9
+    kernels.check_status("cuda")

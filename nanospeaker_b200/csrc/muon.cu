@@ -190,8 +190,8 @@ __global__ void __launch_bounds__(MU_THREADS)
 // its A, s on its result).
 // What bounds it: the tensor pipe and its operand reads from shared memory; per tall iteration at
 // n = 576 2.6 us of Gram, 1.6 us of A A and 5.4 us of update MMAs at full rate.
-// Warps: 0 copies tiles in and out, 1 issues MMAs, 2..9 convert accumulators.
-constexpr int NS_EPI_WARPS = 8;
+// Warps: 0 copies tiles in and out, 1 issues MMAs, 2..17 convert accumulators.
+constexpr int NS_EPI_WARPS = 16;
 constexpr int NS_THREADS = 64 + 32 * NS_EPI_WARPS;
 constexpr uint32_t NS_BOX = 16384;
 constexpr int NS_MAX_SLOTS = 6;
@@ -430,7 +430,8 @@ struct Ns {
   static __device__ void converts(const NsJob& job, const NsJobs& js, int group, uint32_t tiles,
                                   uint32_t poly, uint32_t tmem, NsBars* bars) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int quad = warp & 3, side = (warp - 2) >> 2;     // columns of side 0 / 1 of every pair of boxes
+    // a quadrant's four warps: side 0 / 1 of every pair of boxes, half 0 / 1 of a box's columns
+    const int quad = warp & 3, side = ((warp - 2) >> 2) & 1, half = (warp - 2) >> 3;
     const int row = quad * 32 + lane;
     const uint32_t lanes = tmem + (uint32_t(quad * 32) << 16);
     const int nt = (job.length + 127) / 128;
@@ -458,11 +459,11 @@ struct Ns {
       tc_fence_after();
       if (!(s2 > 0.f))   // a norm that overflows: the direction is zero, its products may be infinite
 #pragma unroll 1
-        for (int c = 0; c < 8 * BLOCKS; ++c)
+        for (int c = 4 * half; c < 8 * BLOCKS; c += (c & 3) == 3 ? 5 : 1)
           st_shared_v4(poly + uint32_t(2 * (c >> 3) + side) * NS_BOX + uint32_t(row) * 128u + (c & 7) * 16,
                        0u, 0u, 0u, 0u);
 #pragma unroll 1
-      for (int c = s2 > 0.f ? 0 : 2 * BLOCKS; c < 2 * BLOCKS; ++c)
+      for (int c = s2 > 0.f ? half : 2 * BLOCKS; c < 2 * BLOCKS; c += 2)
         convert32<false>(lanes + uint32_t(c >> 1) * 128u + uint32_t(side) * 64u + uint32_t(c & 1) * 32u,
                          poly + uint32_t((c & ~1) + side) * NS_BOX, row, c & 1,
                          [&](float, float g) { return s2 * g; });
@@ -470,7 +471,7 @@ struct Ns {
       wait(&bars->acc_full, 1);
       tc_fence_after();
 #pragma unroll 1
-      for (int c = 0; c < 2 * BLOCKS; ++c)
+      for (int c = half; c < 2 * BLOCKS; c += 2)
         convert32<true>(lanes + uint32_t(c >> 1) * 128u + uint32_t(side) * 64u + uint32_t(c & 1) * 32u,
                         poly + uint32_t((c & ~1) + side) * NS_BOX, row, c & 1,
                         [&](float g, float g2) { return js.b * g + js.c * g2; });
@@ -486,7 +487,7 @@ struct Ns {
         const uint32_t x = tiles + uint32_t(sl) * TILE_BYTES;
         if (!TALL || quad * 32 < live) {
 #pragma unroll 1
-          for (int c = 0; c < BOXES; ++c) {
+          for (int c = half; c < BOXES; c += 2) {
             const int box = (c & ~1) + side;
             if (!TALL && box * 64 + (c & 1) * 32 >= live) continue;
             convert32<true>(d + uint32_t(box) * 64u + uint32_t(c & 1) * 32u,

@@ -380,7 +380,8 @@ def build_stages(m, x):
                                           d_aux, counts, 1e-2, ld)),
             ("router wgrad x^T@dl (gemm + reduce)", TF, 2.0 * T * D * E, 1,
              lambda i: K.wgrad(xr[i % 3], dl[i % 3], None, 1)),
-            ("router dx dl@W^T (atomic adds into dx)", TF, 2.0 * T * D * E, 1,
+            # (past 4096 tokens part of the dX launch)
+            ("router dx dl@W^T (atomic adds into dx)", TF, 2.0 * T * D * E, int(T <= 4096),
              lambda i: K.dx_gemm_acc(dl[i % 3].unsqueeze(0), wp, None, None, 1, None, 0, 1,
                                      acc[i % 3])),
         ]

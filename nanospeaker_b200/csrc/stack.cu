@@ -73,11 +73,9 @@ struct StackItem {
   int expert;        // < E routed, else shared
   int slice, t0, n;  // shared: its token block; routed: n = -1
 };
-// Up and down; the last, partial round's extra items go to the CTAs at the end, away from the shared experts'
-// items and the first tokens (with them on the first CTAs: a layer + 2 us).
-__host__ __device__ __forceinline__ int stack_position(int r, int cta, int grid, int rounds) {
-  return r * grid + ((r & 1) || (r > 0 && r == rounds - 1) ? grid - 1 - cta : cta);
-}
+__host__ __device__ __forceinline__ int stack_position(int r, int cta, int grid) {
+  return r * grid + ((r & 1) ? grid - 1 - cta : cta);   // up and down: the last, partial round's extra
+}                                                       // items go to CTAs without a shared one
 __device__ __forceinline__ StackItem stack_item(const StackArgs& p, int pos) {
   StackItem it;
   const int n_sh = p.S * ST_SLICES * p.sh_blocks;
@@ -202,7 +200,6 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   uint64_t* empty = full + ST_PARTS;                             // [ST_PARTS] their stages are free again
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.misc);
   volatile int* go_on = abort_flag + 1;   // written by compute thread 0 alone
-  volatile int* issued = abort_flag + 2;  // parts whose loads are on their way; by the TMA warp
   int* cnt = reinterpret_cast<int*>(smem + L.misc + 16);
   StackItem* items = reinterpret_cast<StackItem*>(smem + L.misc + 16 + ST_MAX_ITEMS * 4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -213,15 +210,14 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
   const int kS = p.k + p.S;
   // this CTA's items (all but the last round are full)
   const int rounds = (p.n_items + G - 1) / G;
-  const int n_mine = rounds - (stack_position(rounds - 1, cta, G, rounds) < p.n_items ? 0 : 1);
+  const int n_mine = rounds - (stack_position(rounds - 1, cta, G) < p.n_items ? 0 : 1);
 
   if (tid == 0) {
     for (int s = 0; s < 2 * ST_PARTS; ++s) mbar_init(full + s, 1);
     *abort_flag = 0;
-    *issued = 0;
     fence_mbar_init();
   }
-  if (tid < n_mine) items[tid] = stack_item(p, stack_position(tid, cta, G, rounds));
+  if (tid < n_mine) items[tid] = stack_item(p, stack_position(tid, cta, G));
   __syncthreads();
   pdl_wait();   // the counters, x and the weights may come from the kernels before this one
 
@@ -244,10 +240,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
           uint64_t* bar = full + part % ST_PARTS;
 #pragma unroll 1
           for (int c = 0; c < n && ok; ++c) {
-            if (ahead == 0) {   // this stage was part old_part's (given back unseen by an item without
-                                // tokens: its loads may still be landing)
+            if (ahead == 0) {   // this stage was part old_part's
               ok = mbar_wait(empty + old_part % ST_PARTS, (old_part / ST_PARTS) & 1, p.status) &&
-                   mbar_wait(full + old_part % ST_PARTS, (old_part / ST_PARTS) & 1, p.status) &&
                    *abort_flag == 0;
               if (!ok) break;
               ahead = old_part & 1 ? n_out : n_in;
@@ -266,13 +260,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
             }
             if (++slot == NS) slot = 0;
           }
-          if (ok) *issued = part + 1;
         }
       }
-      // nothing may still be landing when the CTA leaves
-#pragma unroll 1
-      for (; ok && old_part < part; ++old_part)
-        ok = mbar_wait(full + old_part % ST_PARTS, (old_part / ST_PARTS) & 1, p.status);
       if (!ok) {   // given up: let what is in flight land before the CTA may leave
         *abort_flag = 1;
         atomicExch(p.status, ST_WAIT_TIMEOUT);
@@ -322,14 +311,6 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
       atomicExch(p.status, ST_WAIT_TIMEOUT);
       *abort_flag = 1;
     }
-  };
-
-  // An item without tokens gives its stages back as soon as their loads are under way: waiting for them to
-  // land held up the item behind it, and the CTA's token, by 1.2 us each.
-  auto issue_wait = [&](int q) {
-#pragma unroll 1
-    for (uint32_t n = 0; *issued <= q && *abort_flag == 0; ++n)
-      if (n > (1u << 24)) *abort_flag = 1;   // (the TMA warp flags the status)
   };
 
   // router weight: a thread owns four columns (4 * (tid % P)) of every Q-th row
@@ -557,7 +538,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
 #pragma unroll 1
       for (int half = 0; half < 2; ++half, ++part) {   // up/gate, then down; each gives its stages back
         if (n == 0) {
-          if (tid == 0) issue_wait(part);
+          if (tid == 0) part_wait(part);
         } else if (half == 0) {
           // up/gate + GLU: 64 outputs (gate, up: two mma rows each) x 16 tokens; the four warps of an
           // mma row take a quarter of every 64-deep stage each

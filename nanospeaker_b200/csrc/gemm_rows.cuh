@@ -634,13 +634,14 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
                          wd[3]);
           }
           fence_proxy_async();
-          // the buffer filled next was handed to TMA OUT_BOXES - 1 stores ago: wait for that read
+          // the buffer filled next was handed to TMA OUT_BOXES - 1 boxes ago: wait for that read
           if (issuer) bulk_wait_read<OUT_BOXES - 2>();
           epi_bar_sync(EPI_WARPS * 32);
-          if (issuer && tc.n0 + jb * 64 < p.n_dim) {
-            tma_store_3d(&tmOut, smem + L::STAGING_OFFSET + (box_count % OUT_BOXES) * OUT_BOX_BYTES,
-                         tc.n0 + jb * 64, tc.m_tile * BM, tc.z);
-            bulk_commit();
+          if (issuer) {
+            if (tc.n0 + jb * 64 < p.n_dim)
+              tma_store_3d(&tmOut, smem + L::STAGING_OFFSET + (box_count % OUT_BOXES) * OUT_BOX_BYTES,
+                           tc.n0 + jb * 64, tc.m_tile * BM, tc.z);
+            bulk_commit();   // (of a box past the last column too: the wait above counts one group per box)
           }
         }
       } else if constexpr (EPI == EPI_RAW_RED || EPI == EPI_SCALE_RED) {

@@ -197,6 +197,30 @@ def test_shared_expert_schedule_on_unpermuted_tokens(T):
     K().check_status("cuda")
 
 
+@pytest.mark.parametrize("D", [64, 256, 320, 512, 576])
+def test_stored_tiles_with_columns_past_the_last_one(D):
+    """A 192-column tile leaves in three boxes of 64 columns, of which those past D are not stored (two,
+    two, one, one, none of them in a row's last tile); many tiles per CTA, so that the boxes' buffers come
+    round. Every value by itself: half a bf16 ulp (8 bits: 2^-8 of the value at most), and the fp32 sums'
+    K 2^-24 of the sum of the products' absolute values."""
+    T, H = 40000, 128
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    hid, da1 = rnd(T, H).bfloat16(), rnd(T, 2 * H).bfloat16()
+    wo, wi = (rnd(1, H, D) * H ** -0.5).bfloat16(), (rnd(1, D, 2 * H) * D ** -0.5).bfloat16()
+
+    def off(y, a, w):
+        ref, size = a.double() @ w.double(), a.double().abs() @ w.double().abs()
+        return int(((y.double() - ref).abs() > 2.0 ** -8 * ref.abs() + 3 * a.shape[1] * 2.0 ** -24 * size).sum())
+
+    for _ in range(10):
+        y, ydx = (K().down_gemm(hid, wo, None, None, 1, None, None, 0),
+                  K().dx_gemm(da1, wi, None, None, 1))
+        assert off(y[0], hid, wo[0]) == 0
+        assert off(ydx[0], da1, wi[0].t()) == 0
+    K().check_status("cuda")
+
+
 @pytest.mark.parametrize("T,S", [(1, 1), (127, 2), (300, 2), (1000, 3), (2048, 2)])
 def test_group_summed_gemms_store_the_shared_experts_share(T, S):
     """out[t] = sum_g A[offsets[g] + t] @ B_g with plain stores: the shared experts' share of the

@@ -16,7 +16,7 @@ SHIM = os.path.join(HERE, "_moe_shim.so")
 SHIM_SOURCE = "shim.cpp"
 SOURCES = ["api.cu", "routing.cu", "router_fused.cu", "router_front.cu", "movement.cu", "norm.cu", "gemm.cu", "ep.cu", "block.cu", "stack.cu",
            "muon.cu"]
-HEADERS = ["act.cuh", "agree.cuh", "stack_shape.cuh", "stages.cuh", "tma_map.cuh", "ptx.cuh", "pdl.cuh", "gemm.cuh", "gemm_rows.cuh", "gemm_rows2.cuh", "gemm_wgrad2.cuh", "gemm_wgrad.cuh", "routing.cuh", "dispatch_scatter.cuh", "route_token.cuh", "per_device.cuh", os.path.join("..", "..", "include", "moe_b200.h")]
+HEADERS = ["act.cuh", "agree.cuh", "wgrad_order.cuh", "stack_shape.cuh", "stages.cuh", "tma_map.cuh", "ptx.cuh", "pdl.cuh", "gemm.cuh", "gemm_rows.cuh", "gemm_rows2.cuh", "gemm_wgrad2.cuh", "gemm_wgrad.cuh", "routing.cuh", "dispatch_scatter.cuh", "route_token.cuh", "per_device.cuh", os.path.join("..", "..", "include", "moe_b200.h")]
 
 
 def _stale(out: str, files) -> bool:

@@ -8,9 +8,11 @@
 // that fit one chunk (the common case for routed experts) store bf16 directly and skip the second
 // pass. An empty run still owns one work item, which writes zeros.
 #pragma once
+#include "wgrad_order.cuh"
 
 namespace moe {
 
+static_assert(WGRAD_BK == BK, "a stage is one K block");
 constexpr int WGRAD_THREADS = 320;   // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
 constexpr int WGRAD_GATHER_WARPS = 4;
 constexpr int WGRAD_THREADS_GATHER = 320 + (WGRAD_GATHER_WARPS - 1) * 32;  // + producer warps 10..12
@@ -52,11 +54,6 @@ struct WgradSmem {
   static constexpr int DYNAMIC = TOTAL + 1024;
   static_assert(DYNAMIC <= 232448, "one CTA's shared memory");
 };
-
-// Number of split-K work items of a run of `rows` rows.
-__host__ __device__ __forceinline__ int wgrad_chunks(int rows, int ks_rows) {
-  return rows <= ks_rows ? 1 : (rows + ks_rows - 1) / ks_rows;
-}
 
 // Run g's start and end for g = 32 i + lane, i < 8 (one warp); every load is on its way before the first
 // is used.
@@ -127,12 +124,10 @@ __device__ __forceinline__ WgradUnit wgrad_item(const WgradArgs& p, const WgradT
   u.group = group;
   u.item = j;
   u.n_c = t.first_item[group + 1] - t.first_item[group];
-  const int start = t.run_start[group];
-  const int end = p.pad_offsets != nullptr ? t.run_start[group + 1] : p.rows_host;
-  u.row0 = start + (j - t.first_item[group]) * p.ks_rows;
-  int rows = end - u.row0;
-  rows = rows < 0 ? 0 : (rows > p.ks_rows ? p.ks_rows : rows);
-  u.num_k = (rows + BK - 1) / BK;
+  const WgradRuns runs{t.run_start, p.pad_offsets != nullptr ? -1 : p.rows_host};
+  const WgradRows w = wgrad_rows(runs, p.ks_rows, group, j - t.first_item[group]);
+  u.row0 = w.row0;
+  u.num_k = w.blocks;
   return u;
 }
 __device__ __forceinline__ int wgrad_group_of(const WgradTable& t, int n_groups, int j) {
@@ -188,10 +183,8 @@ __device__ __forceinline__ WgradWalk wgrad_plan(const WgradArgs& p, WgradTable& 
   if (walk.sorted) {
     if (p.n_groups > 8) {          // a thread per run
       for (int g = threadIdx.x; g < p.n_groups; g += blockDim.x) {
-        WgradUnit u = wgrad_item(p, t, g, t.first_item[g]);
-        const int end = t.run_start[g + 1];
-        for (int j = u.item; j < u.item + u.n_c; ++j, u.row0 += p.ks_rows) {
-          t.size[j] = (min(end - u.row0, p.ks_rows) + BK - 1) / BK;
+        for (int j = t.first_item[g]; j < t.first_item[g + 1]; ++j) {
+          t.size[j] = wgrad_item(p, t, g, j).num_k;
           t.group[j] = uint8_t(g);
         }
       }
@@ -202,7 +195,7 @@ __device__ __forceinline__ WgradWalk wgrad_plan(const WgradArgs& p, WgradTable& 
         t.group[j] = uint8_t(g);
       }
     }
-    if (threadIdx.x < 16 && n_items + threadIdx.x < WGRAD_SORT_MAX) t.size[n_items + threadIdx.x] = -1;
+    if (threadIdx.x < 3 && n_items + threadIdx.x < WGRAD_SORT_MAX) t.size[n_items + threadIdx.x] = WGRAD_NO_ITEM;
     __syncthreads();
     // four lanes per item, four others at a time
     for (int base = 0; base < n_items; base += blockDim.x / 4) {
@@ -212,8 +205,8 @@ __device__ __forceinline__ WgradWalk wgrad_plan(const WgradArgs& p, WgradTable& 
 #pragma unroll 2
       for (int k = 4 * (threadIdx.x & 3); k < n_items; k += 16) {
         const int4 o = *reinterpret_cast<const int4*>(t.size + k);
-        rank += (o.x > size || (o.x == size && k < i)) + (o.y > size || (o.y == size && k + 1 < i)) +
-                (o.z > size || (o.z == size && k + 2 < i)) + (o.w > size || (o.w == size && k + 3 < i));
+        rank += int(wgrad_before(o.x, k, size, i)) + int(wgrad_before(o.y, k + 1, size, i)) +
+                int(wgrad_before(o.z, k + 2, size, i)) + int(wgrad_before(o.w, k + 3, size, i));
       }
       rank += __shfl_xor_sync(0xffffffffu, rank, 1);
       rank += __shfl_xor_sync(0xffffffffu, rank, 2);

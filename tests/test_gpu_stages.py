@@ -276,6 +276,23 @@ def test_wgrad_split_k_is_deterministic_and_chunk_size_independent():
     K().check_status("cuda")
 
 
+@pytest.mark.parametrize("G,T,ks", [(9, 576, 256), (9, 320, 192), (10, 640, 128), (11, 577, 256), (37, 300, 64),
+                                    (8, 300, 64), (256, 300, 64)])
+@pytest.mark.parametrize("m,n", [(256, 256), (96, 192), (128, 256)])
+def test_wgrad_of_fixed_groups_cut_into_chunks(G, T, ks, m, n):
+    """The fixed schedule on either side of the eight groups from where a thread plans a run, two to five
+    chunks a run, items of every remainder by the four that are compared at a time, and more of them than are
+    sorted; on CTA pairs, and single CTAs of both tile widths. fp32 sums rounded once: 2^-8 of a value, and
+    T 2^-24 of the sum of the products' absolute values."""
+    gen = torch.Generator(device="cuda").manual_seed(G)
+    a = torch.randn(G, T, m, generator=gen, device="cuda").bfloat16()
+    b = torch.randn(G, T, n, generator=gen, device="cuda").bfloat16()
+    got = K().wgrad(a, b, None, G, ks_rows=ks, a_grouped=True, b_grouped=True)
+    ref, size = a.double().mT @ b.double(), a.double().abs().mT @ b.double().abs()
+    assert not ((got.double() - ref).abs() > 2.0 ** -8 * ref.abs() + 3 * T * 2.0 ** -24 * size).any()
+    K().check_status("cuda")
+
+
 def test_entry_points_reject_bad_arguments():
     x = torch.randn(4, 100, device="cuda").bfloat16()          # d_model % 8 != 0
     with pytest.raises(RuntimeError, match="shape|covered"):

@@ -60,6 +60,26 @@ def test_kernel_newton_schulz_matches_the_oracle(shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(10, 576, 256), (13, 576, 128), (11, 576, 256)])
+def test_kernel_newton_schulz_on_stacks_cut_into_chunks(shape):
+    """More than eight matrices whose Gram products are cut into three chunks each: 30, 39 and 33 work items.
+    Every matrix against the fp32 iteration, to the bar of the test above."""
+    from nanospeaker_b200 import kernels
+    from nanospeaker_b200.muon import _kernel_ok, newton_schulz5
+    g = (torch.randn(*shape) * 0.02).bfloat16().cuda()
+    assert _kernel_ok(g)
+    got = newton_schulz5(g).float()
+    x = g.double().mT
+    x = x / (x.norm(dim=(-2, -1), keepdim=True) + 1e-7)
+    for _ in range(5):
+        a = x @ x.mT
+        x = 3.4445 * x + (-4.7750 * a + 2.0315 * (a @ a)) @ x
+    off = (got - x.mT).norm(dim=(-2, -1)) / x.norm(dim=(-2, -1))
+    assert float(off.max()) < 3e-2
+    kernels.check_status("cuda")
+
+
+@pytest.mark.gpu
 def test_muon_step_on_the_blocks_gradients():
     """One optimizer step on a block's stacked expert weights with the gradients its backward left,
     on the GPU (kernel Newton-Schulz) against the oracle's step on the CPU."""

@@ -95,7 +95,7 @@ inline int prep(const PrepArgs& a, cudaStream_t st) {
 
 // fp32 -> bf16 (the bias gradients' last step).
 __global__ void __launch_bounds__(256)
-    to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int32_t n) {
+    to_bf16_kernel(const float* src, __nv_bfloat16* dst, int32_t n) {
   moe::pdl_trigger();
   moe::pdl_wait();
   for (int i = int(blockIdx.x * blockDim.x + threadIdx.x); i < n; i += int(gridDim.x * blockDim.x))

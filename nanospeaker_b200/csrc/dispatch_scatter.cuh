@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "pdl.cuh"
 #include "routing.cuh"
 
 namespace moe {
@@ -19,7 +20,7 @@ constexpr int DISPATCH_MAX_BLOCKS = 128;
 // L2, never through the read-only path.
 template <bool SAME_KERNEL>
 __device__ __forceinline__ int32_t ld_i32(const int32_t* p) {
-  return SAME_KERNEL ? __ldcg(p) : __ldg(p);
+  return SAME_KERNEL ? __ldcg(p) : ld_prev(p);
 }
 template <bool SAME_KERNEL>
 __device__ __forceinline__ int64_t ld_i64(const int64_t* p) {
@@ -56,7 +57,7 @@ __device__ __forceinline__ void finish_forward(const FinishArgs& f, const int32_
       const float c = float(ci);
       dot += c * (FROM == FINISH_SHARED        ? f.colsum[e]
                   : FROM == FINISH_SAME_KERNEL ? __ldcg(f.colsum + e)
-                                               : __ldg(f.colsum + e));
+                                               : ld_prev(f.colsum + e));
       tot += c;
     }
   }

@@ -40,11 +40,11 @@ struct PeerTable {
 // ranks' pairs in rank order). As an owner: own_offs [E_r + 1], own_counts [E_r], own_npp [1],
 // own_eids [cap_tiles] (tile -> local expert, 0 past the live length).
 __global__ void __launch_bounds__(256)
-    ep_plan_kernel(const int32_t* __restrict__ cnt_all, const int32_t* __restrict__ bounds,
-                   int n_ranks, int n_experts, int rank, int32_t* __restrict__ owner_of,
-                   int32_t* __restrict__ send_row0, int32_t* __restrict__ own_offs,
-                   int32_t* __restrict__ own_counts, int32_t* __restrict__ own_npp,
-                   int32_t* __restrict__ own_eids, int64_t cap_tiles) {
+    ep_plan_kernel(const int32_t* cnt_all, const int32_t* bounds,
+                   int n_ranks, int n_experts, int rank, int32_t* owner_of,
+                   int32_t* send_row0, int32_t* own_offs,
+                   int32_t* own_counts, int32_t* own_npp,
+                   int32_t* own_eids, int64_t cap_tiles) {
   pdl_trigger();
   pdl_wait();
   __shared__ int32_t tot[MAX_EXPERTS], before[MAX_EXPERTS], owner[MAX_EXPERTS];
@@ -106,11 +106,11 @@ __global__ void __launch_bounds__(256)
 // shared experts' pairs (expert id >= n_experts) point at the local extra buffer, laid out
 // [n_shared, n_tokens, .]: rank n_ranks, row s * n_tokens + t.
 __global__ void __launch_bounds__(256)
-    ep_pair_map_kernel(const int64_t* __restrict__ idx_all, const int32_t* __restrict__ inv_ids,
-                       const int32_t* __restrict__ local_offs, const int32_t* __restrict__ owner_of,
-                       const int32_t* __restrict__ send_row0, int64_t n_pairs, int k_all,
-                       int n_experts, int n_ranks, int64_t n_tokens, int32_t* __restrict__ pair_rank,
-                       int32_t* __restrict__ pair_row) {
+    ep_pair_map_kernel(const int64_t* idx_all, const int32_t* inv_ids,
+                       const int32_t* local_offs, const int32_t* owner_of,
+                       const int32_t* send_row0, int64_t n_pairs, int k_all,
+                       int n_experts, int n_ranks, int64_t n_tokens, int32_t* pair_rank,
+                       int32_t* pair_row) {
   pdl_trigger();
   pdl_wait();
   for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n_pairs;
@@ -140,25 +140,25 @@ struct alignas(16) Chunk16 {
 // one GPU's NVLink ingress; rank r starts at its first pair for rank r + 1 instead (measured on 8
 // GPUs: 1.2-1.9 ms per push without the rotation).
 __global__ void __launch_bounds__(256)
-    ep_push_rows_kernel(const Chunk16* __restrict__ src, const int32_t* __restrict__ sorted_ids,
-                        const int32_t* __restrict__ n_live_slots,
-                        const int32_t* __restrict__ first_slot, int64_t n_pairs, int k_all,
-                        const int32_t* __restrict__ pair_rank, const int32_t* __restrict__ pair_row,
+    ep_push_rows_kernel(const Chunk16* src, const int32_t* sorted_ids,
+                        const int32_t* n_live_slots,
+                        const int32_t* first_slot, int64_t n_pairs, int k_all,
+                        const int32_t* pair_rank, const int32_t* pair_row,
                         PeerTable rows, PeerTable sid, PeerTable pw,
-                        const __nv_bfloat16* __restrict__ w_all, int chunks_per_row) {
+                        const __nv_bfloat16* w_all, int chunks_per_row) {
   pdl_trigger();
   pdl_wait();
-  const int live = __ldg(n_live_slots);
-  int rot = first_slot != nullptr ? __ldg(first_slot) : 0;
+  const int live = ld_prev(n_live_slots);
+  int rot = first_slot != nullptr ? ld_prev(first_slot) : 0;
   if (rot < 0 || rot >= live) rot = 0;
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int s0 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s0 < live; s0 += warps) {
     const int s = s0 + rot < live ? s0 + rot : s0 + rot - live;
-    const int pair = __ldg(sorted_ids + s);
+    const int pair = ld_prev(sorted_ids + s);
     if (pair >= n_pairs) continue;
-    const int r = __ldg(pair_rank + pair);
-    const int64_t row = __ldg(pair_row + pair);
+    const int r = ld_prev(pair_rank + pair);
+    const int64_t row = ld_prev(pair_row + pair);
     const Chunk16* from = src + int64_t(pair / k_all) * chunks_per_row;
     Chunk16* to = static_cast<Chunk16*>(rows.p[r]) + row * chunks_per_row;
     // a lane's loads of the row are all issued before its first (remote) store: written as one
@@ -184,9 +184,9 @@ __global__ void __launch_bounds__(256)
 // Owner side: the pad slots of every local run -- rows [offs[e] + counts[e], offs[e + 1]) -- get
 // zero rows (the GEMMs rely on them) and, when sid is given, the sentinel id.
 __global__ void __launch_bounds__(256)
-    ep_pad_fix_kernel(const int32_t* __restrict__ own_offs, const int32_t* __restrict__ own_counts,
-                      int n_local, Chunk16* __restrict__ rows, int chunks_per_row,
-                      int32_t* __restrict__ sid, int32_t sentinel) {
+    ep_pad_fix_kernel(const int32_t* own_offs, const int32_t* own_counts,
+                      int n_local, Chunk16* rows, int chunks_per_row,
+                      int32_t* sid, int32_t sentinel) {
   pdl_trigger();
   pdl_wait();
   for (int e = blockIdx.x; e < n_local; e += gridDim.x) {
@@ -212,10 +212,10 @@ __device__ __forceinline__ void ep_acc8(float* acc, const Chunk16& r) {
 // out[t, :] = sum_j y.p[pair_rank[p]][pair_row[p], :]  (+ extra[t, :])  in fp32 (pair order j, as the
 // single-GPU combine), stored as bf16. One thread per 16-byte chunk of a token row.
 __global__ void __launch_bounds__(256)
-    ep_pull_combine_kernel(PeerTable y, const int32_t* __restrict__ pair_rank,
-                           const int32_t* __restrict__ pair_row, int64_t n_tokens, int k_all,
-                           int chunks_per_row, const Chunk16* __restrict__ extra,
-                           Chunk16* __restrict__ out) {
+    ep_pull_combine_kernel(PeerTable y, const int32_t* pair_rank,
+                           const int32_t* pair_row, int64_t n_tokens, int k_all,
+                           int chunks_per_row, const Chunk16* extra,
+                           Chunk16* out) {
   pdl_trigger();
   pdl_wait();
   const int64_t total = n_tokens * chunks_per_row;
@@ -252,9 +252,9 @@ __global__ void __launch_bounds__(256)
 
 // out[p] = v.p[pair_rank[p]][pair_row[p]] for the routed pairs (columns j < top_k), 0 for the rest.
 __global__ void __launch_bounds__(256)
-    ep_pull_vec_kernel(PeerTable v, const int32_t* __restrict__ pair_rank,
-                       const int32_t* __restrict__ pair_row, int64_t n_pairs, int k_all, int top_k,
-                       __nv_bfloat16* __restrict__ out) {
+    ep_pull_vec_kernel(PeerTable v, const int32_t* pair_rank,
+                       const int32_t* pair_row, int64_t n_pairs, int k_all, int top_k,
+                       __nv_bfloat16* out) {
   pdl_trigger();
   pdl_wait();
   for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n_pairs;

@@ -128,8 +128,8 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
                "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
                : "memory");
 }
-__device__ __forceinline__ void ld_global_nc_v8(const void* p, uint32_t* w) {
-  asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+__device__ __forceinline__ void ld_global_v8(const void* p, uint32_t* w) {
+  asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]),
                  "=r"(w[7])
                : "l"(p));

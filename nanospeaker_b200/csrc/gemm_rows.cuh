@@ -84,17 +84,17 @@ __device__ __forceinline__ TileRef tile_ref(const RowsArgs& p, int t, int m_tile
   const int rest = t / p.n_chunks;
   if (p.n_fixed_groups > 0) return TileRef{rest % m_tiles, rest / m_tiles};
   if (p.order != nullptr) {
-    const int2 r = __ldg(p.order + rest);
+    const int2 r = ld_prev(p.order + rest);
     return TileRef{r.x, r.y};
   }
-  return TileRef{rest, __ldg(p.expert_ids + rest)};
+  return TileRef{rest, ld_prev(p.expert_ids + rest)};
 }
 // t -> (group slice z, 128-row block, N chunk), without the owner of a routed tile.
 __device__ __forceinline__ TileCoord decode_tile(const RowsArgs& p, int t, int m_tiles, int bn) {
   TileCoord c;
   const int rest = t / p.n_chunks;
   c.z = p.n_fixed_groups > 0 ? rest / m_tiles : 0;
-  c.m_tile = p.n_fixed_groups > 0 ? rest - c.z * m_tiles : p.order != nullptr ? __ldg(&p.order[rest].x) : rest;
+  c.m_tile = p.n_fixed_groups > 0 ? rest - c.z * m_tiles : p.order != nullptr ? ld_prev(&p.order[rest].x) : rest;
   c.n0 = (t - rest * p.n_chunks) * bn;
   c.group = -1;
   return c;
@@ -104,7 +104,7 @@ __device__ __forceinline__ TileCoord decode_tile(const RowsArgs& p, int t, int m
 __device__ __forceinline__ void add_bias32(float* v, const __nv_bfloat16* bias) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const uint4 r = __ldg(reinterpret_cast<const uint4*>(bias) + i);
+    const uint4 r = ld_prev(reinterpret_cast<const uint4*>(bias) + i);
     const uint32_t w[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
   // (every thread waits for the preceding kernels itself before its first read of their data; a
   // CTA beyond the end of the list runs no loop iteration and only gives its TMEM back)
   pdl_wait();
-  const int live = p.n_fixed_groups > 0 ? p.rows_host : __ldg(p.n_post_pad);
+  const int live = p.n_fixed_groups > 0 ? p.rows_host : ld_prev(p.n_post_pad);
   const int m_tiles = (live + BM - 1) / BM;
   const int total_tiles = m_tiles * p.n_chunks * (p.n_fixed_groups > 0 ? p.n_fixed_groups : 1);
 
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
     const int r4 = lane >> 3, c = lane & 7;
     // the next tile's pairs are fetched with the current tile, the place of the one after that, too
     auto load_pair = [&](const TileRef& r) {
-      return r.group >= 0 ? __ldg(p.sorted_ids + int64_t(r.m_tile) * BM + gw * 32 + lane) : p.n_pairs;
+      return r.group >= 0 ? ld_prev(p.sorted_ids + int64_t(r.m_tile) * BM + gw * 32 + lane) : p.n_pairs;
     };
     TileRef next = tile_ref(p, blockIdx.x, m_tiles, total_tiles);
     TileRef after = tile_ref(p, blockIdx.x + gridDim.x, m_tiles, total_tiles);
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
       // rows in the slot-ordered buffer; their A rows are the token-major source itself, row =
       // slot - start of the group's run. The run start is fetched with the next tile's owner.
       auto run_start_of = [&](int group) {
-        return (group >= p.a2_first_group && group >= 0) ? __ldg(p.a2_offsets + group) : 0;
+        return (group >= p.a2_first_group && group >= 0) ? ld_prev(p.a2_offsets + group) : 0;
       };
       TileRef next = tile_ref(p, blockIdx.x, m_tiles, total_tiles);
       TileRef after = tile_ref(p, blockIdx.x + gridDim.x, m_tiles, total_tiles);
@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
           const int k0 = (kt - g_sum * p.num_k) * BK;
           if (p.sum_groups > 0)
             tma_load_3d(sA, &tmA, full_bar + s, k0,
-                        tc.m_tile * BM + __ldg(p.sum_offsets + g_sum), 0);
+                        tc.m_tile * BM + ld_prev(p.sum_offsets + g_sum), 0);
           else if (a_alt)
             tma_load_3d(sA, &tmA2, full_bar + s, k0, tc.m_tile * BM - a_start, 0);
           else if (!GATHER_A)
@@ -524,11 +524,11 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
     auto load_pair = [&](int t) {
       if (t >= total_tiles || fixed || p.sorted_ids == nullptr) return p.n_pairs;
       const int rest = t / p.n_chunks;
-      return __ldg(p.sorted_ids + int64_t(p.order != nullptr ? __ldg(&p.order[rest].x) : rest) * BM + row);
+      return ld_prev(p.sorted_ids + int64_t(p.order != nullptr ? ld_prev(&p.order[rest].x) : rest) * BM + row);
     };
     auto load_w = [&](int pr) {
       if (p.pair_w == nullptr) return 1.f;
-      return pr < p.n_pairs ? __bfloat162float(__ldg(p.pair_w + pr)) : 0.f;
+      return pr < p.n_pairs ? __bfloat162float(ld_prev(p.pair_w + pr)) : 0.f;
     };
     int pair = load_pair(blockIdx.x);
     int pair_n = load_pair(blockIdx.x + gridDim.x);
@@ -550,8 +550,8 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
           for (int jb = 0; jb < BN / 64; ++jb) {
             const int col = tc.n0 + jb * 64 + half * 32;
             if (r < p.rows_host && col < p.n_dim) {
-              ld_global_nc_v8(p.addend + r * p.ld_out + col, add_w[jb]);
-              ld_global_nc_v8(p.addend + r * p.ld_out + col + 16, add_w[jb] + 8);
+              ld_global_v8(p.addend + r * p.ld_out + col, add_w[jb]);
+              ld_global_v8(p.addend + r * p.ld_out + col + 16, add_w[jb] + 8);
             } else {
 #pragma unroll
               for (int i = 0; i < 16; ++i) add_w[jb][i] = 0u;
@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
       [[maybe_unused]] const __nv_bfloat16* bias_row = nullptr;
       if constexpr (EPI == EPI_GLU || EPI == EPI_SCALE || EPI == EPI_SCALE_RED) {
         if (p.bias != nullptr) {
-          const int grp = fixed ? tc.z : __ldg(p.expert_ids + tc.m_tile);
+          const int grp = fixed ? tc.z : ld_prev(p.expert_ids + tc.m_tile);
           bias_row = p.bias + int64_t(grp) * p.n_dim;   // one row per group of both weight stacks
         }
       }

@@ -392,11 +392,11 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
       if (u.left <= 0 || p.sorted_ids == nullptr) return p.n_pairs;
       const Unit2 c = unit_of(u);
       if (c.beside) return c.m_tile * BM + row;   // a token
-      return c.valid ? __ldg(p.sorted_ids + int64_t(c.m_tile) * BM + row) : p.n_pairs;
+      return c.valid ? ld_prev(p.sorted_ids + int64_t(c.m_tile) * BM + row) : p.n_pairs;
     };
     auto load_w = [&](int pr) {
       if (p.pair_w == nullptr) return 1.f;
-      return pr < p.n_pairs ? __bfloat162float(__ldg(p.pair_w + pr)) : 0.f;
+      return pr < p.n_pairs ? __bfloat162float(ld_prev(p.pair_w + pr)) : 0.f;
     };
     Walk ahead = walk();
     int pair = load_pair(ahead);

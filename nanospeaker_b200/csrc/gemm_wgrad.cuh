@@ -67,8 +67,8 @@ __device__ __forceinline__ RunEnds load_run_ends(const int32_t* offsets, int n_g
     r.lo[i] = r.hi[i] = 0;
     if (32 * i < n_groups) {
       const int g = 32 * i + lane;
-      r.lo[i] = __ldg(offsets + min(g, n_groups));
-      r.hi[i] = __ldg(offsets + min(g + 1, n_groups));
+      r.lo[i] = ld_prev(offsets + min(g, n_groups));
+      r.hi[i] = ld_prev(offsets + min(g + 1, n_groups));
     }
   }
   return r;
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
         auto fetch_tok = [&](int kt) {
           int tok = -1;
           if (gather && lane < ROWS_PER_WARP && kt < w.num_k) {
-            const int pair = __ldg(p.sorted_ids + w.row0 + kt * BK + gw * ROWS_PER_WARP + lane);
+            const int pair = ld_prev(p.sorted_ids + w.row0 + kt * BK + gw * ROWS_PER_WARP + lane);
             tok = pair < p.n_pairs ? pair / p.top_k : -1;
           }
           return tok;
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(256)
     int n = 0;
     for (int base = 0; base < p.n_groups; base += 32) {
       const int g = base + int(threadIdx.x);
-      const bool split = g < p.n_groups && __ldg(p.item_table + g + 1) - __ldg(p.item_table + g) > 1;
+      const bool split = g < p.n_groups && ld_prev(p.item_table + g + 1) - ld_prev(p.item_table + g) > 1;
       const unsigned m = __ballot_sync(0xffffffffu, split);
       if (split) split_runs[n + __popc(m & ((1u << threadIdx.x) - 1u))] = g;
       n += __popc(m);
@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(256)
   const int n_split = n_split_s;
   for (int i = blockIdx.y; i < n_split; i += gridDim.y) {
     const int g = split_runs[i];
-    const int first = __ldg(p.item_table + g), n_c = __ldg(p.item_table + g + 1) - first;
+    const int first = ld_prev(p.item_table + g), n_c = ld_prev(p.item_table + g + 1) - first;
     for (int f = slice * per_slice + threadIdx.x; f < (slice + 1) * per_slice; f += blockDim.x) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       const float4* src = reinterpret_cast<const float4*>(

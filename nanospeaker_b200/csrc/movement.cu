@@ -13,7 +13,7 @@ namespace moe {
 
 __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
   uint4 r;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
                : "l"(p));
   return r;
@@ -22,18 +22,18 @@ __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
 // xs[slot, :] = x[sorted_ids[slot] / top_k, :] for live slots, zero rows for pad slots.
 // row_bytes is a multiple of 16. One thread moves one 16-byte chunk.
 __global__ void __launch_bounds__(256)
-    permute_rows_kernel(const uint4* __restrict__ x, const int32_t* __restrict__ sorted_ids,
-                        const int32_t* __restrict__ n_post_pad, int32_t n_pairs, int32_t top_k,
-                        int32_t chunks_per_row, uint4* __restrict__ xs) {
+    permute_rows_kernel(const uint4* x, const int32_t* sorted_ids,
+                        const int32_t* n_post_pad, int32_t n_pairs, int32_t top_k,
+                        int32_t chunks_per_row, uint4* xs) {
   pdl_trigger();
   pdl_wait();
-  const int32_t live = __ldg(n_post_pad);
+  const int32_t live = ld_prev(n_post_pad);
   const int64_t total = int64_t(live) * chunks_per_row;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += int64_t(gridDim.x) * blockDim.x) {
     const int32_t slot = int32_t(i / chunks_per_row);
     const int32_t c = int32_t(i - int64_t(slot) * chunks_per_row);
-    const int32_t pair = __ldg(sorted_ids + slot);
+    const int32_t pair = ld_prev(sorted_ids + slot);
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (pair < n_pairs) v = ld_stream(x + int64_t(pair / top_k) * chunks_per_row + c);
     xs[i] = v;
@@ -48,7 +48,7 @@ struct alignas(32) Chunk32 {
 __device__ __forceinline__ Chunk32 ld_keep32(const Chunk32* p) {
   Chunk32 r;
   asm volatile(
-      "ld.global.nc.L1::no_allocate.L2::evict_last.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      "ld.global.L1::no_allocate.L2::evict_last.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
       : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]),
         "=r"(r.w[6]), "=r"(r.w[7])
       : "l"(p));
@@ -65,18 +65,18 @@ __device__ __forceinline__ void st32(Chunk32* p, const Chunk32& r) {
 // one flat run of 8 * chunks_per_row chunks, PERMUTE_UNROLL independent loads per lane in flight.
 constexpr int PERMUTE_UNROLL = 3;
 __global__ void __launch_bounds__(256)
-    permute_rows32_kernel(const Chunk32* __restrict__ x, const int32_t* __restrict__ sorted_ids,
-                          const int32_t* __restrict__ n_post_pad, int32_t n_pairs, int32_t top_k,
-                          int32_t chunks_per_row, Chunk32* __restrict__ xs) {
+    permute_rows32_kernel(const Chunk32* x, const int32_t* sorted_ids,
+                          const int32_t* n_post_pad, int32_t n_pairs, int32_t top_k,
+                          int32_t chunks_per_row, Chunk32* xs) {
   pdl_trigger();
   pdl_wait();
-  const int32_t live = __ldg(n_post_pad);  // a multiple of 128
+  const int32_t live = ld_prev(n_post_pad);  // a multiple of 128
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   const int per_group = 8 * chunks_per_row;
   for (int32_t row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 8; row0 < live;
        row0 += warps * 8) {
-    const int32_t pair = __ldg(sorted_ids + row0 + (lane & 7));
+    const int32_t pair = ld_prev(sorted_ids + row0 + (lane & 7));
     const int32_t my_tok = pair < n_pairs ? pair / top_k : -1;  // token of row row0 + lane % 8
     Chunk32* dst = xs + int64_t(row0) * chunks_per_row;
     for (int base = 0; base < per_group; base += 32 * PERMUTE_UNROLL) {
@@ -114,10 +114,10 @@ __device__ __forceinline__ void acc_bf16x8(float* acc, uint4 r) {
 // out[t, :] = sum_j y[inv_ids[t*top_k + j], :]  (+ extra[t, :])  in fp32, stored as bf16.
 template <int TOPK>
 __global__ void __launch_bounds__(256)
-    combine_rows_kernel(const uint4* __restrict__ y, const int32_t* __restrict__ inv_ids,
+    combine_rows_kernel(const uint4* y, const int32_t* inv_ids,
                         int64_t n_tokens, int32_t top_k_rt, int32_t chunks_per_row,
-                        const uint4* __restrict__ extra, const uint4* __restrict__ extra2,
-                        uint4* __restrict__ out) {
+                        const uint4* extra, const uint4* extra2,
+                        uint4* out) {
   pdl_trigger();
   pdl_wait();
   const int top_k = TOPK > 0 ? TOPK : top_k_rt;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(256)
       uint4 rows[TOPK > 0 ? TOPK : 1];
 #pragma unroll
       for (int j = 0; j < TOPK; ++j) {
-        const int32_t slot = __ldg(inv_ids + t * TOPK + j);   // < 0: the pair has no row (dropped)
+        const int32_t slot = ld_prev(inv_ids + t * TOPK + j);   // < 0: the pair has no row (dropped)
         rows[j] = slot >= 0 ? ld_stream(y + int64_t(slot) * chunks_per_row + c)
                             : make_uint4(0u, 0u, 0u, 0u);
       }
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256)
       for (int j = 0; j < TOPK; ++j) acc_bf16x8(acc, rows[j]);
     } else {
       for (int j = 0; j < top_k; ++j) {
-        const int32_t slot = __ldg(inv_ids + t * top_k + j);
+        const int32_t slot = ld_prev(inv_ids + t * top_k + j);
         if (slot >= 0) acc_bf16x8(acc, ld_stream(y + int64_t(slot) * chunks_per_row + c));
       }
     }
@@ -159,32 +159,32 @@ __global__ void __launch_bounds__(256)
 // (tile, 256-column chunk); thread = one 8-column piece of one of 8 row phases; the phases are
 // folded through shared memory, then one fp32 atomic per column.
 __global__ void __launch_bounds__(256)
-    segment_colsum_kernel(const uint4* __restrict__ buf, int32_t pieces_per_row,
-                          const int32_t* __restrict__ expert_ids,
-                          const int32_t* __restrict__ n_post_pad,
-                          const int32_t* __restrict__ pad_offsets,
-                          const int32_t* __restrict__ sorted_ids,
-                          const __nv_bfloat16* __restrict__ pair_w, int32_t n_pairs,
-                          const uint4* __restrict__ alt, int64_t alt_rows, int32_t first_alt_group,
-                          float* __restrict__ out) {
+    segment_colsum_kernel(const uint4* buf, int32_t pieces_per_row,
+                          const int32_t* expert_ids,
+                          const int32_t* n_post_pad,
+                          const int32_t* pad_offsets,
+                          const int32_t* sorted_ids,
+                          const __nv_bfloat16* pair_w, int32_t n_pairs,
+                          const uint4* alt, int64_t alt_rows, int32_t first_alt_group,
+                          float* out) {
   pdl_trigger();
   pdl_wait();
   const int tile = blockIdx.x;
-  if (int64_t(tile) * 128 >= __ldg(n_post_pad)) return;
-  const int group = __ldg(expert_ids + tile);
+  if (int64_t(tile) * 128 >= ld_prev(n_post_pad)) return;
+  const int group = ld_prev(expert_ids + tile);
   const int piece = blockIdx.y * 32 + (threadIdx.x & 31);   // 16-byte piece (8 columns) of the row
   const int phase = threadIdx.x >> 5;                        // rows phase, phase + 8, ...
   __shared__ float part[8][32][8];
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const bool from_alt = alt != nullptr && group >= first_alt_group;
-  const int64_t run0 = from_alt ? __ldg(pad_offsets + group) : 0;
+  const int64_t run0 = from_alt ? ld_prev(pad_offsets + group) : 0;
   if (piece < pieces_per_row) {
     for (int r = phase; r < 128; r += 8) {
       const int64_t slot = int64_t(tile) * 128 + r;
       float w = 1.f;
       if (pair_w != nullptr) {
-        const int32_t pr = __ldg(sorted_ids + slot);
-        w = pr < n_pairs ? __bfloat162float(__ldg(pair_w + pr)) : 0.f;
+        const int32_t pr = ld_prev(sorted_ids + slot);
+        w = pr < n_pairs ? __bfloat162float(ld_prev(pair_w + pr)) : 0.f;
       }
       uint4 v;
       if (from_alt) {
@@ -220,8 +220,8 @@ __global__ void __launch_bounds__(256)
 // sumsq[g] += sum of squares of group g's elements (fp32; the caller zeroes it). x [groups, per_group]
 // bf16, per_group a multiple of 8. One block-level reduction and one atomic per block.
 __global__ void __launch_bounds__(256)
-    group_sumsq_kernel(const uint4* __restrict__ x, int64_t pieces_per_group,
-                       float* __restrict__ sumsq) {
+    group_sumsq_kernel(const uint4* x, int64_t pieces_per_group,
+                       float* sumsq) {
   pdl_trigger();
   pdl_wait();
   const int g = blockIdx.y;
@@ -252,15 +252,15 @@ __global__ void __launch_bounds__(256)
 // out = alpha * s_g * x + beta * y, element-wise in fp32, one rounding to bf16. s_g = 1 / (sqrt(
 // sumsq[g]) + eps) when sumsq is given (the Frobenius normalisation of group g), else 1; y may be null.
 __global__ void __launch_bounds__(256)
-    axpby_kernel(const uint4* __restrict__ x, const uint4* __restrict__ y, uint4* __restrict__ out,
+    axpby_kernel(const uint4* x, const uint4* y, uint4* out,
                  int64_t pieces_per_group, int64_t total, float alpha, float beta,
-                 const float* __restrict__ sumsq, float eps) {
+                 const float* sumsq, float eps) {
   pdl_trigger();
   pdl_wait();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += int64_t(gridDim.x) * blockDim.x) {
     float a = alpha;
-    if (sumsq != nullptr) a *= 1.f / (sqrtf(__ldg(sumsq + i / pieces_per_group)) + eps);
+    if (sumsq != nullptr) a *= 1.f / (sqrtf(ld_prev(sumsq + i / pieces_per_group)) + eps);
     const uint4 vx = ld_stream(x + i);
     uint4 vy = make_uint4(0u, 0u, 0u, 0u);
     if (y != nullptr) vy = ld_stream(y + i);
@@ -280,8 +280,8 @@ __global__ void __launch_bounds__(256)
 // dst[r, c] = c < cols ? src[r, c] : 0 for c < dst_ld: pads a matrix's rows to a TMA-friendly
 // stride (the router weight [D, E] -> [D, ld]) or drops the pad columns again.
 __global__ void __launch_bounds__(256)
-    copy_cols_kernel(const uint16_t* __restrict__ src, int64_t rows, int32_t cols, int32_t src_ld,
-                     uint16_t* __restrict__ dst, int32_t dst_ld) {
+    copy_cols_kernel(const uint16_t* src, int64_t rows, int32_t cols, int32_t src_ld,
+                     uint16_t* dst, int32_t dst_ld) {
   pdl_trigger();
   pdl_wait();
   const int64_t total = rows * dst_ld;

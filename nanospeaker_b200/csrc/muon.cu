@@ -80,7 +80,7 @@ __device__ __forceinline__ const MuonTensor& muon_tensor(const MuonTensors& ts, 
 // the same from run to run). HBM-bound: 8 bytes per value (grad and buf read, buf and dir written).
 __global__ void __launch_bounds__(MU_THREADS)
     muon_direction_kernel(const __grid_constant__ MuonTensors ts, float w_grad, float momentum,
-                          float* __restrict__ norms) {
+                          float* norms) {
   pdl_trigger();
   pdl_wait();
   if (norms != nullptr && blockIdx.x == 0 && threadIdx.x < 3) norms[threadIdx.x] = 0.f;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(MU_THREADS)
 // (norms[2] is its ticket). HBM-bound: 6 bytes per value in bf16.
 __global__ void __launch_bounds__(MU_THREADS)
     muon_apply_kernel(const __grid_constant__ MuonTensors ts, float decay,
-                      float* __restrict__ partials, float* norms) {
+                      float* partials, float* norms) {
   pdl_trigger();
   pdl_wait();
   const MuonTensor& t = muon_tensor(ts, blockIdx.x);

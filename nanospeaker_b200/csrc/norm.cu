@@ -43,9 +43,9 @@ __device__ __forceinline__ float warp_sum(float v) {
 // h[t, :] = x[t, :] * rstd[t] * gamma,  rstd[t] = rsqrt(mean(x[t, :]^2) + eps)  (kept for the backward)
 template <int NCH>
 __global__ void __launch_bounds__(NORM_WARPS * 32)
-    rmsnorm_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ gamma,
+    rmsnorm_fwd_kernel(const uint4* x, const uint4* gamma,
                        int64_t n_rows, int32_t chunks_per_row, float eps, float inv_d,
-                       uint4* __restrict__ h, float* __restrict__ rstd) {
+                       uint4* h, float* rstd) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -92,10 +92,10 @@ __global__ void __launch_bounds__(NORM_WARPS * 32)
 // busy). Blocks per SM: as many as are resident.
 template <int NCH>
 __global__ void __launch_bounds__(NORM_WARPS * 32)
-    rmsnorm_bwd_kernel(const uint4* __restrict__ dh, const uint4* __restrict__ x,
-                       const float* __restrict__ rstd, const uint4* __restrict__ gamma,
-                       const uint4* __restrict__ add, int64_t n_rows, int32_t chunks_per_row,
-                       float inv_d, uint4* __restrict__ dx, float* __restrict__ dgamma) {
+    rmsnorm_bwd_kernel(const uint4* dh, const uint4* x,
+                       const float* rstd, const uint4* gamma,
+                       const uint4* add, int64_t n_rows, int32_t chunks_per_row,
+                       float inv_d, uint4* dx, float* dgamma) {
   pdl_trigger();
   pdl_wait();
   extern __shared__ float dg_s[];  // [chunks_per_row * 8]

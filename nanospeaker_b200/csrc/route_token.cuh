@@ -6,6 +6,7 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include "pdl.cuh"
 #include "routing.cuh"
 
 namespace moe {
@@ -78,7 +79,7 @@ __device__ __forceinline__ void route_token(const RouteArgs& a, Load load, int64
       const float f = __uint_as_float((i & 1) ? w & 0xffff0000u : w << 16);
       float v = e0 + i < a.n_experts ? f + b[i] : -CUDART_INF_F;
       if (a.noise != nullptr && e0 + i < a.n_experts)   // exploration noise, one value per (token, expert)
-        v += __ldg(a.noise + tc * a.n_experts + e0 + i);
+        v += ld_prev(a.noise + tc * a.n_experts + e0 + i);
       key[i] = __float_as_uint(v);
       mx = fmaxf(mx, v);
     }
@@ -230,8 +231,8 @@ __device__ __forceinline__ void route_warp(const RouteArgs& a, const __nv_bfloat
     v[i] = -CUDART_INF_F;
     key[i] = 0u;   // (no key of a value is 0)
     if (e < E) {
-      v[i] = __bfloat162float(lg[e]) + (bias != nullptr ? __ldg(bias + e) : 0.f);
-      if (a.noise != nullptr) v[i] += __ldg(a.noise + t * E + e);
+      v[i] = __bfloat162float(lg[e]) + (bias != nullptr ? ld_prev(bias + e) : 0.f);
+      if (a.noise != nullptr) v[i] += ld_prev(a.noise + t * E + e);
       key[i] = float_key(v[i]);
     }
     mx = fmaxf(mx, v[i]);

@@ -186,9 +186,9 @@ __global__ void __launch_bounds__(FRONT_THREADS, 1) router_front_kernel(const Fr
 // per thread. Every global load is on its way before the first is used (a pair's expert beside the
 // histogram table), the ranks inside the block are made under the plan, and two barriers remain.
 __global__ void __launch_bounds__(FRONT_THREADS)
-    router_front_scatter_kernel(const int64_t* __restrict__ idx_all, int32_t n_pairs, int n_experts,
-                                int chunk, const int32_t* __restrict__ block_hist,
-                                const float* __restrict__ block_colsum, int32_t* __restrict__ sorted_ids,
+    router_front_scatter_kernel(const int64_t* idx_all, int32_t n_pairs, int n_experts,
+                                int chunk, const int32_t* block_hist,
+                                const float* block_colsum, int32_t* sorted_ids,
                                 const ScatterArgs sc) {
   constexpr int WARPS = FRONT_THREADS / 32, MAX_WARPS = FRONT_TOKENS * 32 / 32;
   pdl_trigger();
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(FRONT_THREADS)
   pdl_wait();
   const int64_t pair = int64_t(blk) * chunk + tid;
   const bool live_pair = tid < chunk && pair < n_pairs;
-  const int e_mine = live_pair ? int(__ldg(reinterpret_cast<const long long*>(idx_all) + pair)) : -1;
+  const int e_mine = live_pair ? int(ld_prev(reinterpret_cast<const long long*>(idx_all) + pair)) : -1;
   const bool finish = sc.fin.counts != nullptr && blk == 0;
   constexpr int U = 6;   // experts of a warp at a time
   for (int e0 = warp; e0 < n_experts; e0 += U * WARPS) {
@@ -214,9 +214,9 @@ __global__ void __launch_bounds__(FRONT_THREADS)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int e = e0 + u * WARPS, b = lane + 32 * j;
-        v[u][j] = e < n_experts && b < n_blocks ? __ldg(block_hist + e * n_blocks + b) : 0;
+        v[u][j] = e < n_experts && b < n_blocks ? ld_prev(block_hist + e * n_blocks + b) : 0;
         f[u][j] = finish && block_colsum != nullptr && e < sc.fin.n_experts && b < n_blocks
-                      ? __ldg(block_colsum + e * n_blocks + b)
+                      ? ld_prev(block_colsum + e * n_blocks + b)
                       : 0.f;
       }
 #pragma unroll

@@ -29,12 +29,12 @@ constexpr int RF_WARPS = 8;
 // fill of sorted_ids, so that dispatch_scatter_kernel can follow directly.
 template <int NSLOT, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
-    router_fused_kernel(const __nv_bfloat16* __restrict__ logits, int ld,
-                        const float* __restrict__ bias, const float* __restrict__ noise, int64_t n_tokens, int n_experts, int top_k,
+    router_fused_kernel(const __nv_bfloat16* logits, int ld,
+                        const float* bias, const float* noise, int64_t n_tokens, int n_experts, int top_k,
                         int n_shared, int normalize, int full_softmax,
-                        __nv_bfloat16* __restrict__ w_all, int64_t* __restrict__ idx_all,
-                        float* __restrict__ colsum, int tokens_per_block,
-                        int32_t* __restrict__ block_hist, int32_t* __restrict__ sorted_ids,
+                        __nv_bfloat16* w_all, int64_t* idx_all,
+                        float* colsum, int tokens_per_block,
+                        int32_t* block_hist, int32_t* sorted_ids,
                         int64_t l_cap) {
   pdl_trigger();
   pdl_wait();
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(WARPS * 32)
       const int e = i * 32 + lane;
       const bool in = e < n_experts;
       v[i] = in ? __bfloat162float(row[e]) + b[i] +
-                      (noise != nullptr ? __ldg(noise + t * n_experts + e) : 0.f)
+                      (noise != nullptr ? ld_prev(noise + t * n_experts + e) : 0.f)
                 : -CUDART_INF_F;
       const uint32_t fk = float_key(v[i]);
       key[i] = in ? (fk == 0u ? 1u : fk) : 0u;
@@ -198,12 +198,12 @@ constexpr int RF4_TOKENS = RF4_THREADS / 4;   // tokens per block and pass
 // KT: the smallest of 2, 4, 6, 8 that holds top_k.
 template <int EPL, int KT, bool COLSUM>
 __global__ void __launch_bounds__(RF4_THREADS)
-    router_fused4_kernel(const __nv_bfloat16* __restrict__ logits, int ld,
-                         const float* __restrict__ bias, const float* __restrict__ noise, int64_t n_tokens, int n_experts, int top_k,
+    router_fused4_kernel(const __nv_bfloat16* logits, int ld,
+                         const float* bias, const float* noise, int64_t n_tokens, int n_experts, int top_k,
                          int n_shared, int normalize, int full_softmax,
-                         __nv_bfloat16* __restrict__ w_all, int64_t* __restrict__ idx_all,
-                         float* __restrict__ colsum, int tokens_per_block,
-                         int32_t* __restrict__ block_hist, int32_t* __restrict__ sorted_ids,
+                         __nv_bfloat16* w_all, int64_t* idx_all,
+                         float* colsum, int tokens_per_block,
+                         int32_t* block_hist, int32_t* sorted_ids,
                          int64_t l_cap, const ScatterArgs sc) {
   // No early release of the next kernel when a scatter launch follows: with it the step measured
   // 4.5 us slower (the likely reason: the dispatch's scatter blocks, 512 threads each, become
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(RF4_THREADS)
     const bool valid = t < t_hi;
     const int64_t tc = valid ? t : t_hi - 1;   // lanes past the end repeat the last token, write nothing
     route_token<EPL, KT, COLSUM>(
-        args, [&](int e) { return __ldg(reinterpret_cast<const uint2*>(logits + tc * ld + e)); }, t, tc,
+        args, [&](int e) { return ld_prev(reinterpret_cast<const uint2*>(logits + tc * ld + e)); }, t, tc,
         valid, b, csum, list, chunked ? hist : nullptr);
   }
 
@@ -371,15 +371,15 @@ static void launch_rf4(int epl, int top_k, bool want_colsum, unsigned grid, bool
 //   => d colsum[e] = d_aux * aux_scale_T * counts[e] / (T * top_k), added to every d p[t, e].
 template <int NSLOT>
 __global__ void __launch_bounds__(RF_WARPS * 32)
-    router_fused_bwd_kernel(const __nv_bfloat16* __restrict__ logits, int ld,
-                            const float* __restrict__ bias, const float* __restrict__ noise, const int64_t* __restrict__ idx_all,
-                            const __nv_bfloat16* __restrict__ dw_all,
-                            const __nv_bfloat16* __restrict__ extra_dw, int extra_ld,
-                            const int32_t* __restrict__ inv_ids, int64_t n_tokens,
+    router_fused_bwd_kernel(const __nv_bfloat16* logits, int ld,
+                            const float* bias, const float* noise, const int64_t* idx_all,
+                            const __nv_bfloat16* dw_all,
+                            const __nv_bfloat16* extra_dw, int extra_ld,
+                            const int32_t* inv_ids, int64_t n_tokens,
                             int n_experts, int top_k, int n_shared, int normalize,
-                            int full_softmax, const float* __restrict__ d_aux,
-                            const int32_t* __restrict__ counts, float aux_scale_T,
-                            __nv_bfloat16* __restrict__ dl, int ld_out) {
+                            int full_softmax, const float* d_aux,
+                            const int32_t* counts, float aux_scale_T,
+                            __nv_bfloat16* dl, int ld_out) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(RF_WARPS * 32)
     for (int i = 0; i < NSLOT; ++i) {
       const int e = i * 32 + lane;
       v[i] = e < n_experts ? __bfloat162float(row[e]) + b[i] +
-                                 (noise != nullptr ? __ldg(noise + t * n_experts + e) : 0.f)
+                                 (noise != nullptr ? ld_prev(noise + t * n_experts + e) : 0.f)
                            : -CUDART_INF_F;
       mx = fmaxf(mx, v[i]);
       dp[i] = dcs[i];
@@ -527,9 +527,9 @@ __global__ void __launch_bounds__(RF_WARPS * 32)
 }
 
 // aux[0] = coef * E * sum_e (counts[e] / sum counts) * (colsum[e] / T)   (one warp)
-__global__ void balance_loss_kernel(const float* __restrict__ colsum,
-                                    const int32_t* __restrict__ counts, int n_experts,
-                                    int64_t n_tokens, float coef, float* __restrict__ aux) {
+__global__ void balance_loss_kernel(const float* colsum,
+                                    const int32_t* counts, int n_experts,
+                                    int64_t n_tokens, float coef, float* aux) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x;

@@ -30,9 +30,9 @@ namespace moe {
 //                     normalize == 0 -> the full-softmax probabilities of the winners.
 template <int NSLOT>
 __global__ void __launch_bounds__(256)
-    router_topk_kernel(const float* __restrict__ logits, int64_t n_tokens, int n_experts, int top_k,
-                       int normalize, int full_softmax, float* __restrict__ topk_w,
-                       int64_t* __restrict__ topk_idx, float* __restrict__ probs) {
+    router_topk_kernel(const float* logits, int64_t n_tokens, int n_experts, int top_k,
+                       int normalize, int full_softmax, float* topk_w,
+                       int64_t* topk_idx, float* probs) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -134,10 +134,10 @@ __global__ void __launch_bounds__(256)
 //   !full_softmax, !normalize    : dp_i = dw_i on S, softmax Jacobian
 template <int NSLOT>
 __global__ void __launch_bounds__(256)
-    router_topk_bwd_kernel(const float* __restrict__ logits, const int64_t* __restrict__ topk_idx,
-                           const float* __restrict__ d_topk_w, const float* __restrict__ d_probs,
+    router_topk_bwd_kernel(const float* logits, const int64_t* topk_idx,
+                           const float* d_topk_w, const float* d_probs,
                            int64_t n_tokens, int n_experts, int top_k, int normalize,
-                           int full_softmax, float* __restrict__ d_logits) {
+                           int full_softmax, float* d_logits) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -256,9 +256,9 @@ static int64_t dispatch_chunk(int64_t n_pairs) {
 // Pass 1: per-block histogram of expert ids -> block_hist[expert][block]; also paints this block's
 // share of sorted_ids with the sentinel so pad slots need no separate fill launch.
 __global__ void __launch_bounds__(DISPATCH_THREADS)
-    dispatch_hist_kernel(const int64_t* __restrict__ topk_idx, int64_t n_pairs, int n_experts,
-                         int chunk, int32_t* __restrict__ block_hist,
-                         int32_t* __restrict__ sorted_ids, int64_t l_cap, int32_t* status) {
+    dispatch_hist_kernel(const int64_t* topk_idx, int64_t n_pairs, int n_experts,
+                         int chunk, int32_t* block_hist,
+                         int32_t* sorted_ids, int64_t l_cap, int32_t* status) {
   pdl_trigger();
   pdl_wait();
   __shared__ int32_t hist[MAX_EXPERTS];
@@ -287,12 +287,12 @@ __global__ void __launch_bounds__(DISPATCH_THREADS)
 
 // Pass 2 (dispatch_scatter.cuh): plan + stable scatter, one block per chunk.
 __global__ void __launch_bounds__(DISPATCH_THREADS)
-    dispatch_scatter_kernel(const int64_t* __restrict__ topk_idx, int64_t n_pairs, int n_experts,
-                            int chunk, int n_blocks, const int32_t* __restrict__ block_hist,
-                            int32_t* __restrict__ counts, int32_t* __restrict__ pad_offsets,
-                            int32_t* __restrict__ n_post_pad, int32_t* __restrict__ expert_ids,
-                            int64_t n_tiles_cap, int32_t* __restrict__ sorted_ids,
-                            int32_t* __restrict__ inv_ids, int32_t capacity, int32_t n_capped,
+    dispatch_scatter_kernel(const int64_t* topk_idx, int64_t n_pairs, int n_experts,
+                            int chunk, int n_blocks, const int32_t* block_hist,
+                            int32_t* counts, int32_t* pad_offsets,
+                            int32_t* n_post_pad, int32_t* expert_ids,
+                            int64_t n_tiles_cap, int32_t* sorted_ids,
+                            int32_t* inv_ids, int32_t capacity, int32_t n_capped,
                             const FinishArgs fin) {
   pdl_trigger();
   pdl_wait();

@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
       const int rstep = Q * P, rn = last ? 0 : router_rows;   // (in chunks of four columns)
 #pragma unroll
       for (int i = 0; i < ST_ROUTER_PRE; ++i)
-        wr[i] = i < rn ? __ldg(rsrc + i * rstep) : make_uint2(0u, 0u);
+        wr[i] = i < rn ? ld_prev(rsrc + i * rstep) : make_uint2(0u, 0u);
 #pragma unroll 1
       for (int i = ST_ROUTER_PRE; i < min(rn, ST_ROUTER_PRE + router_room); ++i)
         cp_async_8(smem_u32(router_s) + ((i - ST_ROUTER_PRE) * ST_CT + tid) * 8, rsrc + i * rstep);
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
         const int i_late = ST_ROUTER_PRE + router_room;
 #pragma unroll
         for (int u = 0; u < ST_ROUTER_LATE; ++u)
-          wl[u] = i_late + u < rn ? __ldg(rsrc + (i_late + u) * rstep) : make_uint2(0u, 0u);
+          wl[u] = i_late + u < rn ? ld_prev(rsrc + (i_late + u) * rstep) : make_uint2(0u, 0u);
         ct_sync();
 #pragma unroll 1
         for (int d = 2 * tid; d < dpad; d += 2 * ST_CT) {
@@ -426,12 +426,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stack_kernel(const StackArgs p)
             for (int u = 0; u < ST_ROUTER_LATE; ++u) add(wl[u], xrow[min(rq + (i + u) * Q, D - 1)]);
 #pragma unroll
             for (int u = 0; u < ST_ROUTER_LATE; ++u)
-              wl[u] = i + ST_ROUTER_LATE + u < rn ? __ldg(rsrc + (i + ST_ROUTER_LATE + u) * rstep)
+              wl[u] = i + ST_ROUTER_LATE + u < rn ? ld_prev(rsrc + (i + ST_ROUTER_LATE + u) * rstep)
                                                   : make_uint2(0u, 0u);
           }
           *reinterpret_cast<float4*>(red_s + rq * p.E + 4 * rp) = make_float4(a0, a1, a2, a3);
         }
-        const float b = bias != nullptr && tid < p.E ? __ldg(bias + tid) : 0.f;
+        const float b = bias != nullptr && tid < p.E ? ld_prev(bias + tid) : 0.f;
         ct_sync();
         if (tid < p.E) {   // (at most 256 experts: one thread each)
           float s = 0.f;

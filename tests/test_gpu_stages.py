@@ -72,6 +72,39 @@ def test_permute_and_combine_are_bit_exact(T, E, k, D, skew):
         assert torch.equal(out, acc.bfloat16())
 
 
+def test_a_chain_reads_what_the_kernel_before_it_wrote():
+    """Dispatch and permute back to back in a graph, where the permute starts early and reads the live rows as
+    its first value: the plan is another one at every replay, from a few live tiles to one per expert."""
+    T, E, k, D = 300, 64, 2, 96
+    gen = torch.Generator().manual_seed(1)
+    x = torch.randn(T, D, generator=gen).bfloat16()
+    plans = [torch.stack([torch.arange(T) % n, (torch.arange(T) + 1) % n], 1) for n in (2, 64, 3, 33, 5, 64, 2)]
+    idx, xc = plans[0].cuda(), x.cuda()
+
+    def chain():
+        sids, eids, offs, counts, npp, inv = K().dispatch(idx, E)
+        return sids, npp, K().permute(xc, k, sids, npp)
+
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        chain()
+    side.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        sids, npp, xs = chain()
+    for plan in plans:
+        idx.copy_(plan)
+        xs.fill_(7)
+        torch.cuda.synchronize()
+        graph.replay()
+        want = O.dispatch(plan, E)
+        nl = int(want[4])
+        assert int(npp) == nl and torch.equal(sids.cpu()[:nl], want[0][:nl])
+        assert torch.equal(xs.cpu()[:nl], _slot_rows(x, want[0], k, nl, T * k)[0])
+        assert (xs[nl:] == 7).all()
+    K().check_status("cuda")
+
+
 @pytest.mark.parametrize("T,E,k,D,skew", CASES)
 def test_forward_gemm_stages(T, E, k, D, skew):
     H = 128

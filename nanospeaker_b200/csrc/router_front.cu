@@ -200,6 +200,7 @@ __global__ void __launch_bounds__(FRONT_THREADS)
   const int warps = (chunk + 31) / 32;
   for (int i = tid; i < warps * (MAX_EXPERTS / 2); i += FRONT_THREADS)
     reinterpret_cast<uint32_t*>(mine)[i] = 0u;
+  __syncthreads();   // (a warp counts into its row below; ahead of the wait the barrier costs nothing)
   pdl_wait();
   const int64_t pair = int64_t(blk) * chunk + tid;
   const bool live_pair = tid < chunk && pair < n_pairs;

@@ -848,6 +848,32 @@ def test_small_front_equals_the_general_path(T, D, E, k, S, norm, full, noise):
     assert rel_l2(a[0], b[0]) < ATOMIC_TOL * (k + S) / 3
 
 
+@pytest.mark.parametrize("T,E,k,S", [(2048, 128, 8, 2), (2041, 8, 8, 0), (333, 76, 6, 2), (17, 4, 4, 2)])
+def test_small_front_gives_every_pair_its_slot_each_time(T, E, k, S):
+    """The small batch's plan, call after call: three to five warps of counts a block, all tokens at the same
+    experts. The slots are a permutation in stable order whatever the warps' timing."""
+    from nanospeaker_b200 import kernels
+    D = 128
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    si, so = (rnd(S, D, 256).bfloat16(), rnd(S, 128, D).bfloat16()) if S else (None, None)
+    args = (rnd(T, D).bfloat16(), (rnd(D, E) * 0.05).bfloat16(), rnd(E) * 0.3, rnd(E, D, 256).bfloat16(),
+            rnd(E, 128, D).bfloat16(), si, so, k, True, True, 0.01, "silu", True, None, True, None, False)
+    first = None
+    for _ in range(50):
+        with torch.no_grad():
+            r = torch.ops.moe_b200.moe_block(*args)
+        idx, sids, inv = r[7], r[8], r[13]
+        first = r if first is None else first
+        if r is first:   # against a stable sort of the pairs by expert
+            order = idx.reshape(-1).argsort(stable=True)
+            live = sids[: int(r[12])]
+            assert torch.equal(live[live < T * (k + S)].long(), order)
+            assert torch.equal(live[inv.long()].long(), torch.arange(T * (k + S), device="cuda"))
+        assert torch.equal(inv, first[13]) and torch.equal(sids[: live.numel()], live)
+    kernels.check_status("cuda")
+
+
 @pytest.mark.parametrize("T,E,k,S,skew", [(32768, 8, 2, 2, 0.0), (33001, 76, 1, 0, 2.0), (40000, 5, 5, 1, 0.3)])
 def test_large_inference_walks_every_tile_once(T, E, k, S, skew):
     """From 32768 tokens on the inference forward walks its tiles window by window: runs of unequal length,

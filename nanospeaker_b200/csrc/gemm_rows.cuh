@@ -200,7 +200,6 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
   // The prologue below (barriers, TMEM, descriptor prefetch) touches nothing an earlier kernel
   // wrote, so it runs BEFORE the wait for the preceding kernels: under programmatic dependent launch
   // this CTA is resident while the previous grid's last CTAs still work.
-  pdl_trigger();
   using L = RowsSmem<BN, STAGES, EPI, OUT_BOXES>;
   constexpr bool GATHER_A = GATHER != GATHER_NO;
   constexpr bool TMA_OUT = epi_uses_tma_store(EPI);
@@ -254,6 +253,7 @@ __global__ void __launch_bounds__(rows_threads(EPI, GATHER), 1)
   if (warp == 1) {
     tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
+    pdl_trigger();
   }
   tc_fence_before();
   __syncthreads();

@@ -143,7 +143,6 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
                       const __grid_constant__ CUtensorMap tmOut, const RowsArgs p) {
   // (the prologue up to the wait touches nothing an earlier kernel wrote: barriers, TMEM and the
   // pair's meeting take 1.8 us)
-  pdl_trigger();
   using L = Rows2Smem<BN, STAGES, EPI>;
   static_assert(BN % 32 == 0 && BN <= 256, "BN must be a multiple of 32 up to 256");
   static_assert(!B_MN || BN % 128 == 0, "an MN-major weight half must be whole 64-column boxes");
@@ -198,6 +197,7 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
   if (warp == 1) {
     tmem_alloc2(tmem_slot, TMEM_COLS);
     tmem_relinquish2();
+    pdl_trigger();
   }
   tc_fence_before();
   cluster_sync_all();     // both CTAs' barriers are initialised and both have their TMEM

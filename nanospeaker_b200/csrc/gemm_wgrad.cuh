@@ -227,8 +227,8 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
                       const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmAlt, const WgradArgs p, int tiles_x,
                       int tiles_y) {
-  pdl_trigger();   // (the wait for the preceding kernels comes after the part of the prologue
-                   // that reads nothing of theirs: barriers and TMEM)
+  // (the wait for the preceding kernels comes after the part of the prologue that reads nothing of theirs:
+  // barriers and TMEM)
   using L = WgradSmem<BN, STAGES>;
   constexpr uint32_t TMEM_BUF = BN <= 128 ? 128 : 256;
   constexpr uint32_t TMEM_COLS = 2 * TMEM_BUF;
@@ -268,6 +268,7 @@ __global__ void __launch_bounds__(GATHER ? WGRAD_THREADS_GATHER : WGRAD_THREADS,
   if (warp == 1) {
     tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
+    pdl_trigger();
   }
   tc_fence_before();
   __syncthreads();

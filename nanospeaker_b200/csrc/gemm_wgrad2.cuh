@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(WGRAD_THREADS, 1)
                        const __grid_constant__ CUtensorMap tmB,
                        const __grid_constant__ CUtensorMap tmAlt, const WgradArgs p, int tiles_x,
                        int tiles_y) {
-  pdl_trigger();   // (the prologue up to the wait touches nothing an earlier kernel wrote)
+  // (the prologue up to the wait touches nothing an earlier kernel wrote)
   using L = Wgrad2Smem<BN, STAGES>;
   constexpr uint32_t TMEM_BUF = BN <= 128 ? 128 : 256;
   constexpr uint32_t TMEM_COLS = 2 * TMEM_BUF;
@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(WGRAD_THREADS, 1)
   if (warp == 1) {
     tmem_alloc2(tmem_slot, TMEM_COLS);
     tmem_relinquish2();
+    pdl_trigger();
   }
   tc_fence_before();
   cluster_sync_all();

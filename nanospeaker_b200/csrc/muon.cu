@@ -511,7 +511,6 @@ __global__ void __launch_bounds__(NS_THREADS, 1)
   while (k + 1 < js.n && js.job[k + 1].first_block <= int(blockIdx.x)) ++k;
   const NsJob& job = js.job[k];
   const int group = int(blockIdx.x) - job.first_block;
-  pdl_trigger();
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&job.map);
     for (int s = 0; s < NS_MAX_SLOTS; ++s) {
@@ -530,6 +529,7 @@ __global__ void __launch_bounds__(NS_THREADS, 1)
   if (warp == 1) {
     tmem_alloc(&bars->tmem, 512);
     tmem_relinquish();
+    pdl_trigger();
   }
   tc_fence_before();
   __syncthreads();

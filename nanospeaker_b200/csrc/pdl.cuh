@@ -1,7 +1,9 @@
 // Programmatic dependent launch. Every kernel of the library starts with pdl_trigger() + pdl_wait()
 // and is launched with launch_pdl(): the next kernel in the stream may then be scheduled while this
 // one still runs (its CTAs become resident as SMs free up and park in pdl_wait()), which hides the
-// launch latency between two dependent kernels. pdl_wait() returns once the preceding kernel has
+// launch latency between two dependent kernels. A kernel that uses TMEM triggers when it holds it: a
+// parked CTA that had taken the SM's TMEM first would wait for this one, and this one for the TMEM, both
+// for good (the allocation's wait has no limit). pdl_wait() returns once the preceding kernel has
 // completed and its writes are visible; it must be executed by every CTA before any global access
 // and before exit, otherwise a later kernel could overtake an earlier one it depends on.
 #pragma once

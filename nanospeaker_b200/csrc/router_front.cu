@@ -66,7 +66,6 @@ __host__ __device__ __forceinline__ FrontSmem front_smem(int d_model, int n_expe
 // NS: ceil(E / 32); epl: experts per lane of the four-lane form.
 template <int NS>
 __global__ void __launch_bounds__(FRONT_THREADS, 1) router_front_kernel(const FrontArgs p, int epl) {
-  pdl_trigger();
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t mma_done;
   __shared__ uint32_t tmem_slot;
@@ -85,6 +84,7 @@ __global__ void __launch_bounds__(FRONT_THREADS, 1) router_front_kernel(const Fr
   if (warp == 1) {
     tmem_alloc(&tmem_slot, 128);
     tmem_relinquish();
+    pdl_trigger();
   }
   for (int e = tid; e < E + p.route.n_shared; e += FRONT_THREADS) hist[e] = 0;
   pdl_wait();

@@ -137,6 +137,19 @@ inline Sizes sizes(int64_t n_tokens, int32_t n_experts, int32_t n_shared, int32_
   return s;
 }
 
+// A token has a row in a run once at most, and runs are padded to whole tiles.
+inline int64_t longest_run(int64_t n_tokens) { return (n_tokens + 127) / 128 * 128; }
+// Rows per split-K chunk of the three weight gradients.
+struct Chunks {
+  int32_t in, out, router;
+};
+inline Chunks chunks_of(const Sizes& z, int64_t n_tokens, int32_t d_model, int32_t d_hidden) {
+  return Chunks{
+      moe::wgrad_chunk_rows(d_model, 2 * d_hidden, z.l_cap, z.n_all, 1, longest_run(n_tokens)),
+      moe::wgrad_chunk_rows(d_hidden, d_model, z.l_cap, z.n_all, 1, longest_run(n_tokens)),
+      moe::wgrad_chunk_rows(d_model, z.ld, n_tokens, 1, 0, n_tokens)};
+}
+
 // What the forward makes besides its results. A training forward keeps all of it for the backward.
 struct Kept {
   void *xs, *a1;                  // [L, D] permuted rows, [L, 2H] pre-activations (training only)
@@ -226,6 +239,7 @@ int carve_bwd(void* p, int64_t n_tokens, int32_t d_model, int32_t d_hidden, int3
               int32_t n_shared, int32_t top_k, bool store, bool bias_in, bool bias_out,
               BwdScratch* b) {
   const Sizes z = sizes(n_tokens, n_experts, n_shared, top_k);
+  const Chunks ks = chunks_of(z, n_tokens, d_model, d_hidden);
   Carver c(p);
   *b = BwdScratch{};
   b->douts = c.take(size_t(z.l_cap) * d_model * 2);
@@ -234,12 +248,13 @@ int carve_bwd(void* p, int64_t n_tokens, int32_t d_model, int32_t d_hidden, int3
   b->dtw = c.take(size_t(z.m) * 2);
   b->dl = c.take(size_t(n_tokens) * z.ld * 2);
   b->d_router_padded = c.take(size_t(d_model) * z.ld * 2);
-  int rc = moe_b200_wgrad_scratch_bytes(d_model, 2 * d_hidden, z.l_cap, z.n_all, 1, 0,
+  int rc = moe_b200_wgrad_scratch_bytes(d_model, 2 * d_hidden, z.l_cap, z.n_all, 1, ks.in,
                                         &b->part_in_bytes);
   if (rc != MOE_B200_OK) return rc;
-  rc = moe_b200_wgrad_scratch_bytes(d_hidden, d_model, z.l_cap, z.n_all, 1, 0, &b->part_out_bytes);
+  rc = moe_b200_wgrad_scratch_bytes(d_hidden, d_model, z.l_cap, z.n_all, 1, ks.out,
+                                    &b->part_out_bytes);
   if (rc != MOE_B200_OK) return rc;
-  rc = moe_b200_wgrad_scratch_bytes(d_model, z.ld, n_tokens, 1, 0, 0, &b->part_r_bytes);
+  rc = moe_b200_wgrad_scratch_bytes(d_model, z.ld, n_tokens, 1, 0, ks.router, &b->part_r_bytes);
   if (rc != MOE_B200_OK) return rc;
   b->part_in = c.take(b->part_in_bytes);
   b->part_out = c.take(b->part_out_bytes);
@@ -456,8 +471,8 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
   const int32_t* first_shared = b.k.pad_offsets + E;
   const int32_t* live = S ? first_shared : b.k.n_post_pad;
   const bool store = d.store_combine != 0;
-  // a token has a row in a run once at most; runs are padded to whole tiles
-  const int64_t longest_run = (T + 127) / 128 * 128;
+  const int64_t longest = longest_run(T);
+  const Chunks ks = chunks_of(z, T, D, H);
   const int32_t* offs = S ? b.k.pad_offsets : nullptr;
 
   STEP(moe::dhidden_glu_bwd(b.grad_out, z.l_cap, D, d.w_out, E, d.w_sh_out, S, H, b.k.expert_ids,
@@ -485,13 +500,13 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
       STEP(zero_words(b.dx, T * D / 2, main_st));
     if (!dx_with_router) CU(cudaEventRecord(ev->dx, main_st));
   }
-  STEP(moe::wgrad(b.k.xs, 0, D, b.s.da1, 0, 2 * H, z.l_cap, b.k.pad_offsets, z.n_all, 0, nullptr, 0,
+  STEP(moe::wgrad(b.k.xs, 0, D, b.s.da1, 0, 2 * H, z.l_cap, b.k.pad_offsets, z.n_all, ks.in, nullptr, 0,
                   0, 0, b.dw_in, E, S ? b.dw_sh_in : nullptr, b.s.part_in, b.s.part_in_bytes,
-                  S ? d.x : nullptr, S ? T : 0, S ? 1 : 0, longest_run, 2 * H, d.status, stream));
+                  S ? d.x : nullptr, S ? T : 0, S ? 1 : 0, longest, 2 * H, d.status, stream));
   // side a: dW_out, then the bias gradients (column sums over the runs)
-  STEP(moe::wgrad(b.s.hidw, 0, H, b.s.douts, 0, D, z.l_cap, b.k.pad_offsets, z.n_all, 0, nullptr, 0,
+  STEP(moe::wgrad(b.s.hidw, 0, H, b.s.douts, 0, D, z.l_cap, b.k.pad_offsets, z.n_all, ks.out, nullptr, 0,
                   0, 0, b.dw_out, E, S ? b.dw_sh_out : nullptr, b.s.part_out, b.s.part_out_bytes,
-                  S ? b.grad_out : nullptr, S ? T : 0, S ? 2 : 0, longest_run, D, d.status, sa));
+                  S ? b.grad_out : nullptr, S ? T : 0, S ? 2 : 0, longest, D, d.status, sa));
   // side b: the router's backward. With b_out a pair's d(topk_w) gains <dOut[t], b_out[e]>: one row GEMM
   // dOut @ b_out^T over all experts, read at the pair's column by the router kernel.
   if (b.s.b_extra)
@@ -528,8 +543,8 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
   }
   // side b: the router's weight gradient (a product of one chunk is stored with the padded width and
   // copied), and its share of dx: as rows of their own with a stored combine, or added
-  const bool padded = E != z.ld && T <= moe::wgrad_chunk_rows(D, z.ld, T, 1, 0);
-  STEP(moe::wgrad(d.x, 0, D, b.s.dl, 0, z.ld, T, nullptr, 1, 0, nullptr, 0, 0, 0,
+  const bool padded = E != z.ld && T <= ks.router;
+  STEP(moe::wgrad(d.x, 0, D, b.s.dl, 0, z.ld, T, nullptr, 1, ks.router, nullptr, 0, 0, 0,
                   padded ? b.s.d_router_padded : b.d_router, 1, nullptr, b.s.part_r,
                   b.s.part_r_bytes, nullptr, 0, 0, T, padded ? z.ld : E, d.status, sb));
   if (padded) STEP(moe_b200_copy_cols(b.s.d_router_padded, D, E, z.ld, b.d_router, E, sb));
@@ -554,9 +569,7 @@ int run_backward(const Bwd& b, int32_t* n_launches, cudaStream_t main_st) {
   if (store)
     STEP(moe_b200_combine(b.s.ydx, b.k.inv_ids, T, z.ks, D, b.s.dx_router, nullptr, b.dx, stream));
   // the weight gradients' reduction passes
-  launched += (longest_run > moe::wgrad_chunk_rows(D, 2 * H, z.l_cap, z.n_all, 1)) +
-              (longest_run > moe::wgrad_chunk_rows(H, D, z.l_cap, z.n_all, 1)) +
-              (T > moe::wgrad_chunk_rows(D, z.ld, T, 1, 0));
+  launched += (longest > ks.in) + (longest > ks.out) + (T > ks.router);
   if (n_launches) *n_launches = launched;
   return MOE_B200_OK;
 }

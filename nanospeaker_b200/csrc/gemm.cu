@@ -833,27 +833,37 @@ static int64_t wgrad_items(int64_t rows, int n_groups, int routed, int ks_rows) 
   return routed ? rows / ks_rows + n_groups : int64_t(n_groups) * wgrad_chunks(int(rows), ks_rows);
 }
 
-// Rows per split-K chunk when the caller leaves the choice to the library. Expert runs are cut so that a
-// chunk is about a CTA's share of the work, which grows with the slot rows: shorter chunks mean more fp32
-// partial tiles, longer ones a longer tail behind the longest run (a shared expert's: every token). 78
-// experts, dW_in / dW_out, us:
-//   tokens (slot rows)     1024         1536         2048         3072         4096 rows a chunk
-//   2048  (26 K)       20.9 / 16.5  23.0 / 18.6  21.4 / 17.7  21.4 / 17.7  21.5 / 17.9
-//   4096  (43 K)       29.3 / 22.0  26.6 / 21.9  27.5 / 22.8  31.7 / 27.2  32.5 / 28.9
-//   8192  (75 K)       46.0 / 31.3  38.2 / 29.6  38.6 / 31.0  38.9 / 32.4  41.3 / 35.8
-//   16384 (141 K)      86.6 / 60.3  73.1 / 51.7  64.5 / 44.6  57.2 / 43.6  57.2 / 45.2
-// Below 36 K rows the pass that sums the partial tiles costs the step more (2048 graphed 159 against 164),
-// and so it does where every run would be cut (10000 tokens, 8 experts: 207 against 212): not below twice
-// the mean run.
+// Rows per split-K chunk when the caller leaves the choice to the library. Expert runs (of at most max_run rows)
+// are cut so that a chunk is about a CTA's share of the work: the slot rows times the 128-row tiles of C that a
+// chunk fills (on CTA pairs an even number of them), over the SMs. Shorter chunks mean more fp32 partial
+// tiles, longer ones a longer tail behind the longest run (a shared expert's: every token). Not below twice
+// the mean run, where every run would be cut, nor below half of WGRAD_UNCUT_ROWS; and runs up to that are
+// left whole, since the pass that sums the tiles costs the step what it saves there (2048 tokens graphed 159
+// against 164 us). dW_in / dW_out alone, us, runs of a skewed routing and two shared experts; first the share:
+//   d_model  experts  tokens         share        1024         1536         2048         3072         4096 rows
+//   256      76       4096       578 / 289    17.4 / 16.9  19.3 / 18.8  20.2 / 20.0  24.5 / 24.4  25.7 / 25.6
+//   256      76       16384     1906 / 953    50.5 / 38.1  44.9 / 34.4  39.7 / 33.2  39.2 / 37.0  39.2 / 38.6
+//   576      76       4096      1733 / 867    24.4 / 18.7  25.1 / 19.1  26.0 / 20.2  30.3 / 24.4  30.6 / 26.2
+//   576      76       16384     5718 / 2859   87.5 / 58.4  74.0 / 52.9  65.1 / 46.1  59.0 / 45.6  54.5 / 44.8
+//   576      16       8192      1422 / 711    25.8 / 16.0  22.4 / 18.6  21.1 / 19.5  24.9 / 24.0  28.6 / 28.1
+//   1024     76       4096      2311 / 1155   35.9 / 27.8  34.7 / 29.0  35.6 / 30.0  40.1 / 35.1  41.7 / 37.4
+//   1024     76       8192      4082 / 2041   69.2 / 52.4  56.9 / 44.2  48.9 / 41.9  48.5 / 44.6  50.3 / 48.2
+//   1024     16       16384     3667 / 1834   57.8 / 43.0  51.5 / 41.2  45.9 / 33.5  42.0 / 36.3  40.2 / 40.1
+// In the step the best chunk is longer than alone, the summing passes standing beside other streams' kernels:
+// without the two floors the step at 8192 tokens of d_model 256 took 207 us, with them 202.
 // On the fixed schedule (few groups, every row) the chunks are sized so that the work items fill the SMs
 // about once.
-static int auto_ks_rows(int32_t m_dim, int32_t n_dim, int64_t rows, int n_groups, int routed) {
-  if (routed) {
-    const int64_t share = std::max<int64_t>(rows / 28, 2 * rows / n_groups);
-    return rows < 36864 ? 3072 : int(std::min<int64_t>(3072, (share + 256) / 512 * 512));
-  }
+constexpr int WGRAD_UNCUT_ROWS = 3072;
+static int auto_ks_rows(int32_t m_dim, int32_t n_dim, int64_t rows, int n_groups, int routed, int64_t max_run) {
   const int bn = n_dim % 256 == 0 ? 256 : 192;
-  const int64_t tiles = int64_t((m_dim + BM - 1) / BM) * ((n_dim + bn - 1) / bn) * n_groups;
+  const int64_t tx = (m_dim + BM - 1) / BM, ty = (n_dim + bn - 1) / bn;
+  if (routed) {
+    if (max_run <= WGRAD_UNCUT_ROWS) return WGRAD_UNCUT_ROWS;
+    const int64_t share = rows * (tx > 1 ? (tx + 1) / 2 * 2 : 1) * ty / sm_count();
+    const int64_t chunk = (std::max<int64_t>(share, 2 * rows / n_groups) + 256) / 512 * 512;
+    return int(std::min<int64_t>(WGRAD_UNCUT_ROWS, std::max<int64_t>(WGRAD_UNCUT_ROWS / 2, chunk)));
+  }
+  const int64_t tiles = tx * ty * n_groups;
   int64_t splits = sm_count() / (tiles > 0 ? tiles : 1);
   if (splits < 1) splits = 1;
   int64_t ks = ((rows + splits - 1) / splits + 63) / 64 * 64;
@@ -864,8 +874,9 @@ static int auto_ks_rows(int32_t m_dim, int32_t n_dim, int64_t rows, int n_groups
 }  // extern "C"
 
 namespace moe {
-int wgrad_chunk_rows(int32_t m_dim, int32_t n_dim, int64_t rows, int32_t n_groups, int32_t routed) {
-  return auto_ks_rows(m_dim, n_dim, rows, n_groups, routed);
+int wgrad_chunk_rows(int32_t m_dim, int32_t n_dim, int64_t rows, int32_t n_groups, int32_t routed,
+                     int64_t max_run) {
+  return auto_ks_rows(m_dim, n_dim, rows, n_groups, routed, max_run);
 }
 }  // namespace moe
 
@@ -876,7 +887,7 @@ int moe_b200_wgrad_scratch_bytes(int32_t m_dim, int32_t n_dim, int64_t rows, int
   if (m_dim < 1 || n_dim < 1 || rows < 0 || n_groups < 1 || ks_rows < 0 || ks_rows % 64 != 0 ||
       !partial_bytes)
     return MOE_B200_ERR_SHAPE;
-  if (ks_rows == 0) ks_rows = auto_ks_rows(m_dim, n_dim, rows, n_groups, routed);
+  if (ks_rows == 0) ks_rows = auto_ks_rows(m_dim, n_dim, rows, n_groups, routed, rows);
   const int bn = n_dim % 256 == 0 ? 256 : 192;
   const int64_t tiles_xy = int64_t((m_dim + BM - 1) / BM) * ((n_dim + bn - 1) / bn);
   *partial_bytes = WGRAD_TABLE_BYTES + size_t(wgrad_items(rows, n_groups, routed, ks_rows)) *
@@ -912,7 +923,7 @@ int wgrad(const void* a, int32_t a_grouped, int32_t m_dim, const void* b,
       !aligned16(dw_extra))
     return MOE_B200_ERR_ALIGN;
   const int routed = pad_offsets != nullptr;
-  if (ks_rows == 0) ks_rows = auto_ks_rows(m_dim, n_dim, rows, n_groups, routed);
+  if (ks_rows == 0) ks_rows = auto_ks_rows(m_dim, n_dim, rows, n_groups, routed, rows);
   size_t need_p = 0;
   moe_b200_wgrad_scratch_bytes(m_dim, n_dim, rows, n_groups, routed, ks_rows, &need_p);
   if (partial_bytes < need_p) return MOE_B200_ERR_SCRATCH;

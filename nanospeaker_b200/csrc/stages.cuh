@@ -48,6 +48,7 @@ int wgrad(const void* a, int32_t a_grouped, int32_t m_dim, const void* b,
           int32_t n_first, void* dw_extra, void* partials, size_t partial_bytes,
           const void* alt, int64_t alt_rows, int32_t alt_which, int64_t max_run, int32_t out_cols, int32_t* status,
           void* stream);
-// Rows per split-K chunk that moe_b200_wgrad picks.
-int wgrad_chunk_rows(int32_t m_dim, int32_t n_dim, int64_t rows, int32_t n_groups, int32_t routed);
+// Rows per split-K chunk for runs of at most max_run rows. moe_b200_wgrad picks it with max_run = rows.
+int wgrad_chunk_rows(int32_t m_dim, int32_t n_dim, int64_t rows, int32_t n_groups, int32_t routed,
+                     int64_t max_run);
 }  // namespace moe

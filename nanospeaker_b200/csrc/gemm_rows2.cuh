@@ -362,9 +362,7 @@ __global__ void __launch_bounds__(rows2_bound(EPI), 1)
         if (!mbar_wait(afull_bar + b, (uint32_t(j) >> 1) & 1, p.status))
           atomicExch(p.status, ST_WAIT_TIMEOUT);
         const int ncols = min(BN, p.n_dim - tc.n0);
-        // A row goes as one bulk reduction, lane l of the warp the rows rw + 4 l. (With half of the rows as
-        // vector red instructions instead the load/store unit is the slower of the two paths: 16384 tokens
-        // down 36.7 -> 33.4 us, dX 41.5 -> 41.3; 4096 13.7 -> 12.1 and 17.5 -> 16.5.)
+        // (a row per lane, as in rows_gemm_kernel)
         const int r = warp - (2 + EPI_WARPS) + RED_WARPS * lane;
         const int tok = tok_all[b * BM + r];
         if (tok >= 0)

@@ -50,7 +50,7 @@ METRIC = "MoE-block tokens/s (fwd+bwd)"
 # been captured with ncu on this workload; see profiles/ncu_block_kernels_T16384.md.
 NCU_TRAFFIC_BYTES = {"permute (routed rows; shared experts read x in place)": 82.0e6,
                      "up_gemm+glu (gathers, keeps rows and a1)": 234.7e6,
-                     "dhidden+glu_bwd (gathers, keeps rows)": 312.4e6,
+                     "dhidden+glu_bwd (gathers, keeps rows)": 312.7e6,
                      "wgrad_in (gemm + reduce)": 242.6e6, "wgrad_out (gemm + reduce)": 185.7e6}
 # (filled from the ncu summaries under profiles/; a kernel without a capture reports null)
 

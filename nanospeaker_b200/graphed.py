@@ -3,8 +3,8 @@
 A block's training step is 15 to 17 launches; one native call per direction issues them in about
 160 us of host time with autograd, which is what a step takes up to 2048 tokens. Nothing in the kernel
 path reads a value on the host or has a data-dependent shape, so forward and backward can each be
-captured once per input shape and replayed: 129 us at 300 tokens (167 eager), 147 at 2048 (162). Past that the copies into the graphs' buffers cost more than the launches (16384: 441
-against 405), and the block called directly is the faster one.
+captured once per input shape and replayed: 129 us at 300 tokens (167 eager), 146 at 2048 (162). Past that the copies into the graphs' buffers cost more
+than the launches (16384: 421 against 390), and the block called directly is the faster one.
 `GraphedMoEBlock` does that and stays a drop-in for the block: same call, same post-forward
 attributes (`aux_loss`, `expert_counts`, `dropped`), autograd works as usual (the two graphs are
 tied together by a native autograd node; by torch.cuda.make_graphed_callables where the weights are

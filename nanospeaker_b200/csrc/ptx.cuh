@@ -50,8 +50,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait. try_wait itself suspends for a hardware-chosen slice, so the
-// limit below is several seconds of wall time, far beyond any healthy wait.
+// Bounded wait. try_wait itself suspends for a hardware-chosen slice (2 us), so the
+// limit below is 8 seconds of wall time, far beyond any healthy wait.
 #ifndef MOE_WAIT_LIMIT
 #define MOE_WAIT_LIMIT (1u << 22)
 #endif
